@@ -411,17 +411,20 @@ struct AdamWConstants {
     float beta1, rest1, beta2, rest2, eps, weight_decay;
 };
 // One launch over every tensor of `d_tensors` (a device array of `tensors` entries; `chunks` =
-// d_chunk_tensor/d_chunk_start entries of kUpdateChunk elements each). p, m, v are updated in
-// place with the reference's 16 rounded f32 operations per element.
-constexpr uint32_t kUpdateChunk = 4096;
+// d_chunk_tensor/d_chunk_start entries of update_chunk(all elements) elements each). p, m, v are
+// updated in place with the reference's 16 rounded f32 operations per element.
+constexpr uint32_t kSmallUpdateChunk = 1024, kLargeUpdateChunk = 4096;
+// Short chunks while they all fit the device at once (8 blocks of 256 threads on 148 SMs): the
+// launch then ends after one turn of each thread.
+inline uint32_t update_chunk(uint64_t elements) { return elements <= 148ull * 8 * kSmallUpdateChunk ? kSmallUpdateChunk : kLargeUpdateChunk; }
 void adamw(cudaStream_t s, const UpdateTensor* d_tensors, const uint32_t* d_chunk_tensor,
-           const uint32_t* d_chunk_start, uint32_t chunks, AdamWConstants c, const float* lr_t,
+           const uint32_t* d_chunk_start, uint32_t chunks, uint32_t chunk, AdamWConstants c, const float* lr_t,
            const float* c1, const float* c2);
 // p16[i] = bf16(p[i]): the working copy of a parameter after its f32 master was uploaded.
 void working_copy(cudaStream_t s, const float* p, void* p16, uint64_t n);
 // p -= lr * g, `lr` a device scalar.
 void sgd(cudaStream_t s, const UpdateTensor* d_tensors, const uint32_t* d_chunk_tensor,
-         const uint32_t* d_chunk_start, uint32_t chunks, const float* lr);
+         const uint32_t* d_chunk_start, uint32_t chunks, uint32_t chunk, const float* lr);
 
 }  // namespace k
 }  // namespace msx

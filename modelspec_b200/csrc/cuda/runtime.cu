@@ -803,9 +803,12 @@ struct Scheduler {
         msx_plan* plan = P;
         // Device tables: tensors, then the chunk -> (tensor, start) map.
         std::vector<uint32_t> chunk_tensor, chunk_start;
+        uint64_t elements = 0;
+        for (const Update& u : updates) elements += prog.params[u.param].ty.count();
+        const uint32_t chunk = k::update_chunk(elements);
         for (uint32_t t = 0; t < updates.size(); ++t) {
             uint64_t count = prog.params[updates[t].param].ty.count();
-            for (uint64_t c = 0; c * k::kUpdateChunk < count; ++c) {
+            for (uint64_t c = 0; c * chunk < count; ++c) {
                 chunk_tensor.push_back(t);
                 chunk_start.push_back(static_cast<uint32_t>(c));
             }
@@ -815,11 +818,7 @@ struct Scheduler {
         update_chunk_tensor = chunk_tensor;
         update_chunk_start = chunk_start;
         std::vector<uint32_t> reads, writes;
-        uint64_t elements = 0;
-        for (const Update& u : updates) {
-            reads.push_back(u.grad_pos);
-            elements += prog.params[u.param].ty.count();
-        }
+        for (const Update& u : updates) reads.push_back(u.grad_pos);
         Node pseudo;
         pseudo.id = node(updates[0].grad_pos).id;
         bool adamw = prog.optimizer.rule == msx::Rule::AdamW;
@@ -843,7 +842,7 @@ struct Scheduler {
             Launch& l = emit("adamw_multi_tensor", pseudo, reads, writes, [=](cudaStream_t s) {
                 auto* tensors = static_cast<k::UpdateTensor*>(plan->d_update_tables);
                 auto* ct = reinterpret_cast<uint32_t*>(tensors + n_updates);
-                k::adamw(s, tensors, ct, ct + chunks, chunks, constants, plan->f(static_cast<uint32_t>(lr_t)),
+                k::adamw(s, tensors, ct, ct + chunks, chunks, chunk, constants, plan->f(static_cast<uint32_t>(lr_t)),
                          plan->f(static_cast<uint32_t>(c1)), plan->f(static_cast<uint32_t>(c2)));
             });
             l.flop = 16 * elements;
@@ -859,7 +858,7 @@ struct Scheduler {
             Launch& l = emit("sgd_multi_tensor", pseudo, reads, writes, [=](cudaStream_t s) {
                 auto* tensors = static_cast<k::UpdateTensor*>(plan->d_update_tables);
                 auto* ct = reinterpret_cast<uint32_t*>(tensors + n_updates);
-                k::sgd(s, tensors, ct, ct + chunks, chunks, plan->f(rate));
+                k::sgd(s, tensors, ct, ct + chunks, chunks, chunk, plan->f(rate));
             });
             l.flop = 2 * elements;
             optimizer_bytes = 12 * elements;
