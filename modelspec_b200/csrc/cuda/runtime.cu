@@ -26,6 +26,7 @@
 #include "../core/rng.hpp"
 #include "common.cuh"
 #include "kernels.cuh"
+#include "host_copy.hpp"
 #include "plan.hpp"
 
 using msx::Launch;
@@ -107,6 +108,7 @@ struct Bucket {
 struct msx_device {
     int ordinal = 0;
     std::string error;
+    msx::HostCopier copier;  // downloads of this device's plans into pageable memory
 };
 
 struct InputCheck {
@@ -2763,7 +2765,10 @@ int msx_open(int ordinal, msx_device** out) {
     });
 }
 
-void msx_close(msx_device* device) { delete device; }
+void msx_close(msx_device* device) {
+    if (device) cudaSetDevice(device->ordinal);  // where the copier's streams and buffers live
+    delete device;
+}
 
 const char* msx_last_error(const msx_device* device) { return device ? device->error.c_str() : g_open_error.c_str(); }
 
@@ -2846,10 +2851,13 @@ static int transfer(msx_plan* plan, float* device_ptr, uint64_t expect, void* ho
         if (bytes != expect)
             throw StatusError(MSX_BAD_ARGUMENT, std::string(what) + ": " + std::to_string(bytes) + " bytes given, " + std::to_string(expect) + " expected");
         cuda_ok(cudaSetDevice(plan->device->ordinal), "cudaSetDevice");
-        if (upload) cuda_ok(cudaMemcpyAsync(device_ptr, host, bytes, cudaMemcpyHostToDevice, plan->stream), what);
-        else cuda_ok(cudaMemcpyAsync(host, device_ptr, bytes, cudaMemcpyDeviceToHost, plan->stream), what);
+        if (upload) {
+            cuda_ok(cudaMemcpyAsync(device_ptr, host, bytes, cudaMemcpyHostToDevice, plan->stream), what);
+            cuda_ok(cudaStreamSynchronize(plan->stream), what);
+        } else {
+            cuda_ok(plan->device->copier.to_host(plan->device->ordinal, host, device_ptr, bytes, plan->stream), what);
+        }
         (upload ? plan->bytes_uploaded : plan->bytes_downloaded) += bytes;
-        cuda_ok(cudaStreamSynchronize(plan->stream), what);
         return MSX_OK;
     });
 }
@@ -3182,8 +3190,7 @@ int msx_value_download(msx_plan* plan, uint32_t value_id, void* host, uint64_t b
         if (bytes != expect) throw StatusError(MSX_BAD_ARGUMENT, "msx_value_download: " + std::to_string(expect) + " bytes expected");
         int rc = wait_all(plan, 0);
         if (rc != MSX_OK) return rc;
-        cuda_ok(cudaMemcpyAsync(host, plan->ptr(static_cast<uint32_t>(at)), bytes, cudaMemcpyDeviceToHost, plan->stream), "cudaMemcpyAsync");
-        cuda_ok(cudaStreamSynchronize(plan->stream), "cudaStreamSynchronize");
+        cuda_ok(plan->device->copier.to_host(plan->device->ordinal, host, plan->ptr(static_cast<uint32_t>(at)), bytes, plan->stream), "msx_value_download");
         return MSX_OK;
     });
 }
