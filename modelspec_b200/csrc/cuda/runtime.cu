@@ -3,8 +3,8 @@
 // A plan is built once from the text of a Tensor IR program: the scheduler below walks the live
 // nodes in definition order and emits kernel launches (plan.hpp lists the fusions), a linear-scan
 // allocator places every intermediate in one arena by liveness, and the launches are captured
-// into one CUDA graph at the first step. A step is then one host-to-device copy of the staged
-// inputs, one graph launch and one 4-byte read-back of the loss, all on the plan's stream; the
+// into one CUDA graph at the first step. A step is then one graph launch on the plan's stream, whose
+// first kernel takes over the staged inputs and whose last puts the loss where the host reads it; the
 // host never waits inside msx_run unless all of its staging slots are still in flight.
 #include <cuda_runtime.h>
 #include <dlfcn.h>
@@ -43,6 +43,14 @@ constexpr uint64_t kAlign = 256;
 constexpr uint64_t kGuardBytes = 64;          // 16 sentinel words after every value of a MSX_PLAN_GUARD plan
 constexpr uint32_t kGuardWord = 0xA5C3A5C3u;
 constexpr int kStagingSlots = 8;  // steps in flight before msx_run waits (the reference's SUBMIT_STEPS)
+// The end events of this many steps are kept: the last kStagingSlots steps' and, as the begin of a
+// step submitted behind a running one, their predecessors'.
+constexpr int kStepEvents = 2 * kStagingSlots;
+// Inputs of more than kDirectInputBytes cross PCIe on a stream of their own, beside the step before,
+// into one of two slots on the device; smaller ones are read from the pinned slot by the step's first
+// kernel (which 16 blocks do in one trip over PCIe; at 200 KB the copy beside the step before wins).
+constexpr uint64_t kDirectInputBytes = 64ull << 10;
+constexpr int kDeviceSlots = 2;
 
 uint64_t align_up(uint64_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
@@ -147,15 +155,23 @@ struct msx_plan {
     float* backup = nullptr;
     uint64_t backup_floats = 0;
     bool backup_filled = false;
-    std::vector<char> owns_param16;
+    char* state = nullptr;   // the parameters, moments and working copies this plan owns
+    char* tables = nullptr;  // its inputs, their staging, constants, status, counters and job tables
     char* d_inputs = nullptr;
     uint64_t input_bytes = 0;
     std::vector<char> blob;  // the staged inputs, host side
     bool blob_dirty = true;  // staged since the last upload
-    char* pinned[kStagingSlots] = {};
+    char* pinned = nullptr;        // kStagingSlots slots of slot_bytes
+    uint64_t slot_bytes = 0;
+    char* d_staging = nullptr;     // large inputs: kDeviceSlots slots on the device, filled on copy_stream
+    cudaStream_t copy_stream = nullptr;
+    cudaEvent_t copied[kDeviceSlots] = {};
+    uint32_t* d_turn = nullptr;    // the slot of the step that runs next, kept by the step itself
     float* pinned_loss = nullptr;  // kStagingSlots floats
-    cudaEvent_t slot_begin[kStagingSlots] = {}, slot_done[kStagingSlots] = {};  // around each submitted step
-    bool slot_used[kStagingSlots] = {};
+    // Step n ends with step_done[n % kStepEvents]. It begins with step_begin[...] when the stream was
+    // idle as it was submitted, else where the step before it ends.
+    cudaEvent_t step_begin[kStepEvents] = {}, step_done[kStepEvents] = {};
+    bool began_idle[kStepEvents] = {};
     std::vector<float> consts;
     float* d_consts = nullptr;
     uint32_t* d_status = nullptr;
@@ -183,8 +199,10 @@ struct msx_plan {
     uint64_t steps = 0;
     uint64_t shard_rows_before = 0;
 
-    cudaGraphExec_t graph = nullptr;
-    cudaEvent_t clock_start = nullptr, clock_stop = nullptr;
+    // The captured step: [1] takes its inputs over first, [0] runs on what is staged already. Each is
+    // made when a step of its kind first runs.
+    cudaGraphExec_t graphs[2] = {};
+    cudaEvent_t clock_start = nullptr;  // before the first step since the last msx_elapsed_ms
     uint64_t clock_steps = 0;
 
     uint64_t live_nodes = 0, param_bytes = 0;
@@ -650,7 +668,6 @@ struct Scheduler {
         P->v.assign(np, nullptr);
         P->owns_param.assign(np, 0);
         P->params16.assign(np, nullptr);
-        P->owns_param16.assign(np, 0);
         uint64_t offset = 0;
         for (uint32_t at = 0; at < prog.nodes.size(); ++at) {
             const Node& nd = node(at);
@@ -2284,6 +2301,17 @@ void allocate(msx_plan* P, const Scheduler& sched) {
         if (s.kind == Slot::Param) param_used[s.index] = 1;
         if (s.kind == Slot::Moment) moment_used[s.index] = 1;
     }
+    // Parameters, moments and working copies of the plan's own are pieces of one allocation, and so
+    // are its inputs, constants, status, counters and tables: a device allocation takes a millisecond
+    // or more, and a BERT-base step has 800 such pieces. Each piece starts on a 256-byte boundary.
+    uint64_t state_bytes = 0;
+    std::vector<std::pair<void**, uint64_t>> state_pieces;
+    auto state_piece = [&](void** to, uint64_t bytes) {
+        state_pieces.push_back({to, state_bytes});
+        state_bytes += align_up(bytes);
+        P->param_bytes += bytes;
+    };
+    std::vector<size_t> new_copies;
     for (size_t p = 0; p < prog.params.size(); ++p) {
         uint64_t bytes = std::max<uint64_t>(prog.params[p].ty.count() * 4, 4);
         if (param_used[p]) {
@@ -2296,10 +2324,8 @@ void allocate(msx_plan* P, const Scheduler& sched) {
             if (shared) {
                 P->params[p] = shared;
             } else {
-                cuda_ok(plan_malloc(P, &P->params[p], bytes), "cudaMalloc(parameter)");
-                cuda_ok(cudaMemset(P->params[p], 0, bytes), "cudaMemset(parameter)");
+                state_piece(reinterpret_cast<void**>(&P->params[p]), bytes);
                 P->owns_param[p] = 1;
-                P->param_bytes += bytes;
             }
         }
         // Mixed precision: every matrix parameter gets the bf16 working copy the matmuls read
@@ -2313,43 +2339,68 @@ void allocate(msx_plan* P, const Scheduler& sched) {
             if (shared16) {
                 P->params16[p] = shared16;
             } else {
-                cuda_ok(plan_malloc(P, &P->params16[p], bytes / 2), "cudaMalloc(parameter working copy)");
-                P->owns_param16[p] = 1;
-                P->param_bytes += bytes / 2;
-                k::working_copy(P->stream, P->params[p], P->params16[p], prog.params[p].ty.count());
+                state_piece(&P->params16[p], bytes / 2);
+                new_copies.push_back(p);
             }
         }
         if (moment_used[p]) {
-            cuda_ok(plan_malloc(P, &P->m[p], bytes), "cudaMalloc(moment)");
-            cuda_ok(plan_malloc(P, &P->v[p], bytes), "cudaMalloc(moment)");
-            cuda_ok(cudaMemset(P->m[p], 0, bytes), "cudaMemset(moment)");
-            cuda_ok(cudaMemset(P->v[p], 0, bytes), "cudaMemset(moment)");
-            P->param_bytes += 2 * bytes;
+            state_piece(reinterpret_cast<void**>(&P->m[p]), bytes);
+            state_piece(reinterpret_cast<void**>(&P->v[p]), bytes);
         }
     }
-    uint64_t in_bytes = std::max<uint64_t>(P->input_bytes, kAlign);
-    cuda_ok(plan_malloc(P, &P->d_inputs, in_bytes), "cudaMalloc(inputs)");
-    cuda_ok(cudaMemset(P->d_inputs, 0, in_bytes), "cudaMemset(inputs)");
-    P->blob.assign(in_bytes, 0);
-    for (int s = 0; s < kStagingSlots; ++s) {
-        cuda_ok(cudaMallocHost(&P->pinned[s], in_bytes), "cudaMallocHost(staging)");
-        cuda_ok(cudaEventCreate(&P->slot_begin[s]), "cudaEventCreate");
-        cuda_ok(cudaEventCreate(&P->slot_done[s]), "cudaEventCreate");
+    if (state_bytes) {
+        cuda_ok(plan_malloc(P, &P->state, state_bytes), "cudaMalloc(parameters and moments)");
+        cuda_ok(cudaMemsetAsync(P->state, 0, state_bytes, P->stream), "cudaMemset(parameters and moments)");
+        for (const auto& [to, at] : state_pieces) *to = P->state + at;
+        // A working copy beside a shared master is filled now; one beside a master of its own follows
+        // the master's upload.
+        for (size_t p : new_copies) k::working_copy(P->stream, P->params[p], P->params16[p], prog.params[p].ty.count());
     }
-    cuda_ok(cudaMallocHost(&P->pinned_loss, kStagingSlots * sizeof(float)), "cudaMallocHost(loss)");
-    cuda_ok(cudaMallocHost(&P->pinned_status, kStagingSlots * sizeof(uint32_t)), "cudaMallocHost(status)");
-    std::memset(P->pinned_status, 0, kStagingSlots * sizeof(uint32_t));
-    uint64_t const_bytes = std::max<uint64_t>(P->consts.size() * 4, 4);
-    cuda_ok(plan_malloc(P, &P->d_consts, const_bytes), "cudaMalloc(constants)");
+    const uint64_t in_bytes = std::max<uint64_t>(P->input_bytes, kAlign);
+    const bool staged = P->input_bytes > kDirectInputBytes;
+    const uint64_t const_bytes = std::max<uint64_t>(P->consts.size() * 4, 4);
+    const uint64_t counter_bytes = std::max<uint64_t>(P->counters_used, 1) * 4;
+    const uint64_t tensor_bytes = sched.updates.size() * sizeof(k::UpdateTensor), chunk_bytes = sched.update_chunk_tensor.size() * 4;
+    {
+        const std::pair<void**, uint64_t> pieces[] = {
+            {reinterpret_cast<void**>(&P->d_inputs), in_bytes},
+            {reinterpret_cast<void**>(&P->d_staging), staged ? kDeviceSlots * in_bytes : 0},
+            {reinterpret_cast<void**>(&P->d_consts), const_bytes},
+            {reinterpret_cast<void**>(&P->d_status), 8},
+            {reinterpret_cast<void**>(&P->d_counters), counter_bytes},
+            {&P->d_row_sum_jobs, sched.deferred_rows.size() * sizeof(k::RowSumJob)},
+            {&P->d_sum_jobs, sched.deferred.size() * sizeof(k::SumJob)},
+            {&P->d_update_tables, tensor_bytes + 2 * chunk_bytes}};
+        uint64_t bytes = 0;
+        for (const auto& piece : pieces) bytes += align_up(piece.second);
+        cuda_ok(plan_malloc(P, &P->tables, bytes), "cudaMalloc(inputs and tables)");
+        cuda_ok(cudaMemsetAsync(P->tables, 0, bytes, P->stream), "cudaMemset(inputs and tables)");
+        cuda_ok(cudaStreamSynchronize(P->stream), "cudaStreamSynchronize");  // before the copies below fill the tables
+        char* at = P->tables;
+        for (const auto& piece : pieces) {
+            if (piece.second) *piece.first = at;
+            at += align_up(piece.second);
+        }
+    }
+    P->blob.assign(in_bytes, 0);
+    // One pinned allocation: the input slots, then each slot's loss and status word.
+    P->slot_bytes = in_bytes;
+    cuda_ok(cudaMallocHost(&P->pinned, kStagingSlots * in_bytes + 2 * kStagingSlots * 4), "cudaMallocHost(staging)");
+    P->pinned_loss = reinterpret_cast<float*>(P->pinned + kStagingSlots * in_bytes);
+    P->pinned_status = reinterpret_cast<uint32_t*>(P->pinned_loss + kStagingSlots);
+    std::memset(P->pinned_loss, 0, 2 * kStagingSlots * 4);
+    for (int s = 0; s < kStepEvents; ++s) {
+        cuda_ok(cudaEventCreate(&P->step_begin[s]), "cudaEventCreate");
+        cuda_ok(cudaEventCreate(&P->step_done[s]), "cudaEventCreate");
+    }
+    if (staged) {
+        cuda_ok(cudaStreamCreateWithFlags(&P->copy_stream, cudaStreamNonBlocking), "cudaStreamCreate");
+        for (cudaEvent_t& e : P->copied) cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+    }
     if (!P->consts.empty())
         cuda_ok(cudaMemcpy(P->d_consts, P->consts.data(), P->consts.size() * 4, cudaMemcpyHostToDevice), "cudaMemcpy(constants)");
-    cuda_ok(plan_malloc(P, &P->d_status, 4), "cudaMalloc(status)");
-    cuda_ok(cudaMemset(P->d_status, 0, 4), "cudaMemset(status)");
-    uint64_t counter_bytes = std::max<uint64_t>(P->counters_used, 1) * 4;
-    cuda_ok(plan_malloc(P, &P->d_counters, counter_bytes), "cudaMalloc(counters)");
-    cuda_ok(cudaMemset(P->d_counters, 0, counter_bytes), "cudaMemset(counters)");
+    P->d_turn = P->d_status + 1;
     cuda_ok(cudaEventCreate(&P->clock_start), "cudaEventCreate");
-    cuda_ok(cudaEventCreate(&P->clock_stop), "cudaEventCreate");
     P->side_fork.assign(P->launches.size(), nullptr);
     P->side_done.assign(P->launches.size(), nullptr);
     for (size_t l = 0; l < P->launches.size(); ++l) {
@@ -2368,7 +2419,6 @@ void allocate(msx_plan* P, const Scheduler& sched) {
                                           d.ld, first_block));
             first_block += k::row_sum_job_blocks(d.rows, d.width);
         }
-        cuda_ok(plan_malloc(P, &P->d_row_sum_jobs, jobs.size() * sizeof(k::RowSumJob)), "cudaMalloc(row sum jobs)");
         cuda_ok(cudaMemcpy(P->d_row_sum_jobs, jobs.data(), jobs.size() * sizeof(k::RowSumJob), cudaMemcpyHostToDevice), "cudaMemcpy(row sum jobs)");
     }
     if (!sched.deferred.empty()) {
@@ -2385,7 +2435,6 @@ void allocate(msx_plan* P, const Scheduler& sched) {
             first_block += k::sum_job_blocks(d.chunks, d.width);
             jobs.push_back(job);
         }
-        cuda_ok(plan_malloc(P, &P->d_sum_jobs, jobs.size() * sizeof(k::SumJob)), "cudaMalloc(sum jobs)");
         cuda_ok(cudaMemcpy(P->d_sum_jobs, jobs.data(), jobs.size() * sizeof(k::SumJob), cudaMemcpyHostToDevice), "cudaMemcpy(sum jobs)");
     }
     if (!sched.updates.empty()) {
@@ -2400,13 +2449,10 @@ void allocate(msx_plan* P, const Scheduler& sched) {
             t.p16 = P->params16[u.param];
             tensors.push_back(t);
         }
-        size_t table_bytes = tensors.size() * sizeof(k::UpdateTensor);
-        size_t chunk_bytes = sched.update_chunk_tensor.size() * 4;
-        cuda_ok(plan_malloc(P, &P->d_update_tables, table_bytes + 2 * chunk_bytes), "cudaMalloc(update tables)");
         char* base = static_cast<char*>(P->d_update_tables);
-        cuda_ok(cudaMemcpy(base, tensors.data(), table_bytes, cudaMemcpyHostToDevice), "cudaMemcpy(update tables)");
-        cuda_ok(cudaMemcpy(base + table_bytes, sched.update_chunk_tensor.data(), chunk_bytes, cudaMemcpyHostToDevice), "cudaMemcpy");
-        cuda_ok(cudaMemcpy(base + table_bytes + chunk_bytes, sched.update_chunk_start.data(), chunk_bytes, cudaMemcpyHostToDevice), "cudaMemcpy");
+        cuda_ok(cudaMemcpy(base, tensors.data(), tensor_bytes, cudaMemcpyHostToDevice), "cudaMemcpy(update tables)");
+        cuda_ok(cudaMemcpy(base + tensor_bytes, sched.update_chunk_tensor.data(), chunk_bytes, cudaMemcpyHostToDevice), "cudaMemcpy");
+        cuda_ok(cudaMemcpy(base + tensor_bytes + chunk_bytes, sched.update_chunk_start.data(), chunk_bytes, cudaMemcpyHostToDevice), "cudaMemcpy");
     }
 }
 
@@ -2414,7 +2460,8 @@ void release(msx_plan* P) {
     if (!P) return;
     cudaSetDevice(P->device->ordinal);
     if (P->stream) cudaStreamSynchronize(P->stream);
-    if (P->graph) cudaGraphExecDestroy(P->graph);
+    for (cudaGraphExec_t g : P->graphs)
+        if (g) cudaGraphExecDestroy(g);
     if (P->comm_stream) cudaStreamSynchronize(P->comm_stream);
     for (Bucket& b : P->buckets) {
         if (b.ready) cudaEventDestroy(b.ready);
@@ -2427,18 +2474,8 @@ void release(msx_plan* P) {
         if (e) cudaEventDestroy(e);
     cudaFree(P->d_weight_total);
     cudaFree(P->arena);
-    for (size_t p = 0; p < P->params.size(); ++p) {
-        if (P->owns_param[p]) cudaFree(P->params[p]);
-        if (P->owns_param16[p]) cudaFree(P->params16[p]);
-        cudaFree(P->m[p]);
-        cudaFree(P->v[p]);
-    }
-    cudaFree(P->d_inputs);
-    cudaFree(P->d_consts);
-    cudaFree(P->d_status);
-    cudaFree(P->d_counters);
-    cudaFree(P->d_update_tables);
-    cudaFree(P->d_sum_jobs);
+    cudaFree(P->state);
+    cudaFree(P->tables);
     if (P->side_stream) {
         cudaStreamSynchronize(P->side_stream);
         cudaStreamDestroy(P->side_stream);
@@ -2447,17 +2484,19 @@ void release(msx_plan* P) {
         if (e) cudaEventDestroy(e);
     for (cudaEvent_t e : P->side_done)
         if (e) cudaEventDestroy(e);
-    cudaFree(P->d_row_sum_jobs);
-    for (int s = 0; s < kStagingSlots; ++s) {
-        if (P->pinned[s]) cudaFreeHost(P->pinned[s]);
-        if (P->slot_begin[s]) cudaEventDestroy(P->slot_begin[s]);
-        if (P->slot_done[s]) cudaEventDestroy(P->slot_done[s]);
+    if (P->copy_stream) {
+        cudaStreamSynchronize(P->copy_stream);
+        cudaStreamDestroy(P->copy_stream);
+    }
+    for (cudaEvent_t e : P->copied)
+        if (e) cudaEventDestroy(e);
+    for (int s = 0; s < kStepEvents; ++s) {
+        if (P->step_begin[s]) cudaEventDestroy(P->step_begin[s]);
+        if (P->step_done[s]) cudaEventDestroy(P->step_done[s]);
     }
     if (P->backup) cudaFree(P->backup);
-    if (P->pinned_loss) cudaFreeHost(P->pinned_loss);
-    if (P->pinned_status) cudaFreeHost(P->pinned_status);
+    if (P->pinned) cudaFreeHost(P->pinned);
     if (P->clock_start) cudaEventDestroy(P->clock_start);
-    if (P->clock_stop) cudaEventDestroy(P->clock_stop);
     if (P->stream) cudaStreamDestroy(P->stream);
     delete P;
 }
@@ -2672,11 +2711,23 @@ int wait_all(msx_plan* P, uint32_t timeout_ms) {
         cuda_ok(cudaStreamSynchronize(P->stream), "cudaStreamSynchronize");
         return MSX_OK;
     }
-    int slot = static_cast<int>((P->steps - 1) % kStagingSlots);
-    int rc = wait_event(P->slot_done[slot], timeout_ms == 0 ? 600000u : timeout_ms);
+    int rc = wait_event(P->step_done[(P->steps - 1) % kStepEvents], timeout_ms == 0 ? 600000u : timeout_ms);
     if (rc != MSX_OK) return rc;
-    check_status(P, slot);
+    check_status(P, static_cast<int>((P->steps - 1) % kStagingSlots));
     return MSX_OK;
+}
+
+// What a step is beside its launches: it takes its inputs over from the slot of its turn, and at its
+// end puts its loss and the status word into pinned memory and moves the turn on. Both ends are
+// kernels of the step's graph: a copy engine's turn costs several microseconds of an otherwise idle
+// device each (an 8-kernel step: 30 us with a copy in front and two 4-byte copies behind, 18 us so).
+void enqueue_step(msx_plan* P, bool take_inputs) {
+    if (take_inputs)
+        k::take_inputs(P->stream, P->d_staging ? P->d_staging : P->pinned, P->slot_bytes, P->d_staging ? kDeviceSlots : kStagingSlots, P->input_bytes,
+                       P->d_inputs, P->d_turn);
+    enqueue_all(P);
+    k::publish_step(P->stream, P->loss_pos >= 0 ? P->f(static_cast<uint32_t>(P->loss_pos)) : nullptr, P->d_status, P->pinned_loss, P->pinned_status,
+                    P->d_turn, kStagingSlots);
 }
 
 template <class F> int guarded(msx_device* device, F body) {
@@ -2964,10 +3015,12 @@ int msx_set_shard(msx_plan* plan, uint64_t rows_before, uint64_t global_rows) {
     if (!plan) return MSX_BAD_ARGUMENT;
     (void)global_rows;
     return guarded(plan->device, [&]() -> int {
-        if (plan->shard_rows_before != rows_before && plan->graph) {
+        if (plan->shard_rows_before != rows_before) {
             cuda_ok(cudaStreamSynchronize(plan->stream), "cudaStreamSynchronize");
-            cuda_ok(cudaGraphExecDestroy(plan->graph), "cudaGraphExecDestroy");
-            plan->graph = nullptr;
+            for (cudaGraphExec_t& graph : plan->graphs) {
+                if (graph) cuda_ok(cudaGraphExecDestroy(graph), "cudaGraphExecDestroy");
+                graph = nullptr;
+            }
         }
         plan->shard_rows_before = rows_before;
         return MSX_OK;
@@ -2978,13 +3031,16 @@ int msx_run(msx_plan* plan) {
     if (!plan) return MSX_BAD_ARGUMENT;
     return guarded(plan->device, [&]() -> int {
         cuda_ok(cudaSetDevice(plan->device->ordinal), "cudaSetDevice");
-        int slot = static_cast<int>(plan->steps % kStagingSlots);
-        if (plan->slot_used[slot]) {
-            int rc = wait_event(plan->slot_done[slot], 600000u);
+        const int slot = static_cast<int>(plan->steps % kStagingSlots), at = static_cast<int>(plan->steps % kStepEvents);
+        if (plan->steps >= kStagingSlots) {
+            int rc = wait_event(plan->step_done[(plan->steps - kStagingSlots) % kStepEvents], 600000u);
             if (rc != MSX_OK) throw StatusError(rc, "msx_run: a step submitted " + std::to_string(kStagingSlots) + " steps ago has not finished");
         }
         if (plan->clock_steps == 0) cuda_ok(cudaEventRecord(plan->clock_start, plan->stream), "cudaEventRecord");
-        cuda_ok(cudaEventRecord(plan->slot_begin[slot], plan->stream), "cudaEventRecord");
+        // A step submitted behind a running one begins where that one ends; only on an idle stream
+        // does it need an event of its own (a recorded event costs the stream about 2 us).
+        plan->began_idle[at] = plan->steps == 0 || cudaEventQuery(plan->step_done[(plan->steps - 1) % kStepEvents]) == cudaSuccess;
+        if (plan->began_idle[at]) cuda_ok(cudaEventRecord(plan->step_begin[at], plan->stream), "cudaEventRecord");
         if (!plan->timing_begun) {
             plan->timing_begun = true;
             plan->first_submit = plan->last_wait = std::chrono::steady_clock::now();
@@ -2992,41 +3048,45 @@ int msx_run(msx_plan* plan) {
         ++plan->submits;
         plan->dispatches += plan->launches.size();
         plan->bytes_downloaded += (plan->loss_pos >= 0 ? 4 : 0) + 4;
-        if (plan->input_bytes && plan->blob_dirty) {
+        const bool take_inputs = plan->input_bytes && plan->blob_dirty;
+        if (take_inputs) {
             plan->bytes_uploaded += plan->input_bytes;
             plan->blob_dirty = false;
-            std::memcpy(plan->pinned[slot], plan->blob.data(), plan->input_bytes);
-            cuda_ok(cudaMemcpyAsync(plan->d_inputs, plan->pinned[slot], plan->input_bytes, cudaMemcpyHostToDevice, plan->stream),
-                    "cudaMemcpyAsync(inputs)");
+            char* const from = plan->pinned + slot * plan->slot_bytes;
+            std::memcpy(from, plan->blob.data(), plan->input_bytes);
+            if (plan->d_staging) {
+                // The slot on the device is free once the step that last used it has run.
+                const int half = slot % kDeviceSlots;
+                if (plan->steps >= kDeviceSlots)
+                    cuda_ok(cudaStreamWaitEvent(plan->copy_stream, plan->step_done[(plan->steps - kDeviceSlots) % kStepEvents], 0), "cudaStreamWaitEvent");
+                cuda_ok(cudaMemcpyAsync(plan->d_staging + half * plan->slot_bytes, from, plan->input_bytes, cudaMemcpyHostToDevice, plan->copy_stream),
+                        "cudaMemcpyAsync(inputs)");
+                cuda_ok(cudaEventRecord(plan->copied[half], plan->copy_stream), "cudaEventRecord");
+                cuda_ok(cudaStreamWaitEvent(plan->stream, plan->copied[half], 0), "cudaStreamWaitEvent");
+            }
         }
         if (plan->flags & MSX_PLAN_NO_GRAPH) {
-            enqueue_all(plan);
+            enqueue_step(plan, take_inputs);
         } else {
-            if (!plan->graph) {
+            cudaGraphExec_t& exec = plan->graphs[take_inputs ? 1 : 0];
+            if (!exec) {
                 cudaGraph_t graph = nullptr;
                 cuda_ok(cudaStreamBeginCapture(plan->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
                 try {
-                    enqueue_all(plan);
+                    enqueue_step(plan, take_inputs);
                 } catch (...) {
                     cudaStreamEndCapture(plan->stream, &graph);
                     if (graph) cudaGraphDestroy(graph);
                     throw;
                 }
                 cuda_ok(cudaStreamEndCapture(plan->stream, &graph), "cudaStreamEndCapture");
-                cudaError_t e = cudaGraphInstantiate(&plan->graph, graph, 0);
+                cudaError_t e = cudaGraphInstantiate(&exec, graph, 0);
                 cudaGraphDestroy(graph);
                 cuda_ok(e, "cudaGraphInstantiate");
             }
-            cuda_ok(cudaGraphLaunch(plan->graph, plan->stream), "cudaGraphLaunch");
+            cuda_ok(cudaGraphLaunch(exec, plan->stream), "cudaGraphLaunch");
         }
-        if (plan->loss_pos >= 0)
-            cuda_ok(cudaMemcpyAsync(plan->pinned_loss + slot, plan->ptr(static_cast<uint32_t>(plan->loss_pos)), 4, cudaMemcpyDeviceToHost,
-                                    plan->stream),
-                    "cudaMemcpyAsync(loss)");
-        cuda_ok(cudaMemcpyAsync(plan->pinned_status + slot, plan->d_status, 4, cudaMemcpyDeviceToHost, plan->stream), "cudaMemcpyAsync(status)");
-        cuda_ok(cudaEventRecord(plan->clock_stop, plan->stream), "cudaEventRecord");
-        cuda_ok(cudaEventRecord(plan->slot_done[slot], plan->stream), "cudaEventRecord");
-        plan->slot_used[slot] = true;
+        cuda_ok(cudaEventRecord(plan->step_done[at], plan->stream), "cudaEventRecord");
         ++plan->steps;
         ++plan->clock_steps;
         return MSX_OK;
@@ -3057,7 +3117,7 @@ int msx_loss_of(msx_plan* plan, uint64_t step_number, float* loss, uint32_t time
             throw StatusError(MSX_BAD_ARGUMENT, "msx_loss_of: only the last " + std::to_string(kStagingSlots) + " submitted steps keep their loss");
         if (plan->loss_pos < 0) throw StatusError(MSX_BAD_ARGUMENT, "msx_loss_of: the program has no rank-0 loss");
         int slot = static_cast<int>(step_number % kStagingSlots);
-        int rc = wait_event(plan->slot_done[slot], timeout_ms == 0 ? 600000u : timeout_ms);
+        int rc = wait_event(plan->step_done[step_number % kStepEvents], timeout_ms == 0 ? 600000u : timeout_ms);
         if (rc != MSX_OK) return rc;
         check_status(plan, slot);
         *loss = plan->pinned_loss[slot];
@@ -3087,8 +3147,8 @@ int msx_profile_step_repeated(msx_plan* plan, uint32_t repeats, float* launch_ms
         std::vector<cudaEvent_t> events(2 * count);
         for (cudaEvent_t& e : events) cuda_ok(cudaEventCreate(&e), "cudaEventCreate");
         if (plan->input_bytes) {
-            std::memcpy(plan->pinned[0], plan->blob.data(), plan->input_bytes);
-            cuda_ok(cudaMemcpyAsync(plan->d_inputs, plan->pinned[0], plan->input_bytes, cudaMemcpyHostToDevice, plan->stream), "cudaMemcpyAsync");
+            std::memcpy(plan->pinned, plan->blob.data(), plan->input_bytes);
+            cuda_ok(cudaMemcpyAsync(plan->d_inputs, plan->pinned, plan->input_bytes, cudaMemcpyHostToDevice, plan->stream), "cudaMemcpyAsync");
         }
         begin_side_work(plan);
         for (size_t l = 0; l < count; ++l) {
@@ -3120,10 +3180,11 @@ int msx_step_ms(msx_plan* plan, uint64_t step_number, float* ms) {
     return guarded(plan->device, [&]() -> int {
         if (step_number >= plan->steps || step_number + kStagingSlots < plan->steps)
             throw StatusError(MSX_BAD_ARGUMENT, "msx_step_ms: only the last " + std::to_string(kStagingSlots) + " submitted steps keep their time");
-        int slot = static_cast<int>(step_number % kStagingSlots);
-        int rc = wait_event(plan->slot_done[slot], 600000u);
+        const int at = static_cast<int>(step_number % kStepEvents);
+        int rc = wait_event(plan->step_done[at], 600000u);
         if (rc != MSX_OK) return rc;
-        cuda_ok(cudaEventElapsedTime(ms, plan->slot_begin[slot], plan->slot_done[slot]), "cudaEventElapsedTime");
+        const cudaEvent_t begin = plan->began_idle[at] ? plan->step_begin[at] : plan->step_done[(step_number - 1) % kStepEvents];
+        cuda_ok(cudaEventElapsedTime(ms, begin, plan->step_done[at]), "cudaEventElapsedTime");
         return MSX_OK;
     });
 }
@@ -3536,9 +3597,8 @@ int msx_elapsed_ms(msx_plan* plan, double* total_ms, uint64_t* steps) {
         if (plan->clock_steps == 0) return MSX_OK;
         int rc = wait_all(plan, 0);
         if (rc != MSX_OK) return rc;
-        cuda_ok(cudaEventSynchronize(plan->clock_stop), "cudaEventSynchronize");
         float ms = 0.0f;
-        cuda_ok(cudaEventElapsedTime(&ms, plan->clock_start, plan->clock_stop), "cudaEventElapsedTime");
+        cuda_ok(cudaEventElapsedTime(&ms, plan->clock_start, plan->step_done[(plan->steps - 1) % kStepEvents]), "cudaEventElapsedTime");
         *total_ms = ms;
         plan->clock_steps = 0;
         return MSX_OK;
