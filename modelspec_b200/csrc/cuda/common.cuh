@@ -4,6 +4,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <initializer_list>
 #include <stdexcept>
@@ -27,6 +28,16 @@ inline void check(cudaError_t e, const char* what) {
 // earlier (the host application's own, or an earlier launch here) is reported once and does not
 // fail every later launch.
 inline void check_launch(const char* kernel) { check(cudaGetLastError(), kernel); }
+
+// Allows `kernel` its dynamic shared memory on the current device. The attribute is per device: it is
+// set when the device changes (a second thread that sees a stale value only sets it once more).
+template <class Kernel> inline void set_shared_memory(Kernel kernel, int bytes, std::atomic<int>& configured_device) {
+    int device = 0;
+    check(cudaGetDevice(&device), "cudaGetDevice");
+    if (device == configured_device.load(std::memory_order_relaxed)) return;
+    check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes), "dynamic shared memory");
+    configured_device.store(device, std::memory_order_relaxed);
+}
 
 // ---- elements of either storage type ------------------------------------------------------------
 // A mixed-precision plan stores activations as bf16; the kernels that touch them are templates on

@@ -262,7 +262,9 @@ void matmul(cudaStream_t s, const float* a, bool a_t, const float* b, bool b_t, 
 // `leave_partials` a split k stops at the partial tiles, workspace[split][m][n], for
 // finalize_sums (no bias then).
 struct MatmulTcPlan {
-    uint32_t bm, bn, splits, kblocks_per_split;  // tile rows (64 or 128) and width, k split
+    uint32_t bm, bn, splits, kblocks_per_split;  // tile rows and width, k split
+    bool fma;                                    // on the FMA units (gemm_small.cu),
+    uint32_t cluster;                            // the k of a tile shared by that many CTAs
     uint64_t workspace_floats;
 };
 // `problems` > 1: that many independent batched products in one launch (k is then not split);
@@ -304,8 +306,19 @@ struct MatmulJob {
     float* workspace;  // matmul_tc_job_plan(m, n, k).workspace_floats floats, or null when that is 0
     uint64_t m, n, k;
 };
+// The TMA-fed tiles (gemm_tf32.cu) with the tile and split of `p`. `chain` > 1: the `count` = chain
+// products are summed into products[0].c (k unsplit).
+void matmul_tf32(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* products, uint32_t count, bool a_t, bool b_t, uint64_t m, uint64_t n, uint64_t k,
+                 uint32_t chain, MatmulPitches pitches, uint32_t* status);
+// Small products on the FMA units (gemm_small.cu).
+void matmul_small(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* products, uint32_t count, bool a_t, bool b_t, uint64_t m, uint64_t n, uint64_t k,
+                  MatmulPitches pitches);
 constexpr uint32_t kMatmulJobs = 24;  // jobs one launch carries
 MatmulTcPlan matmul_tc_job_plan(uint64_t m, uint64_t n, uint64_t k);
+// The jobs on the TMA-fed 128 x 128 tile, when TMA can address every operand and result; false when it
+// cannot.
+bool matmul_tf32_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, bool a_t, bool b_t, uint32_t* status);
+void matmul_small_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, bool a_t, bool b_t);
 void matmul_tc_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, bool a_t, bool b_t, uint32_t* status);
 
 // outer x inner independent products through one launch (grid.z = problem): matrix z of an
