@@ -39,6 +39,19 @@ template <class Kernel> inline void set_shared_memory(Kernel kernel, int bytes, 
     configured_device.store(device, std::memory_order_relaxed);
 }
 
+// The SMs of the current device.
+inline uint32_t device_sm_count() {
+    static std::atomic<int> counted_device{-1};
+    static std::atomic<uint32_t> count{0};
+    int device = 0, sms = 0;
+    check(cudaGetDevice(&device), "cudaGetDevice");
+    if (device == counted_device.load(std::memory_order_acquire)) return count.load(std::memory_order_relaxed);
+    check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
+    count.store(static_cast<uint32_t>(sms), std::memory_order_relaxed);
+    counted_device.store(device, std::memory_order_release);
+    return static_cast<uint32_t>(sms);
+}
+
 // ---- elements of either storage type ------------------------------------------------------------
 // A mixed-precision plan stores activations as bf16; the kernels that touch them are templates on
 // the element type and compute in f32 whatever it is. One element, or four consecutive ones (16

@@ -569,7 +569,7 @@ bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 //     leave SMs idle), or pairs of CTAs on 256 x 256 tiles once there are enough of those;
 //   * the rest, and batched products, the 64-row tiles of this file.
 // A split k adds the reduce launch and its partial tiles.
-MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems, uint64_t group, bool tma_ok) {
+MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems, uint64_t group, bool tma_ok, uint64_t chain) {
     enum Kernel { Fma, Tma, Rows64 };
     struct Candidate {
         Kernel kernel;
@@ -594,7 +594,7 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
     double best_cost = 0.0;
     for (const Candidate& c : candidates) {
         const bool single = problems == 1 && kblocks > 0;  // batched and empty products stay on the 64-row tiles
-        if (c.kernel == Fma ? !single : (c.kernel == Tma) != (single && tma_ok)) continue;
+        if (c.kernel == Fma ? !single || chain > 1 : (c.kernel == Tma) != (single && tma_ok)) continue;
         const uint64_t m_tiles = (m + c.bm - 1) / c.bm, n_tiles = (n + c.bn - 1) / c.bn, tiles = m_tiles * n_tiles * problems * group;
         auto consider = [&](double cost, uint64_t splits, uint64_t per, uint32_t cluster) {
             if (best.bn != 0 && cost >= best_cost) return;
@@ -612,7 +612,7 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
             consider(chain > streamed ? chain : streamed, 1, kblocks, cluster);
             continue;
         }
-        const uint64_t most = problems > 1 ? 1 : (kblocks / 2 > 0 ? kblocks / 2 : 1);
+        const uint64_t most = problems > 1 || chain > 1 ? 1 : (kblocks / 2 > 0 ? kblocks / 2 : 1);
         for (uint64_t splits = 1; splits <= most && splits <= 64; ++splits) {
             const uint64_t per = (kblocks + splits - 1) / splits;
             const uint64_t used = kblocks == 0 ? 1 : (kblocks + per - 1) / per;
@@ -620,7 +620,7 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
             const double waves = std::ceil(static_cast<double>(tiles * splits) / c.at_once);
             double cost;
             if (c.kernel == Tma) {
-                cost = c.fixed + waves * (static_cast<double>(per) * c.block + c.tile);
+                cost = c.fixed + waves * (static_cast<double>(per * chain) * c.block + c.tile);
             } else {
                 const double paired = waves * (c.fixed + static_cast<double>(per) * c.block);
                 const double streamed = std::ceil(static_cast<double>(tiles * splits) / 148.0) * static_cast<double>(per) * c.tile;

@@ -73,68 +73,62 @@ template <int CG, int BN> struct Tile {
 
 struct Job {
     float* c;  // the result, or the job's split-k workspace
-    uint32_t m, n, ldc, splits, kblocks, first_unit;
+    uint32_t m, n, kblocks, first_unit;
+    tc::Divisor splits;
+    tc::TileWalk walk;
 };
 struct Args {
-    uint32_t units, m, n, ldc, splits, products;
-    uint32_t kblocks;                         // of one product
-    uint32_t chain;                           // > 1: that many products are summed into one result
-    uint32_t c_tma, c_vec, c_padded;          // C by TMA stores; else 16-byte stores; padding between n and ldc may be overwritten
-    float* c[MAX_PRODUCTS];                   // C, or the split-k workspace [splits][m][n]
-    const float* bias[MAX_PRODUCTS];          // null for none
-    uint32_t* status;
+    uint32_t units = 0, m = 0, n = 0, ldc = 0;
+    tc::TileWalk walk;
+    tc::Divisor splits;
+    uint32_t kblocks = 0;                       // of one product
+    uint32_t chain = 1;                         // > 1: that many products are summed into one result
+    uint32_t c_tma = 1, c_vec = 1, c_padded = 0;  // C by TMA stores; else 16-byte stores; padding between n and ldc may be overwritten
+    float* c[MAX_PRODUCTS] = {};                // C, or the split-k workspace [splits][m][n]
+    const float* bias[MAX_PRODUCTS] = {};       // null for none
+    uint32_t* status = nullptr;
 };
 struct Maps {
     CUtensorMap a[MAX_PRODUCTS], b[MAX_PRODUCTS], c[MAX_PRODUCTS];
 };
 // Products of different shapes and one storage form in one launch.
 struct JobArgs : Args {
-    uint32_t job_count;
-    Job jobs[MAX_JOBS];
+    uint32_t job_count = 0;
+    Job jobs[MAX_JOBS] = {};
 };
 struct JobMaps {
     CUtensorMap a[MAX_JOBS], b[MAX_JOBS], c[MAX_JOBS];
 };
 
-// Unit `u` of a launch: tiles of one column of tiles are neighbours (they share their block of B), then
-// come the splits of a tile, then the columns, then the products or jobs.
+// Unit `u` of a launch: its tile, then the split, and the product or job.
 struct Unit {
     uint32_t m0, n0, split, splits, product, kblocks;
     uint32_t m, n, ldc;
     float* c;
     const float* bias;
 };
-template <int CG, int BN> __device__ __forceinline__ Unit unit_of(const Args& args, uint32_t u) {
+__device__ __forceinline__ Unit unit_of(const Args& args, uint32_t u) {
     Unit w;
-    w.m = args.m; w.n = args.n; w.ldc = args.ldc; w.splits = args.splits;
-    const uint32_t down = (w.m + 128u * CG - 1) / (128u * CG), across = (w.n + BN - 1) / BN;
-    w.m0 = (u % down) * (128u * CG);
-    u /= down;
-    w.split = u % w.splits;
-    u /= w.splits;
-    w.n0 = (u % across) * BN;
-    w.product = u / across;
+    w.m = args.m; w.n = args.n; w.ldc = args.ldc; w.splits = args.splits.d;
+    u = args.walk.take(u, &w.m0, &w.n0);
+    w.product = args.splits.quotient(u);
+    w.split = u - w.product * args.splits.d;
     w.c = args.c[w.product];
     w.bias = args.bias[w.product];
-    w.kblocks = args.chain > 1 ? args.kblocks * args.chain : (args.kblocks - w.split + w.splits - 1) / w.splits;
+    w.kblocks = args.chain > 1 ? args.kblocks * args.chain : args.splits.quotient(args.kblocks - w.split + w.splits - 1);
     return w;
 }
-template <int CG, int BN> __device__ __forceinline__ Unit unit_of(const JobArgs& args, uint32_t u) {
+__device__ __forceinline__ Unit unit_of(const JobArgs& args, uint32_t u) {
     uint32_t j = 0;
     while (j + 1 < args.job_count && args.jobs[j + 1].first_unit <= u) ++j;
     const Job& job = args.jobs[j];
-    u -= job.first_unit;
     Unit w;
-    w.m = job.m; w.n = job.n; w.ldc = job.ldc; w.splits = job.splits;
-    const uint32_t down = (w.m + 128u * CG - 1) / (128u * CG);
-    w.m0 = (u % down) * (128u * CG);
-    u /= down;
-    w.split = u % w.splits;
-    w.n0 = (u / w.splits) * BN;
+    w.m = job.m; w.n = w.ldc = job.n; w.splits = job.splits.d;
+    w.split = job.walk.take(u - job.first_unit, &w.m0, &w.n0);
     w.product = j;
     w.c = job.c;
     w.bias = nullptr;
-    w.kblocks = (job.kblocks - w.split + w.splits - 1) / w.splits;
+    w.kblocks = job.splits.quotient(job.kblocks - w.split + w.splits - 1);
     return w;
 }
 
@@ -150,43 +144,6 @@ template <int CG, int REUSE> __device__ __forceinline__ void mma_tf32(uint32_t t
     else MSX_MMA("2", "");
 #undef MSX_MMA
 }
-// Arrives on `bar` (of both CTAs of a pair) when the MMAs issued so far have completed.
-template <int CG> __device__ __forceinline__ void commit(uint32_t bar) {
-    if constexpr (CG == 1) tc::mma_commit(bar);
-    else
-        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-                     ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
-}
-// Arrives on the first CTA's barrier at the same offset.
-template <int CG> __device__ __forceinline__ void arrive_first(uint32_t bar) {
-    if constexpr (CG == 1) tc::mbar_arrive(bar);
-    else
-        asm volatile("{\n\t.reg .b32 far;\n\tmapa.shared::cluster.u32 far, %0, 0;\n\tmbarrier.arrive.release.cluster.shared::cluster.b64 _, [far];\n\t}"
-                     ::"r"(bar) : "memory");
-}
-template <int CG> __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
-    if constexpr (CG == 1) return tc::mbar_try_wait(bar, parity);
-    uint32_t ok;
-    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
-                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
-    return ok != 0;
-}
-// Waits for `parity` of `bar`, all lanes of a warp together; false when the wait ran out or another
-// role gave up.
-template <int CG> __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* status) {
-    bool ok = false;
-    for (uint32_t spin = 0; spin < tc::WAIT_LIMIT; ++spin) {
-        if (try_wait<CG>(bar, parity)) { ok = true; break; }
-        if ((spin & 255u) == 255u && *abort_flag) break;
-    }
-    ok = __all_sync(0xffffffffu, ok);
-    if (!ok && *abort_flag == 0) {
-        *abort_flag = 1;
-        atomicOr(status, 2u);
-    }
-    return ok;
-}
-
 // Tiles of a (column, row[, split]) tensor map.
 __device__ __forceinline__ void load(uint32_t dst, const CUtensorMap* map, uint32_t bar, uint32_t x, uint32_t row) {
     asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
@@ -202,10 +159,6 @@ __device__ __forceinline__ void store_add(const CUtensorMap* map, uint32_t src, 
     asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
                  ::"l"(map), "r"(src), "r"(x), "r"(row), "r"(split) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-
-__device__ __forceinline__ void cluster_barrier() {
-    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
 // The part of x below its top 11 significant bits, exactly.
@@ -229,8 +182,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
     volatile uint32_t* const abort_flag = tmem_slot + 1;
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-    uint32_t rank = 0;
-    if constexpr (CG == 2) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    const uint32_t rank = tc::cta_rank<CG>();
     const uint32_t first_unit = blockIdx.x / CG, step = gridDim.x / CG, units = args.units;
 
     if (tid == 0) {
@@ -247,16 +199,10 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == T::MMA_WARP) {
-        if constexpr (CG == 1) {
-            asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(T::TMEM_COLUMNS) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-        } else {
-            asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(tc::smem_u32(tmem_slot)), "r"(T::TMEM_COLUMNS) : "memory");
-            asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
-        }
+        tc::tmem_alloc<CG>(tc::smem_u32(tmem_slot), T::TMEM_COLUMNS);
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    if constexpr (CG == 2) cluster_barrier();  // the other CTA's barriers exist before anything arrives on them
+    if constexpr (CG == 2) tc::cluster_barrier();  // the other CTA's barriers exist before anything arrives on them
     else __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
@@ -267,13 +213,13 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
         // stage: a block is a chain of about a thousand cycles (wait, read, write, the proxy fence, the
         // arrival) that more warps on one block do not shorten, so blocks are worked on side by side.
         uint32_t total = 0;
-        for (uint32_t u = first_unit; u < units; u += step) total += unit_of<CG, BN>(args, u).kblocks;
+        for (uint32_t u = first_unit; u < units; u += step) total += unit_of(args, u).kblocks;
         const uint32_t stage = tid / GROUP_THREADS, in_group = tid % GROUP_THREADS;
         bool alive = true;
         uint32_t parity = 0;
         for (uint32_t g = stage; g < total && alive; g += STAGES, parity ^= 1u) {
             char* const at = smem + stage * T::STAGE_BYTES + in_group * 16;
-            alive = warp_wait<1>(tc::smem_u32(&raw_full[stage]), parity, abort_flag, args.status);
+            alive = tc::warp_wait<1>(tc::smem_u32(&raw_full[stage]), parity, abort_flag, args.status);
             if (!alive) break;
             constexpr int PER_THREAD = T::RAW_BYTES / 16 / GROUP_THREADS, OF_A = T::A_BYTES / 16 / GROUP_THREADS;
             constexpr int BATCH = PER_THREAD % 8 == 0 ? 8 : 10;
@@ -293,7 +239,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
             // Visible to the tensor core's async-proxy reads before the MMA warp is told.
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) arrive_first<CG>(tc::smem_u32(&lo_full[stage]));
+            if (lane == 0) tc::arrive_first<CG>(tc::smem_u32(&lo_full[stage]));
         }
     } else if (warp == T::MMA_WARP) {
         // ---- the MMA warp (the pair's first CTA) -------------------------------------------------------
@@ -317,14 +263,14 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
             bool alive = true;
             uint32_t stage = 0, parity = 0, turn = 0;
             for (uint32_t u = first_unit; u < units && alive; u += step) {
-                const uint32_t kblocks = unit_of<CG, BN>(args, u).kblocks;
+                const uint32_t kblocks = unit_of(args, u).kblocks;
                 for (uint32_t kb = 0; kb < kblocks && alive; ++kb) {
                     const uint32_t in_segment = kb % LENGTH, acc = turn & 1u;
                     if (in_segment == 0) {
-                        alive = warp_wait<CG>(tc::smem_u32(&acc_empty[acc]), ((turn >> 1) & 1u) ^ 1u, abort_flag, args.status);
+                        alive = tc::warp_wait<CG>(tc::smem_u32(&acc_empty[acc]), ((turn >> 1) & 1u) ^ 1u, abort_flag, args.status);
                         if (!alive) break;
                     }
-                    alive = warp_wait<CG>(tc::smem_u32(&lo_full[stage]), parity, abort_flag, args.status);
+                    alive = tc::warp_wait<CG>(tc::smem_u32(&lo_full[stage]), parity, abort_flag, args.status);
                     if (!alive) break;
                     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                     if (lane == 0) {
@@ -345,8 +291,8 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
                                 mma_tf32<CG, 0>(to, a_lo, b_hi, idesc_bn, 1u);
                             }
                         }
-                        commit<CG>(tc::smem_u32(&empty[stage]));
-                        if (in_segment + 1 == LENGTH || kb + 1 == kblocks) commit<CG>(tc::smem_u32(&acc_full[acc]));
+                        tc::commit<CG>(tc::smem_u32(&empty[stage]));
+                        if (in_segment + 1 == LENGTH || kb + 1 == kblocks) tc::commit<CG>(tc::smem_u32(&acc_full[acc]));
                     }
                     if (in_segment + 1 == LENGTH || kb + 1 == kblocks) ++turn;
                     if (++stage == STAGES) { stage = 0; parity ^= 1u; }
@@ -360,11 +306,11 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
         uint32_t stage = 0, parity = 1;  // the parity a free stage shows
         uint32_t issued = 0;
         for (uint32_t u = first_unit; u < units && alive; u += step) {
-            const Unit w = unit_of<CG, BN>(args, u);
+            const Unit w = unit_of(args, u);
             const uint32_t m0 = w.m0 + rank * 128u, n0 = w.n0 + rank * T::BN_CTA;
             uint32_t product = w.product, k_at = w.split;  // k block of the product
             for (uint32_t kb = 0; kb < w.kblocks && alive; ++kb, ++issued) {
-                alive = warp_wait<CG>(tc::smem_u32(&empty[stage]), parity, abort_flag, args.status);
+                alive = tc::warp_wait<CG>(tc::smem_u32(&empty[stage]), parity, abort_flag, args.status);
                 if (!alive) break;
                 if (lane == 0) {
                     const uint32_t bar = tc::smem_u32(&raw_full[stage]);
@@ -411,8 +357,8 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
         bool alive = true;
         uint32_t turn = 0;
         for (uint32_t u = first_unit; u < units && alive; u += step)
-        for (uint32_t segment = 0, left = unit_of<CG, BN>(args, u).kblocks; left > 0 && alive; left -= left < LENGTH ? left : LENGTH, ++segment, ++turn) {
-            const Unit w = unit_of<CG, BN>(args, u);
+        for (uint32_t segment = 0, left = unit_of(args, u).kblocks; left > 0 && alive; left -= left < LENGTH ? left : LENGTH, ++segment, ++turn) {
+            const Unit w = unit_of(args, u);
             const uint32_t acc = turn & 1u;
             // The bias of the warp's columns, fetched before the wait for the tile (a load issued in the drain
             // would queue behind all the SM has in flight) and put where every lane reads all of it. The
@@ -430,7 +376,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
                     if (bias_at + 3 < w.n) bias4.w = __ldg(w.bias + bias_at + 3);
                 }
             }
-            alive = warp_wait<CG>(tc::smem_u32(&acc_full[acc]), (turn >> 1) & 1u, abort_flag, args.status);
+            alive = tc::warp_wait<CG>(tc::smem_u32(&acc_full[acc]), (turn >> 1) & 1u, abort_flag, args.status);
             if (!alive) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             float* const my_bias = bias_tile + acc * BN + first_col;
@@ -515,39 +461,27 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
             // The warp's share of the accumulator and of the bias has been read.
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             __syncwarp();
-            if (lane == 0) arrive_first<CG>(tc::smem_u32(&acc_empty[acc]));
+            if (lane == 0) tc::arrive_first<CG>(tc::smem_u32(&acc_empty[acc]));
         }
         // The slab must outlive the store that reads it.
         if (args.c_tma && lane == 0) tc::tma_store_wait_read<0>();
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncwarp();
-    if constexpr (CG == 2) cluster_barrier();  // the pair's remote arrivals have landed before either CTA goes away
+    if constexpr (CG == 2) tc::cluster_barrier();  // the pair's remote arrivals have landed before either CTA goes away
     else __syncthreads();
     if (warp == T::MMA_WARP) {
-        if constexpr (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(T::TMEM_COLUMNS) : "memory");
-        else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(T::TMEM_COLUMNS) : "memory");
+        tc::tmem_dealloc<CG>(tmem_base, T::TMEM_COLUMNS);
     }
 }
 
 template <int CG, int BN, bool A_T, bool B_T, class A, class M> void launch(cudaStream_t s, const A& args, const M& maps) {
     using T = Tile<CG, BN>;
     auto kernel = tf32_kernel<CG, BN, A_T, B_T, A, M>;
-    // The attribute is per device: set it when the device changes (a second thread that sees a
-    // stale value only sets it once more).
     static std::atomic<int> configured_device{-1};
-    static std::atomic<uint32_t> sm_count{0};
-    int device = 0;
-    check(cudaGetDevice(&device), "cudaGetDevice");
-    if (device != configured_device.load(std::memory_order_relaxed)) {
-        check(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(T::TOTAL)), "matmul_tf32 shared memory");
-        int sms = 0;
-        check(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device), "cudaDeviceGetAttribute");
-        sm_count.store(static_cast<uint32_t>(sms), std::memory_order_relaxed);
-        configured_device.store(device, std::memory_order_relaxed);
-    }
+    set_shared_memory(kernel, static_cast<int>(T::TOTAL), configured_device);
     // One CTA per SM, alone or in pairs, each walking its share of the units.
-    const uint32_t most = sm_count.load(std::memory_order_relaxed) / CG;
+    const uint32_t most = device_sm_count() / CG;
     cudaLaunchConfig_t config = {};
     config.gridDim = dim3((args.units < most ? args.units : most) * CG);
     config.blockDim = dim3(T::THREADS);
@@ -598,7 +532,7 @@ bool tma_addressable(const float* base, uint64_t pitch) { return aligned16(base)
 
 void matmul_tf32(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* products, uint32_t count, bool a_t, bool b_t, uint64_t m, uint64_t n, uint64_t k,
                  uint32_t chain, MatmulPitches pitches, uint32_t* status) {
-    Args args = {};
+    Args args;
     Maps maps = {};
     const bool partial = p.splits > 1;
     const uint32_t lda = pitches.a ? pitches.a : static_cast<uint32_t>(a_t ? m : k), ldb = pitches.b ? pitches.b : static_cast<uint32_t>(b_t ? k : n);
@@ -606,13 +540,13 @@ void matmul_tf32(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* pr
     args.n = static_cast<uint32_t>(n);
     // Partial tiles of a split k are dense; the pitch of C applies to the CTAs that write C itself.
     args.ldc = pitches.c && !partial ? pitches.c : static_cast<uint32_t>(n);
-    args.splits = p.splits;
+    args.splits = tc::Divisor(p.splits);
+    args.walk = tc::TileWalk(m, n, p.bm, p.bn);
     args.kblocks = static_cast<uint32_t>((k + BK - 1) / BK);
     args.chain = chain;
     args.status = status;
     args.c_padded = pitches.c != 0 && !partial;
     args.c_vec = args.ldc % 4 == 0;
-    args.c_tma = 1;
     const uint32_t results = chain > 1 ? 1 : count, group = p.bm / 128;
     for (uint32_t g = 0; g < count; ++g) {
         encode_operands(maps, g, products[g].a, lda, products[g].b, ldb, a_t, b_t, m, n, k, p.bn / group);
@@ -623,8 +557,7 @@ void matmul_tf32(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* pr
         args.c_tma = args.c_tma && tma_addressable(args.c[g], args.ldc);
     }
     for (uint32_t g = 0; g < results && args.c_tma; ++g) maps.c[g] = encode(args.c[g], n, m, args.ldc, p.splits, 32, false);
-    args.products = results;
-    args.units = static_cast<uint32_t>(((m + p.bm - 1) / p.bm) * ((n + p.bn - 1) / p.bn)) * p.splits * results;
+    args.units = args.walk.count() * p.splits * results;
     if (p.bm == 256) launch_form<2, 256>(s, a_t, b_t, args, maps);
     else if (p.bn == 128) launch_form<1, 128>(s, a_t, b_t, args, maps);
     else if (p.bn == 64) launch_form<1, 64>(s, a_t, b_t, args, maps);
@@ -632,11 +565,9 @@ void matmul_tf32(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* pr
 }
 
 bool matmul_tf32_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, bool a_t, bool b_t, uint32_t* status) {
-    JobArgs args = {};
+    JobArgs args;
     JobMaps maps = {};
     args.status = status;
-    args.c_tma = args.c_vec = 1;
-    args.chain = 1;
     for (uint32_t j = 0; j < count; ++j) {
         const MatmulJob& job = jobs[j];
         const MatmulTcPlan p = matmul_tc_job_plan(job.m, job.n, job.k);
@@ -647,11 +578,12 @@ bool matmul_tf32_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, boo
         Job& to = args.jobs[args.job_count++];
         to.c = c;
         to.m = static_cast<uint32_t>(job.m);
-        to.n = to.ldc = static_cast<uint32_t>(job.n);
-        to.splits = p.splits;
+        to.n = static_cast<uint32_t>(job.n);
+        to.splits = tc::Divisor(p.splits);
+        to.walk = tc::TileWalk(job.m, job.n, 128, 128);
         to.kblocks = static_cast<uint32_t>((job.k + BK - 1) / BK);
         to.first_unit = args.units;
-        args.units += static_cast<uint32_t>(((job.m + 127) / 128) * ((job.n + 127) / 128)) * p.splits;
+        args.units += to.walk.count() * p.splits;
         encode_operands(maps, j, job.a, lda, job.b, ldb, a_t, b_t, job.m, job.n, job.k, 128);
         maps.c[j] = encode(c, job.n, job.m, job.n, p.splits, 32, false);
     }

@@ -270,9 +270,9 @@ struct MatmulTcPlan {
 // `problems` > 1: that many independent batched products in one launch (k is then not split);
 // `group` > 1: that many products of this shape in one launch of matmul_tc_group (the workspace
 // size is per product).
-// `wide_ok`: the operands can be TMA sources (bases on 16 bytes, row pitches multiples of 4
-// floats), which the 128 x 128 tile needs.
-MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems = 1, uint64_t group = 1, bool wide_ok = true);
+// `tma_ok`: the operands can be TMA sources (bases on 16 bytes, row pitches multiples of 4 floats).
+// `chain` > 1: for matmul_tf32, which sums that many products (their k unsplit).
+MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems = 1, uint64_t group = 1, bool tma_ok = true, uint64_t chain = 1);
 void matmul_tc(cudaStream_t s, const float* a, bool a_t, const float* b, bool b_t, float* c, uint64_t m,
                uint64_t n, uint64_t k, float* workspace, uint32_t* status, const float* bias = nullptr,
                bool leave_partials = false);
@@ -356,12 +356,36 @@ struct MatmulBf16Plan {
     uint32_t bn, splits, kblocks_per_split;
     uint64_t workspace_floats;  // split-k partial tiles [split][m][n]; 0 when k is not split
 };
-MatmulBf16Plan matmul_bf16_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems = 1);
+// `problems`: batched matrices times products of one launch; `chain`: products summed into one result.
+// Either keeps k unsplit when above 1.
+MatmulBf16Plan matmul_bf16_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems = 1, uint64_t chain = 1);
 // `workspace` holds matmul_bf16_plan(m, n, k, outer * inner).workspace_floats floats. With
 // `leave_partials` a split k stops at the partial tiles for finalize_sums (no bias then). A wait
 // that runs out inside the kernel raises bit 1 of *status.
 void matmul_bf16(cudaStream_t s, const HalfMatrix& a, const HalfMatrix& b, const HalfResult& c, uint64_t m, uint64_t n, uint64_t k,
                  uint32_t outer, uint32_t inner, float* workspace, const float* bias, uint32_t* status, bool leave_partials = false);
+// What is applied to a bf16 result as it drains: nothing; gelu, stored in `beside` while C keeps its
+// argument; the gradient of gelu at the argument in `beside`, times the product, stored in C.
+enum class Epilogue { None, Gelu, GeluGrad };
+struct HalfProduct {
+    HalfMatrix a, b;
+    HalfResult c;
+    const float* bias;
+    float* workspace;
+};
+// Up to four products of one shape and storage form in one launch. `chain` > 1: the count = chain products
+// are summed into products[0].c, with its bias.
+void matmul_bf16_group(cudaStream_t s, const HalfProduct* products, uint32_t count, uint64_t m, uint64_t n, uint64_t k, uint32_t outer, uint32_t inner,
+                       uint32_t chain, Epilogue epilogue, const HalfResult& beside, uint32_t* status, bool leave_partials = false);
+// Products of different shapes, one storage form, in one launch: each writes its partial tiles
+// [split][m][n] (f32; one when its k is not split), matmul_bf16_job_plan(m, n, k).workspace_floats floats.
+struct HalfJob {
+    HalfMatrix a, b;
+    float* partial;
+    uint64_t m, n, k;
+};
+MatmulBf16Plan matmul_bf16_job_plan(uint64_t m, uint64_t n, uint64_t k);
+void matmul_bf16_jobs(cudaStream_t s, const HalfJob* jobs, uint32_t count, uint32_t* status);
 
 // ---- attention (attention.cu) -----------------------------------------------------------------
 struct AttentionShape {

@@ -15,6 +15,10 @@
 //   * (=) add_rows(matmul(x, w), b): the bias is added in the matmul's epilogue;
 //   * (=) up to four matmuls of one shape and storage form whose operands exist (the Q, K, V
 //     projections of a layer, their input gradients) are one launch;
+//   * products of one such launch that are addends of the same layer norm's adjoint (the input
+//     gradients of Q, K and V) are one product over their k ranges laid end to end;
+//   * (=) a gelu or gelu_grad that alone takes the result of a product element by element runs as the
+//     product's tiles drain (mixed-precision plans; of the result as it is stored);
 //   * gradient-tagged matmuls whose result only the optimizer reads (weight gradients) wait for
 //     the end of the backward pass and run as jobs of one launch per storage form (their k split
 //     left as partial tiles for the finalize launch);

@@ -295,7 +295,8 @@ void close_peer_reduce(msx_plan* P);
 // Tuning switch: MSX_FUSE is a bit mask of optional fusions (default: all). 1 sublayer tails
 // (dropout + residual + layer norm), 2 adjoint sums inside layer-norm backward, 4 weight-gradient
 // matmuls as jobs of one launch, 8 heavy launches with late readers on a side stream, 16
-// dropout_grad inside the layer-norm backward that makes or reads its operand, 32 the fused
+// dropout_grad inside the layer-norm backward that makes or reads its operand and, in a
+// mixed-precision plan, gelu and gelu_grad inside the product that makes theirs, 32 the fused
 // attention kernels of a mixed-precision plan (off: batched products with row kernels between),
 // 64 the keep decisions of a dropout site stored by the forward launch that draws them, one bit
 // per element, and read by the site's dropout_grad (off: every launch draws again).
@@ -397,7 +398,17 @@ struct Scheduler {
                 pseudo.id = node(part[0].result).id;
                 msx_plan* plan = P;
                 const bool a_t = (form & 2) != 0, b_t = (form & 1) != 0;
+                const bool half = mixed();
                 Launch& l = emit("matmul_jobs", pseudo, reads, writes, [=](cudaStream_t s) {
+                    if (half) {
+                        std::vector<k::HalfJob> jobs;
+                        for (const DeferredMatmul& d : part)
+                            jobs.push_back({{plan->h16(d.a), static_cast<uint32_t>(a_t ? d.m : d.k), 0, 0, a_t},
+                                            {plan->h16(d.b), static_cast<uint32_t>(b_t ? d.k : d.n), 0, 0, b_t},
+                                            plan->f(static_cast<uint32_t>(d.workspace)), d.m, d.n, d.k});
+                        k::matmul_bf16_jobs(s, jobs.data(), static_cast<uint32_t>(jobs.size()), plan->d_status);
+                        return;
+                    }
                     std::vector<k::MatmulJob> jobs;
                     for (const DeferredMatmul& d : part)
                         jobs.push_back({plan->f(d.a), plan->f(d.b), plan->f(static_cast<uint32_t>(d.workspace)),
@@ -574,10 +585,15 @@ struct Scheduler {
         static const char* const names[] = {"embedding", "embedding_grad", "add_layer_norm", "add_layer_norm_dropout", "dropout_add_layer_norm",
                                             "dropout_add", "gelu_layer_norm", "layer_norm", "matmul", "attention_forward", "attention_backward",
                                             "gelu", "unary", "gelu_grad", "dropout", "layer_norm_backward", "cross_entropy_with_grad",
-                                            "cross_entropy", "sum_rows", "sum_rows_batched"};
+                                            "cross_entropy", "sum_rows", "sum_rows_batched", "matmul_jobs"};
         for (const char* name : names)
             if (kernel == name) return true;
         return false;
+    }
+    // A bf16 activation of the arena, through the transposes folded into it.
+    bool arena_half(uint32_t p) const {
+        while (P->slots[p].kind == Slot::View) p = P->slots[p].index;
+        return P->slots[p].kind == Slot::Arena && P->slots[p].half;
     }
 
     uint32_t scratch(uint64_t bytes) {
@@ -1025,19 +1041,19 @@ struct Scheduler {
                 uint64_t m = nd.ty.shape[0], n = nd.ty.shape[1], kk = cols_of(in[0]);
                 std::vector<Product> group = {claim_product(at)};
                 const bool pitched = pitch_of(group[0].a) || pitch_of(group[0].b) || pitchable(group[0].result);
-                if ((fusion_mask() & 4u) && !(P->flags & MSX_PLAN_EXACT_MATMUL) && !mixed() && !pitched && group[0].bias < 0 &&
-                    nd.tag == msx::Tag::Gradient && deferrable(group[0].result)) {
+                if ((fusion_mask() & 4u) && !(P->flags & MSX_PLAN_EXACT_MATMUL) && !pitched && group[0].bias < 0 &&
+                    nd.tag == msx::Tag::Gradient && deferrable(group[0].result) && (!mixed() || (arena_half(group[0].a) && arena_half(group[0].b)))) {
                     const uint64_t operand_bytes = (m * kk + kk * n) * 4;
                     // Only products too small to fill the device on their own: a large one is better
                     // off with the tile the plan model picks for it.
                     if (2 * m * n * kk <= kDeferredMatmulFlop && deferred_matmul_bytes + operand_bytes <= kDeferredMatmulBytes) {
                         deferred_matmul_bytes += operand_bytes;
                         const Product& p = group[0];
-                        const k::MatmulTcPlan job = k::matmul_tc_job_plan(m, n, kk);
+                        const uint32_t splits = mixed() ? k::matmul_bf16_job_plan(m, n, kk).splits : k::matmul_tc_job_plan(m, n, kk).splits;
                         // An unsplit job writes one "partial" tile too: the launch then touches no
                         // output, only scratch that the finalize launch reads, and may run beside others.
-                        const int ws = static_cast<int>(scratch(std::max<uint64_t>(job.workspace_floats, m * n) * 4));
-                        deferred.push_back({static_cast<uint32_t>(ws), 0, job.splits, m * n, p.result});
+                        const int ws = static_cast<int>(scratch(splits * m * n * 4));
+                        deferred.push_back({static_cast<uint32_t>(ws), 0, splits, m * n, p.result});
                         uint32_t a = p.a, b = p.b;
                         const int form = (P->transposed(a) ? 2 : 0) + (P->transposed(b) ? 1 : 0);
                         while (P->slots[a].kind == Slot::View) a = P->slots[a].index;
@@ -1048,7 +1064,7 @@ struct Scheduler {
                 }
                 // Later matmuls of the same shape and storage form whose operands already exist
                 // (the three projections of an attention layer, their gradients) join the launch.
-                if (!(P->flags & MSX_PLAN_EXACT_MATMUL) && !mixed() && !pitched)
+                if (!(P->flags & MSX_PLAN_EXACT_MATMUL) && !pitched)
                     for (uint32_t later = at + 1; later < prog.nodes.size() && later < at + 64 && group.size() < 4; ++later)
                         if (joins(later, group[0], at, m, n, kk)) group.push_back(claim_product(later));
                 emit_matmul(nd, group, m, n, kk);
@@ -1621,6 +1637,7 @@ struct Scheduler {
         std::vector<uint32_t> adjoint = {source};
         auto summed = adjoint_sums.find(source);
         if (summed != adjoint_sums.end()) adjoint = summed->second;
+        chain_addends(adjoint);
         // dropout_grad of dx (the adjoint of the projection under this sublayer's dropout) is a
         // second output of the launch.
         int dropped = -1;
@@ -1807,6 +1824,45 @@ struct Scheduler {
         return deferrable(p.result) == deferrable(first.result);
     }
 
+    // Products of one launch whose results are addends of the same layer norm's adjoint (the input
+    // gradients of the Q, K and V projections) become one product with their k behind one another: one
+    // result is written and read instead of three. Whether they do shows when that layer norm's backward
+    // is scheduled; until then the launch only notes that they may.
+    struct Chainable {
+        uint32_t launch_value;
+        std::vector<uint32_t> results;
+        std::shared_ptr<bool> chained;
+    };
+    std::vector<Chainable> chainables;
+    std::shared_ptr<bool> chainable(const Node& nd, const std::vector<Product>& group) {
+        if (group.size() < 2) return nullptr;
+        Chainable c = {nd.id, {}, std::make_shared<bool>(false)};
+        for (const Product& p : group) {
+            if (p.bias >= 0 || users[p.result].size() != 1 || is_output_value(p.result)) return nullptr;
+            c.results.push_back(p.result);
+        }
+        chainables.push_back(c);
+        return c.chained;
+    }
+    void chain_addends(std::vector<uint32_t>& addends) {
+        for (const Chainable& c : chainables) {
+            if (*c.chained) continue;
+            bool all = true;
+            for (uint32_t r : c.results) all = all && std::count(addends.begin(), addends.end(), r) == 1;
+            if (!all) continue;
+            for (Launch& l : P->launches) {
+                if (l.kernel != "matmul" || l.value != c.launch_value) continue;
+                *c.chained = true;
+                l.writes = {c.results[0]};
+                for (size_t i = 1; i < c.results.size(); ++i) {
+                    P->slots[c.results[i]].kind = Slot::Dead;
+                    addends.erase(std::find(addends.begin(), addends.end(), c.results[i]));
+                }
+                break;
+            }
+        }
+    }
+
     // C[m, n] = op(a) x op(b) for every product of `group` (one shape, one storage form): the exact
     // f32 chain kernel under MSX_PLAN_EXACT_MATMUL (one product), else the tensor cores.
     void emit_matmul(const Node& nd, const std::vector<Product>& group, uint64_t m, uint64_t n, uint64_t kk) {
@@ -1820,7 +1876,7 @@ struct Scheduler {
         const Product first = group[0];
         const bool a_t_flip = first.flip_a, b_t_flip = first.flip_b;
         if (mixed()) {
-            emit_matmul_bf16(nd, first, reads, m, n, kk);
+            emit_matmul_bf16(nd, group, reads, m, n, kk);
             return;
         }
         if (P->flags & MSX_PLAN_EXACT_MATMUL) {
@@ -1843,6 +1899,9 @@ struct Scheduler {
         // A split k whose sum only the optimizer reads (a weight gradient) stays as partial
         // tiles: the finalize launch adds them with every other deferred sum.
         const bool defer = tc.workspace_floats != 0 && first.bias < 0 && deferrable(first.result);
+        const bool tma_ok = a_pitch % 4 == 0 && b_pitch % 4 == 0;
+        const std::shared_ptr<bool> chained = tma_ok && !tc.fma ? chainable(nd, group) : nullptr;
+        const k::MatmulTcPlan chain_plan = chained ? k::matmul_tc_plan(m, n, kk, 1, 1, true, count) : tc;
         k::MatmulPitches pitches;
         pitches.a = pitch_of(first.a);
         pitches.b = pitch_of(first.b);
@@ -1872,8 +1931,9 @@ struct Scheduler {
                 operands[g].bias = p.bias >= 0 ? plan->f(static_cast<uint32_t>(p.bias)) : nullptr;
                 operands[g].workspace = workspaces[g] >= 0 ? plan->f(static_cast<uint32_t>(workspaces[g])) : nullptr;
             }
-            k::matmul_tc_group(s, operands, count, plan->transposed(first.a) != a_t_flip, plan->transposed(first.b) != b_t_flip, m, n, kk,
-                               plan->d_status, defer, pitches);
+            const bool a_t = plan->transposed(first.a) != a_t_flip, b_t = plan->transposed(first.b) != b_t_flip;
+            if (chained && *chained) k::matmul_tf32(s, chain_plan, operands, count, a_t, b_t, m, n, kk, count, pitches, plan->d_status);
+            else k::matmul_tc_group(s, operands, count, a_t, b_t, m, n, kk, plan->d_status, defer, pitches);
         });
         l.flop = 2 * m * n * kk * count;
     }
@@ -1983,41 +2043,94 @@ struct Scheduler {
     // The product of a mixed-precision plan: bf16 operands in place (an activation, or the working
     // copy of a parameter), the result in the storage type of its slot, a split k reduced by the
     // launch or, for a weight gradient, left as f32 partial tiles for the finalize launch.
-    void emit_matmul_bf16(const Node& nd, const Product& p, const std::vector<uint32_t>& reads, uint64_t m, uint64_t n, uint64_t kk) {
+    // The gelu or gelu_grad that alone takes the result of a product element by element runs as the
+    // product's tiles drain: gelu beside its argument (which its gradient reads later), gelu_grad in the
+    // place of the adjoint it multiplies. -1: neither.
+    int gelu_behind(const Product& p) const {
+        if (!(fusion_mask() & 16u) || is_output_value(p.result)) return -1;
+        for (uint32_t u : users[p.result]) {
+            const Node& un = node(u);
+            if (handled[u] || !stored_half(un)) continue;
+            if (un.op == Op::Gelu) {
+                // One that a layer norm reads is a launch with that layer norm.
+                for (uint32_t reader : users[u])
+                    if (node(reader).op == Op::LayerNorm) return -1;
+                return static_cast<int>(u);
+            }
+            if (un.op == Op::GeluGrad && users[p.result].size() == 1 && p.bias < 0 && pos(un.operands[1]) == p.result && pos(un.operands[0]) != p.result &&
+                pos(un.operands[0]) < p.node && arena_half(pos(un.operands[0])) && P->slots[pos(un.operands[0])].kind == Slot::Arena)
+                return static_cast<int>(u);
+        }
+        return -1;
+    }
+
+    void emit_matmul_bf16(const Node& nd, const std::vector<Product>& group, std::vector<uint32_t> reads, uint64_t m, uint64_t n, uint64_t kk) {
         msx_plan* plan = P;
-        for (uint32_t operand : {p.a, p.b}) {
-            uint32_t home = operand;
-            while (P->slots[home].kind == Slot::View) home = P->slots[home].index;
-            const Slot& slot = P->slots[home];
-            const bool ok = (slot.kind == Slot::Arena && slot.half) || (slot.kind == Slot::Param && node(home).ty.rank() == 2);
-            if (!ok) unsupported(nd, "a bf16 plan multiplies bf16 activations and matrix parameters; %" + std::to_string(node(home).id) + " is neither");
+        for (const Product& p : group)
+            for (uint32_t operand : {p.a, p.b}) {
+                uint32_t home = operand;
+                while (P->slots[home].kind == Slot::View) home = P->slots[home].index;
+                const Slot& slot = P->slots[home];
+                const bool ok = (slot.kind == Slot::Arena && slot.half) || (slot.kind == Slot::Param && node(home).ty.rank() == 2);
+                if (!ok) unsupported(nd, "a bf16 plan multiplies bf16 activations and matrix parameters; %" + std::to_string(node(home).id) + " is neither");
+            }
+        const Product first = group[0];
+        const uint32_t count = static_cast<uint32_t>(group.size());
+        const k::MatmulBf16Plan tc = k::matmul_bf16_plan(m, n, kk, count);
+        const bool defer = tc.workspace_floats != 0 && first.bias < 0 && deferrable(first.result);
+        if (count == 1 && pitchable(first.result)) set_pitch(first.result);
+        const int behind = count == 1 && tc.splits == 1 && n % 8 == 0 && P->slots[first.result].half ? gelu_behind(first) : -1;
+        const k::Epilogue epilogue = behind < 0 ? k::Epilogue::None
+                                     : node(static_cast<uint32_t>(behind)).op == Op::Gelu ? k::Epilogue::Gelu : k::Epilogue::GeluGrad;
+        uint32_t result_of_first = first.result, beside = 0;
+        if (behind >= 0) {
+            const uint32_t u = static_cast<uint32_t>(behind);
+            handled[u] = 1;
+            make_arena(P->slots[u], node(u));
+            if (epilogue == k::Epilogue::Gelu) {
+                beside = u;
+            } else {
+                beside = pos(node(u).operands[0]);
+                reads.push_back(beside);
+                P->slots[first.result].kind = Slot::Dead;
+                result_of_first = u;
+            }
         }
-        const k::MatmulBf16Plan tc = k::matmul_bf16_plan(m, n, kk);
-        const bool defer = tc.workspace_floats != 0 && p.bias < 0 && deferrable(p.result);
-        if (pitchable(p.result)) set_pitch(p.result);
+        const std::shared_ptr<bool> chained = chainable(nd, group);
         std::vector<uint32_t> writes;
-        int ws = -1;
-        if (tc.workspace_floats) {
-            ws = static_cast<int>(scratch(tc.workspace_floats * 4));
-            writes.push_back(static_cast<uint32_t>(ws));
+        std::vector<int> workspaces;
+        for (const Product& p : group) {
+            int ws = -1;
+            if (tc.workspace_floats) {
+                ws = static_cast<int>(scratch(tc.workspace_floats * 4));
+                writes.push_back(static_cast<uint32_t>(ws));
+            }
+            workspaces.push_back(ws);
+            if (defer) deferred.push_back({static_cast<uint32_t>(ws), 0, tc.splits, m * n, p.result});
+            else writes.push_back(&p == &group[0] ? result_of_first : p.result);
         }
-        if (defer) deferred.push_back({static_cast<uint32_t>(ws), 0, tc.splits, m * n, p.result});
-        else writes.push_back(p.result);
-        const bool a_t = P->transposed(p.a) != p.flip_a, b_t = P->transposed(p.b) != p.flip_b;
-        const uint32_t a_pitch = pitch_of(p.a) ? pitch_of(p.a) : static_cast<uint32_t>(a_t ? m : kk);
-        const uint32_t b_pitch = pitch_of(p.b) ? pitch_of(p.b) : static_cast<uint32_t>(b_t ? kk : n);
-        const uint32_t c_pitch = P->slots[p.result].pitch;
-        const uint32_t a = p.a, b = p.b, result = p.result;
-        const int bias = p.bias;
+        if (epilogue == k::Epilogue::Gelu) writes.push_back(beside);
+        const bool a_t = P->transposed(first.a) != first.flip_a, b_t = P->transposed(first.b) != first.flip_b;
+        const uint32_t a_pitch = pitch_of(first.a) ? pitch_of(first.a) : static_cast<uint32_t>(a_t ? m : kk);
+        const uint32_t b_pitch = pitch_of(first.b) ? pitch_of(first.b) : static_cast<uint32_t>(b_t ? kk : n);
+        const uint32_t c_pitch = P->slots[first.result].pitch;
+        const std::vector<Product> products = group;
         Launch& l = emit("matmul", nd, reads, writes, [=](cudaStream_t s) {
-            const k::HalfMatrix A = {plan->h16(a), a_pitch, 0, 0, a_t};
-            const k::HalfMatrix B = {plan->h16(b), b_pitch, 0, 0, b_t};
-            const k::HalfResult C = {plan->ptr(result), plan->half(result), c_pitch, 0, 0};
-            if (!A.base || !B.base) throw StatusError(MSX_LAUNCH_FAILED, "a matmul operand of a bf16 plan has no bf16 storage");
-            k::matmul_bf16(s, A, B, C, m, n, kk, 1, 1, ws >= 0 ? plan->f(static_cast<uint32_t>(ws)) : nullptr,
-                           bias >= 0 ? plan->f(static_cast<uint32_t>(bias)) : nullptr, plan->d_status, defer);
+            k::HalfProduct operands[4];
+            for (uint32_t g = 0; g < count; ++g) {
+                const Product& p = products[g];
+                const uint32_t result = g == 0 ? result_of_first : p.result;
+                operands[g].a = {plan->h16(p.a), a_pitch, 0, 0, a_t};
+                operands[g].b = {plan->h16(p.b), b_pitch, 0, 0, b_t};
+                if (!operands[g].a.base || !operands[g].b.base) throw StatusError(MSX_LAUNCH_FAILED, "a matmul operand of a bf16 plan has no bf16 storage");
+                operands[g].c = {plan->ptr(result), plan->half(result), c_pitch, 0, 0};
+                operands[g].bias = p.bias >= 0 ? plan->f(static_cast<uint32_t>(p.bias)) : nullptr;
+                operands[g].workspace = workspaces[g] >= 0 ? plan->f(static_cast<uint32_t>(workspaces[g])) : nullptr;
+            }
+            const k::HalfResult aside = {epilogue == k::Epilogue::None ? nullptr : plan->ptr(beside), true, 0, 0, 0};
+            k::matmul_bf16_group(s, operands, count, m, n, kk, 1, 1, chained && *chained ? count : 1, epilogue, aside, plan->d_status, defer);
         });
-        l.flop = 2 * m * n * kk;
+        l.flop = 2 * m * n * kk * count;
     }
 
     std::map<std::array<uint32_t, 5>, uint32_t> forward_probabilities;  // (q, k, v, mask, heads) -> scratch slot

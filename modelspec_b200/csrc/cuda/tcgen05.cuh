@@ -103,6 +103,131 @@ template <int Pending> __device__ __forceinline__ void tma_store_wait_read() {
     asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(Pending) : "memory");
 }
 
+// ---- the tiles of a product --------------------------------------------------------------------------
+// Division by a number known at launch: a multiplication (of dividends below 2^31; Granlund and
+// Montgomery, PLDI 1994, figure 4.1). A persistent CTA finds its next tile in every role, and five
+// divisions one after the other are half a microsecond each time.
+struct Divisor {
+    uint32_t d = 1, multiplier = 1, shift = 0;
+    Divisor() = default;
+    explicit Divisor(uint32_t by) : d(by) {
+        while (shift < 32 && (1ull << shift) < by) ++shift;
+        multiplier = static_cast<uint32_t>((1ull << 32) * ((1ull << shift) - by) / by + 1);
+    }
+    __device__ __forceinline__ uint32_t quotient(uint32_t x) const { return (__umulhi(x, multiplier) + x) >> shift; }
+};
+// Tiles are walked in bands of 8 rows of tiles, column by column: the tiles that the device works on at a
+// time then form a block about as high as it is wide, and read the fewest different rows of A and columns
+// of B (18,944 x 3,072 x 3,072 in bf16: 302 us down whole columns, 242 in bands of 4 to 16).
+struct TileWalk {
+    static constexpr uint32_t BAND = 8;
+    uint32_t down = 1, rows = 0, columns = 0;  // rows of tiles; rows and columns of one
+    Divisor tiles, band_tiles, last_band;
+    TileWalk() = default;
+    TileWalk(uint64_t m, uint64_t n, uint32_t tile_rows, uint32_t tile_columns)
+        : down(static_cast<uint32_t>((m + tile_rows - 1) / tile_rows)), rows(tile_rows), columns(tile_columns) {
+        const uint32_t across = static_cast<uint32_t>((n + tile_columns - 1) / tile_columns);
+        tiles = Divisor(down * across);
+        band_tiles = Divisor(BAND * across);
+        last_band = Divisor(down % BAND ? down % BAND : BAND);
+    }
+    uint32_t count() const { return tiles.d; }
+    // Splits `u` into a tile's first row and column and what follows the tiles.
+    __device__ __forceinline__ uint32_t take(uint32_t u, uint32_t* m0, uint32_t* n0) const {
+        const uint32_t rest = tiles.quotient(u), tile = u - rest * tiles.d;
+        const uint32_t band = band_tiles.quotient(tile), in_band = tile - band * band_tiles.d;
+        const bool last = (band + 1) * BAND > down;
+        const uint32_t column = last ? last_band.quotient(in_band) : in_band / BAND;
+        *m0 = (band * BAND + in_band - column * (last ? last_band.d : BAND)) * rows;
+        *n0 = column * columns;
+        return rest;
+    }
+};
+
+// ---- one CTA, or a pair of CTAs of a cluster (CG = 2) that share their MMAs ---------------------------
+template <int CG> __device__ __forceinline__ uint32_t cta_rank() {
+    uint32_t rank = 0;
+    if constexpr (CG == 2) asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    return rank;
+}
+// By one warp of each CTA of the group.
+template <int CG> __device__ __forceinline__ void tmem_alloc(uint32_t slot, uint32_t columns) {
+    if constexpr (CG == 1) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(columns) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    } else {
+        asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(slot), "r"(columns) : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+    }
+}
+template <int CG> __device__ __forceinline__ void tmem_dealloc(uint32_t base, uint32_t columns) {
+    if constexpr (CG == 1) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns) : "memory");
+    else asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(base), "r"(columns) : "memory");
+}
+// Arrives on `bar` (of both CTAs of a pair) when the MMAs issued so far have completed.
+template <int CG> __device__ __forceinline__ void commit(uint32_t bar) {
+    if constexpr (CG == 1) mma_commit(bar);
+    else
+        asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                     ::"r"(bar), "h"(static_cast<uint16_t>(3)) : "memory");
+}
+// Arrives on the first CTA's barrier at the same offset.
+template <int CG> __device__ __forceinline__ void arrive_first(uint32_t bar) {
+    if constexpr (CG == 1) mbar_arrive(bar);
+    else
+        asm volatile("{\n\t.reg .b32 far;\n\tmapa.shared::cluster.u32 far, %0, 0;\n\tmbarrier.arrive.release.cluster.shared::cluster.b64 _, [far];\n\t}"
+                     ::"r"(bar) : "memory");
+}
+template <int CG> __device__ __forceinline__ bool try_wait(uint32_t bar, uint32_t parity) {
+    if constexpr (CG == 1) return mbar_try_wait(bar, parity);
+    uint32_t ok;
+    asm volatile("{\n\t.reg .pred p;\n\tmbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\tselp.u32 %0, 1, 0, p;\n\t}"
+                 : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    return ok != 0;
+}
+// Waits for `parity` of `bar`, all lanes of a warp together; false when the wait ran out or another
+// role gave up.
+template <int CG> __device__ __forceinline__ bool warp_wait(uint32_t bar, uint32_t parity, volatile uint32_t* abort_flag, uint32_t* status) {
+    bool ok = false;
+    for (uint32_t spin = 0; spin < WAIT_LIMIT; ++spin) {
+        if (try_wait<CG>(bar, parity)) { ok = true; break; }
+        if ((spin & 255u) == 255u && *abort_flag) break;
+    }
+    ok = __all_sync(0xffffffffu, ok);
+    if (!ok && *abort_flag == 0) {
+        *abort_flag = 1;
+        atomicOr(status, 2u);
+    }
+    return ok;
+}
+
+__device__ __forceinline__ void cluster_barrier() {
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// The first CTA's shared memory at the same offset.
+template <int CG> __device__ __forceinline__ uint32_t first_cta(uint32_t address) {
+    if constexpr (CG == 1) return address;
+    uint32_t far;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, 0;" : "=r"(far) : "r"(address));
+    return far;
+}
+// One box of a (column, row, inner, outer) tensor map into this CTA's shared memory (its bytes counted, for a
+// pair, on a barrier of either CTA), and back.
+template <int CG> __device__ __forceinline__ void load_tile(uint32_t dst, const CUtensorMap* map, uint32_t bar, uint32_t x, uint32_t row, uint32_t inner, uint32_t outer) {
+    if constexpr (CG == 1)
+        asm volatile("cp.async.bulk.tensor.4d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                     ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(row), "r"(inner), "r"(outer) : "memory");
+    else
+        asm volatile("cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4, %5, %6}], [%2];"
+                     ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(row), "r"(inner), "r"(outer) : "memory");
+}
+__device__ __forceinline__ void store_tile(const CUtensorMap* map, uint32_t src, uint32_t x, uint32_t row, uint32_t inner, uint32_t outer) {
+    asm volatile("cp.async.bulk.tensor.4d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+                 ::"l"(map), "r"(src), "r"(x), "r"(row), "r"(inner), "r"(outer) : "memory");
+    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+}
+
 // Byte offset of the 16-byte chunk `c16` (8 bf16 elements) of row `row` in a tile of 128-byte rows
 // with the 128-byte swizzle TMA writes and tcgen05 reads: 8-row groups of 1024 bytes, the chunk
 // index xor-ed with the row within its group.
