@@ -1834,8 +1834,10 @@ struct Scheduler {
         std::shared_ptr<bool> chained;
     };
     std::vector<Chainable> chainables;
-    std::shared_ptr<bool> chainable(const Node& nd, const std::vector<Product>& group) {
-        if (group.size() < 2) return nullptr;
+    static constexpr uint64_t kChainedTiles = 148;  // of 128 x 128: one for every SM
+    std::shared_ptr<bool> chainable(const Node& nd, const std::vector<Product>& group, uint64_t m, uint64_t n) {
+        // Side by side the products of a small result keep more SMs busy than one with a longer k would.
+        if (group.size() < 2 || (m + 127) / 128 * ((n + 127) / 128) < kChainedTiles) return nullptr;
         Chainable c = {nd.id, {}, std::make_shared<bool>(false)};
         for (const Product& p : group) {
             if (p.bias >= 0 || users[p.result].size() != 1 || is_output_value(p.result)) return nullptr;
@@ -1900,7 +1902,7 @@ struct Scheduler {
         // tiles: the finalize launch adds them with every other deferred sum.
         const bool defer = tc.workspace_floats != 0 && first.bias < 0 && deferrable(first.result);
         const bool tma_ok = a_pitch % 4 == 0 && b_pitch % 4 == 0;
-        const std::shared_ptr<bool> chained = tma_ok && !tc.fma ? chainable(nd, group) : nullptr;
+        const std::shared_ptr<bool> chained = tma_ok && !tc.fma ? chainable(nd, group, m, n) : nullptr;
         const k::MatmulTcPlan chain_plan = chained ? k::matmul_tc_plan(m, n, kk, 1, 1, true, count) : tc;
         k::MatmulPitches pitches;
         pitches.a = pitch_of(first.a);
@@ -2096,7 +2098,7 @@ struct Scheduler {
                 result_of_first = u;
             }
         }
-        const std::shared_ptr<bool> chained = chainable(nd, group);
+        const std::shared_ptr<bool> chained = chainable(nd, group, m, n);
         std::vector<uint32_t> writes;
         std::vector<int> workspaces;
         for (const Product& p : group) {
