@@ -19,40 +19,77 @@ namespace k {
 
 namespace {
 
-// One warp per score row: p = softmax over the unmasked keys of acc * scale, in place.
-__global__ void masked_softmax_kernel(float* __restrict__ scores, const float* __restrict__ mask, uint32_t rows,
-                                      uint32_t rows_per_sequence, uint32_t s, float scale) {
-    uint32_t row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+// One warp per score row, the row in registers (key lane + 32 i is item i of a lane; ITEMS x 32 keys or
+// fewer): a score is read once and a probability written once, with every load of a row in flight together.
+constexpr uint32_t ROW_BLOCK_WARPS = 8;
+
+// p = softmax over the unmasked keys of acc * scale, in place.
+template <int ITEMS>
+__global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(float* __restrict__ scores, const float* __restrict__ mask, uint32_t rows,
+                                                                              uint32_t rows_per_sequence, uint32_t s, float scale) {
+    const uint32_t row = blockIdx.x * ROW_BLOCK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
-    int lane = threadIdx.x & 31;
     float* p = scores + static_cast<uint64_t>(row) * s;
     const float* m = mask + static_cast<uint64_t>(row / rows_per_sequence) * s;
+    float x[ITEMS];
+    uint32_t counts = 0;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t j = min(lane + 32 * i, s - 1);
+        x[i] = p[j];
+        counts |= (lane + 32 * i < s && __ldg(m + j) != 0.0f ? 1u : 0u) << i;
+    }
     float best = -INFINITY;
-    for (uint32_t j = lane; j < s; j += 32)
-        if (m[j] != 0.0f) best = fmaxf(best, p[j] * scale);
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+        if ((counts >> i) & 1u) best = fmaxf(best, x[i] * scale);
     best = warp_max(best);
     float total = 0.0f;
-    for (uint32_t j = lane; j < s; j += 32) {
-        float e = m[j] != 0.0f ? expf(p[j] * scale - best) : 0.0f;
-        p[j] = e;
-        total += e;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        x[i] = (counts >> i) & 1u ? expf(x[i] * scale - best) : 0.0f;
+        total += x[i];
     }
     total = warp_sum(total);
-    for (uint32_t j = lane; j < s; j += 32) p[j] = p[j] / total;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+        if (lane + 32 * i < s) p[lane + 32 * i] = x[i] / total;
 }
 
 // dS = scale * P * (dP - sum_j P dP), written over dP.
-__global__ void score_grad_kernel(const float* __restrict__ p, float* __restrict__ dp, uint32_t rows, uint32_t s, float scale) {
-    uint32_t row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
+template <int ITEMS>
+__global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) score_grad_kernel(const float* __restrict__ p, float* __restrict__ dp, uint32_t rows, uint32_t s,
+                                                                          float scale) {
+    const uint32_t row = blockIdx.x * ROW_BLOCK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
-    int lane = threadIdx.x & 31;
     const float* pr = p + static_cast<uint64_t>(row) * s;
     float* dr = dp + static_cast<uint64_t>(row) * s;
+    float x[ITEMS], d[ITEMS];
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i) {
+        const uint32_t j = min(lane + 32 * i, s - 1);
+        x[i] = __ldg(pr + j);
+        d[i] = dr[j];
+    }
     float dot = 0.0f;
-    for (uint32_t j = lane; j < s; j += 32) dot = fmaf(pr[j], dr[j], dot);
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+        if (lane + 32 * i < s) dot = fmaf(x[i], d[i], dot);
     dot = warp_sum(dot);
-    for (uint32_t j = lane; j < s; j += 32) dr[j] = pr[j] * (dr[j] - dot) * scale;
+#pragma unroll
+    for (int i = 0; i < ITEMS; ++i)
+        if (lane + 32 * i < s) dr[lane + 32 * i] = x[i] * (d[i] - dot) * scale;
 }
+
+// The kernel of the narrowest row that holds `s` keys (at most 512).
+#define MSX_FOR_KEYS(kernel, s, ...)                          \
+    do {                                                      \
+        const dim3 grid((rows + ROW_BLOCK_WARPS - 1) / ROW_BLOCK_WARPS), block(32 * ROW_BLOCK_WARPS); \
+        if ((s) <= 64) kernel<2><<<grid, block, 0, stream>>>(__VA_ARGS__);        \
+        else if ((s) <= 128) kernel<4><<<grid, block, 0, stream>>>(__VA_ARGS__);  \
+        else if ((s) <= 256) kernel<8><<<grid, block, 0, stream>>>(__VA_ARGS__);  \
+        else kernel<16><<<grid, block, 0, stream>>>(__VA_ARGS__);                 \
+    } while (0)
 
 struct Heads {
     uint32_t b, l, s, a, d, h;
@@ -79,7 +116,8 @@ void probabilities(cudaStream_t s, const float* q, const float* k, const float* 
     // S[i, j] = sum_c q[i, c] k[j, c]: B is the keys stored [n, k].
     matmul_tc_batched(s, hd.q(q), transposed(hd.kv(k)), hd.scores(p), hd.l, hd.s, hd.d, hd.b, hd.a, status);
     uint32_t rows = hd.rows();
-    masked_softmax_kernel<<<(rows + 7) / 8, 256, 0, s>>>(p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
+    const cudaStream_t stream = s;
+    MSX_FOR_KEYS(masked_softmax_kernel, hd.s, p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
     check_launch("attention masked_softmax");
 }
 
@@ -109,7 +147,8 @@ void attention_tc_backward(cudaStream_t s, const float* q, const float* k, const
     // dP[i, j] = sum_c g[i, c] v[j, c]
     matmul_tc_batched(s, hd.q(g), transposed(hd.kv(v)), hd.scores(dp), hd.l, hd.s, hd.d, hd.b, hd.a, status);
     uint32_t rows = hd.rows();
-    score_grad_kernel<<<(rows + 7) / 8, 256, 0, s>>>(p, dp, rows, hd.s, hd.scale);
+    const cudaStream_t stream = s;
+    MSX_FOR_KEYS(score_grad_kernel, hd.s, p, dp, rows, hd.s, hd.scale);
     check_launch("attention score_grad");
     // dQ[i, c] = sum_j dS[i, j] k[j, c];  dK[j, c] = sum_i dS[i, j] q[i, c]
     if (dq) matmul_tc_batched(s, hd.scores(dp), hd.kv(k), hd.q(dq), hd.l, hd.d, hd.s, hd.b, hd.a, status);
