@@ -525,7 +525,7 @@ CUtensorMap encode_b(const HalfMatrix& b, uint64_t n, uint64_t k, uint32_t inner
 // gradients: few tiles, k = the batch's rows). Measured, earlier 128 x 256 tiles of one CTA -> now:
 // 16,384 x 768 x 3,072 73 -> 62 us (1,240 TFLOP/s), 16,384 x 3,072 x 768 75 -> 58, 4,096 x 128 x 512
 // 8.5 -> 6.3, 4,096 x 512 x 128 8.3 -> 6.6.
-MatmulBf16Plan matmul_bf16_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems, uint64_t chain) {
+MatmulBf16Plan matmul_bf16_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t products, uint64_t chain, uint64_t batch) {
     struct Candidate {
         uint32_t bm, bn;
         double fixed, block, drain, at_once;
@@ -536,13 +536,13 @@ MatmulBf16Plan matmul_bf16_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t pro
     MatmulBf16Plan best = {};
     double best_cost = 0.0;
     for (const Candidate& c : candidates) {
-        const uint64_t tiles = (m + c.bm - 1) / c.bm * ((n + c.bn - 1) / c.bn) * problems;
-        const uint64_t most = problems > 1 || chain > 1 ? 1 : std::max<uint64_t>(1, std::min<uint64_t>(32, kblocks / 4));
+        const uint64_t tiles = (m + c.bm - 1) / c.bm * ((n + c.bn - 1) / c.bn) * products * batch;
+        const uint64_t most = batch > 1 || chain > 1 ? 1 : std::max<uint64_t>(1, std::min<uint64_t>(32, kblocks / 4));
         for (uint64_t splits = 1; splits <= most; ++splits) {
             const uint64_t per = (kblocks + splits - 1) / splits;
             if (kblocks && (kblocks + per - 1) / per != splits) continue;
             double cost = c.fixed + std::ceil(static_cast<double>(tiles * splits) / c.at_once) * std::max(static_cast<double>(per * chain) * c.block, c.drain);
-            if (splits > 1) cost += kReduceFixed + static_cast<double>(m * n * (splits + 1)) * 4.0 / kReduceBytesPerUs;
+            if (splits > 1) cost += kReduceFixed + static_cast<double>(products * m * n * (splits + 1)) * 4.0 / kReduceBytesPerUs;
             if (best.bn != 0 && cost >= best_cost) continue;
             best_cost = cost;
             best.bn = c.bn;
@@ -560,7 +560,7 @@ void matmul_bf16_group(cudaStream_t s, const HalfProduct* products, uint32_t cou
     if (count > MAX_PRODUCTS) throw std::invalid_argument("matmul_bf16: more products than one launch carries");
     const uint64_t problems = static_cast<uint64_t>(outer) * inner;
     const uint32_t results = chain > 1 ? 1 : count;
-    const MatmulBf16Plan p = matmul_bf16_plan(m, n, k, problems * results, chain);
+    const MatmulBf16Plan p = matmul_bf16_plan(m, n, k, results, chain, problems);
     const bool partial = p.splits > 1;
     Args args;
     Maps maps = {};

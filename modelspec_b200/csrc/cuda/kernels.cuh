@@ -356,10 +356,10 @@ struct MatmulBf16Plan {
     uint32_t bn, splits, kblocks_per_split;
     uint64_t workspace_floats;  // split-k partial tiles [split][m][n]; 0 when k is not split
 };
-// `problems`: batched matrices times products of one launch; `chain`: products summed into one result.
-// Either keeps k unsplit when above 1.
-MatmulBf16Plan matmul_bf16_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems = 1, uint64_t chain = 1);
-// `workspace` holds matmul_bf16_plan(m, n, k, outer * inner).workspace_floats floats. With
+// `products` of one launch (workspace_floats is that of each), `chain` products summed into one result,
+// `batch` matrices of each. A chain or a batch keeps k unsplit.
+MatmulBf16Plan matmul_bf16_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t products = 1, uint64_t chain = 1, uint64_t batch = 1);
+// `workspace` holds matmul_bf16_plan(m, n, k, 1, 1, outer * inner).workspace_floats floats. With
 // `leave_partials` a split k stops at the partial tiles for finalize_sums (no bias then). A wait
 // that runs out inside the kernel raises bit 1 of *status.
 void matmul_bf16(cudaStream_t s, const HalfMatrix& a, const HalfMatrix& b, const HalfResult& c, uint64_t m, uint64_t n, uint64_t k,
