@@ -54,7 +54,7 @@ struct FusedArgs {
     void* dv;
     uint32_t* status;
     uint32_t batch, q_len, k_len, heads, d, h;
-    float scale;
+    float scale, scale_log2;  // 1 / sqrt(d), and times log2(e)
     CoordOrder order;    // of every [rows, H] operand's tensor map
 };
 
@@ -64,6 +64,19 @@ __device__ __forceinline__ uint32_t keys_that_count(const float* __restrict__ ma
     const uint32_t key = first + lane;
     const bool counts = key < k_len && mask[static_cast<uint64_t>(seq) * k_len + key] != 0.0f;
     return __ballot_sync(0xffffffffu, counts);
+}
+
+// The row work is bound by instructions (16,384 scores a tile), so an element gets as few as there are:
+// the maximum over the products as they are, then exp(scale (x - max)) as one fused multiply-add and one
+// base-2 exponential, and a mask only where one of the 32 keys is masked: -inf, whose exponential is 0.
+// (A product, a difference, a product with log2(e) and a test of the mask each, before the maximum and
+// again behind it, came to 27 instructions an element: forward 165 us, backward 264 at
+// 32 x 12 x 512 x 64; now 121 and 182.)
+__device__ __forceinline__ void hide_masked(uint32_t (&r)[32], uint32_t counts) {
+    if (counts == 0xffffffffu) return;
+#pragma unroll
+    for (int c = 0; c < 32; ++c)
+        if (!((counts >> c) & 1u)) r[c] = 0xff800000u;
 }
 
 // One [128 rows, 64 columns] tile of a [rows, H] operand: rows row0.. of sequence `seq`, head `head`.
@@ -240,7 +253,7 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
         const uint32_t quarter = warp & 3u, chunk = (warp - 2) >> 2, t = quarter * 32 + lane;
         const uint32_t lane_base = (quarter * 32u) << 16;
         const uint32_t row = q0 + t;
-        float best = -INFINITY, total = 0.0f;  // total: over this thread's columns only, until the end
+        float best = -INFINITY, total = 0.0f;  // best: of the products q . k, before the scale; total: over this thread's columns only, until the end
         float o[16];
 #pragma unroll
         for (int c = 0; c < 16; ++c) o[c] = 0.0f;
@@ -273,7 +286,7 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             tmem_load16(tmem_pv + (j & 1u) * 64 + lane_base + chunk * 16, pv);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int c = 0; c < 16; ++c) o[c] = o[c] * pending_shrink + __uint_as_float(pv[c]);
+            for (int c = 0; c < 16; ++c) o[c] = fmaf(o[c], pending_shrink, __uint_as_float(pv[c]));
             asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
             return true;
         };
@@ -287,26 +300,24 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
             uint32_t r[32];
             tmem_load32(tmem_base + stage * 128 + lane_base + chunk * 32, r);
             asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-            float sc[32];
-            float mine = -INFINITY;
+            hide_masked(r, counts);
+            float most[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
 #pragma unroll
-            for (int c = 0; c < 32; ++c) {
-                sc[c] = ((counts >> c) & 1u) ? __uint_as_float(r[c]) * args.scale : -INFINITY;
-                mine = fmaxf(mine, sc[c]);
-            }
+            for (int c = 0; c < 32; ++c) most[c & 3] = fmaxf(most[c & 3], __uint_as_float(r[c]));
             float parts[4];
-            alive = exchange_with_row(mine, parts);
+            alive = exchange_with_row(fmaxf(fmaxf(most[0], most[1]), fmaxf(most[2], most[3])), parts);
             if (!alive) break;
             const float new_best = fmaxf(fmaxf(best, fmaxf(parts[0], parts[1])), fmaxf(parts[2], parts[3]));
             // exp(-inf - -inf) never forms: a row that has seen no key yet keeps zeros.
-            const float shrink = best == -INFINITY ? 0.0f : __expf(best - new_best);
-            float tile_total = 0.0f;
+            const float shrink = best == -INFINITY ? 0.0f : exp2_fast((best - new_best) * args.scale_log2);
+            const float shift = new_best == -INFINITY ? 0.0f : new_best * args.scale_log2;
+            float sc[32], sums[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
             for (int c = 0; c < 32; ++c) {
-                sc[c] = ((counts >> c) & 1u) ? __expf(sc[c] - new_best) : 0.0f;
-                tile_total += sc[c];
+                sc[c] = exp2_fast(fmaf(__uint_as_float(r[c]), args.scale_log2, -shift));
+                sums[c & 3] += sc[c];
             }
-            total = total * shrink + tile_total;
+            total = fmaf(total, shrink, (sums[0] + sums[1]) + (sums[2] + sums[3]));
             best = new_best;
             // This stage of P is free: P_j-2 V_j-2 was complete before this thread added it, a tile ago.
             store_chunk_bf16(p_tile(stage), t, chunk, sc);
@@ -334,7 +345,7 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 store_part_bf16(args.out, global_row * args.h + head * args.d, o, chunk * 16, args.d);
                 if (args.stats != nullptr && chunk == 0) {
                     float* st = args.stats + (global_row * args.heads + head) * 2;
-                    st[0] = best;
+                    st[0] = best * args.scale;
                     st[1] = sum;
                 }
             }
@@ -347,11 +358,11 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
 
 // ---- backward -------------------------------------------------------------------------------------
 // Shared memory: K_j, V_j, two stages of (Q_i, G_i), P (two tiles), dS (two tiles): 160 KB; then
-// barriers and the row statistics of every query (max, 1 / sum, D).
+// barriers and the row statistics of every query (the shift of its exponents, D).
 // Tensor memory (512 columns): S / dP [0, 128), dV [128, 192), dK [192, 256), dQ_i [256 + 64 i, ..).
 constexpr uint32_t BWD_TILES = 10 * TILE_BYTES;
 constexpr uint32_t BWD_ROWS = 512;
-constexpr uint32_t BWD_SMEM = BWD_TILES + 1024 /* alignment slack */ + 256 /* barriers */ + 3 * BWD_ROWS * 4;
+constexpr uint32_t BWD_SMEM = BWD_TILES + 1024 /* alignment slack */ + 256 /* barriers */ + 2 * BWD_ROWS * 4;
 constexpr uint32_t BWD_TMEM = 512;
 
 __global__ void __launch_bounds__(THREADS, 1)
@@ -375,9 +386,9 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
            DQ_FULL, STATS_MET, BARS };
     uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + BARS);
     volatile uint32_t* abort_flag = reinterpret_cast<volatile uint32_t*>(tmem_slot + 1);
-    float* row_best = reinterpret_cast<float*>(tiles + BWD_TILES + 256);  // [BWD_ROWS]
-    float* row_inverse = row_best + BWD_ROWS;                             // 1 / sum of exp
-    float* row_dot = row_inverse + BWD_ROWS;                              // D_i
+    // P = exp(score - max) / sum = 2^(x scale_log2 - shift), shift = max log2(e) + log2(sum).
+    float* row_shift = reinterpret_cast<float*>(tiles + BWD_TILES + 256);  // [BWD_ROWS]
+    float* row_dot = row_shift + BWD_ROWS;                                 // D_i
 
     const uint32_t tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
     const uint32_t head = blockIdx.x, seq = blockIdx.y;
@@ -437,23 +448,29 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         const uint32_t idesc_queries = instruction_descriptor(TILE, 64, false, true);     // dS K
         bool alive = true;
         uint32_t pair = 0;
+        // S = Q_i K_j^T of a pair, once its Q and G are there.
+        auto scores = [&](uint32_t of) -> bool {
+            const uint32_t stage = of & 1u;
+            if (!mbar_wait(bar(QG_FULL0 + stage), (of >> 1) & 1u, abort_flag, args.status)) return false;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (lane == 0) {
+#pragma unroll
+                for (uint32_t ks = 0; ks < 4; ++ks)
+                    mma_bf16(tmem_sp, tile_descriptor(smem_u32(q_tile(stage)) + ks * 32, 16), tile_descriptor(smem_u32(k_tile) + ks * 32, 16), idesc_scores, ks != 0);
+                mma_commit(bar(S_FULL));
+            }
+            __syncwarp();
+            return true;
+        };
         for (uint32_t j = 0; j < key_tiles && alive; ++j) {
             alive = mbar_wait(bar(KV_FULL), j & 1u, abort_flag, args.status);
             // dV_j and dK_j start from zero: the previous key tile's must have been drained.
             if (alive) alive = mbar_wait(bar(ACC_EMPTY), (j & 1u) ^ 1u, abort_flag, args.status);
             for (uint32_t i = 0; i < query_tiles && alive; ++i, ++pair) {
-                const uint32_t stage = pair & 1u, use = pair >> 1, ph = pair & 1u;
+                const uint32_t stage = pair & 1u, ph = pair & 1u;
                 const uint32_t q_at = smem_u32(q_tile(stage)), g_at = smem_u32(g_tile(stage));
-                alive = mbar_wait(bar(QG_FULL0 + stage), use & 1u, abort_flag, args.status);
+                if (i == 0) alive = scores(pair);
                 if (!alive) break;
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
-#pragma unroll
-                    for (uint32_t ks = 0; ks < 4; ++ks)
-                        mma_bf16(tmem_sp, tile_descriptor(q_at + ks * 32, 16), tile_descriptor(smem_u32(k_tile) + ks * 32, 16), idesc_scores, ks != 0);
-                    mma_commit(bar(S_FULL));
-                }
-                __syncwarp();
                 // The row threads have read S and written P: dP may take the region, P^T G may read P.
                 alive = mbar_wait(bar(P_DONE), ph, abort_flag, args.status);
                 if (!alive) break;
@@ -474,6 +491,10 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
                 alive = mbar_wait(bar(DS_DONE), ph, abort_flag, args.status);
                 if (!alive) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                // The row threads have read dP as well: the next queries' S goes ahead of this pair's dK and
+                // dQ, which then run under its softmax.
+                if (i + 1 < query_tiles) alive = scores(pair + 1);
+                if (!alive) break;
                 if (lane == 0) {
                     // dK_j += dS^T Q_i, and dQ_i += dS K_j: k = the 128 keys, 16 per MMA (32 bytes of
                     // a dS row, 16 rows of the K tile).
@@ -506,12 +527,11 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
         // max and sum, and D = sum_c O g over the head's columns.
         {
             const uint32_t row = chunk * TILE + t;
-            float best = 0.0f, inverse = 0.0f, dot = 0.0f;
+            float shift = INFINITY, dot = 0.0f;  // +inf: a row past the end, or of masked keys alone: its probabilities are zeros
             if (row < args.q_len) {
                 const uint64_t global_row = static_cast<uint64_t>(seq) * args.q_len + row;
                 const float* st = args.stats + (global_row * args.heads + head) * 2;
-                best = st[0];
-                inverse = st[1] > 0.0f ? 1.0f / st[1] : 0.0f;
+                if (st[1] > 0.0f) shift = fmaf(st[0], 1.4426950408889634f, log2f(st[1]));
                 const bf16* o = static_cast<const bf16*>(args.o) + global_row * args.h + head * args.d;
                 const bf16* g = static_cast<const bf16*>(args.g) + global_row * args.h + head * args.d;
                 for (uint32_t c = 0; c + 8 <= args.d; c += 8) {
@@ -520,8 +540,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
                     dot = fmaf(a.hi.x, b.hi.x, dot); dot = fmaf(a.hi.y, b.hi.y, dot); dot = fmaf(a.hi.z, b.hi.z, dot); dot = fmaf(a.hi.w, b.hi.w, dot);
                 }
             }
-            row_best[row] = best;
-            row_inverse[row] = inverse;  // 0 for a row past the end: its probabilities are zeros
+            row_shift[row] = shift;
             row_dot[row] = dot;
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(STATS_MET));
@@ -534,7 +553,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
             for (uint32_t i = 0; i < query_tiles; ++i, ++pair) {
                 const uint32_t ph = pair & 1u;
                 const uint32_t row = i * TILE + t;
-                const float best = row_best[row], inverse = row_inverse[row], dot = row_dot[row];
+                const float shift = row_shift[row], dot = row_dot[row];
                 alive = mbar_wait(bar(S_FULL), ph, abort_flag, args.status);
                 // The P tile is free once the P^T G of the previous pair has been read by the tensor core.
                 if (alive) alive = mbar_wait(bar(P_FREE), ph ^ 1u, abort_flag, args.status);
@@ -544,9 +563,10 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
                 uint32_t r[32];
                 tmem_load32(tmem_sp + lane_base + chunk * 32, r);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+                hide_masked(r, counts);
                 float p[32];
 #pragma unroll
-                for (int c = 0; c < 32; ++c) p[c] = ((counts >> c) & 1u) ? __expf(__uint_as_float(r[c]) * args.scale - best) * inverse : 0.0f;
+                for (int c = 0; c < 32; ++c) p[c] = exp2_fast(fmaf(__uint_as_float(r[c]), args.scale_log2, -shift));
                 store_chunk_bf16(p_tile, t, chunk, p);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -560,7 +580,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
                 tmem_load32(tmem_sp + lane_base + chunk * 32, r);
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-                for (int c = 0; c < 32; ++c) p[c] = p[c] * (__uint_as_float(r[c]) - dot) * args.scale;  // dS
+                for (int c = 0; c < 32; ++c) p[c] = p[c] * (__uint_as_float(r[c]) - dot);  // dS, its scale left to dK and dQ
                 store_chunk_bf16(ds_tile, t, chunk, p);
                 asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                 asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -582,7 +602,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 float v[16];
 #pragma unroll
-                for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(raw[c]);
+                for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(raw[c]) * (which == 0 ? 1.0f : args.scale);
                 void* to = which == 0 ? args.dv : args.dk;
                 if (to != nullptr && key < args.k_len) store_part_bf16(to, key_at, v, chunk * 16, args.d);
             }
@@ -602,7 +622,7 @@ attention_backward_kernel(const __grid_constant__ CUtensorMap map_q, const __gri
                 asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
                 float v[16];
 #pragma unroll
-                for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(raw[c]);
+                for (int c = 0; c < 16; ++c) v[c] = __uint_as_float(raw[c]) * args.scale;
                 const uint32_t row = i * TILE + t;
                 if (row < args.q_len) store_part_bf16(args.dq, (static_cast<uint64_t>(seq) * args.q_len + row) * args.h + head * args.d, v, chunk * 16, args.d);
             }
@@ -631,6 +651,7 @@ FusedArgs fused_args(const float* mask, AttentionShape sh, uint32_t* status) {
     a.d = sh.head_dim;
     a.h = sh.heads * sh.head_dim;
     a.scale = 1.0f / sqrtf(static_cast<float>(sh.head_dim));
+    a.scale_log2 = a.scale * 1.4426950408889634f;
     return a;
 }
 
