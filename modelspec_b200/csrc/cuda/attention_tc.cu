@@ -1,5 +1,6 @@
 // Attention and its gradients on the tensor cores: each contraction is one batched tcgen05
-// matmul over every (sequence, head) (gemm_tc.cu, 3xTF32), with two row kernels between them.
+// matmul over every (sequence, head) (gemm_tf32.cu, or gemm_tc.cu for widths off 16 bytes; 3xTF32), with two
+// row kernels between them.
 //
 //   forward   S = Q_h K_h^T            -> P = masked softmax(S / sqrt(d))   -> O_h = P V_h
 //   backward  P as the forward left it (or computed again as above);  dP = G_h V_h^T;  dS = scale P (dP - rowsum(P dP));
@@ -19,25 +20,35 @@ namespace k {
 
 namespace {
 
-// One warp per score row, the row in registers (key lane + 32 i is item i of a lane; ITEMS x 32 keys or
-// fewer): a score is read once and a probability written once, with every load of a row in flight together.
+// One warp per score row, the row in registers (ITEMS x 32 keys or fewer): a score is read once and a
+// probability written once, with every load of a row in flight together. Rows on 16 bytes (V = 4) are read
+// and written four keys a lane.
 constexpr uint32_t ROW_BLOCK_WARPS = 8;
 
 // p = softmax over the unmasked keys of acc * scale, in place.
-template <int ITEMS>
+template <int ITEMS, int V>
 __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(float* __restrict__ scores, const float* __restrict__ mask, uint32_t rows,
                                                                               uint32_t rows_per_sequence, uint32_t s, float scale) {
     const uint32_t row = blockIdx.x * ROW_BLOCK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
     float* p = scores + static_cast<uint64_t>(row) * s;
     const float* m = mask + static_cast<uint64_t>(row / rows_per_sequence) * s;
+    auto key_of = [lane](int i) { return static_cast<uint32_t>(i / V * 32 * V + i % V) + lane * V; };  // of item i
     float x[ITEMS];
     uint32_t counts = 0;
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i) {
-        const uint32_t j = min(lane + 32 * i, s - 1);
-        x[i] = p[j];
-        counts |= (lane + 32 * i < s && __ldg(m + j) != 0.0f ? 1u : 0u) << i;
+    for (int i = 0; i < ITEMS; i += V) {
+        const uint32_t j = min(key_of(i), s - V);
+        float4 mask4;
+        if constexpr (V == 4) {
+            const float4 x4 = *reinterpret_cast<const float4*>(p + j);
+            x[i] = x4.x; x[i + 1] = x4.y; x[i + 2] = x4.z; x[i + 3] = x4.w;
+            mask4 = make_float4(__ldg(m + j), __ldg(m + j + 1), __ldg(m + j + 2), __ldg(m + j + 3));
+            if (key_of(i) < s) counts |= ((mask4.x != 0.0f ? 1u : 0u) | (mask4.y != 0.0f ? 2u : 0u) | (mask4.z != 0.0f ? 4u : 0u) | (mask4.w != 0.0f ? 8u : 0u)) << i;
+        } else {
+            x[i] = p[j];
+            counts |= (key_of(i) < s && __ldg(m + j) != 0.0f ? 1u : 0u) << i;
+        }
     }
     float best = -INFINITY;
 #pragma unroll
@@ -51,9 +62,19 @@ __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(fl
         total += x[i];
     }
     total = warp_sum(total);
+    // x / total: the product with the reciprocal, corrected by its own remainder.
+    const float inverse = 1.0f / total;
 #pragma unroll
-    for (int i = 0; i < ITEMS; ++i)
-        if (lane + 32 * i < s) p[lane + 32 * i] = x[i] / total;
+    for (int i = 0; i < ITEMS; ++i) {
+        const float first = x[i] * inverse;
+        x[i] = fmaf(fmaf(-first, total, x[i]), inverse, first);
+    }
+#pragma unroll
+    for (int i = 0; i < ITEMS; i += V) {
+        if (key_of(i) >= s) continue;
+        if constexpr (V == 4) *reinterpret_cast<float4*>(p + key_of(i)) = make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]);
+        else p[key_of(i)] = x[i];
+    }
 }
 
 // dS = scale * P * (dP - sum_j P dP), written over dP.
@@ -81,16 +102,6 @@ __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) score_grad_kernel(const 
         if (lane + 32 * i < s) dr[lane + 32 * i] = x[i] * (d[i] - dot) * scale;
 }
 
-// The kernel of the narrowest row that holds `s` keys (at most 512).
-#define MSX_FOR_KEYS(kernel, s, ...)                          \
-    do {                                                      \
-        const dim3 grid((rows + ROW_BLOCK_WARPS - 1) / ROW_BLOCK_WARPS), block(32 * ROW_BLOCK_WARPS); \
-        if ((s) <= 64) kernel<2><<<grid, block, 0, stream>>>(__VA_ARGS__);        \
-        else if ((s) <= 128) kernel<4><<<grid, block, 0, stream>>>(__VA_ARGS__);  \
-        else if ((s) <= 256) kernel<8><<<grid, block, 0, stream>>>(__VA_ARGS__);  \
-        else kernel<16><<<grid, block, 0, stream>>>(__VA_ARGS__);                 \
-    } while (0)
-
 struct Heads {
     uint32_t b, l, s, a, d, h;
     float scale;
@@ -112,12 +123,23 @@ BatchedOperand transposed(BatchedOperand o) {
     return o;
 }
 
+void product(cudaStream_t s, const BatchedProduct& one, uint64_t m, uint64_t n, uint64_t k, const Heads& hd, uint32_t* status) {
+    matmul_tc_batched(s, &one, 1, m, n, k, hd.b, hd.a, status);
+}
+
 void probabilities(cudaStream_t s, const float* q, const float* k, const float* mask, float* p, const Heads& hd, uint32_t* status) {
     // S[i, j] = sum_c q[i, c] k[j, c]: B is the keys stored [n, k].
-    matmul_tc_batched(s, hd.q(q), transposed(hd.kv(k)), hd.scores(p), hd.l, hd.s, hd.d, hd.b, hd.a, status);
+    product(s, {hd.q(q), transposed(hd.kv(k)), hd.scores(p)}, hd.l, hd.s, hd.d, hd, status);
     uint32_t rows = hd.rows();
-    const cudaStream_t stream = s;
-    MSX_FOR_KEYS(masked_softmax_kernel, hd.s, p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
+    const bool wide = hd.s % 4 == 0 && reinterpret_cast<uintptr_t>(p) % 16 == 0;
+    const dim3 grid((rows + ROW_BLOCK_WARPS - 1) / ROW_BLOCK_WARPS), block(32 * ROW_BLOCK_WARPS);
+    if (wide && hd.s <= 128) masked_softmax_kernel<4, 4><<<grid, block, 0, s>>>(p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
+    else if (wide && hd.s <= 256) masked_softmax_kernel<8, 4><<<grid, block, 0, s>>>(p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
+    else if (wide) masked_softmax_kernel<16, 4><<<grid, block, 0, s>>>(p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
+    else if (hd.s <= 64) masked_softmax_kernel<2, 1><<<grid, block, 0, s>>>(p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
+    else if (hd.s <= 128) masked_softmax_kernel<4, 1><<<grid, block, 0, s>>>(p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
+    else if (hd.s <= 256) masked_softmax_kernel<8, 1><<<grid, block, 0, s>>>(p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
+    else masked_softmax_kernel<16, 1><<<grid, block, 0, s>>>(p, mask, rows, hd.a * hd.l, hd.s, hd.scale);
     check_launch("attention masked_softmax");
 }
 
@@ -133,7 +155,7 @@ void attention_tc_forward(cudaStream_t s, const float* q, const float* k, const 
     Heads hd = heads_of(sh);
     probabilities(s, q, k, mask, p, hd, status);
     // O[i, c] = sum_j P[i, j] v[j, c]
-    matmul_tc_batched(s, hd.scores(p), hd.kv(v), hd.q(out), hd.l, hd.d, hd.s, hd.b, hd.a, status);
+    product(s, {hd.scores(p), hd.kv(v), hd.q(out)}, hd.l, hd.d, hd.s, hd, status);
 }
 
 void attention_tc_backward(cudaStream_t s, const float* q, const float* k, const float* v, const float* mask, const float* g,
@@ -141,18 +163,31 @@ void attention_tc_backward(cudaStream_t s, const float* q, const float* k, const
     if (sh.batch == 0 || sh.q_len == 0) return;
     Heads hd = heads_of(sh);
     if (!p_ready) probabilities(s, q, k, mask, p, hd, status);
-    // dV[j, c] = sum_i P[i, j] g[i, c]: A is P stored [k, m].
-    if (dv) matmul_tc_batched(s, transposed(hd.scores(p)), hd.q(g), hd.kv(dv), hd.s, hd.d, hd.l, hd.b, hd.a, status);
-    if (!dq && !dk) return;
+    // dV[j, c] = sum_i P[i, j] g[i, c] and dK[j, c] = sum_i dS[i, j] q[i, c], one launch: A is P or dS
+    // stored [k, m].
+    auto key_gradients = [&] {
+        BatchedProduct both[2];
+        uint32_t count = 0;
+        if (dv) both[count++] = {transposed(hd.scores(p)), hd.q(g), hd.kv(dv)};
+        if (dk) both[count++] = {transposed(hd.scores(dp)), hd.q(q), hd.kv(dk)};
+        if (count) matmul_tc_batched(s, both, count, hd.s, hd.d, hd.l, hd.b, hd.a, status);
+    };
+    if (!dq && !dk) {
+        key_gradients();
+        return;
+    }
     // dP[i, j] = sum_c g[i, c] v[j, c]
-    matmul_tc_batched(s, hd.q(g), transposed(hd.kv(v)), hd.scores(dp), hd.l, hd.s, hd.d, hd.b, hd.a, status);
+    product(s, {hd.q(g), transposed(hd.kv(v)), hd.scores(dp)}, hd.l, hd.s, hd.d, hd, status);
     uint32_t rows = hd.rows();
-    const cudaStream_t stream = s;
-    MSX_FOR_KEYS(score_grad_kernel, hd.s, p, dp, rows, hd.s, hd.scale);
+    const dim3 grid((rows + ROW_BLOCK_WARPS - 1) / ROW_BLOCK_WARPS), block(32 * ROW_BLOCK_WARPS);
+    if (hd.s <= 64) score_grad_kernel<2><<<grid, block, 0, s>>>(p, dp, rows, hd.s, hd.scale);
+    else if (hd.s <= 128) score_grad_kernel<4><<<grid, block, 0, s>>>(p, dp, rows, hd.s, hd.scale);
+    else if (hd.s <= 256) score_grad_kernel<8><<<grid, block, 0, s>>>(p, dp, rows, hd.s, hd.scale);
+    else score_grad_kernel<16><<<grid, block, 0, s>>>(p, dp, rows, hd.s, hd.scale);
     check_launch("attention score_grad");
-    // dQ[i, c] = sum_j dS[i, j] k[j, c];  dK[j, c] = sum_i dS[i, j] q[i, c]
-    if (dq) matmul_tc_batched(s, hd.scores(dp), hd.kv(k), hd.q(dq), hd.l, hd.d, hd.s, hd.b, hd.a, status);
-    if (dk) matmul_tc_batched(s, transposed(hd.scores(dp)), hd.q(q), hd.kv(dk), hd.s, hd.d, hd.l, hd.b, hd.a, status);
+    key_gradients();
+    // dQ[i, c] = sum_j dS[i, j] k[j, c]
+    if (dq) product(s, {hd.scores(dp), hd.kv(k), hd.q(dq)}, hd.l, hd.d, hd.s, hd, status);
 }
 
 // ---- mixed precision ----------------------------------------------------------------------------

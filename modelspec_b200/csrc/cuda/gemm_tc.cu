@@ -567,9 +567,9 @@ bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 //   * small tiles on the FMA units while the product fits a few of them per SM;
 //   * operands TMA can address: 128-row tiles 32, 64 or 128 wide (the narrow ones when the wide ones would
 //     leave SMs idle), or pairs of CTAs on 256 x 256 tiles once there are enough of those;
-//   * the rest, and batched products, the 64-row tiles of this file.
+//   * the rest, and empty products, the 64-row tiles of this file.
 // A split k adds the reduce launch and its partial tiles.
-MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems, uint64_t group, bool tma_ok, uint64_t chain) {
+MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems, uint64_t group, bool tma_ok, uint64_t chain, bool batched) {
     enum Kernel { Fma, Tma, Rows64 };
     struct Candidate {
         Kernel kernel;
@@ -593,8 +593,7 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
     MatmulTcPlan best = {};
     double best_cost = 0.0;
     for (const Candidate& c : candidates) {
-        const bool single = problems == 1 && kblocks > 0;  // batched and empty products stay on the 64-row tiles
-        if (c.kernel == Fma ? !single || chain > 1 : (c.kernel == Tma) != (single && tma_ok)) continue;
+        if (c.kernel == Fma ? batched || kblocks == 0 || chain > 1 : (c.kernel == Tma) != (kblocks > 0 && tma_ok)) continue;
         const uint64_t m_tiles = (m + c.bm - 1) / c.bm, n_tiles = (n + c.bn - 1) / c.bn, tiles = m_tiles * n_tiles * problems * group;
         auto consider = [&](double cost, uint64_t splits, uint64_t per, uint32_t cluster) {
             if (best.bn != 0 && cost >= best_cost) return;
@@ -612,7 +611,7 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
             consider(chain > streamed ? chain : streamed, 1, kblocks, cluster);
             continue;
         }
-        const uint64_t most = problems > 1 || chain > 1 ? 1 : (kblocks / 2 > 0 ? kblocks / 2 : 1);
+        const uint64_t most = batched || chain > 1 ? 1 : (kblocks / 2 > 0 ? kblocks / 2 : 1);
         for (uint64_t splits = 1; splits <= most && splits <= 64; ++splits) {
             const uint64_t per = (kblocks + splits - 1) / splits;
             const uint64_t used = kblocks == 0 ? 1 : (kblocks + per - 1) / per;
@@ -760,9 +759,10 @@ void matmul_tc_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, bool 
     launch_tile(s, args, dim3(blocks), 64, a_t, b_t);
 }
 
-void matmul_tc_batched(cudaStream_t s, const BatchedOperand& a, const BatchedOperand& b, const BatchedOperand& c, uint64_t m,
-                       uint64_t n, uint64_t k, uint32_t outer, uint32_t inner, uint32_t* status) {
-    if (m == 0 || n == 0 || outer == 0 || inner == 0) return;
+namespace {
+// One batched product on the 64-row tiles: operands that TMA cannot address.
+void launch_batched(cudaStream_t s, const BatchedOperand& a, const BatchedOperand& b, const BatchedOperand& c, uint64_t m, uint64_t n, uint64_t k,
+                    uint32_t outer, uint32_t inner, uint32_t* status) {
     TcArgs args = {};
     args.a[0] = a.base;
     args.b[0] = b.base;
@@ -785,9 +785,16 @@ void matmul_tc_batched(cudaStream_t s, const BatchedOperand& a, const BatchedOpe
     args.b_outer = b.stride_outer; args.b_inner = b.stride_inner;
     args.c_outer = c.stride_outer; args.c_inner = c.stride_inner;
     args.status = status;
-    const MatmulTcPlan p = matmul_tc_plan(m, n, k, static_cast<uint64_t>(outer) * inner);
+    const MatmulTcPlan p = matmul_tc_plan(m, n, k, static_cast<uint64_t>(outer) * inner, 1, false, 1, true);
     dim3 grid(static_cast<uint32_t>((n + p.bn - 1) / p.bn), static_cast<uint32_t>((m + p.bm - 1) / p.bm), outer * inner);
     launch_tile(s, args, grid, p.bn, a.transposed, b.transposed);
+}
+}  // namespace
+
+void matmul_tc_batched(cudaStream_t s, const BatchedProduct* products, uint32_t count, uint64_t m, uint64_t n, uint64_t k, uint32_t outer, uint32_t inner,
+                       uint32_t* status) {
+    if (m == 0 || n == 0 || outer == 0 || inner == 0 || matmul_tf32_batched(s, products, count, m, n, k, outer, inner, status)) return;
+    for (uint32_t g = 0; g < count; ++g) launch_batched(s, products[g].a, products[g].b, products[g].c, m, n, k, outer, inner, status);
 }
 
 }  // namespace k

@@ -83,6 +83,7 @@ struct Args {
     tc::Divisor splits;
     uint32_t kblocks = 0;                       // of one product
     uint32_t chain = 1;                         // > 1: that many products are summed into one result
+    tc::Divisor batch{1}, batch_inner{1};       // matrices of each product, (outer, inner) of them (k unsplit)
     uint32_t c_tma = 1, c_vec = 1, c_padded = 0;  // C by TMA stores; else 16-byte stores; padding between n and ldc may be overwritten
     float* c[MAX_PRODUCTS] = {};                // C, or the split-k workspace [splits][m][n]
     const float* bias[MAX_PRODUCTS] = {};       // null for none
@@ -100,9 +101,9 @@ struct JobMaps {
     CUtensorMap a[MAX_JOBS], b[MAX_JOBS], c[MAX_JOBS];
 };
 
-// Unit `u` of a launch: its tile, then the split, and the product or job.
+// Unit `u` of a launch: its tile, then the split, the matrix of a batch, and the product or job.
 struct Unit {
-    uint32_t m0, n0, split, splits, product, kblocks;
+    uint32_t m0, n0, split, splits, product, kblocks, z_inner, z_outer;
     uint32_t m, n, ldc;
     float* c;
     const float* bias;
@@ -111,8 +112,12 @@ __device__ __forceinline__ Unit unit_of(const Args& args, uint32_t u) {
     Unit w;
     w.m = args.m; w.n = args.n; w.ldc = args.ldc; w.splits = args.splits.d;
     u = args.walk.take(u, &w.m0, &w.n0);
-    w.product = args.splits.quotient(u);
-    w.split = u - w.product * args.splits.d;
+    const uint32_t after_split = args.splits.quotient(u);
+    w.split = u - after_split * args.splits.d;
+    w.product = args.batch.quotient(after_split);
+    const uint32_t z = after_split - w.product * args.batch.d;
+    w.z_outer = args.batch_inner.quotient(z);
+    w.z_inner = z - w.z_outer * args.batch_inner.d;
     w.c = args.c[w.product];
     w.bias = args.bias[w.product];
     w.kblocks = args.chain > 1 ? args.kblocks * args.chain : args.splits.quotient(args.kblocks - w.split + w.splits - 1);
@@ -126,6 +131,7 @@ __device__ __forceinline__ Unit unit_of(const JobArgs& args, uint32_t u) {
     w.m = job.m; w.n = w.ldc = job.n; w.splits = job.splits.d;
     w.split = job.walk.take(u - job.first_unit, &w.m0, &w.n0);
     w.product = j;
+    w.z_inner = w.z_outer = 0;
     w.c = job.c;
     w.bias = nullptr;
     w.kblocks = job.splits.quotient(job.kblocks - w.split + w.splits - 1);
@@ -144,20 +150,9 @@ template <int CG, int REUSE> __device__ __forceinline__ void mma_tf32(uint32_t t
     else MSX_MMA("2", "");
 #undef MSX_MMA
 }
-// Tiles of a (column, row[, split]) tensor map.
-__device__ __forceinline__ void load(uint32_t dst, const CUtensorMap* map, uint32_t bar, uint32_t x, uint32_t row) {
-    asm volatile("cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-                 ::"r"(dst), "l"(map), "r"(bar), "r"(x), "r"(row) : "memory");
-}
-__device__ __forceinline__ void store(const CUtensorMap* map, uint32_t src, uint32_t x, uint32_t row, uint32_t split) {
-    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-                 ::"l"(map), "r"(src), "r"(x), "r"(row), "r"(split) : "memory");
-    asm volatile("cp.async.bulk.commit_group;" ::: "memory");
-}
-
-__device__ __forceinline__ void store_add(const CUtensorMap* map, uint32_t src, uint32_t x, uint32_t row, uint32_t split) {
-    asm volatile("cp.reduce.async.bulk.tensor.3d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4}], [%1];"
-                 ::"l"(map), "r"(src), "r"(x), "r"(row), "r"(split) : "memory");
+__device__ __forceinline__ void store_add(const CUtensorMap* map, uint32_t src, uint32_t x, uint32_t row, uint32_t inner, uint32_t outer) {
+    asm volatile("cp.reduce.async.bulk.tensor.4d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3, %4, %5}], [%1];"
+                 ::"l"(map), "r"(src), "r"(x), "r"(row), "r"(inner), "r"(outer) : "memory");
     asm volatile("cp.async.bulk.commit_group;" ::: "memory");
 }
 
@@ -316,18 +311,19 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
                     const uint32_t bar = tc::smem_u32(&raw_full[stage]);
                     const uint32_t to_a = tc::smem_u32(smem + stage * T::STAGE_BYTES), to_b = to_a + 2 * T::A_BYTES;
                     const uint32_t k0 = k_at * BK;
+                    auto load = [&](uint32_t to, const CUtensorMap* map, uint32_t x, uint32_t row) { tc::load_tile<1>(to, map, bar, x, row, w.z_inner, w.z_outer); };
                     tc::mbar_expect_tx(bar, T::RAW_BYTES);
                     if (A_T) {  // stored [k, m]: four boxes of 32 m by 32 k
 #pragma unroll
-                        for (uint32_t p = 0; p < 4; ++p) load(to_a + p * 4096u, &maps.a[product], bar, m0 + 32u * p, k0);
+                        for (uint32_t p = 0; p < 4; ++p) load(to_a + p * 4096u, &maps.a[product], m0 + 32u * p, k0);
                     } else {    // stored [m, k]: one box of 32 k by 128 m
-                        load(to_a, &maps.a[product], bar, k0, m0);
+                        load(to_a, &maps.a[product], k0, m0);
                     }
                     if (B_T) {  // stored [n, k]
-                        load(to_b, &maps.b[product], bar, k0, n0);
+                        load(to_b, &maps.b[product], k0, n0);
                     } else {    // stored [k, n]
 #pragma unroll
-                        for (uint32_t p = 0; p < T::BN_CTA / 32; ++p) load(to_b + p * 4096u, &maps.b[product], bar, n0 + 32u * p, k0);
+                        for (uint32_t p = 0; p < T::BN_CTA / 32; ++p) load(to_b + p * 4096u, &maps.b[product], n0 + 32u * p, k0);
                     }
                 }
                 if (++stage == STAGES) { stage = 0; parity ^= 1u; }
@@ -427,8 +423,9 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
                     if (lane == 0 && first_row < w.m) {
-                        if (segment == 0) store(&maps.c[w.product], tc::smem_u32(slab), gn0, first_row, w.split);
-                        else store_add(&maps.c[w.product], tc::smem_u32(slab), gn0, first_row, w.split);
+                        const uint32_t inner = w.splits > 1 ? w.split : w.z_inner;
+                        if (segment == 0) tc::store_tile(&maps.c[w.product], tc::smem_u32(slab), gn0, first_row, inner, w.z_outer);
+                        else store_add(&maps.c[w.product], tc::smem_u32(slab), gn0, first_row, inner, w.z_outer);
                     }
                     continue;
                 }
@@ -507,26 +504,43 @@ template <int CG, int BN, class A, class M> void launch_form(cudaStream_t s, boo
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
 
-// A matrix of `rows` rows of `cols` floats, `pitch` apart, as a tensor map of boxes of 32 floats by
-// `box_rows` rows; `splits` > 0: that many dense ones behind one another (a third coordinate).
-CUtensorMap encode(const float* base, uint64_t cols, uint64_t rows, uint64_t pitch, uint32_t splits, uint32_t box_rows, bool chunks_of_32) {
-    const cuuint64_t size[3] = {cols, rows, splits ? splits : 1}, stride[2] = {pitch * 4, pitch * rows * 4};
-    const cuuint32_t box[3] = {32, box_rows, 1}, element[3] = {1, 1, 1};
+// Where the matrices of a batch lie: `inner` of them stride_inner apart, `outer` such rows stride_outer apart.
+struct Batch {
+    uint64_t inner, stride_inner, outer, stride_outer;
+};
+// A matrix of `rows` rows of `cols` floats, `pitch` apart, or a batch of them as two more coordinates,
+// as a tensor map of boxes of 32 floats by `box_rows` rows.
+CUtensorMap encode(const float* base, uint64_t cols, uint64_t rows, uint64_t pitch, const Batch& z, uint32_t box_rows, bool chunks_of_32) {
+    // A dimension of one element may carry any stride.
+    const uint64_t whole = pitch * rows;
+    const cuuint64_t size[4] = {cols, rows, z.inner, z.outer};
+    const cuuint64_t stride[3] = {pitch * 4, (z.inner > 1 ? z.stride_inner : whole) * 4, (z.outer > 1 ? z.stride_outer : whole) * 4};
+    const cuuint32_t box[4] = {32, box_rows, 1, 1}, element[4] = {1, 1, 1, 1};
     CUtensorMap map;
-    const CUresult r = tc::encode_tiled()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, splits ? 3 : 2, const_cast<float*>(base), size, stride, box, element,
+    const CUresult r = tc::encode_tiled()(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT32, 4, const_cast<float*>(base), size, stride, box, element,
                                           CU_TENSOR_MAP_INTERLEAVE_NONE, chunks_of_32 ? CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B : CU_TENSOR_MAP_SWIZZLE_128B,
                                           CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) throw std::invalid_argument("matmul_tf32: cuTensorMapEncodeTiled refused a matrix (" + std::to_string(static_cast<int>(r)) + ")");
     return map;
 }
+constexpr Batch ONE = {1, 0, 1, 0};
+Batch splits_of(uint64_t splits, uint64_t m, uint64_t n) { return {splits, m * n, 1, 0}; }  // the split-k workspace
 // The tensor maps of one product's operands: boxes of 32 floats by the CTA's rows for an operand stored
 // with k along its rows, 32 by 32 in the swizzle of 32-byte chunks for one with k down its columns.
 template <class M> void encode_operands(M& maps, uint32_t at, const float* a, uint32_t lda, const float* b, uint32_t ldb, bool a_t, bool b_t, uint64_t m, uint64_t n,
-                                        uint64_t k, uint32_t b_rows) {
-    maps.a[at] = a_t ? encode(a, m, k, lda, 0, 32, true) : encode(a, k, m, lda, 0, 128, false);
-    maps.b[at] = b_t ? encode(b, k, n, ldb, 0, b_rows, false) : encode(b, n, k, ldb, 0, 32, true);
+                                        uint64_t k, uint32_t b_rows, const Batch& of_a = ONE, const Batch& of_b = ONE) {
+    maps.a[at] = a_t ? encode(a, m, k, lda, of_a, 32, true) : encode(a, k, m, lda, of_a, 128, false);
+    maps.b[at] = b_t ? encode(b, k, n, ldb, of_b, b_rows, false) : encode(b, n, k, ldb, of_b, 32, true);
 }
 bool tma_addressable(const float* base, uint64_t pitch) { return aligned16(base) && pitch % 4 == 0; }
+bool tma_addressable(const BatchedOperand& x) { return tma_addressable(x.base, x.pitch) && x.stride_outer % 4 == 0 && x.stride_inner % 4 == 0; }
+
+void launch_plan(cudaStream_t s, const MatmulTcPlan& p, bool a_t, bool b_t, const Args& args, const Maps& maps) {
+    if (p.bm == 256) launch_form<2, 256>(s, a_t, b_t, args, maps);
+    else if (p.bn == 128) launch_form<1, 128>(s, a_t, b_t, args, maps);
+    else if (p.bn == 64) launch_form<1, 64>(s, a_t, b_t, args, maps);
+    else launch_form<1, 32>(s, a_t, b_t, args, maps);
+}
 
 }  // namespace
 
@@ -556,12 +570,46 @@ void matmul_tf32(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* pr
         args.c_vec = args.c_vec && aligned16(args.c[g]);
         args.c_tma = args.c_tma && tma_addressable(args.c[g], args.ldc);
     }
-    for (uint32_t g = 0; g < results && args.c_tma; ++g) maps.c[g] = encode(args.c[g], n, m, args.ldc, p.splits, 32, false);
+    for (uint32_t g = 0; g < results && args.c_tma; ++g) maps.c[g] = encode(args.c[g], n, m, args.ldc, splits_of(p.splits, m, n), 32, false);
     args.units = args.walk.count() * p.splits * results;
-    if (p.bm == 256) launch_form<2, 256>(s, a_t, b_t, args, maps);
-    else if (p.bn == 128) launch_form<1, 128>(s, a_t, b_t, args, maps);
-    else if (p.bn == 64) launch_form<1, 64>(s, a_t, b_t, args, maps);
-    else launch_form<1, 32>(s, a_t, b_t, args, maps);
+    launch_plan(s, p, a_t, b_t, args, maps);
+}
+
+bool matmul_tf32_batched(cudaStream_t s, const BatchedProduct* products, uint32_t count, uint64_t m, uint64_t n, uint64_t k, uint32_t outer, uint32_t inner,
+                         uint32_t* status) {
+    if (k == 0) return false;
+    for (uint32_t g = 0; g < count; ++g)
+        for (const BatchedOperand* x : {&products[g].a, &products[g].b, &products[g].c})
+            if (!tma_addressable(*x)) return false;
+    const uint64_t problems = static_cast<uint64_t>(outer) * inner;
+    // One product whose 64 x 32 tiles all find an SM of their own is 0.7 us sooner on those (16 heads of 128
+    // queries x 128 keys x 64: attention forward 12.9 -> 11.5 us); from two tiles to an SM on, or with two products
+    // to share a launch, these tiles win (64 such heads: forward 16.3 -> 14.9 us, backward 29.9 -> 21.0;
+    // 384 heads of 512 x 512 x 64: forward 745 -> 414 us, backward 1,151 -> 643).
+    if (count == 1 && (m + 63) / 64 * ((n + 31) / 32) * problems <= device_sm_count()) return false;
+    const MatmulTcPlan p = matmul_tc_plan(m, n, k, problems, count, true, 1, true);
+    Args args;
+    Maps maps = {};
+    args.m = static_cast<uint32_t>(m);
+    args.n = static_cast<uint32_t>(n);
+    args.ldc = products[0].c.pitch;
+    args.splits = tc::Divisor(1);
+    args.batch = tc::Divisor(static_cast<uint32_t>(problems));
+    args.batch_inner = tc::Divisor(inner);
+    args.walk = tc::TileWalk(m, n, p.bm, p.bn);
+    args.kblocks = static_cast<uint32_t>((k + BK - 1) / BK);
+    args.status = status;
+    const bool a_t = products[0].a.transposed, b_t = products[0].b.transposed;
+    for (uint32_t g = 0; g < count; ++g) {
+        const BatchedProduct& q = products[g];
+        auto batch = [&](const BatchedOperand& x) { return Batch{inner, x.stride_inner, outer, x.stride_outer}; };
+        encode_operands(maps, g, q.a.base, q.a.pitch, q.b.base, q.b.pitch, a_t, b_t, m, n, k, p.bn / (p.bm / 128), batch(q.a), batch(q.b));
+        maps.c[g] = encode(q.c.base, n, m, q.c.pitch, batch(q.c), 32, false);
+        args.c[g] = const_cast<float*>(q.c.base);
+    }
+    args.units = static_cast<uint32_t>(args.walk.count() * problems * count);
+    launch_plan(s, p, a_t, b_t, args, maps);
+    return true;
 }
 
 bool matmul_tf32_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, bool a_t, bool b_t, uint32_t* status) {
@@ -585,7 +633,7 @@ bool matmul_tf32_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, boo
         to.first_unit = args.units;
         args.units += to.walk.count() * p.splits;
         encode_operands(maps, j, job.a, lda, job.b, ldb, a_t, b_t, job.m, job.n, job.k, 128);
-        maps.c[j] = encode(c, job.n, job.m, job.n, p.splits, 32, false);
+        maps.c[j] = encode(c, job.n, job.m, job.n, splits_of(p.splits, job.m, job.n), 32, false);
     }
     launch_form<1, 128>(s, a_t, b_t, args, maps);
     return true;

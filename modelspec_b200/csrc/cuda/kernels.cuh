@@ -267,12 +267,12 @@ struct MatmulTcPlan {
     uint32_t cluster;                            // the k of a tile shared by that many CTAs
     uint64_t workspace_floats;
 };
-// `problems` > 1: that many independent batched products in one launch (k is then not split);
+// `batched`: for matmul_tc_batched, `problems` independent matrices of each product (k is then not split);
 // `group` > 1: that many products of this shape in one launch of matmul_tc_group (the workspace
 // size is per product).
 // `tma_ok`: the operands can be TMA sources (bases on 16 bytes, row pitches multiples of 4 floats).
 // `chain` > 1: for matmul_tf32, which sums that many products (their k unsplit).
-MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems = 1, uint64_t group = 1, bool tma_ok = true, uint64_t chain = 1);
+MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problems = 1, uint64_t group = 1, bool tma_ok = true, uint64_t chain = 1, bool batched = false);
 void matmul_tc(cudaStream_t s, const float* a, bool a_t, const float* b, bool b_t, float* c, uint64_t m,
                uint64_t n, uint64_t k, float* workspace, uint32_t* status, const float* bias = nullptr,
                bool leave_partials = false);
@@ -331,8 +331,15 @@ struct BatchedOperand {
     uint64_t stride_outer, stride_inner;
     bool transposed;
 };
-void matmul_tc_batched(cudaStream_t s, const BatchedOperand& a, const BatchedOperand& b, const BatchedOperand& c,
-                       uint64_t m, uint64_t n, uint64_t k, uint32_t outer, uint32_t inner, uint32_t* status);
+struct BatchedProduct {
+    BatchedOperand a, b, c;
+};
+// Up to 4 such products of one shape and storage form, sharing a launch where TMA can address them.
+void matmul_tc_batched(cudaStream_t s, const BatchedProduct* products, uint32_t count, uint64_t m, uint64_t n, uint64_t k, uint32_t outer, uint32_t inner,
+                       uint32_t* status);
+// On the TMA-fed tiles (gemm_tf32.cu); false, and nothing launched, when TMA cannot address an operand.
+bool matmul_tf32_batched(cudaStream_t s, const BatchedProduct* products, uint32_t count, uint64_t m, uint64_t n, uint64_t k, uint32_t outer, uint32_t inner,
+                         uint32_t* status);
 
 // ---- matmul on bf16 operands (gemm_bf16.cu) ---------------------------------------------------
 // Mixed-precision plans: operands stored as bf16, products by tcgen05.mma kind::f16 fed by TMA,
