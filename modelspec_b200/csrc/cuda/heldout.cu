@@ -89,7 +89,7 @@ __global__ void __launch_bounds__(THREADS) heldout_rows_kernel(const float* __re
     __shared__ float row_total;
     __shared__ uint32_t last;
     __shared__ double staged[4 * THREADS];
-    __shared__ uint32_t warp_hits[THREADS / 32];
+    __shared__ uint32_t warp_hits[THREADS / 32], kept_of[4 * THREADS / 32];
 
     const uint32_t n = blockIdx.x;
     const float* row = logits + static_cast<uint64_t>(n) * pitch;
@@ -149,23 +149,42 @@ __global__ void __launch_bounds__(THREADS) heldout_rows_kernel(const float* __re
     __syncthreads();
     if (!last) return;
 
-    // The last block of the batch: the rows' terms in ascending row order onto the state.
+    // The last block of the batch: the rows' terms in ascending row order onto the state. A chain of f64
+    // additions takes 16 cycles a term, 35 us for 4,096 rows, so the +0 of a row that does not count (five
+    // rows in six of a masked-token batch) is left out: x + 0 is x, but for a sum of -0, which is seen to
+    // below. (4,096 x 30,522 with 15 % selected: 121 -> 106 us.)
     __threadfence();
     uint32_t counted = 0;
     double sum = state->numerator;
-    bool started = state->started != 0u;
+    bool started = state->started != 0u, left_out = false;
     for (uint32_t base = 0; base < rows; base += 4 * THREADS) {
-        const uint32_t here = min(static_cast<uint32_t>(4 * THREADS), rows - base);
-        for (uint32_t i = threadIdx.x; i < here; i += THREADS) {
-            staged[i] = __ldcg(terms + base + i);
-            counted += __ldcg(hits + base + i);
+        double mine[4];
+        uint32_t kept[4];
+#pragma unroll
+        for (uint32_t u = 0; u < 4; ++u) {
+            const uint32_t i = base + u * THREADS + threadIdx.x;
+            mine[u] = i < rows ? __ldcg(terms + i) : 0.0;
+            counted += i < rows ? __ldcg(hits + i) : 0u;
+            kept[u] = __ballot_sync(0xffffffffu, __double_as_longlong(mine[u]) != 0);
+            if (lane == 0) kept_of[u * (THREADS / 32) + warp] = __popc(kept[u]);
         }
+        __syncthreads();
+        uint32_t here = 0;
+#pragma unroll
+        for (uint32_t g = 0; g < 4 * THREADS / 32; ++g) {
+            if (g % (THREADS / 32) == warp) {
+                const uint32_t u = g / (THREADS / 32);
+                if ((kept[u] >> lane) & 1u) staged[here + __popc(kept[u] & ((1u << lane) - 1u))] = mine[u];
+            }
+            here += kept_of[g];
+        }
+        left_out = left_out || here < min(static_cast<uint32_t>(4 * THREADS), rows - base);
         __syncthreads();
         if (threadIdx.x == 0) {
             // The first term starts the sum; each later one is added (its product is exact, so
             // the host's fused multiply-add rounds to the same f64).
             uint32_t i = 0;
-            if (!started) {
+            if (!started && here > 0) {
                 sum = staged[0];
                 started = true;
                 i = 1;
@@ -187,8 +206,8 @@ __global__ void __launch_bounds__(THREADS) heldout_rows_kernel(const float* __re
     if (threadIdx.x == 0) {
         unsigned long long correct = 0;
         for (int w = 0; w < THREADS / 32; ++w) correct += warp_hits[w];
-        state->numerator = sum;
-        state->started = started ? 1u : 0u;
+        state->numerator = sum == 0.0 && left_out ? 0.0 : sum;
+        state->started = started || left_out ? 1u : 0u;
         state->correct += correct;
         state->arrived = 0u;  // the next batch counts its own rows
     }
