@@ -284,7 +284,9 @@ __global__ void __launch_bounds__(256) scatter_kernel(const TG* __restrict__ g, 
 // does; the other positions have nothing to do. A step names a few thousand of a vocabulary's
 // 30,522 rows, so this visits n positions where the row walk visits every row twice (two
 // searches); a hot row's run is long, so two hot rows never start within one block's eight
-// positions and the block-wide path below takes at most one of them.
+// positions and the block-wide path below takes at most one of them. The hot row's chain of additions
+// is what the launch waits for, so each group of columns has a block of its own (as a loop within the
+// block, 16,384 ids and 768 columns took 211 us; now 65).
 template <int VEC, class TG, class TO>
 __global__ void __launch_bounds__(256) scatter_in_place_kernel(const TG* __restrict__ g, const int32_t* __restrict__ sorted_id,
                                                                const int32_t* __restrict__ sorted_n, uint32_t n, TO* out, uint32_t rows,
@@ -293,9 +295,9 @@ __global__ void __launch_bounds__(256) scatter_in_place_kernel(const TG* __restr
     constexpr int LOADS = kHotChunk * span / VEC / 256;
     __shared__ float stage[kHotChunk][span];
     __shared__ uint32_t hot_row, hot_at, hot_count, hot_group;
-    const uint32_t groups = (h + span - 1) / span;
+    const uint32_t group = blockIdx.y;  // of `span` columns
     const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (uint32_t group = 0; group < groups; ++group) {
+    {
         if (threadIdx.x == 0) hot_count = 0;
         __syncthreads();
         const uint32_t p = blockIdx.x * 8 + warp, col = group * span + lane * VEC;
@@ -362,7 +364,7 @@ __global__ void __launch_bounds__(256) scatter_in_place_kernel(const TG* __restr
         // The block's hot row, if one starts here, by the whole block: 32 occurrences at a time
         // into shared memory, two chunks of loads in flight while a third is added in order.
         const uint32_t count = hot_count;
-        if (count == 0) continue;
+        if (count == 0) return;
         const uint32_t row = hot_row, at = hot_at, col0 = hot_group * span;
         float4 held4[2][VEC == 4 ? LOADS : 1];
         float held1[2][VEC == 1 ? LOADS : 1];
@@ -456,9 +458,9 @@ void launch_scatter(cudaStream_t s, const TG* g, TO* out, uint64_t n, uint64_t r
     const uint64_t span = vec ? 128 : 32;
     if (n > 0 && static_cast<const void*>(base) == static_cast<const void*>(out)) {
         // In place: only the rows some id names change, a warp per sorted position.
-        const uint32_t positions = static_cast<uint32_t>((n + 7) / 8);
-        if (vec) scatter_in_place_kernel<4><<<positions, 256, 0, s>>>(g, sorted_id, sorted_n, static_cast<uint32_t>(n), out, static_cast<uint32_t>(rows), static_cast<uint32_t>(h));
-        else scatter_in_place_kernel<1><<<positions, 256, 0, s>>>(g, sorted_id, sorted_n, static_cast<uint32_t>(n), out, static_cast<uint32_t>(rows), static_cast<uint32_t>(h));
+        const dim3 grid(static_cast<uint32_t>((n + 7) / 8), static_cast<uint32_t>((h + span - 1) / span));
+        if (vec) scatter_in_place_kernel<4><<<grid, 256, 0, s>>>(g, sorted_id, sorted_n, static_cast<uint32_t>(n), out, static_cast<uint32_t>(rows), static_cast<uint32_t>(h));
+        else scatter_in_place_kernel<1><<<grid, 256, 0, s>>>(g, sorted_id, sorted_n, static_cast<uint32_t>(n), out, static_cast<uint32_t>(rows), static_cast<uint32_t>(h));
         check_launch("embedding_grad");
         return;
     }
