@@ -200,6 +200,27 @@ __global__ void finalize_sums_kernel(const SumJob* __restrict__ jobs, uint32_t c
     __shared__ uint32_t which;
     const SumJob job = jobs[job_of_block(jobs, count, &which)];
     const uint32_t block = blockIdx.x - job.first_block;
+    if (sum_job_wide(job.chunks, job.width)) {
+        // The same order, four columns a thread.
+        const uint32_t c = (block * 256 + threadIdx.y * 32 + threadIdx.x) * 4;
+        if (c >= job.width) return;
+        float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (((reinterpret_cast<uintptr_t>(job.partial) | reinterpret_cast<uintptr_t>(job.out)) & 15u) == 0) {
+#pragma unroll 8
+            for (uint32_t k = 0; k < job.chunks; ++k) {
+                const float4 v = *reinterpret_cast<const float4*>(job.partial + static_cast<uint64_t>(k) * job.width + c);
+                acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
+            }
+            *reinterpret_cast<float4*>(job.out + c) = acc;
+            return;
+        }
+        for (uint32_t k = 0; k < job.chunks; ++k) {
+            const float* v = job.partial + static_cast<uint64_t>(k) * job.width + c;
+            acc.x += v[0]; acc.y += v[1]; acc.z += v[2]; acc.w += v[3];
+        }
+        job.out[c] = acc.x; job.out[c + 1] = acc.y; job.out[c + 2] = acc.z; job.out[c + 3] = acc.w;
+        return;
+    }
     if (job.chunks <= 64) {
         // Plain ascending order, one thread per column (what the two-launch forms of sum_rows and
         // the split-K reduction do).
