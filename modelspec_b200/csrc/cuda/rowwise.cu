@@ -653,8 +653,10 @@ __device__ __forceinline__ uint32_t keep_mask(const DropoutDraw& draw, uint64_t 
 // sum_out may be null when only the layer norm is wanted.
 // EXACT: the row is ITEMS x 32 wide, so that no column has to be tested. The test of every value, a
 // branch around a load or a store each, cost more than the arithmetic (16,384 bf16 rows of 768: 75 -> 59 us, of which some 40 are the Philox rounds).
+// The Philox rounds are what it waits for: of rows of 768, three blocks to an SM (80 registers) keep the
+// integer units busier than the two of 92 (68 -> 59 us).
 template <int ITEMS, int V, bool EXACT, class T>
-__global__ void __launch_bounds__(256) dropout_add_layer_norm_kernel(
+__global__ void __launch_bounds__(256, !EXACT ? 1 : ITEMS >= 32 ? 2 : ITEMS >= 24 ? 3 : 4) dropout_add_layer_norm_kernel(
     const T* __restrict__ x, const T* __restrict__ residual, DropoutDraw x_draw, const float* __restrict__ gamma,
     const float* __restrict__ beta, T* __restrict__ sum_out, T* __restrict__ out, DropoutDraw out_draw,
     T* __restrict__ out_dropped, uint32_t rows, uint32_t width_given, bool gelu_first) {
