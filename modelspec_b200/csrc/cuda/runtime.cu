@@ -2042,9 +2042,6 @@ struct Scheduler {
         l.flop = pair_flop * (1 + (dv >= 0) + ((dq >= 0 || dk >= 0) ? 1 : 0) + (dq >= 0) + (dk >= 0));
     }
 
-    // The product of a mixed-precision plan: bf16 operands in place (an activation, or the working
-    // copy of a parameter), the result in the storage type of its slot, a split k reduced by the
-    // launch or, for a weight gradient, left as f32 partial tiles for the finalize launch.
     // The gelu or gelu_grad that alone takes the result of a product element by element runs as the
     // product's tiles drain: gelu beside its argument (which its gradient reads later), gelu_grad in the
     // place of the adjoint it multiplies. -1: neither.
@@ -2066,6 +2063,9 @@ struct Scheduler {
         return -1;
     }
 
+    // The products of one launch of a mixed-precision plan: bf16 operands in place (an activation, or the working
+    // copy of a parameter), the result in the storage type of its slot, a split k reduced by the
+    // launch or, for a weight gradient, left as f32 partial tiles for the finalize launch.
     void emit_matmul_bf16(const Node& nd, const std::vector<Product>& group, std::vector<uint32_t> reads, uint64_t m, uint64_t n, uint64_t kk) {
         msx_plan* plan = P;
         for (const Product& p : group)
