@@ -25,7 +25,7 @@
 //                which a TMA store writes to C.
 // The tensor core's f32 accumulation truncates: a sum of N MMAs comes out low by about N 2^-24 of its
 // terms' magnitude (3 10^-4 of a sum of 16,384 positive products). So the sums of a tile leave tensor
-// memory every 24 (or 128) k blocks and go on in C, the first by a TMA store and the later ones by TMA's f32
+// memory every 24 (or 256) k blocks and go on in C, the first by a TMA store and the later ones by TMA's f32
 // reduction in the L2 (each after the one before it has landed, so in one order), and on the tiles of
 // one CTA the two cross products, whose terms are 2^-11 of the others', have an accumulator of their own.
 //
@@ -46,9 +46,10 @@ constexpr int BK = 32;
 constexpr int GROUP_THREADS = 64;  // of the warps that make one stage's lo blocks
 constexpr int MAX_PRODUCTS = 4, MAX_JOBS = 24;
 // k blocks summed in tensor memory before the sum goes to C: 24 (768 deep, error 6 10^-6 of a product's
-// norm on the paired tiles); 128 for products of two operands stored with k down their columns, the
-// weight gradients, whose k is the rows of a batch (16,384: 6 10^-5; 1.2 10^-4 as one sum).
-constexpr uint32_t SEGMENT = 24, SEGMENT_ROWS = 128;
+// norm on the paired tiles); 256 for products of two operands stored with k down their columns, the
+// weight gradients, whose k is the rows of a batch and mostly split (8,192 deep at most, where one sum over
+// 16,384 was 1.2 10^-4 off).
+constexpr uint32_t SEGMENT = 24, SEGMENT_ROWS = 256;
 
 template <int CG, int BN> struct Tile {
     static constexpr int BN_CTA = BN / CG;  // columns of B a CTA holds
