@@ -14,6 +14,7 @@
 #include <atomic>
 #include <cstdint>
 #include <cstring>
+#include <exception>
 #include <mutex>
 #include <thread>
 #include <vector>
@@ -28,7 +29,8 @@ public:
     ~HostCopier() { release(); }
 
     // Copies `bytes` from the device to `host` behind what `stream` holds, and returns when they have
-    // arrived. The first error of any thread is the result.
+    // arrived. The first error of any thread is the result. A share whose thread cannot be started (a
+    // process at its limit of threads or memory) is moved by the caller's.
     cudaError_t to_host(int device, void* host, const void* from, uint64_t bytes, cudaStream_t stream) {
         cudaPointerAttributes where;
         const bool pageable = bytes >= kSmallest && cudaPointerGetAttributes(&where, host) == cudaSuccess && where.type == cudaMemoryTypeUnregistered;
@@ -46,12 +48,19 @@ public:
         auto work = [&](uint32_t l) {
             cudaError_t mine = cudaSetDevice(device);
             if (mine == cudaSuccess) mine = move_pieces(lanes_[l], static_cast<char*>(host), static_cast<const char*>(from), bytes, l, pieces, lanes);
-            if (mine != cudaSuccess) failed = static_cast<int>(mine);
+            int none = static_cast<int>(cudaSuccess);
+            if (mine != cudaSuccess) failed.compare_exchange_strong(none, static_cast<int>(mine));
         };
-        std::vector<std::thread> others;
-        for (uint32_t l = 1; l < lanes; ++l) others.emplace_back(work, l);
+        std::thread others[kMostLanes];
+        uint32_t started = 1;
+        try {
+            for (; started < lanes; ++started) others[started] = std::thread(work, started);
+        } catch (const std::exception&) {
+        }
         work(0);
-        for (std::thread& t : others) t.join();
+        for (uint32_t l = started; l < lanes; ++l) work(l);
+        for (std::thread& t : others)
+            if (t.joinable()) t.join();
         return static_cast<cudaError_t>(failed.load());
     }
 
