@@ -25,7 +25,7 @@
 //                which a TMA store writes to C.
 // The tensor core's f32 accumulation truncates: a sum of N MMAs comes out low by about N 2^-24 of its
 // terms' magnitude (3 10^-4 of a sum of 16,384 positive products). So the sums of a tile leave tensor
-// memory every 24 (or 256) k blocks and go on in C, the first by a TMA store and the later ones by TMA's f32
+// memory every 24 k blocks and go on in C, the first by a TMA store and the later ones by TMA's f32
 // reduction in the L2 (each after the one before it has landed, so in one order), and on the tiles of
 // one CTA the two cross products, whose terms are 2^-11 of the others', have an accumulator of their own.
 //
@@ -45,11 +45,11 @@ namespace {
 constexpr int BK = 32;
 constexpr int GROUP_THREADS = 64;  // of the warps that make one stage's lo blocks
 constexpr int MAX_PRODUCTS = 4, MAX_JOBS = 24;
-// k blocks summed in tensor memory before the sum goes to C: 24 (768 deep, error 6 10^-6 of a product's
-// norm on the paired tiles); 256 for products of two operands stored with k down their columns, the
-// weight gradients, whose k is the rows of a batch and mostly split (8,192 deep at most, where one sum over
-// 16,384 was 1.2 10^-4 off).
-constexpr uint32_t SEGMENT = 24, SEGMENT_ROWS = 256;
+// k blocks summed in tensor memory before the sum goes to C (768 deep: 6 10^-6 of a product's norm on the
+// paired tiles, however deep the product). The sums into C cost a weight gradient 768 x 3,072 x 16,384
+// nothing (309 us; 312 with 64 blocks, 322 with 256) and 3,072 x 768 x 16,384 up to 5 % (328 us; 321 and
+// 308), for errors of 6 10^-6 (1.5 10^-5 and 5.9 10^-5) of their norm.
+constexpr uint32_t SEGMENT = 24;
 
 template <int CG, int BN> struct Tile {
     static constexpr int BN_CTA = BN / CG;  // columns of B a CTA holds
@@ -164,7 +164,6 @@ template <int CG, int BN, bool A_T, bool B_T, class A, class M>
 __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __grid_constant__ A args, const __grid_constant__ M maps) {
     using T = Tile<CG, BN>;
     constexpr int STAGES = T::STAGES;
-    constexpr uint32_t LENGTH = A_T && !B_T ? SEGMENT_ROWS : SEGMENT;
     extern __shared__ __align__(1024) char smem[];  // tiles on 1,024 bytes: the swizzle pattern is a function of address bits
     char* const slabs = smem + STAGES * T::STAGE_BYTES;
     float* const bias_tile = reinterpret_cast<float*>(slabs + T::DRAIN_WARPS * T::SLAB_BYTES);  // two of BN columns
@@ -261,7 +260,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
             for (uint32_t u = first_unit; u < units && alive; u += step) {
                 const uint32_t kblocks = unit_of(args, u).kblocks;
                 for (uint32_t kb = 0; kb < kblocks && alive; ++kb) {
-                    const uint32_t in_segment = kb % LENGTH, acc = turn & 1u;
+                    const uint32_t in_segment = kb % SEGMENT, acc = turn & 1u;
                     if (in_segment == 0) {
                         alive = tc::warp_wait<CG>(tc::smem_u32(&acc_empty[acc]), ((turn >> 1) & 1u) ^ 1u, abort_flag, args.status);
                         if (!alive) break;
@@ -288,9 +287,9 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
                             }
                         }
                         tc::commit<CG>(tc::smem_u32(&empty[stage]));
-                        if (in_segment + 1 == LENGTH || kb + 1 == kblocks) tc::commit<CG>(tc::smem_u32(&acc_full[acc]));
+                        if (in_segment + 1 == SEGMENT || kb + 1 == kblocks) tc::commit<CG>(tc::smem_u32(&acc_full[acc]));
                     }
-                    if (in_segment + 1 == LENGTH || kb + 1 == kblocks) ++turn;
+                    if (in_segment + 1 == SEGMENT || kb + 1 == kblocks) ++turn;
                     if (++stage == STAGES) { stage = 0; parity ^= 1u; }
                     __syncwarp();
                 }
@@ -354,7 +353,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
         bool alive = true;
         uint32_t turn = 0;
         for (uint32_t u = first_unit; u < units && alive; u += step)
-        for (uint32_t segment = 0, left = unit_of(args, u).kblocks; left > 0 && alive; left -= left < LENGTH ? left : LENGTH, ++segment, ++turn) {
+        for (uint32_t segment = 0, left = unit_of(args, u).kblocks; left > 0 && alive; left -= left < SEGMENT ? left : SEGMENT, ++segment, ++turn) {
             const Unit w = unit_of(args, u);
             const uint32_t acc = turn & 1u;
             // The bias of the warp's columns, fetched before the wait for the tile (a load issued in the drain

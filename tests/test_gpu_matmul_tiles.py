@@ -42,3 +42,29 @@ def test_f32_products_at_the_edges_of_their_kernels(device, m, n, k, form):
     assert int(status.item()) == 0
     worst = float((off.abs() / size).max())
     assert worst <= (6e-6 if k <= 1024 else 2e-5), worst
+
+
+# Weight gradients as deep as a batch has rows: on pairs of CTAs (unsplit and split) and on tiles of one
+# CTA. What truncates is a segment of 96 k slices in tensor memory, three MMAs a slice, each at most
+# 2^-23 of a sum that grows to the segment's: 96 * 3 * 2^-23 / 2 = 1.7e-5 of sum |a||b| if every MMA lost
+# a whole unit in the last place, half of it on average (a sum of 256 k blocks was 2.8e-5 low).
+@pytest.mark.parametrize("m,n,k", [(768, 3072, 16384), (3072, 768, 16384), (768, 768, 16384), (396, 1024, 60000), (96, 64, 20000), (4096, 260, 9001)])
+def test_deep_weight_gradients_do_not_come_out_low(device, m, n, k):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(m + 3 * n + 7 * k)
+    a = torch.randn((k, m), device="cuda", generator=gen) + 0.5
+    b = torch.randn((k, n), device="cuda", generator=gen) + 0.5
+    c = torch.full((m, n), float("nan"), device="cuda")
+    L = M.lib()
+    need = L.msx_op_matmul_workspace(m, n, k)
+    ws = torch.empty(max(need, 1), device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    torch.cuda.synchronize()
+    rc = L.msx_op_matmul(ptr(a), 1, ptr(b), 0, ptr(c), m, n, k, ptr(ws), need, ptr(status), C.c_void_p(torch.cuda.current_stream().cuda_stream), 0)
+    assert rc == M.OK, L.msx_last_error(None)
+    size = a.double().abs().t() @ b.double().abs()
+    off = (c.double() - a.double().t() @ b.double()).abs()
+    assert int(status.item()) == 0
+    worst = float((off / size).max())
+    assert worst <= 8.6e-6, worst
