@@ -930,11 +930,8 @@ void launch_cross_entropy_one_read(cudaStream_t s, const float* logits, const in
                                    const float* den, float* row_loss, float* grad, uint32_t vv, uint32_t l1, uint32_t l2, uint32_t* counter,
                                    float* loss, uint64_t rows, bool vec) {
     if (vec && vv > 16384) {
-        static const bool configured = [] {
-            cudaFuncSetAttribute(cross_entropy_fused_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, kSplitSharedBytes);
-            return true;
-        }();
-        (void)configured;
+        static std::atomic<int> configured_device{-1};
+        set_shared_memory(cross_entropy_fused_split_kernel, kSplitSharedBytes, configured_device);
         cross_entropy_fused_split_kernel<<<static_cast<uint32_t>(rows), kSplitThreads, kSplitSharedBytes, s>>>(logits, labels, weights, g, den,
                                                                                                               row_loss, grad, vv, l1, l2,
                                                                                                               counter, loss);
@@ -1096,8 +1093,8 @@ void launch_layer_norm_backward(cudaStream_t s, const T* x, const float* gamma, 
         auto kernel = layer_norm_backward_kernel<N, W, E, T>; \
         constexpr uint32_t bytes = (N >= 16 ? 2u : 1u) * 8u * 32u * N * 4u; \
         if (bytes > 40000u) { \
-            static const bool configured = [kernel] { cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(bytes)); return true; }(); \
-            (void)configured; \
+            static std::atomic<int> configured_device{-1}; \
+            set_shared_memory(kernel, static_cast<int>(bytes), configured_device); \
         } \
         kernel<<<chunks, 256, bytes, s>>>(x, gamma, g, g1, g2, g3, dx, scratch, counter, dgamma, dbeta, want, r, hh, per, in_draw, out_draw, dx_dropped, pre_activation); } while (0)
 #define MSX_LN_BACKWARD(N) do { \

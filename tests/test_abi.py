@@ -38,3 +38,14 @@ def test_null_handles_are_bad_arguments():
     assert L.msx_plan_input_count(None) == 0
     assert L.msx_set_input(None, b"x", None, 0) == M.BAD_ARGUMENT
     assert L.msx_training_steps(None) == 0
+
+
+def test_shared_memory_limits_are_set_per_device():
+    """A kernel's limit of dynamic shared memory belongs to a device: it is set by set_shared_memory, which
+    looks at the device, or in front of every launch (`opt_in`), never once for the whole process."""
+    sources = os.path.join(ROOT, "modelspec_b200", "csrc", "cuda")
+    for name in sorted(os.listdir(sources)):
+        for line in open(os.path.join(sources, name)):
+            assert not ("static" in line and "configured" in line and "std::atomic<int> configured_device" not in line), (name, line)
+            if "cudaFuncSetAttribute(" in line:
+                assert "check(" in line, (name, line)
