@@ -12,7 +12,7 @@
 typedef int cudaError_t;
 typedef void* cudaStream_t;
 typedef void* cudaEvent_t;
-enum { cudaSuccess = 0, cudaMemoryTypeUnregistered = 0, cudaEventDisableTiming = 2, cudaStreamNonBlocking = 1, cudaMemcpyDeviceToHost = 2 };
+enum { cudaSuccess = 0, cudaHostRegisterDefault = 0, cudaMemoryTypeUnregistered = 0, cudaEventDisableTiming = 2, cudaStreamNonBlocking = 1, cudaMemcpyDeviceToHost = 2 };
 struct cudaPointerAttributes {
     int type;
 };
@@ -20,6 +20,7 @@ struct cudaPointerAttributes {
 namespace fake {
 inline std::atomic<int> copies{0};
 inline int fail_after = 1 << 30;
+inline bool may_register = true;
 }  // namespace fake
 
 inline cudaError_t cudaPointerGetAttributes(cudaPointerAttributes* a, const void*) { a->type = cudaMemoryTypeUnregistered; return cudaSuccess; }
@@ -27,6 +28,9 @@ inline cudaError_t cudaGetLastError() { return cudaSuccess; }
 inline cudaError_t cudaSetDevice(int) { return cudaSuccess; }
 inline cudaError_t cudaMallocHost(char** p, uint64_t bytes) { *p = static_cast<char*>(std::malloc(bytes)); return cudaSuccess; }
 inline cudaError_t cudaFreeHost(void* p) { std::free(p); return cudaSuccess; }
+inline cudaError_t cudaHostRegister(void*, uint64_t, int) { return fake::may_register ? cudaSuccess : 1; }
+inline cudaError_t cudaHostUnregister(void*) { return cudaSuccess; }
+inline cudaError_t cudaHostGetDevicePointer(void** device, void* host, int) { *device = host; return cudaSuccess; }
 inline cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, int) { *s = s; return cudaSuccess; }
 inline cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
 inline cudaError_t cudaStreamSynchronize(cudaStream_t) { return cudaSuccess; }

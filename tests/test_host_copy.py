@@ -14,12 +14,13 @@ def check(tmp_path_factory):
     program = str(tmp_path_factory.mktemp("host_copy") / "check")
     subprocess.run(["g++", "-std=c++17", "-O1", "-I" + os.path.join(HERE, "host"), "-I" + os.path.join(HERE, "..", "modelspec_b200", "csrc", "cuda"),
                     os.path.join(HERE, "host", "host_copy_check.cpp"), "-o", program, "-pthread", "-ldl"], check=True)
-    return lambda threads, fails: subprocess.run([program, str(threads), str(fails)], capture_output=True, text=True, timeout=60)
+    return lambda threads, fails, registers=1: subprocess.run([program, str(threads), str(fails), str(registers)], capture_output=True, text=True, timeout=60)
 
 
-@pytest.mark.parametrize("threads", [0, 1, 3, 7])
-def test_a_download_needs_no_thread(check, threads):
-    ran = check(threads, -1)
+@pytest.mark.parametrize("threads", [0, 1, 3, 7, 1000])
+@pytest.mark.parametrize("registers", [0, 1])
+def test_a_download_needs_no_thread(check, threads, registers):
+    ran = check(threads, -1, registers)
     assert ran.returncode == 0, ran.stderr
     assert ran.stdout == "0 whole\n"
 
