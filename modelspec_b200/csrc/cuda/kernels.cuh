@@ -448,9 +448,14 @@ void attention_fused_backward(cudaStream_t s, const void* q, const void* k, cons
                               const float* stats, void* dq, void* dk, void* dv, AttentionShape shape, uint32_t* status);
 
 // ---- the ends of a step (step_io.cu) -------------------------------------------------------------
-// to[0 .. bytes) = slots[*turn % count]; `bytes` and `slot_bytes` are multiples of 16, the slots pinned
+// to[0 .. bytes) = slots.at[*turn % slots.count]; `bytes` is a multiple of 16, the slots on 16 bytes in pinned
 // host or device memory.
-void take_inputs(cudaStream_t s, const char* slots, uint64_t slot_bytes, uint32_t count, uint64_t bytes, char* to, const uint32_t* turn);
+constexpr int kMostInputSlots = 8;
+struct InputSlots {
+    const char* at[kMostInputSlots];
+    uint32_t count;
+};
+void take_inputs(cudaStream_t s, const InputSlots& slots, uint64_t bytes, char* to, const uint32_t* turn);
 // to_loss[*turn] = *loss (when there is one), to_status[*turn] = *status (pinned host memory), and
 // *turn moves on, modulo `slots`.
 void publish_step(cudaStream_t s, const float* loss, const uint32_t* status, float* to_loss, uint32_t* to_status, uint32_t* turn, uint32_t slots);

@@ -46,11 +46,19 @@ constexpr int kStagingSlots = 8;  // steps in flight before msx_run waits (the r
 // The end events of this many steps are kept: the last kStagingSlots steps' and, as the begin of a
 // step submitted behind a running one, their predecessors'.
 constexpr int kStepEvents = 2 * kStagingSlots;
-// Inputs of more than kDirectInputBytes cross PCIe on a stream of their own, beside the step before,
-// into one of two slots on the device; smaller ones are read from the pinned slot by the step's first
-// kernel (which 16 blocks do in one trip over PCIe; at 200 KB the copy beside the step before wins).
+// The inputs of a step are read from its pinned slot by its first kernel, which 16 blocks do in one trip
+// over PCIe for 64 KB. A plan that steps behind its own steps brings larger ones into one of two slots on
+// the device beside the step before: an MLP of 200 KB a step takes 48 us so against 54 read in place, a transformer
+// block of 1 MB 280 against 302. With no step to run beside, the copy stays on the plan's own stream (8 MB a step,
+// read back at once: the same 2.1 ms without staging; a second stream only adds its waits). Forward programs,
+// which share a step plan's parameters, are waited for and read theirs in place.
 constexpr uint64_t kDirectInputBytes = 64ull << 10;
 constexpr int kDeviceSlots = 2;
+static_assert(kStagingSlots <= k::kMostInputSlots && kDeviceSlots <= k::kMostInputSlots);
+// Up to here a plan's pinned slots are requests of their own, which fit the room left in the driver's 2 MB blocks
+// of pinned memory (eight of 200 KB: 20 us in a process that has such a block, 1.2 to 3 ms as one request);
+// beyond they are one block.
+constexpr uint64_t kPinnedApart = 2ull << 20;
 
 uint64_t align_up(uint64_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
@@ -161,10 +169,10 @@ struct msx_plan {
     uint64_t input_bytes = 0;
     std::vector<char> blob;  // the staged inputs, host side
     bool blob_dirty = true;  // staged since the last upload
-    char* pinned = nullptr;        // kStagingSlots slots of slot_bytes
-    uint64_t slot_bytes = 0;
-    char* d_staging = nullptr;     // large inputs: kDeviceSlots slots on the device, filled on copy_stream
-    cudaStream_t copy_stream = nullptr;
+    msx::PinnedBlock pinned_together;
+    char* pinned[kStagingSlots] = {};  // a slot of input_bytes each, pieces of pinned_together or requests of their own
+    char* d_staging = nullptr;         // large inputs: kDeviceSlots slots on the device
+    cudaStream_t copy_stream = nullptr;  // fills them beside a running step; made when the first one does
     cudaEvent_t copied[kDeviceSlots] = {};
     uint32_t* d_turn = nullptr;    // the slot of the step that runs next, kept by the step itself
     float* pinned_loss = nullptr;  // kStagingSlots floats
@@ -2398,6 +2406,24 @@ template <class T> cudaError_t plan_malloc(msx_plan* P, T** out, size_t bytes) {
     return e;
 }
 
+// Where a plan's inputs wait for their step: its blob, its pinned slots and, where inputs are staged, its
+// slots on the device. A forward program that shares a step plan's parameters makes them when its first input is
+// set: a run has such a plan from its beginning and may never feed it.
+void make_input_slots(msx_plan* P) {
+    if (!P->blob.empty()) return;
+    const uint64_t bytes = std::max<uint64_t>(P->input_bytes, kAlign);
+    if (kStagingSlots * bytes > kPinnedApart) {
+        cuda_ok(P->pinned_together.make(kStagingSlots * bytes), "pinned memory (staging)");
+        for (int s = 0; s < kStagingSlots; ++s) P->pinned[s] = P->pinned_together.data() + s * bytes;
+    } else {
+        for (char*& slot : P->pinned)
+            if (!slot) cuda_ok(cudaMallocHost(&slot, bytes), "cudaMallocHost(staging)");
+    }
+    if (!P->shares && P->input_bytes > kDirectInputBytes && !P->d_staging)
+        cuda_ok(plan_malloc(P, &P->d_staging, kDeviceSlots * bytes), "cudaMalloc(staging)");
+    P->blob.assign(bytes, 0);
+}
+
 void allocate(msx_plan* P, const Scheduler& sched) {
     const Program& prog = P->program;
     cuda_ok(cudaStreamCreateWithFlags(&P->stream, cudaStreamNonBlocking), "cudaStreamCreate");
@@ -2472,14 +2498,12 @@ void allocate(msx_plan* P, const Scheduler& sched) {
         for (size_t p : new_copies) k::working_copy(P->stream, P->params[p], P->params16[p], prog.params[p].ty.count());
     }
     const uint64_t in_bytes = std::max<uint64_t>(P->input_bytes, kAlign);
-    const bool staged = P->input_bytes > kDirectInputBytes;
     const uint64_t const_bytes = std::max<uint64_t>(P->consts.size() * 4, 4);
     const uint64_t counter_bytes = std::max<uint64_t>(P->counters_used, 1) * 4;
     const uint64_t tensor_bytes = sched.updates.size() * sizeof(k::UpdateTensor), chunk_bytes = sched.update_chunk_tensor.size() * 4;
     {
         const std::pair<void**, uint64_t> pieces[] = {
             {reinterpret_cast<void**>(&P->d_inputs), in_bytes},
-            {reinterpret_cast<void**>(&P->d_staging), staged ? kDeviceSlots * in_bytes : 0},
             {reinterpret_cast<void**>(&P->d_consts), const_bytes},
             {reinterpret_cast<void**>(&P->d_status), 8},
             {reinterpret_cast<void**>(&P->d_counters), counter_bytes},
@@ -2497,20 +2521,14 @@ void allocate(msx_plan* P, const Scheduler& sched) {
             at += align_up(piece.second);
         }
     }
-    P->blob.assign(in_bytes, 0);
-    // One pinned allocation: the input slots, then each slot's loss and status word.
-    P->slot_bytes = in_bytes;
-    cuda_ok(cudaMallocHost(&P->pinned, kStagingSlots * in_bytes + 2 * kStagingSlots * 4), "cudaMallocHost(staging)");
-    P->pinned_loss = reinterpret_cast<float*>(P->pinned + kStagingSlots * in_bytes);
+    if (!P->shares) make_input_slots(P);
+    // Each step's loss and status word.
+    cuda_ok(cudaMallocHost(&P->pinned_loss, 2 * kStagingSlots * 4), "cudaMallocHost(loss)");
     P->pinned_status = reinterpret_cast<uint32_t*>(P->pinned_loss + kStagingSlots);
     std::memset(P->pinned_loss, 0, 2 * kStagingSlots * 4);
     for (int s = 0; s < kStepEvents; ++s) {
         cuda_ok(cudaEventCreate(&P->step_begin[s]), "cudaEventCreate");
         cuda_ok(cudaEventCreate(&P->step_done[s]), "cudaEventCreate");
-    }
-    if (staged) {
-        cuda_ok(cudaStreamCreateWithFlags(&P->copy_stream, cudaStreamNonBlocking), "cudaStreamCreate");
-        for (cudaEvent_t& e : P->copied) cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
     }
     if (!P->consts.empty())
         cuda_ok(cudaMemcpy(P->d_consts, P->consts.data(), P->consts.size() * 4, cudaMemcpyHostToDevice), "cudaMemcpy(constants)");
@@ -2610,7 +2628,12 @@ void release(msx_plan* P) {
         if (P->step_done[s]) cudaEventDestroy(P->step_done[s]);
     }
     if (P->backup) cudaFree(P->backup);
-    if (P->pinned) cudaFreeHost(P->pinned);
+    if (P->pinned_loss) cudaFreeHost(P->pinned_loss);
+    if (P->d_staging) cudaFree(P->d_staging);
+    if (!P->pinned_together.data())
+        for (char* slot : P->pinned)
+            if (slot) cudaFreeHost(slot);
+    P->pinned_together.release();
     if (P->clock_start) cudaEventDestroy(P->clock_start);
     if (P->stream) cudaStreamDestroy(P->stream);
     delete P;
@@ -2837,12 +2860,36 @@ int wait_all(msx_plan* P, uint32_t timeout_ms) {
 // kernels of the step's graph: a copy engine's turn costs several microseconds of an otherwise idle
 // device each (an 8-kernel step: 30 us with a copy in front and two 4-byte copies behind, 18 us so).
 void enqueue_step(msx_plan* P, bool take_inputs) {
-    if (take_inputs)
-        k::take_inputs(P->stream, P->d_staging ? P->d_staging : P->pinned, P->slot_bytes, P->d_staging ? kDeviceSlots : kStagingSlots, P->input_bytes,
-                       P->d_inputs, P->d_turn);
+    if (take_inputs) {
+        k::InputSlots slots = {{}, P->d_staging ? kDeviceSlots : kStagingSlots};
+        for (uint32_t s = 0; s < slots.count; ++s) slots.at[s] = P->d_staging ? P->d_staging + s * P->input_bytes : P->pinned[s];
+        k::take_inputs(P->stream, slots, P->input_bytes, P->d_inputs, P->d_turn);
+    }
     enqueue_all(P);
     k::publish_step(P->stream, P->loss_pos >= 0 ? P->f(static_cast<uint32_t>(P->loss_pos)) : nullptr, P->d_status, P->pinned_loss, P->pinned_status,
                     P->d_turn, kStagingSlots);
+}
+
+// A large step's inputs from its pinned slot to its slot on the device: on the plan's stream when that is
+// idle, else beside the step before.
+void stage_inputs(msx_plan* P, int slot, bool idle) {
+    const int half = slot % kDeviceSlots;
+    char* const to = P->d_staging + half * P->input_bytes;
+    if (idle) {
+        cuda_ok(cudaMemcpyAsync(to, P->pinned[slot], P->input_bytes, cudaMemcpyHostToDevice, P->stream), "cudaMemcpyAsync(inputs)");
+        return;
+    }
+    if (!P->copy_stream) {
+        for (cudaEvent_t& e : P->copied)
+            if (!e) cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
+        cuda_ok(cudaStreamCreateWithFlags(&P->copy_stream, cudaStreamNonBlocking), "cudaStreamCreate");
+    }
+    // The slot on the device is free once the step that last used it has run.
+    if (P->steps >= kDeviceSlots)
+        cuda_ok(cudaStreamWaitEvent(P->copy_stream, P->step_done[(P->steps - kDeviceSlots) % kStepEvents], 0), "cudaStreamWaitEvent");
+    cuda_ok(cudaMemcpyAsync(to, P->pinned[slot], P->input_bytes, cudaMemcpyHostToDevice, P->copy_stream), "cudaMemcpyAsync(inputs)");
+    cuda_ok(cudaEventRecord(P->copied[half], P->copy_stream), "cudaEventRecord");
+    cuda_ok(cudaStreamWaitEvent(P->stream, P->copied[half], 0), "cudaStreamWaitEvent");
 }
 
 template <class F> int guarded(msx_device* device, F body) {
@@ -3118,6 +3165,10 @@ int msx_set_input(msx_plan* plan, const char* name, const void* host, uint64_t b
             std::string why;
             int rc = check_input(in, host, &why);
             if (rc != MSX_OK) throw StatusError(rc, why);
+            if (plan->blob.empty()) {
+                cuda_ok(cudaSetDevice(plan->device->ordinal), "cudaSetDevice");
+                make_input_slots(plan);
+            }
             std::memcpy(plan->blob.data() + in.offset, host, bytes);
             plan->blob_dirty = true;
             return MSX_OK;
@@ -3165,20 +3216,11 @@ int msx_run(msx_plan* plan) {
         plan->bytes_downloaded += (plan->loss_pos >= 0 ? 4 : 0) + 4;
         const bool take_inputs = plan->input_bytes && plan->blob_dirty;
         if (take_inputs) {
+            make_input_slots(plan);
             plan->bytes_uploaded += plan->input_bytes;
             plan->blob_dirty = false;
-            char* const from = plan->pinned + slot * plan->slot_bytes;
-            std::memcpy(from, plan->blob.data(), plan->input_bytes);
-            if (plan->d_staging) {
-                // The slot on the device is free once the step that last used it has run.
-                const int half = slot % kDeviceSlots;
-                if (plan->steps >= kDeviceSlots)
-                    cuda_ok(cudaStreamWaitEvent(plan->copy_stream, plan->step_done[(plan->steps - kDeviceSlots) % kStepEvents], 0), "cudaStreamWaitEvent");
-                cuda_ok(cudaMemcpyAsync(plan->d_staging + half * plan->slot_bytes, from, plan->input_bytes, cudaMemcpyHostToDevice, plan->copy_stream),
-                        "cudaMemcpyAsync(inputs)");
-                cuda_ok(cudaEventRecord(plan->copied[half], plan->copy_stream), "cudaEventRecord");
-                cuda_ok(cudaStreamWaitEvent(plan->stream, plan->copied[half], 0), "cudaStreamWaitEvent");
-            }
+            std::memcpy(plan->pinned[slot], plan->blob.data(), plan->input_bytes);
+            if (plan->d_staging) stage_inputs(plan, slot, plan->began_idle[at]);
         }
         if (plan->flags & MSX_PLAN_NO_GRAPH) {
             enqueue_step(plan, take_inputs);
@@ -3262,8 +3304,9 @@ int msx_profile_step_repeated(msx_plan* plan, uint32_t repeats, float* launch_ms
         std::vector<cudaEvent_t> events(2 * count);
         for (cudaEvent_t& e : events) cuda_ok(cudaEventCreate(&e), "cudaEventCreate");
         if (plan->input_bytes) {
-            std::memcpy(plan->pinned, plan->blob.data(), plan->input_bytes);
-            cuda_ok(cudaMemcpyAsync(plan->d_inputs, plan->pinned, plan->input_bytes, cudaMemcpyHostToDevice, plan->stream), "cudaMemcpyAsync");
+            make_input_slots(plan);
+            std::memcpy(plan->pinned[0], plan->blob.data(), plan->input_bytes);
+            cuda_ok(cudaMemcpyAsync(plan->d_inputs, plan->pinned[0], plan->input_bytes, cudaMemcpyHostToDevice, plan->stream), "cudaMemcpyAsync");
         }
         begin_side_work(plan);
         for (size_t l = 0; l < count; ++l) {
@@ -3406,6 +3449,7 @@ int msx_heldout_create(msx_plan* plan, uint32_t logits, uint32_t batches, msx_he
             throw StatusError(MSX_BAD_ARGUMENT, "msx_heldout_create: %" + std::to_string(logits) + " is not an f32 output of the plan");
         if (batches == 0) throw StatusError(MSX_BAD_ARGUMENT, "msx_heldout_create: no batches");
         cuda_ok(cudaSetDevice(plan->device->ordinal), "cudaSetDevice");
+        make_input_slots(plan);
         std::unique_ptr<msx_heldout> h(new msx_heldout());
         h->plan = plan;
         h->at = static_cast<uint32_t>(at);

@@ -18,9 +18,9 @@ constexpr int kTakeThreads = 256, kTakeChunks = 4;
 
 // 16-byte chunks, four in flight per thread. No word in pinned memory is read by more than one warp:
 // reads of one host address are served one after the other, about a microsecond each.
-__global__ void __launch_bounds__(kTakeThreads) take_inputs_kernel(const char* __restrict__ slots, uint64_t slot_bytes, uint32_t count, uint64_t chunks,
-                                                                    uint4* __restrict__ to, const uint32_t* __restrict__ turn) {
-    const uint4* from = reinterpret_cast<const uint4*>(slots + *turn % count * slot_bytes);
+__global__ void __launch_bounds__(kTakeThreads) take_inputs_kernel(const __grid_constant__ InputSlots slots, uint64_t chunks, uint4* __restrict__ to,
+                                                                    const uint32_t* __restrict__ turn) {
+    const uint4* from = reinterpret_cast<const uint4*>(slots.at[*turn % slots.count]);
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kTakeThreads;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * kTakeThreads + threadIdx.x; i < chunks; i += kTakeChunks * stride) {
         uint4 v[kTakeChunks];
@@ -43,13 +43,13 @@ __global__ void publish_step_kernel(const float* __restrict__ loss, const uint32
 
 }  // namespace
 
-void take_inputs(cudaStream_t s, const char* slots, uint64_t slot_bytes, uint32_t count, uint64_t bytes, char* to, const uint32_t* turn) {
+void take_inputs(cudaStream_t s, const InputSlots& slots, uint64_t bytes, char* to, const uint32_t* turn) {
     const uint64_t chunks = bytes / 16;
     // A chunk a thread while that keeps the grid within one wave (64 KB from pinned memory is 16
     // blocks); four a thread and a loop beyond.
     uint64_t blocks = (chunks + kTakeThreads - 1) / kTakeThreads;
     if (blocks > 296) blocks = 296;
-    take_inputs_kernel<<<static_cast<uint32_t>(blocks), kTakeThreads, 0, s>>>(slots, slot_bytes, count, chunks, reinterpret_cast<uint4*>(to), turn);
+    take_inputs_kernel<<<static_cast<uint32_t>(blocks), kTakeThreads, 0, s>>>(slots, chunks, reinterpret_cast<uint4*>(to), turn);
     check_launch("take_inputs");
 }
 

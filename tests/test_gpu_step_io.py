@@ -1,5 +1,5 @@
 """What surrounds the launches of a step: inputs handed over through the staging slots (small ones
-read from pinned memory by the step's first kernel, large ones copied ahead on their own stream),
+read from pinned memory by the step's first kernel, large ones copied ahead beside the step before),
 losses published in their step's slot, values read back into memory that is not pinned, and the
 update launch at the edges of its chunks."""
 import numpy as np
@@ -39,6 +39,41 @@ def test_every_step_runs_on_the_inputs_staged_for_it(device, n, flags):
         assert steps == 20 and total > 0.0
     finally:
         plan.destroy()
+
+
+# Read in place, staged, at eight pinned slots of 2 MB in all and one beyond, 8 MB; a plan of its own, and one that
+# shares another's parameters and so reads in place whatever the size. Steps waited for one by one, then
+# steps submitted behind one another, then waited for again, some on what is staged already.
+@pytest.mark.parametrize("n", [16384 - 64, 16384 + 1, 65536, 65536 + 64, 2100001])
+@pytest.mark.parametrize("shared", [False, True])
+def test_large_inputs_of_steps_waited_for_and_of_steps_behind_one_another(device, n, shared):
+    p = ProgramText()
+    a = p.input("a", "f32", [n]); b = p.input("b", "f32", [n])
+    p.output(p.op("Mse", [], [a, b]))
+    plans = [M.Plan(device, p.text())]
+    if shared:
+        plans.append(M.Plan(device, p.text(), shares=plans[0]))
+    plan = plans[-1]
+    r = np.random.default_rng(n)
+    values = [r.standard_normal(n).astype(np.float32) for _ in range(6)]
+    zeros = np.zeros(n, dtype=np.float32)
+    mean_square = [float(np.mean(np.square(v, dtype=np.float64))) for v in values]
+    try:
+        plan.set_input("b", zeros)
+        want, k = [], 0
+        for burst in (1, 1, 5, 1, 11, 2, 1):
+            for _ in range(burst):
+                if k % 4 != 3:
+                    plan.set_input("a", values[k % 6])
+                    last = mean_square[k % 6]
+                plan.run()
+                want.append(last)
+                k += 1
+            for j in range(max(k - burst, k - 8), k):
+                assert abs(float(plan.loss_of(j)) - want[j]) <= 1e-6 * want[j], (j, burst)
+    finally:
+        for one in reversed(plans):
+            one.destroy()
 
 
 # Around the sizes where the copy into pageable memory starts to be staged, takes a second piece, a
