@@ -176,8 +176,8 @@ struct msx_plan {
     cudaEvent_t copied[kDeviceSlots] = {};
     uint32_t* d_turn = nullptr;    // the slot of the step that runs next, kept by the step itself
     float* pinned_loss = nullptr;  // kStagingSlots floats
-    // Step n ends with step_done[n % kStepEvents]. It begins with step_begin[...] when the stream was
-    // idle as it was submitted, else where the step before it ends.
+    // Step n ends with step_done[n % kStepEvents]. It begins with step_begin[...], made on first use, when the
+    // stream was idle as it was submitted, else where the step before it ends.
     cudaEvent_t step_begin[kStepEvents] = {}, step_done[kStepEvents] = {};
     bool began_idle[kStepEvents] = {};
     std::vector<float> consts;
@@ -2526,10 +2526,7 @@ void allocate(msx_plan* P, const Scheduler& sched) {
     cuda_ok(cudaMallocHost(&P->pinned_loss, 2 * kStagingSlots * 4), "cudaMallocHost(loss)");
     P->pinned_status = reinterpret_cast<uint32_t*>(P->pinned_loss + kStagingSlots);
     std::memset(P->pinned_loss, 0, 2 * kStagingSlots * 4);
-    for (int s = 0; s < kStepEvents; ++s) {
-        cuda_ok(cudaEventCreate(&P->step_begin[s]), "cudaEventCreate");
-        cuda_ok(cudaEventCreate(&P->step_done[s]), "cudaEventCreate");
-    }
+    for (cudaEvent_t& e : P->step_done) cuda_ok(cudaEventCreate(&e), "cudaEventCreate");
     if (!P->consts.empty())
         cuda_ok(cudaMemcpy(P->d_consts, P->consts.data(), P->consts.size() * 4, cudaMemcpyHostToDevice), "cudaMemcpy(constants)");
     P->d_turn = P->d_status + 1;
@@ -3206,7 +3203,10 @@ int msx_run(msx_plan* plan) {
         // A step submitted behind a running one begins where that one ends; only on an idle stream
         // does it need an event of its own (a recorded event costs the stream about 2 us).
         plan->began_idle[at] = plan->steps == 0 || cudaEventQuery(plan->step_done[(plan->steps - 1) % kStepEvents]) == cudaSuccess;
-        if (plan->began_idle[at]) cuda_ok(cudaEventRecord(plan->step_begin[at], plan->stream), "cudaEventRecord");
+        if (plan->began_idle[at]) {
+            if (!plan->step_begin[at]) cuda_ok(cudaEventCreate(&plan->step_begin[at]), "cudaEventCreate");
+            cuda_ok(cudaEventRecord(plan->step_begin[at], plan->stream), "cudaEventRecord");
+        }
         if (!plan->timing_begun) {
             plan->timing_begun = true;
             plan->first_submit = plan->last_wait = std::chrono::steady_clock::now();
