@@ -557,6 +557,9 @@ bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 // Which kernel, tile and k split by a cost model in microseconds, fitted to measured times of single
 // products (64 x 10 x 128 to 16,384 x 3,072 x 768, all storage forms): a launch's fixed part (set-up,
 // first loads, last drain), a part per k block, one per tile, and the bytes all SMs pull through the L2.
+// The 64-row tiles' figures are fitted to 470 products on rows off 16 bytes (24 to 50,000 a side), each timed with
+// every tile and up to 36 splits: the choice is 1.8 % above the fastest on average (4.9 % with the figures
+// before, 1.47 times it at most: 92 x 17,609 x 2,207 took 178 us on narrow tiles, 122 on wide ones).
 //   * small tiles on the FMA units while the product fits a few of them per SM;
 //   * operands TMA can address: 128-row tiles 32, 64 or 128 wide (the narrow ones when the wide ones would
 //     leave SMs idle), or pairs of CTAs on 256 x 256 tiles once there are enough of those;
@@ -577,19 +580,22 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
         {Tma, 128, 128, 5.3, 0.6, 1.1, 148.0},
         {Tma, 256, 256, 7.2, 1.02, 1.3, 74.0},
         // Two CTAs share an SM; a k block takes at least the last figure of an SM's time.
-        {Rows64, 64, 32, 4.0, 0.37, 0.21, 296.0},
-        {Rows64, 64, 64, 4.0, 0.5, 0.29, 296.0},
-        {Rows64, 64, 128, 4.0, 1.0, 0.58, 296.0},
+        {Rows64, 64, 32, 3.5, 0.25, 0.60, 296.0},
+        {Rows64, 64, 64, 3.5, 0.47, 0.38, 296.0},
+        {Rows64, 64, 128, 3.5, 0.80, 0.45, 296.0},
     };
-    constexpr double kBytesPerUs = 7.0e6, kReduceFixed = 2.0, kReduceBytesPerUs = 2.5e6;
     const uint64_t kblocks = (k + BK - 1) / BK;
     MatmulTcPlan best = {};
     double best_cost = 0.0;
     for (const Candidate& c : candidates) {
         if (c.kernel == Fma ? batched || kblocks == 0 || chain > 1 : (c.kernel == Tma) != (kblocks > 0 && tma_ok)) continue;
+        const bool rows64 = c.kernel == Rows64;
+        if (rows64 && c.bn > 32 && c.bn / 2 >= n) continue;  // a narrower tile holds the same columns
+        const double bytes_per_us = rows64 ? 8.3e6 : 7.0e6, reduce_fixed = rows64 ? 1.7 : 2.0, reduce_bytes_per_us = rows64 ? 7.3e6 : 2.5e6;
         const uint64_t m_tiles = (m + c.bm - 1) / c.bm, n_tiles = (n + c.bn - 1) / c.bn, tiles = m_tiles * n_tiles * problems * group;
         auto consider = [&](double cost, uint64_t splits, uint64_t per, uint32_t cluster) {
-            if (best.bn != 0 && cost >= best_cost) return;
+            // (A split product's second launch is a microsecond more beside the one launch of the FMA tiles.)
+            if (best.bn != 0 && cost + (rows64 && best.fma && splits > 1 ? 1.0 : 0.0) >= best_cost) return;
             best_cost = cost;
             best = MatmulTcPlan{c.bm, c.bn, static_cast<uint32_t>(splits), static_cast<uint32_t>(per == 0 ? 1 : per), c.kernel == Fma, cluster, 0};
         };
@@ -621,9 +627,9 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
             // Every tile reads its rows of A and columns of B over k.
             const double bytes = 4.0 * static_cast<double>(problems * group) *
                                  (static_cast<double>(m * k * n_tiles) + static_cast<double>(n * k * m_tiles) + static_cast<double>(m * n * splits));
-            const double traffic = bytes / kBytesPerUs;
+            const double traffic = bytes / bytes_per_us;
             if (traffic > cost) cost = traffic;
-            if (splits > 1) cost += kReduceFixed + static_cast<double>(m * n * (splits + 1)) * 4.0 / kReduceBytesPerUs;
+            if (splits > 1) cost += reduce_fixed + static_cast<double>(m * n * (splits + 1)) * 4.0 / reduce_bytes_per_us;
             consider(cost, splits, per, 1);
         }
     }
