@@ -330,7 +330,9 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) bf16_kernel(const __
 #pragma unroll 1
             for (uint32_t c0 = 0; c0 < static_cast<uint32_t>(T::COLUMNS); c0 += slab_columns) {
                 const uint32_t gn0 = w.n0 + first_col + c0;
-                if (gn0 >= w.n) break;  // the same for the whole warp
+                // The same for the whole warp. Rows below C are not drained either: with no store of their own
+                // behind them, the wait below would let them into the slab that the last store may still read.
+                if (gn0 >= w.n || !rows_inside) break;
                 char* const slab = my_slabs + (EPILOGUE == Epilogue::None ? (stores++ & 1u) * SLAB_BYTES : 0u);
                 if (args.c_tma) {
                     // The store that last read the slab (two turns ago, or the last) has finished reading it.
@@ -341,11 +343,9 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) bf16_kernel(const __
                     __syncwarp();
                 }
                 if constexpr (EPILOGUE == Epilogue::GeluGrad) {
-                    if (rows_inside) {
-                        alive = warp_wait<1>(beside_bar, besides & 1u, abort_flag, args.status);
-                        if (!alive) break;
-                        ++besides;
-                    }
+                    alive = warp_wait<1>(beside_bar, besides & 1u, abort_flag, args.status);
+                    if (!alive) break;
+                    ++besides;
                 }
                 if (half_out) {
 #pragma unroll
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) bf16_kernel(const __
                 if (args.c_tma) {
                     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
                     __syncwarp();
-                    if (lane == 0 && rows_inside) {
+                    if (lane == 0) {
                         store_tile(&maps.c[w.product], smem_u32(slab), gn0, first_row, w.splits > 1 ? 0u : w.z_inner, w.splits > 1 ? w.split : w.z_outer);
                         if (EPILOGUE == Epilogue::Gelu) store_tile(&maps.beside, smem_u32(slab + SLAB_BYTES), gn0, first_row, 0, 0);
                         // The warp has read its slab of the argument: the next one may land there.

@@ -40,6 +40,34 @@ def test_bf16_products_at_the_edges_of_their_tiles(device, m, n, k, form, half_o
     assert bool(((c.double() - want).abs() <= bound).all())
 
 
+# One k block a tile, so that a warp's rows below C (whose accumulator is zeros) come right behind the stores
+# of the tile before: the zeros must not reach a slab that such a store still reads. Every run the same bits.
+@pytest.mark.parametrize("m,n,k,form", [(2888, 34848, 32, "nn"), (656, 12064, 24, "nt"), (832, 30528, 64, "nt"), (5000, 12064, 32, "tn"), (72, 40064, 16, "nn")])
+@pytest.mark.parametrize("half_out", [False, True])
+def test_rows_below_the_result_leave_no_zeros_in_it(device, m, n, k, form, half_out):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    a = torch.randn((m, k), device="cuda", generator=gen).to(torch.bfloat16)
+    b = torch.randn((k, n), device="cuda", generator=gen).to(torch.bfloat16)
+    a_t, b_t = form[0] == "t", form[1] == "t"
+    d_a, d_b = (a.t() if a_t else a).contiguous(), (b.t() if b_t else b).contiguous()
+    want, size = a.double() @ b.double(), a.double().abs() @ b.double().abs()
+    bound = 1e-5 + 1e-4 * size + (2.0 ** -8 * want.abs() if half_out else 0.0)
+    L = M.lib()
+    need = L.msx_op_matmul_bf16_workspace(m, n, k)
+    ws = torch.empty(max(need, 1), device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    for _ in range(12):
+        c = torch.full((m, n), float("nan"), device="cuda", dtype=torch.bfloat16 if half_out else torch.float32)
+        torch.cuda.synchronize()
+        rc = L.msx_op_matmul_bf16(ptr(d_a), int(a_t), ptr(d_b), int(b_t), ptr(c), int(half_out), m, n, k, ptr(ws), need, ptr(status),
+                                  C.c_void_p(torch.cuda.current_stream().cuda_stream))
+        assert rc == M.OK, L.msx_last_error(None)
+        assert bool(((c.double() - want).abs() <= bound).all())
+    assert int(status.item()) == 0
+
+
 @pytest.mark.parametrize("shape", [dict(batch=3, seq=24, hidden=48, heads=2, ffn=72), dict(batch=11, seq=200, hidden=200, heads=5, ffn=712),
                                    dict(batch=40, seq=128, hidden=512, heads=8, ffn=2048)])
 def test_products_that_share_launches_against_the_f32_plan(device, shape):
