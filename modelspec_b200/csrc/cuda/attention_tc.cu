@@ -62,7 +62,9 @@ __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(fl
         total += x[i];
     }
     total = warp_sum(total);
-    // x / total: the product with the reciprocal, corrected by its own remainder.
+    // x / total, rounded once: with the rounded reciprocal, the quotient corrected by its exact remainder is the
+    // nearest one (Markstein, IBM J. Res. Dev. 34, 1990, theorem 8.2; total is between 1 and the number of keys. A
+    // quotient too small for its remainder to be exact is off by less than the smallest normal number).
     const float inverse = 1.0f / total;
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {

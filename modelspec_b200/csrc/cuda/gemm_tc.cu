@@ -711,8 +711,10 @@ MatmulTcPlan matmul_tc_job_plan(uint64_t m, uint64_t n, uint64_t k) {
     return p;
 }
 
-// (Up to this many microseconds of FMA work; unaligned jobs, which the 64 x 64 tiles would take, gain up
-// to twice that.)
+// Up to this many microseconds of FMA work. The tensor-core launch takes 8 us and 25 ns a row of the batch, the FMA
+// tiles 5 us and more than their work: below the limit they win (the jobs of two layers 64 wide over 256 rows 12.5 -> 8.0 us, over
+// 512 rows 16.9 -> 10.4). From 6 to 12 us of work they would win with more than about 350 rows (1,600: 49 -> 25 us) and lose
+// with fewer (320: 16 -> 20 us; 80: 10 -> 19).
 constexpr double kSmallJobsUs = 6.0;
 void matmul_tc_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, bool a_t, bool b_t, uint32_t* status) {
     if (count == 0) return;

@@ -582,8 +582,9 @@ bool matmul_tf32_batched(cudaStream_t s, const BatchedProduct* products, uint32_
         for (const BatchedOperand* x : {&products[g].a, &products[g].b, &products[g].c})
             if (!tma_addressable(*x)) return false;
     const uint64_t problems = static_cast<uint64_t>(outer) * inner;
-    // One product whose 64 x 32 tiles all find an SM of their own is 0.7 us sooner on those (16 heads of 128
-    // queries x 128 keys x 64: attention forward 12.9 -> 11.5 us); from two tiles to an SM on, or with two products
+    // One product whose 64 x 32 tiles all find an SM of their own is about a microsecond sooner on those, or as soon
+    // (eleven attentions of 16 to 144 such tiles a product, forward: 2 to 16 heads of 128 queries x 128 keys x 64 18.6 ->
+    // 16.6 us, 12 of 100 x 100 x 40 the same, the others of 32 to 512 keys within 1 us either way); from two tiles to an SM on, or with two products
     // to share a launch, these tiles win (64 such heads: forward 16.3 -> 14.9 us, backward 29.9 -> 21.0;
     // 384 heads of 512 x 512 x 64: forward 745 -> 414 us, backward 1,151 -> 643).
     if (count == 1 && (m + 63) / 64 * ((n + 31) / 32) * problems <= device_sm_count()) return false;

@@ -197,3 +197,40 @@ def test_fused_attention_and_its_gradients_against_the_oracle(device, batch, seq
     # A masked key takes no part: its dK and dV rows are zeros.
     dk = d_out[2].float().cpu().numpy()
     assert not dk[seq - 3:seq].any()
+
+
+# Every element against float64, with what bf16 storage can do to it: a probability and a score gradient are
+# rounded once (2^-9 of themselves, here 2^-8 for f32 sums and base-2 exponentials beside it), the row dot of O and g is
+# taken of the stored O, and a result is rounded once.
+@pytest.mark.parametrize("batch,seq,heads,d", [(2, 128, 2, 64), (1, 512, 3, 64), (2, 200, 2, 32), (3, 16, 2, 16), (1, 384, 1, 64), (2, 72, 3, 40)])
+def test_every_element_of_the_fused_attention_against_float64(device, batch, seq, heads, d):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(batch * 1000 + seq + heads + d)
+    h, rows = heads * d, batch * seq
+    t = {name: torch.randn((rows, h), device="cuda", generator=gen).to(torch.bfloat16) for name in "qkvg"}
+    mask = torch.ones((batch, seq), device="cuda")
+    mask[0, seq - 3:] = 0.0
+    out = [torch.full((rows, h), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+    stats = torch.zeros(rows * heads * 2, device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ptr = lambda x: C.c_void_p(x.data_ptr())
+    rc = M.lib().msx_op_attention_bf16(ptr(t["q"]), ptr(t["k"]), ptr(t["v"]), ptr(mask), ptr(t["g"]), ptr(out[0]), ptr(out[1]), ptr(out[2]), ptr(out[3]),
+                                       ptr(stats), batch, seq, seq, heads, d, ptr(status), None)
+    assert rc == M.OK, M.lib().msx_last_error(None).decode()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0
+    split = lambda x: x.double().reshape(batch, seq, heads, d).transpose(1, 2)
+    q, k, v, g = (split(t[name]) for name in "qkvg")
+    got_o, got_dq, got_dk, got_dv = (split(x) for x in out)
+    scale, turn = d ** -0.5, lambda x: x.transpose(-1, -2)
+    p = torch.softmax((q @ turn(k) * scale).masked_fill(mask[:, None, None, :] == 0.0, float("-inf")), dim=-1)
+    o = p @ v
+    ds = scale * p * (g @ turn(v) - (g * o).sum(-1, keepdim=True))
+    # What the rounding of the stored O moves ds by, and of ds itself.
+    off = scale * p * (g.abs() * o.abs()).sum(-1, keepdim=True) + ds.abs()
+    r = 2.0 ** -8
+    for name, got, want, moved in (("out", got_o, o, p @ v.abs()), ("dv", got_dv, turn(p) @ g, turn(p) @ g.abs()),
+                                   ("dq", got_dq, ds @ k, off @ k.abs()), ("dk", got_dk, turn(ds) @ q, turn(off) @ q.abs())):
+        ratio = float(((got - want).abs() / (r * moved + r * want.abs() + 1e-6)).max())
+        assert ratio <= 1.0, (name, ratio)

@@ -2,13 +2,14 @@
 tiles than the device holds at a time) against float64 products of the same operands, and the products
 of a mixed-precision step that share launches (projections as one launch, their input gradients summed
 as one product, weight gradients as jobs, gelu and its gradient as the tile drains) against the f32
-plan of the same run."""
+plan of the same run. gelu and its gradient are also held to float64, element by element."""
 import ctypes as C
 
 import numpy as np
 import pytest
 
 import modelspec_b200 as M
+from helpers import ProgramText
 from modelspec_b200 import models, synthetic
 
 pytestmark = pytest.mark.gpu
@@ -92,3 +93,53 @@ def test_products_that_share_launches_against_the_f32_plan(device, shape):
     finally:
         for run in runs:
             run.destroy()
+
+
+# One CTA and pairs, ragged rows and columns, several bands of tiles, more tiles than the device holds. The three
+# values are read through products with the identity, which are exact; the product in front of gelu_grad is not
+# stored, so its rounding to bf16 is in the bound: 2^-8 of the value for a rounding that fell the other way, and the
+# kernel tolerance of the f32 sum.
+@pytest.mark.parametrize("m,n,k", [(100, 72, 40), (200, 200, 48), (2200, 712, 200), (5000, 1032, 136), (4096, 3072, 768)])
+def test_every_element_of_gelu_and_its_gradient_as_a_tile_drains(device, m, n, k):
+    import torch
+    p = ProgramText()
+    k2 = k + 8  # a shape of its own: products of one shape would share a launch without an epilogue
+    sizes = {"t1": (m, k), "t2": (m, k2), "w1": (k, n), "w2": (k2, n), "eye": (n, n)}
+    at = {name: p.param(name, list(shape)) for name, shape in sizes.items()}
+    bias = p.param("bias", [n])
+    ids = p.input("ids", "i32", [m])
+    x, x2 = p.op("Embedding", [m, k], [at["t1"], ids]), p.op("Embedding", [m, k2], [at["t2"], ids])
+    z = p.op("AddRows", [m, n], [p.op("MatMul", [m, n], [x, at["w1"]]), bias])
+    y = p.op("Gelu", [m, n], [z])
+    d = p.op("GeluGrad", [m, n], [z, p.op("MatMul", [m, n], [x2, at["w2"]])])
+    outputs = [p.op("MatMul", [m, n], [value, at["eye"]]) for value in (z, y, d)]
+    for value in outputs:
+        p.output(value)
+    plan = M.Plan(device, p.text(), flags=M.PLAN_BF16)
+    try:
+        kernels = [plan_kernel for plan_kernel, _, _, _ in plan.profile_step()]
+        assert "matmul" in kernels and not any("gelu" in name for name in kernels), kernels
+        gen = torch.Generator(device="cuda").manual_seed(m + n + k)
+        half = {name: (torch.randn(shape, device="cuda", generator=gen) * (2.0 if name == "t1" else 1.0) * shape[0] ** (-0.5 if name[0] == "w" else 0.0)).to(torch.bfloat16)
+                for name, shape in sizes.items() if name != "eye"}
+        half["eye"] = torch.eye(n, device="cuda").to(torch.bfloat16)
+        b = torch.randn(n, device="cuda", generator=gen)
+        for i, (path, _) in enumerate(plan.params()):
+            plan.param_upload(i, (b if path == "bias" else half[path].float()).cpu().numpy())
+        plan.set_input("ids", np.arange(m, dtype=np.int32))
+        plan.run()
+        got_z, got_y, got_d = (torch.from_numpy(plan.value(value, m * n)).cuda().double().reshape(m, n) for value in outputs)
+        f = {name: value.double() for name, value in half.items()}
+        want_z, size = f["t1"] @ f["w1"] + b.double(), f["t1"].abs() @ f["w1"].abs() + b.double().abs()
+        assert bool(((got_z - want_z).abs() <= 2.0 ** -8 * want_z.abs() + 1e-5 + 1e-4 * size).all())
+        # Of the stored argument.
+        u = 0.7978845608028654 * (got_z + 0.044715 * got_z ** 3)
+        s = torch.sigmoid(2.0 * u)
+        slope = s + got_z * s * (1.0 - s) * 2.0 * 0.7978845608028654 * (1.0 + 3.0 * 0.044715 * got_z ** 2)
+        want_y = got_z * s
+        assert bool(((got_y - want_y).abs() <= 2.0 ** -8 * want_y.abs() + 1e-6).all())
+        g, size = f["t2"] @ f["w2"], f["t2"].abs() @ f["w2"].abs()
+        bound = slope.abs() * (2.0 ** -8 * g.abs() + 1e-5 + 1e-4 * size) + 2.0 ** -8 * (slope * g).abs() + 1e-6 * (1.0 + g.abs())
+        assert bool(((got_d - slope * g).abs() <= bound).all())
+    finally:
+        plan.destroy()
