@@ -55,10 +55,10 @@ constexpr int kStepEvents = 2 * kStagingSlots;
 constexpr uint64_t kDirectInputBytes = 64ull << 10;
 constexpr int kDeviceSlots = 2;
 static_assert(kStagingSlots <= k::kMostInputSlots && kDeviceSlots <= k::kMostInputSlots);
-// Up to here a plan's pinned slots are requests of their own, which fit the room left in the driver's 2 MB blocks
-// of pinned memory (eight of 200 KB: 20 us in a process that has such a block, 1.2 to 3 ms as one request);
-// beyond they are one block.
-constexpr uint64_t kPinnedApart = 2ull << 20;
+// A plan's pinned slots are one block, but between these sizes requests of their own, which fit the room left in
+// the driver's 2 MB blocks of pinned memory (eight of 200 KB: 20 us in a process that has such a block, 1.2 to 3 ms
+// as one request; eight of 64 KB: 7 us, as one request 1).
+constexpr uint64_t kPinnedApart[2] = {512ull << 10, 2ull << 20};
 
 uint64_t align_up(uint64_t x) { return (x + kAlign - 1) / kAlign * kAlign; }
 
@@ -166,13 +166,14 @@ struct msx_plan {
     char* state = nullptr;   // the parameters, moments and working copies this plan owns
     char* tables = nullptr;  // its inputs, their staging, constants, status, counters and job tables
     char* d_inputs = nullptr;
+    char* d_shared_inputs = nullptr;  // those of a plan that shares its parameters, made with its slots
     uint64_t input_bytes = 0;
     std::vector<char> blob;  // the staged inputs, host side
     bool blob_dirty = true;  // staged since the last upload
     msx::PinnedBlock pinned_together;
     char* pinned[kStagingSlots] = {};  // a slot of input_bytes each, pieces of pinned_together or requests of their own
     char* d_staging = nullptr;         // large inputs: kDeviceSlots slots on the device
-    cudaStream_t copy_stream = nullptr;  // fills them beside a running step; made when the first one does
+    cudaStream_t copy_stream = nullptr;  // fills them beside a running step
     cudaEvent_t copied[kDeviceSlots] = {};
     uint32_t* d_turn = nullptr;    // the slot of the step that runs next, kept by the step itself
     float* pinned_loss = nullptr;  // kStagingSlots floats
@@ -2407,20 +2408,31 @@ template <class T> cudaError_t plan_malloc(msx_plan* P, T** out, size_t bytes) {
 }
 
 // Where a plan's inputs wait for their step: its blob, its pinned slots and, where inputs are staged, its
-// slots on the device. A forward program that shares a step plan's parameters makes them when its first input is
-// set: a run has such a plan from its beginning and may never feed it.
+// slots on the device. A forward program that shares a step plan's parameters makes them, and the region on the
+// device that its launches read, when its first input is set: a run has such a plan from its beginning and may
+// never feed it. (An MLP of 200 KB a step: a run is made in 6.4 ms so, in 8.2 with the forward program's 200 KB on the
+// device beside the rest, which then takes one of the driver's 2 MB blocks more.)
 void make_input_slots(msx_plan* P) {
     if (!P->blob.empty()) return;
     const uint64_t bytes = std::max<uint64_t>(P->input_bytes, kAlign);
-    if (kStagingSlots * bytes > kPinnedApart) {
-        cuda_ok(P->pinned_together.make(kStagingSlots * bytes), "pinned memory (staging)");
+    const uint64_t all = kStagingSlots * bytes;
+    if (all <= kPinnedApart[0] || all > kPinnedApart[1]) {
+        cuda_ok(P->pinned_together.make(all), "pinned memory (staging)");
         for (int s = 0; s < kStagingSlots; ++s) P->pinned[s] = P->pinned_together.data() + s * bytes;
     } else {
         for (char*& slot : P->pinned)
             if (!slot) cuda_ok(cudaMallocHost(&slot, bytes), "cudaMallocHost(staging)");
     }
-    if (!P->shares && P->input_bytes > kDirectInputBytes && !P->d_staging)
+    if (!P->shares && P->input_bytes > kDirectInputBytes && !P->d_staging) {
+        cuda_ok(cudaStreamCreateWithFlags(&P->copy_stream, cudaStreamNonBlocking), "cudaStreamCreate");
+        for (cudaEvent_t& e : P->copied) cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         cuda_ok(plan_malloc(P, &P->d_staging, kDeviceSlots * bytes), "cudaMalloc(staging)");
+    }
+    if (!P->d_inputs) {  // (a plan with parameters of its own has them among its tables)
+        cuda_ok(plan_malloc(P, &P->d_shared_inputs, bytes), "cudaMalloc(inputs)");
+        cuda_ok(cudaMemsetAsync(P->d_shared_inputs, 0, bytes, P->stream), "cudaMemset(inputs)");
+        P->d_inputs = P->d_shared_inputs;
+    }
     P->blob.assign(bytes, 0);
 }
 
@@ -2503,7 +2515,7 @@ void allocate(msx_plan* P, const Scheduler& sched) {
     const uint64_t tensor_bytes = sched.updates.size() * sizeof(k::UpdateTensor), chunk_bytes = sched.update_chunk_tensor.size() * 4;
     {
         const std::pair<void**, uint64_t> pieces[] = {
-            {reinterpret_cast<void**>(&P->d_inputs), in_bytes},
+            {reinterpret_cast<void**>(&P->d_inputs), P->shares ? 0 : in_bytes},
             {reinterpret_cast<void**>(&P->d_consts), const_bytes},
             {reinterpret_cast<void**>(&P->d_status), 8},
             {reinterpret_cast<void**>(&P->d_counters), counter_bytes},
@@ -2627,6 +2639,7 @@ void release(msx_plan* P) {
     if (P->backup) cudaFree(P->backup);
     if (P->pinned_loss) cudaFreeHost(P->pinned_loss);
     if (P->d_staging) cudaFree(P->d_staging);
+    if (P->d_shared_inputs) cudaFree(P->d_shared_inputs);
     if (!P->pinned_together.data())
         for (char* slot : P->pinned)
             if (slot) cudaFreeHost(slot);
@@ -2875,11 +2888,6 @@ void stage_inputs(msx_plan* P, int slot, bool idle) {
     if (idle) {
         cuda_ok(cudaMemcpyAsync(to, P->pinned[slot], P->input_bytes, cudaMemcpyHostToDevice, P->stream), "cudaMemcpyAsync(inputs)");
         return;
-    }
-    if (!P->copy_stream) {
-        for (cudaEvent_t& e : P->copied)
-            if (!e) cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
-        cuda_ok(cudaStreamCreateWithFlags(&P->copy_stream, cudaStreamNonBlocking), "cudaStreamCreate");
     }
     // The slot on the device is free once the step that last used it has run.
     if (P->steps >= kDeviceSlots)

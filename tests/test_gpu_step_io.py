@@ -41,10 +41,11 @@ def test_every_step_runs_on_the_inputs_staged_for_it(device, n, flags):
         plan.destroy()
 
 
-# Read in place, staged, at eight pinned slots of 2 MB in all and one beyond, 8 MB; a plan of its own, and one that
+# One float, below and above the 64 KB that are read in place (and the eight pinned slots one request), eight slots of
+# 2 MB in all and one beyond, 8 MB; a plan of its own, and one that
 # shares another's parameters and so reads in place whatever the size. Steps waited for one by one, then
 # steps submitted behind one another, then waited for again, some on what is staged already.
-@pytest.mark.parametrize("n", [16384 - 64, 16384 + 1, 65536, 65536 + 64, 2100001])
+@pytest.mark.parametrize("n", [1, 8192 - 64, 8192, 16384 + 1, 32768, 32768 + 64, 2100001])
 @pytest.mark.parametrize("shared", [False, True])
 def test_large_inputs_of_steps_waited_for_and_of_steps_behind_one_another(device, n, shared):
     p = ProgramText()
@@ -59,8 +60,10 @@ def test_large_inputs_of_steps_waited_for_and_of_steps_behind_one_another(device
     zeros = np.zeros(n, dtype=np.float32)
     mean_square = [float(np.mean(np.square(v, dtype=np.float64))) for v in values]
     try:
+        plan.run()  # on nothing set: zeros
+        want, k, last = [0.0], 1, 0.0
+        assert plan.loss_of(0) == 0.0
         plan.set_input("b", zeros)
-        want, k = [], 0
         for burst in (1, 1, 5, 1, 11, 2, 1):
             for _ in range(burst):
                 if k % 4 != 3:
