@@ -51,7 +51,8 @@ constexpr int kStepEvents = 2 * kStagingSlots;
 // the device beside the step before: an MLP of 200 KB a step takes 48 us so against 54 read in place, a transformer
 // block of 1 MB 280 against 302. With no step to run beside, the copy stays on the plan's own stream (8 MB a step,
 // read back at once: the same 2.1 ms without staging; a second stream only adds its waits). Forward programs,
-// which share a step plan's parameters, are waited for and read theirs in place.
+// which share a step plan's parameters, are waited for and read theirs in place, but for the one a held-out
+// split goes through.
 constexpr uint64_t kDirectInputBytes = 64ull << 10;
 constexpr int kDeviceSlots = 2;
 static_assert(kStagingSlots <= k::kMostInputSlots && kDeviceSlots <= k::kMostInputSlots);
@@ -2412,7 +2413,7 @@ template <class T> cudaError_t plan_malloc(msx_plan* P, T** out, size_t bytes) {
 // device that its launches read, when its first input is set: a run has such a plan from its beginning and may
 // never feed it. (An MLP of 200 KB a step: a run is made in 6.4 ms so, in 8.2 with the forward program's 200 KB on the
 // device beside the rest, which then takes one of the driver's 2 MB blocks more.)
-void make_input_slots(msx_plan* P) {
+void make_input_slots(msx_plan* P, bool behind_its_own_steps = false) {
     if (!P->blob.empty()) return;
     const uint64_t bytes = std::max<uint64_t>(P->input_bytes, kAlign);
     const uint64_t all = kStagingSlots * bytes;
@@ -2423,7 +2424,7 @@ void make_input_slots(msx_plan* P) {
         for (char*& slot : P->pinned)
             if (!slot) cuda_ok(cudaMallocHost(&slot, bytes), "cudaMallocHost(staging)");
     }
-    if (!P->shares && P->input_bytes > kDirectInputBytes && !P->d_staging) {
+    if ((!P->shares || behind_its_own_steps) && P->input_bytes > kDirectInputBytes && !P->d_staging) {
         cuda_ok(cudaStreamCreateWithFlags(&P->copy_stream, cudaStreamNonBlocking), "cudaStreamCreate");
         for (cudaEvent_t& e : P->copied) cuda_ok(cudaEventCreateWithFlags(&e, cudaEventDisableTiming), "cudaEventCreate");
         cuda_ok(plan_malloc(P, &P->d_staging, kDeviceSlots * bytes), "cudaMalloc(staging)");
@@ -3457,7 +3458,7 @@ int msx_heldout_create(msx_plan* plan, uint32_t logits, uint32_t batches, msx_he
             throw StatusError(MSX_BAD_ARGUMENT, "msx_heldout_create: %" + std::to_string(logits) + " is not an f32 output of the plan");
         if (batches == 0) throw StatusError(MSX_BAD_ARGUMENT, "msx_heldout_create: no batches");
         cuda_ok(cudaSetDevice(plan->device->ordinal), "cudaSetDevice");
-        make_input_slots(plan);
+        make_input_slots(plan, true);  // (its batches follow one another)
         std::unique_ptr<msx_heldout> h(new msx_heldout());
         h->plan = plan;
         h->at = static_cast<uint32_t>(at);

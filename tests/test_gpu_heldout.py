@@ -219,3 +219,33 @@ def test_a_prediction_that_is_not_logits_per_label_is_refused(device):
             gpu.heldout_begin(1, "y", "y")
     finally:
         gpu.destroy()
+
+
+# Batches of less and of more than the 64 KB of inputs a step reads in place: beyond, a batch is brought to the
+# device beside the evaluation of the one before. The predictions are the same ones, read back one by one.
+@pytest.mark.parametrize("batch,seq", [(16, 96), (64, 128)])
+def test_batches_behind_one_another_evaluate_as_their_predictions_do(device, batch, seq):
+    vocab, batches = 300, 5
+    source = models.bert(layers=1, hidden=32, heads=2, ffn=64, vocab=vocab, seq=seq, batch=batch, steps=3, warmup_steps=1)
+    run = M.Training(device, source, models.default_masked_rows(batch * seq))
+    held = [synthetic.mlm_batch(b, vocab=vocab, seq=seq, batch=batch) for b in range(batches)]
+    try:
+        run.heldout_begin(batches, "labels", "weights")
+        numerator, correct, denominator, selected = 0.0, 0, 0.0, 0
+        for b, tensors in enumerate(held):
+            for name, value in tensors.items():
+                run.heldout_set(b, name, value)
+                run.set_input(name, value)
+            logits = run.infer()[0].reshape(-1, vocab).astype(np.float64)
+            labels, weights = tensors["labels"], tensors["weights"].astype(np.float64)
+            top = logits.max(axis=1)
+            numerator += float((weights * (top + np.log(np.exp(logits - top[:, None]).sum(axis=1)) - logits[np.arange(len(labels)), labels])).sum())
+            correct += int(((logits.argmax(axis=1) == labels) & (weights > 0)).sum())
+            denominator += float(weights.sum())
+            selected += int((weights > 0).sum())
+        for _ in range(2):
+            loss, accuracy = run.heldout_evaluate()
+            assert close(float(loss) * denominator, numerator, denominator)
+            assert abs(float(accuracy) * selected - correct) <= 0.5
+    finally:
+        run.destroy()
