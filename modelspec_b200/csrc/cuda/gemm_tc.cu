@@ -584,6 +584,7 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
         {Rows64, 64, 64, 3.5, 0.47, 0.38, 296.0},
         {Rows64, 64, 128, 3.5, 0.80, 0.45, 296.0},
     };
+    constexpr uint64_t kDeepest = 96;
     const uint64_t kblocks = (k + BK - 1) / BK;
     MatmulTcPlan best = {};
     double best_cost = 0.0;
@@ -623,6 +624,9 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
                 const double paired = waves * (c.fixed + static_cast<double>(per) * c.block);
                 const double streamed = std::ceil(static_cast<double>(tiles * splits) / 148.0) * static_cast<double>(per) * c.tile;
                 cost = paired > streamed ? paired : streamed;
+                // These tiles sum their k in tensor memory, which truncates: no deeper than 96 k blocks (7e-6 of a
+                // product's norm; 139 in one sum 1.1e-5) where k can be split.
+                if (per > kDeepest && most > 1) cost *= 4.0;
             }
             // Every tile reads its rows of A and columns of B over k.
             const double bytes = 4.0 * static_cast<double>(problems * group) *

@@ -51,7 +51,7 @@ def test_f32_products_at_the_edges_of_their_kernels(device, m, n, k, form):
 # a whole unit in the last place, half of it on average (a sum of 256 k blocks was 2.8e-5 low). The last two have rows TMA cannot address: a
 # sum of 85 k blocks on the 64-row tiles was 9.0e-6 low.
 @pytest.mark.parametrize("m,n,k", [(768, 3072, 16384), (3072, 768, 16384), (768, 768, 16384), (396, 1024, 60000), (96, 64, 20000), (4096, 260, 9001),
-                                   (429, 1281, 16384), (771, 771, 32001)])
+                                   (429, 1281, 16384), (771, 771, 32001), (1567, 1162, 4455), (33, 29, 200001)])
 def test_deep_weight_gradients_do_not_come_out_low(device, m, n, k):
     import torch
     gen = torch.Generator(device="cuda").manual_seed(m + 3 * n + 7 * k)
