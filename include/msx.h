@@ -157,11 +157,12 @@ int msx_loss(msx_plan* plan, float* loss, uint32_t timeout_ms);
 int msx_loss_of(msx_plan* plan, uint64_t step_number, float* loss, uint32_t timeout_ms);
 uint64_t msx_steps_submitted(const msx_plan* plan);
 
-/* Device time of submitted step `step_number` in milliseconds, between CUDA events recorded on
- * the plan's stream before its input copy and after its loss read-back; the last 8 submitted
- * steps keep theirs. With steps submitted back to back these times add up to the run's: the
- * per-step view of the reference's training clock (cli/src/train.rs:17-33), from which a host
- * takes the median step time the reference's benchmarks quote (vulkan/profile.rs:25). */
+/* Device time of submitted step `step_number` in milliseconds, up to a CUDA event on the plan's
+ * stream behind its last kernel: from the end of the step before it, or, where it was submitted on an
+ * idle stream, from an event in front of its inputs; the last 8 submitted steps keep theirs. With
+ * steps submitted back to back these times add up to the run's: the per-step view of the reference's
+ * training clock (cli/src/train.rs:17-33), from which a host takes the median step time the
+ * reference's benchmarks quote (vulkan/profile.rs:25). */
 int msx_step_ms(msx_plan* plan, uint64_t step_number, float* ms);
 
 /* Waits for every submitted step. */
