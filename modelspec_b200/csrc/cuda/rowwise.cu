@@ -286,18 +286,17 @@ __global__ void cross_entropy_fused_kernel(const T* __restrict__ logits, const i
 // tolerance class every exp-based kernel is in), with one reciprocal of the row sum instead of a
 // division per element: 30,522 exps and divisions per row are otherwise as long as the row's
 // memory traffic.
-// VEC = 4 reads and writes 16 bytes per thread (row pitches that are multiples of 4 floats).
+// For rows that no 16-byte access can be made on; every other row takes one of the kernels below.
 constexpr int kWideThreads = 1024, kWideItems = 32;
-template <int VEC, class T>
+template <class T>
 __global__ void __launch_bounds__(kWideThreads, 1)
 cross_entropy_fused_wide_kernel(const T* __restrict__ logits, const int32_t* __restrict__ labels,
                                 const float* __restrict__ weights, const float* __restrict__ g,
                                 const float* __restrict__ denominator, float* __restrict__ row_loss,
                                 T* __restrict__ out, uint32_t v, uint32_t ld, uint32_t ld_out,
                                 uint32_t* __restrict__ counter, float* __restrict__ loss) {
-    // Element i of this thread is column column_of(i): consecutive threads take consecutive
-    // (groups of VEC) columns.
-    auto column_of = [](int i, uint32_t tid) { return (static_cast<uint32_t>(i / VEC) * kWideThreads + tid) * VEC + i % VEC; };
+    // Element i of this thread is column column_of(i): consecutive threads take consecutive columns.
+    auto column_of = [](int i, uint32_t tid) { return static_cast<uint32_t>(i) * kWideThreads + tid; };
     __shared__ float shared[33];
     __shared__ double shared64[33];
     __shared__ bool is_last;
@@ -321,20 +320,10 @@ cross_entropy_fused_wide_kernel(const T* __restrict__ logits, const int32_t* __r
         if (tid == 0) row_loss[r] = 0.0f;
     } else {
         const T* row = logits + static_cast<uint64_t>(r) * ld;
-        if (VEC == 4) {
-            // Unconditional loads from a clamped column (the pitch covers the whole float4 of the
-            // last valid column), so that all eight are in flight together; what lies past v is
-            // replaced afterwards.
-            const uint32_t last = (v - 1) & ~3u;
+        // Unconditional loads from a clamped column, so that all are in flight together; what lies past v
+        // is replaced afterwards.
 #pragma unroll
-            for (int i = 0; i < kWideItems; i += 4) {
-                const float4 f = load4(row + min(column_of(i, tid), last));
-                x[i] = f.x; x[i + 1] = f.y; x[i + 2] = f.z; x[i + 3] = f.w;
-            }
-        } else {
-#pragma unroll
-            for (int i = 0; i < kWideItems; ++i) x[i] = load1(row + min(column_of(i, tid), v - 1));
-        }
+        for (int i = 0; i < kWideItems; ++i) x[i] = load1(row + min(column_of(i, tid), v - 1));
 #pragma unroll
         for (int i = 0; i < kWideItems; ++i)
             if (column_of(i, tid) >= v) x[i] = -INFINITY;
@@ -388,38 +377,203 @@ cross_entropy_fused_wide_kernel(const T* __restrict__ logits, const int32_t* __r
         const float target = c == label ? 1.0f : 0.0f;
         x[i] = zero ? 0.0f : scale * (x[i] * inverse - target);
     }
-    if (VEC == 4) {
 #pragma unroll
-        for (int i = 0; i < kWideItems; i += 4) {
-            const uint32_t c = column_of(i, tid);
-            // Columns past v inside the pitch are padding nobody reads: the whole float4 is written.
-            if (c < v) store4(o + c, make_float4(x[i], x[i + 1], x[i + 2], x[i + 3]));
-        }
-    } else {
-#pragma unroll
-        for (int i = 0; i < kWideItems; ++i) {
-            const uint32_t c = column_of(i, tid);
-            if (c < v) store1(o + c, x[i]);
-        }
+    for (int i = 0; i < kWideItems; ++i) {
+        const uint32_t c = column_of(i, tid);
+        if (c < v) store1(o + c, x[i]);
     }
 }
 
 inline uint32_t warp_row_blocks(uint64_t rows) { return static_cast<uint32_t>((rows + kWarpsPerBlock - 1) / kWarpsPerBlock); }
 
-// The same for rows of 16-byte pitch, as two blocks per SM: 512 threads hold 32 elements each in
+// A row's 16-byte pieces as a thread holds them: f32 values in place, bf16 ones packed as they were read.
+__device__ __forceinline__ float4 as_floats(const uint4& v) {
+    return make_float4(__uint_as_float(v.x), __uint_as_float(v.y), __uint_as_float(v.z), __uint_as_float(v.w));
+}
+__device__ __forceinline__ float bf16_low(uint32_t pair) { return __uint_as_float(pair << 16); }
+__device__ __forceinline__ float bf16_high(uint32_t pair) { return __uint_as_float(pair & 0xffff0000u); }
+
+// The same for rows on 16-byte boundaries: THREADS threads hold a row in GROUPS pieces of 16 bytes each, ROWS
+// such rows a block (more than one only as a warp a row, which then needs no barrier for its row).
+//
+// Bound for long rows by their one read and one write, for short ones by the chain of dependent steps of a
+// row. So one barrier serves the row's maximum and the weight sum, one the row's sum, each warp adds the
+// warps' shares up for itself, and the atomic that finds the last block is not waited for before the
+// gradient is written. bf16 pieces stay packed (half the registers: two blocks of 512 threads an SM hold
+// rows of 32,768, so that one block's loads and stores run under the other's reductions), and their
+// exponentials are taken twice rather than kept as f32.
+// A launch (with what launching costs): 64 x 10 f32 12.6 -> 6.5 us, 96 x 1,009 f32 12.6 -> 6.5, 384 x 5,003 bf16
+// 24.9 -> 10.6, 832 x 30,522 bf16 47.6 -> 32.4, 2,880 x 30,522 bf16 177 -> 107 (a 1,024-thread block a row before).
+template <int THREADS, int ROWS, int GROUPS, int BLOCKS, class T>
+__global__ void __launch_bounds__(THREADS * ROWS, BLOCKS)
+cross_entropy_row_kernel(const T* __restrict__ logits, const int32_t* __restrict__ labels, const float* __restrict__ weights,
+                         const float* __restrict__ g, const float* __restrict__ denominator, float* __restrict__ row_loss,
+                         T* __restrict__ out, uint32_t rows, uint32_t v, uint32_t ld, uint32_t ld_out, uint32_t* __restrict__ counter,
+                         float* __restrict__ loss) {
+    static_assert(ROWS == 1 || THREADS == 32);
+    constexpr bool HALF = sizeof(T) == 2;
+    constexpr uint32_t E = 16 / sizeof(T), ALL = THREADS * ROWS, WARPS = ALL / 32;
+    __shared__ float shared_max[WARPS], shared_sum[WARPS];
+    __shared__ double shared_weight[WARPS];
+    __shared__ bool is_last;
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5, t = ROWS > 1 ? lane : tid;
+    const uint32_t r = blockIdx.x * ROWS + (ROWS > 1 ? warp : 0);
+    auto column_of = [t](int k) { return (static_cast<uint32_t>(k) * THREADS + t) * E; };
+    const bool here = r < rows;
+    const float w = here ? weights[r] : 0.0f;
+    const uint32_t label = here ? static_cast<uint32_t>(labels[r]) : 0u;
+    const T* row = logits + static_cast<uint64_t>(r) * ld;
+    // Unconditional loads from a clamped column (the pitch covers the whole piece of the last valid column), so
+    // that all are in flight together. A row of weight 0 is not read.
+    uint4 x[GROUPS];
+    float picked = 0.0f;
+    if (w != 0.0f) {
+        const uint32_t last = (v - 1) / E * E;
+#pragma unroll
+        for (int k = 0; k < GROUPS; ++k) x[k] = __ldg(reinterpret_cast<const uint4*>(row + min(column_of(k), last)));
+        if (t == 0 && label < v) picked = load1(row + label);
+    }
+    // The weight sum: given (the whole batch's, data parallel), or summed here by every block in the same
+    // order (f64, one rounding), so that no launch has to precede this one.
+    double weight = 0.0;
+    if (denominator == nullptr)
+        for (uint32_t j = tid; j < rows; j += ALL) weight += static_cast<double>(weights[j]);
+    float m = -INFINITY;
+    if (w != 0.0f) {
+        if constexpr (HALF) {
+            const uint32_t none = 0xff80ff80u;  // a pair of -inf
+            __nv_bfloat162 best = *reinterpret_cast<const __nv_bfloat162*>(&none);
+#pragma unroll
+            for (int k = 0; k < GROUPS; ++k) {
+                uint32_t* pair = &x[k].x;
+                const uint32_t c = column_of(k);
+                if (c + E > v) {
+#pragma unroll
+                    for (uint32_t i = 0; i < 4; ++i) {
+                        if (c + 2 * i >= v) pair[i] = none;
+                        else if (c + 2 * i + 1 >= v) pair[i] = (pair[i] & 0xffffu) | (none & 0xffff0000u);
+                    }
+                }
+#pragma unroll
+                for (int i = 0; i < 4; ++i) best = __hmax2(best, *reinterpret_cast<const __nv_bfloat162*>(&pair[i]));
+            }
+            const uint32_t both = *reinterpret_cast<const uint32_t*>(&best);
+            m = fmaxf(bf16_low(both), bf16_high(both));
+        } else {
+#pragma unroll
+            for (int k = 0; k < GROUPS; ++k) {
+                uint32_t* one = &x[k].x;
+#pragma unroll
+                for (uint32_t i = 0; i < 4; ++i) {
+                    if (column_of(k) + i >= v) one[i] = 0xff800000u;
+                    m = fmaxf(m, __uint_as_float(one[i]));
+                }
+            }
+        }
+        m = warp_max(m);
+    }
+    weight = warp_sum(weight);
+    if (lane == 0) {
+        shared_weight[warp] = weight;
+        if (ROWS == 1) shared_max[warp] = m;
+    }
+    __syncthreads();
+    if (ROWS == 1) m = warp_max(lane < WARPS ? shared_max[lane] : -INFINITY);
+    float total = 0.0f;
+    if (w != 0.0f) {
+        // exp(-inf) is 0: the columns past the row's end add nothing.
+#pragma unroll
+        for (int k = 0; k < GROUPS; ++k) {
+            if constexpr (HALF) {
+                const uint32_t* pair = &x[k].x;
+                float part = 0.0f;
+#pragma unroll
+                for (int i = 0; i < 4; ++i) part += __expf(bf16_low(pair[i]) - m) + __expf(bf16_high(pair[i]) - m);
+                total += part;
+            } else {
+                const float4 f = as_floats(x[k]);
+                const float4 e = make_float4(__expf(f.x - m), __expf(f.y - m), __expf(f.z - m), __expf(f.w - m));
+                total += (e.x + e.y) + (e.z + e.w);
+                x[k] = make_uint4(__float_as_uint(e.x), __float_as_uint(e.y), __float_as_uint(e.z), __float_as_uint(e.w));
+            }
+        }
+        total = warp_sum(total);
+    }
+    if (ROWS == 1 && WARPS > 1) {
+        if (lane == 0) shared_sum[warp] = total;
+        __syncthreads();
+        total = warp_sum(lane < WARPS ? shared_sum[lane] : 0.0f);
+    }
+    weight = denominator != nullptr ? static_cast<double>(denominator[0]) : warp_sum(lane < WARPS ? shared_weight[lane] : 0.0);
+    const float den = static_cast<float>(weight);
+    if (t == 0 && here) row_loss[r] = w == 0.0f ? 0.0f : m + logf(total) - picked;
+    // Which block finishes the loss: only the row losses have to be visible to it, so only their writers
+    // fence, and the answer is not needed before the gradient's stores are on their way.
+    uint32_t before = 0;
+    if (ROWS > 1) {
+        if (lane == 0) __threadfence();
+        __syncthreads();
+    } else if (tid == 0) {
+        __threadfence();
+    }
+    if (tid == 0) before = atomicAdd(counter, 1u);
+    const bool zero = den == 0.0f || w == 0.0f;
+    const float scale = zero ? 0.0f : g[0] * w / den, inverse = zero ? 0.0f : 1.0f / total, both = scale * inverse;
+    T* o = out + static_cast<uint64_t>(r) * ld_out;
+#pragma unroll
+    for (int k = 0; k < GROUPS; ++k) {
+        const uint32_t c = column_of(k);
+        float e[E];
+#pragma unroll
+        for (uint32_t i = 0; i < E; ++i) {
+            const uint32_t bits = (&x[k].x)[HALF ? i / 2 : i];
+            e[i] = !HALF ? __uint_as_float(bits) : __expf((i % 2 ? bf16_high(bits) : bf16_low(bits)) - m);
+        }
+        // scale (p - 1) at the label, scale p elsewhere.
+        const bool has_label = label - c < E;
+        const uint32_t at = label - c;
+#pragma unroll
+        for (uint32_t i = 0; i < E; ++i) {
+            if (has_label && i == at) e[i] = zero ? 0.0f : scale * (e[i] * inverse - 1.0f);
+            else e[i] = zero ? 0.0f : e[i] * both;
+        }
+        if (here && c < v) {
+            // Columns past v inside the pitch are padding nobody reads: the whole piece is written.
+            if constexpr (HALF) store8(reinterpret_cast<bf16*>(o) + c, {make_float4(e[0], e[1], e[2], e[3]), make_float4(e[4], e[5], e[6], e[7])});
+            else store4(o + c, make_float4(e[0], e[1], e[2], e[3]));
+        }
+    }
+    if (tid == 0) {
+        is_last = before + 1u == gridDim.x;
+        if (is_last) *counter = 0u;
+    }
+    __syncthreads();
+    if (!is_last) return;
+    // The loss: sum of w * l over sum of w, f64 sums, one rounding.
+    __threadfence();
+    double num = 0.0;
+    for (uint32_t j = tid; j < rows; j += ALL) num = fma(static_cast<double>(weights[j]), static_cast<double>(__ldcg(row_loss + j)), num);
+    num = warp_sum(num);
+    if (lane == 0) shared_weight[warp] = num;
+    __syncthreads();
+    num = warp_sum(lane < WARPS ? shared_weight[lane] : 0.0);
+    if (tid == 0) loss[0] = weight == 0.0 ? 0.0f : static_cast<float>(num / weight);
+}
+
+// The same for f32 rows of more than 16,384 logits, as two blocks per SM: 512 threads hold 32 elements each in
 // registers and up to 32 more in shared memory (64 KB a block), so that one block's loads and
-// stores run under the other's reductions and exponentials. Elements bound for shared memory go
+// stores run under the other's reductions and exponentials. Rows of more than 32,768 take 1,024 threads. Elements bound for shared memory go
 // there straight from global memory (cp.async, 16 bytes), all in flight with the register loads;
 // every thread reads back only what it copied itself.
-constexpr int kSplitThreads = 512, kSplitRegisterItems = 32, kSplitSharedItems = 32;
-constexpr int kSplitSharedBytes = kSplitSharedItems * kSplitThreads * 4;
-__global__ void __launch_bounds__(kSplitThreads, 2)
+constexpr int kSplitRegisterItems = 32, kSplitSharedItems = 32;
+template <int kSplitThreads>
+__global__ void __launch_bounds__(kSplitThreads, 1024 / kSplitThreads)
 cross_entropy_fused_split_kernel(const float* __restrict__ logits, const int32_t* __restrict__ labels,
                                  const float* __restrict__ weights, const float* __restrict__ g,
                                  const float* __restrict__ denominator, float* __restrict__ row_loss,
                                  float* __restrict__ out, uint32_t v, uint32_t ld, uint32_t ld_out,
                                  uint32_t* __restrict__ counter, float* __restrict__ loss) {
-    // Group k of this thread is the four columns from (k * 512 + tid) * 4 on: groups 0..7 live in
+    // Group k of this thread is the four columns from (k * threads + tid) * 4 on: groups 0..7 live in
     // registers, groups 8..15 in shared memory.
     extern __shared__ float4 parked[];  // [kSplitSharedItems / 4][kSplitThreads]
     __shared__ float shared[33];
@@ -924,34 +1078,41 @@ __global__ void __launch_bounds__(256, ITEMS >= 16 ? 2 : 1) layer_norm_backward_
     }
 }
 
-// The one-read kernels: f32 rows of more than 16,384 logits with a 16-byte pitch as two 512-thread
-// blocks per SM, every other case as one 1,024-thread block with the row in registers.
-void launch_cross_entropy_one_read(cudaStream_t s, const float* logits, const int32_t* labels, const float* weights, const float* g,
-                                   const float* den, float* row_loss, float* grad, uint32_t vv, uint32_t l1, uint32_t l2, uint32_t* counter,
-                                   float* loss, uint64_t rows, bool vec) {
-    if (vec && vv > 16384) {
-        static std::atomic<int> configured_device{-1};
-        set_shared_memory(cross_entropy_fused_split_kernel, kSplitSharedBytes, configured_device);
-        cross_entropy_fused_split_kernel<<<static_cast<uint32_t>(rows), kSplitThreads, kSplitSharedBytes, s>>>(logits, labels, weights, g, den,
-                                                                                                              row_loss, grad, vv, l1, l2,
-                                                                                                              counter, loss);
-    } else if (vec) {
-        cross_entropy_fused_wide_kernel<4><<<static_cast<uint32_t>(rows), kWideThreads, 0, s>>>(logits, labels, weights, g, den, row_loss,
-                                                                                                grad, vv, l1, l2, counter, loss);
-    } else {
-        cross_entropy_fused_wide_kernel<1><<<static_cast<uint32_t>(rows), kWideThreads, 0, s>>>(logits, labels, weights, g, den, row_loss,
-                                                                                                grad, vv, l1, l2, counter, loss);
+// The one-read kernels. Rows on 16-byte boundaries: a warp a row up to 1,024 logits (a row's maximum and sum without a
+// barrier), then the fewest threads that hold the row in 32 registers each, so that more rows share an SM (f32 beyond 16,384: half of it in shared memory). Other rows: 1,024 threads, an element a load.
+constexpr uint64_t kWideRow = static_cast<uint64_t>(kWideThreads) * kWideItems, kLongestRow = 65536;
+template <class T>
+void launch_cross_entropy_one_read(cudaStream_t s, const T* logits, const int32_t* labels, const float* weights, const float* g,
+                                   const float* den, float* row_loss, T* grad, uint32_t vv, uint32_t l1, uint32_t l2, uint32_t* counter,
+                                   float* loss, uint32_t rows, bool vec) {
+    constexpr bool HALF = sizeof(T) == 2;
+    if (!vec) {
+        cross_entropy_fused_wide_kernel<<<rows, kWideThreads, 0, s>>>(logits, labels, weights, g, den, row_loss, grad, vv, l1, l2, counter, loss);
+        return;
     }
-}
-void launch_cross_entropy_one_read(cudaStream_t s, const bf16* logits, const int32_t* labels, const float* weights, const float* g,
-                                   const float* den, float* row_loss, bf16* grad, uint32_t vv, uint32_t l1, uint32_t l2, uint32_t* counter,
-                                   float* loss, uint64_t rows, bool vec) {
-    if (vec)
-        cross_entropy_fused_wide_kernel<4><<<static_cast<uint32_t>(rows), kWideThreads, 0, s>>>(logits, labels, weights, g, den, row_loss,
-                                                                                                grad, vv, l1, l2, counter, loss);
-    else
-        cross_entropy_fused_wide_kernel<1><<<static_cast<uint32_t>(rows), kWideThreads, 0, s>>>(logits, labels, weights, g, den, row_loss,
-                                                                                                grad, vv, l1, l2, counter, loss);
+    constexpr int G = HALF ? 4 : 8;  // pieces of 16 bytes that hold 32 elements
+    auto rows_in_registers = [&](auto kernel, uint32_t threads, uint32_t rows_a_block) {
+        kernel<<<(rows + rows_a_block - 1) / rows_a_block, threads * rows_a_block, 0, s>>>(logits, labels, weights, g, den, row_loss, grad, rows, vv,
+                                                                                           l1, l2, counter, loss);
+    };
+    if (vv <= 128) rows_in_registers(cross_entropy_row_kernel<32, 4, 1, 1, T>, 32, 4);
+    else if (vv <= 1024) rows_in_registers(cross_entropy_row_kernel<32, 4, G, 1, T>, 32, 4);
+    else if (vv <= 4096) rows_in_registers(cross_entropy_row_kernel<128, 1, G, 1, T>, 128, 1);
+    else if (vv <= 8192) rows_in_registers(cross_entropy_row_kernel<256, 1, G, 1, T>, 256, 1);
+    else if (vv <= 16384) rows_in_registers(cross_entropy_row_kernel<512, 1, G, 2, T>, 512, 1);
+    else if constexpr (HALF) {
+        if (vv <= 32768) rows_in_registers(cross_entropy_row_kernel<512, 1, 8, 2, T>, 512, 1);
+        else rows_in_registers(cross_entropy_row_kernel<1024, 1, 8, 1, T>, 1024, 1);
+    } else {
+        auto split = [&](auto kernel, int threads, std::atomic<int>& configured_device) {
+            const int bytes = kSplitSharedItems * threads * 4;
+            set_shared_memory(kernel, bytes, configured_device);
+            kernel<<<rows, threads, bytes, s>>>(logits, labels, weights, g, den, row_loss, grad, vv, l1, l2, counter, loss);
+        };
+        static std::atomic<int> half_device{-1}, whole_device{-1};
+        if (vv <= 32768) split(cross_entropy_fused_split_kernel<512>, 512, half_device);
+        else split(cross_entropy_fused_split_kernel<1024>, 1024, whole_device);
+    }
 }
 
 uint32_t backward_chunks(uint64_t rows, uint64_t h) {
@@ -1176,10 +1337,12 @@ void launch_cross_entropy_with_grad(cudaStream_t s, const T* logits, const int32
                                     bool denominator_ready, float* denominator, float* row_loss, float* loss, T* grad, uint64_t rows,
                                     uint64_t v, uint32_t* counter, uint64_t ld, uint64_t ld_grad) {
     const uint32_t vv = static_cast<uint32_t>(v), l1 = static_cast<uint32_t>(ld), l2 = static_cast<uint32_t>(ld_grad);
-    if (rows > 0 && counter != nullptr && v <= static_cast<uint64_t>(kWideThreads) * kWideItems) {
+    constexpr uint64_t E = 16 / sizeof(T);
+    const bool vec = ld % E == 0 && ld_grad % E == 0 && reinterpret_cast<uintptr_t>(logits) % 16 == 0 && reinterpret_cast<uintptr_t>(grad) % 16 == 0;
+    if (rows > 0 && counter != nullptr && v > 0 && v <= (vec ? kLongestRow : kWideRow)) {
         const float* den = denominator_ready ? denominator : nullptr;
-        const bool vec = ld % 4 == 0 && ld_grad % 4 == 0 && aligned4(logits) && aligned4(grad);
-        launch_cross_entropy_one_read(s, logits, labels, weights, g, den, row_loss, grad, vv, l1, l2, counter, loss, rows, vec);
+        launch_cross_entropy_one_read(s, logits, labels, weights, g, den, row_loss, grad, vv, l1, l2, counter, loss,
+                                      static_cast<uint32_t>(rows), vec);
         check_launch("cross_entropy_with_grad");
         return;
     }
