@@ -169,8 +169,15 @@ struct msx_plan {
     char* d_inputs = nullptr;
     char* d_shared_inputs = nullptr;  // those of a plan that shares its parameters, made with its slots
     uint64_t input_bytes = 0;
-    std::vector<char> blob;  // the staged inputs, host side
-    bool blob_dirty = true;  // staged since the last upload
+    // The inputs as they were last set are the slot `image` (-1: none was made). While `image_open` it is the slot
+    // of the step that runs next: inputs of `image_set` have been written there, the others follow from
+    // `image_before` when the step is submitted.
+    int image = -1, image_before = -1;
+    bool image_open = false;
+    std::vector<char> image_set;
+    // Inputs that the host loop staged itself, and their bytes where msx_set_input has put others in their place.
+    std::vector<char> host_staged;
+    std::vector<std::vector<char>> displaced;
     msx::PinnedBlock pinned_together;
     char* pinned[kStagingSlots] = {};  // a slot of input_bytes each, pieces of pinned_together or requests of their own
     char* d_staging = nullptr;         // large inputs: kDeviceSlots slots on the device
@@ -207,6 +214,7 @@ struct msx_plan {
 
     int loss_pos = -1;
     uint64_t steps = 0;
+    uint64_t finished = 0;  // steps known to have run: the host has waited for the last of them
     uint64_t shard_rows_before = 0;
 
     // The captured step: [1] takes its inputs over first, [0] runs on what is staged already. Each is
@@ -2408,13 +2416,13 @@ template <class T> cudaError_t plan_malloc(msx_plan* P, T** out, size_t bytes) {
     return e;
 }
 
-// Where a plan's inputs wait for their step: its blob, its pinned slots and, where inputs are staged, its
+// Where a plan's inputs wait for their step: its pinned slots and, where inputs are staged, its
 // slots on the device. A forward program that shares a step plan's parameters makes them, and the region on the
 // device that its launches read, when its first input is set: a run has such a plan from its beginning and may
 // never feed it. (An MLP of 200 KB a step: a run is made in 6.4 ms so, in 8.2 with the forward program's 200 KB on the
 // device beside the rest, which then takes one of the driver's 2 MB blocks more.)
 void make_input_slots(msx_plan* P, bool behind_its_own_steps = false) {
-    if (!P->blob.empty()) return;
+    if (!P->image_set.empty()) return;
     const uint64_t bytes = std::max<uint64_t>(P->input_bytes, kAlign);
     const uint64_t all = kStagingSlots * bytes;
     if (all <= kPinnedApart[0] || all > kPinnedApart[1]) {
@@ -2434,7 +2442,9 @@ void make_input_slots(msx_plan* P, bool behind_its_own_steps = false) {
         cuda_ok(cudaMemsetAsync(P->d_shared_inputs, 0, bytes, P->stream), "cudaMemset(inputs)");
         P->d_inputs = P->d_shared_inputs;
     }
-    P->blob.assign(bytes, 0);
+    P->host_staged.assign(P->inputs.size() + 1, 0);
+    P->displaced.resize(P->inputs.size() + 1);
+    P->image_set.assign(P->inputs.size() + 1, 0);
 }
 
 void allocate(msx_plan* P, const Scheduler& sched) {
@@ -2838,6 +2848,15 @@ int wait_event(cudaEvent_t event, uint32_t timeout_ms) {
     }
 }
 
+// Waits for step `step`. The driver is not asked about a step that is known to have run (a query costs the host
+// half a microsecond or more).
+int wait_step(msx_plan* P, uint64_t step, uint32_t timeout_ms) {
+    if (step < P->finished) return MSX_OK;
+    const int rc = wait_event(P->step_done[step % kStepEvents], timeout_ms);
+    if (rc == MSX_OK) P->finished = step + 1;
+    return rc;
+}
+
 // The device status word as the step of staging slot `slot` left it (copied out behind the step's
 // loss): a raised bit means the results of that step, and of every later one, are not valid. The
 // word is sticky on the device until this clears it.
@@ -2860,7 +2879,7 @@ int wait_all(msx_plan* P, uint32_t timeout_ms) {
         cuda_ok(cudaStreamSynchronize(P->stream), "cudaStreamSynchronize");
         return MSX_OK;
     }
-    int rc = wait_event(P->step_done[(P->steps - 1) % kStepEvents], timeout_ms == 0 ? 600000u : timeout_ms);
+    int rc = wait_step(P, P->steps - 1, timeout_ms == 0 ? 600000u : timeout_ms);
     if (rc != MSX_OK) return rc;
     check_status(P, static_cast<int>((P->steps - 1) % kStagingSlots));
     return MSX_OK;
@@ -2879,6 +2898,67 @@ void enqueue_step(msx_plan* P, bool take_inputs) {
     enqueue_all(P);
     k::publish_step(P->stream, P->loss_pos >= 0 ? P->f(static_cast<uint32_t>(P->loss_pos)) : nullptr, P->d_status, P->pinned_loss, P->pinned_status,
                     P->d_turn, kStagingSlots);
+}
+
+// The slot of the step that runs next is open for its inputs: they are written where that step reads them, once
+// (through a host image of the plan's and from there into the slot a megabyte of inputs took 80 us more a step).
+// Waits until the step that last used the slot has run.
+void open_image(msx_plan* P) {
+    if (P->image_open) return;
+    if (P->image_set.empty()) {
+        cuda_ok(cudaSetDevice(P->device->ordinal), "cudaSetDevice");
+        make_input_slots(P);
+    }
+    if (P->steps >= kStagingSlots) {
+        int rc = wait_step(P, P->steps - kStagingSlots, 600000u);
+        if (rc != MSX_OK) throw StatusError(rc, "a step submitted " + std::to_string(kStagingSlots) + " steps ago has not finished");
+    }
+    const int slot = static_cast<int>(P->steps % kStagingSlots);
+    std::fill(P->image_set.begin(), P->image_set.end(), static_cast<char>(slot == P->image));
+    P->image_before = P->image;
+    P->image = slot;
+    P->image_open = true;
+}
+
+// What was not set since the slot was opened comes from the slot before (zeros where there was none).
+void complete_image(msx_plan* P) {
+    for (size_t i = 0; i < P->inputs.size(); ++i) {
+        if (P->image_set[i]) continue;
+        char* const to = P->pinned[P->image] + P->inputs[i].offset;
+        if (P->image_before >= 0) std::memcpy(to, P->pinned[P->image_before] + P->inputs[i].offset, P->inputs[i].bytes);
+        else std::memset(to, 0, P->inputs[i].bytes);
+        P->image_set[i] = 1;
+    }
+}
+
+HostInput* input_of(msx_plan* P, const char* name) {
+    for (HostInput& in : P->inputs)
+        if (in.name == name) return &in;
+    return nullptr;
+}
+
+size_t index_of(const msx_plan* P, const HostInput& in) { return static_cast<size_t>(&in - P->inputs.data()); }
+
+// Where an input lies as it was last set (null: it never was).
+char* staged_value(msx_plan* P, const HostInput& in) {
+    if (P->image < 0) return nullptr;
+    const int slot = P->image_open && !P->image_set[index_of(P, in)] ? P->image_before : P->image;
+    return slot < 0 ? nullptr : P->pinned[slot] + in.offset;
+}
+
+// Input `in` of the step that runs next, unchecked.
+void stage_input(msx_plan* P, const HostInput& in, const void* host, bool by_host_loop) {
+    open_image(P);
+    const size_t i = index_of(P, in);
+    if (P->host_staged[i] && !by_host_loop) {
+        const char* now = staged_value(P, in);
+        P->displaced[i].assign(now, now + in.bytes);
+    } else if (by_host_loop) {
+        P->displaced[i].clear();
+    }
+    P->host_staged[i] = by_host_loop;
+    std::memcpy(P->pinned[P->image] + in.offset, host, in.bytes);
+    P->image_set[i] = 1;
 }
 
 // A large step's inputs from its pinned slot to its slot on the device: on the plan's stream when that is
@@ -3163,23 +3243,49 @@ int msx_state_restore(msx_plan* plan) {
 int msx_set_input(msx_plan* plan, const char* name, const void* host, uint64_t bytes) {
     if (!plan || !name || !host) return MSX_BAD_ARGUMENT;
     return guarded(plan->device, [&]() -> int {
-        for (const HostInput& in : plan->inputs) {
-            if (in.name != name) continue;
-            if (bytes != in.bytes)
-                throw StatusError(MSX_BAD_ARGUMENT, "msx_set_input: `" + in.name + "` takes " + std::to_string(in.bytes) + " bytes, " +
+        if (const HostInput* in = input_of(plan, name)) {
+            if (bytes != in->bytes)
+                throw StatusError(MSX_BAD_ARGUMENT, "msx_set_input: `" + in->name + "` takes " + std::to_string(in->bytes) + " bytes, " +
                                                         std::to_string(bytes) + " given");
             std::string why;
-            int rc = check_input(in, host, &why);
+            int rc = check_input(*in, host, &why);
             if (rc != MSX_OK) throw StatusError(rc, why);
-            if (plan->blob.empty()) {
-                cuda_ok(cudaSetDevice(plan->device->ordinal), "cudaSetDevice");
-                make_input_slots(plan);
-            }
-            std::memcpy(plan->blob.data() + in.offset, host, bytes);
-            plan->blob_dirty = true;
+            stage_input(plan, *in, host, false);
             return MSX_OK;
         }
         throw StatusError(MSX_BAD_ARGUMENT, std::string("msx_set_input: the step reads no input `") + name + "`");
+    });
+}
+
+// For the host loop above this file. An input written straight into the slot of the step that runs next; where
+// its value lies until the loop sets it again; its check before a step is submitted (on the value the loop set,
+// put back first where msx_set_input has displaced it).
+int msx_internal_stage_input(msx_plan* plan, const char* name, const void* host, uint64_t bytes) {
+    return guarded(plan->device, [&]() -> int {
+        const HostInput* in = input_of(plan, name);
+        if (!in || in->bytes != bytes) throw StatusError(MSX_BAD_ARGUMENT, std::string("no input `") + name + "` of that size");
+        stage_input(plan, *in, host, true);
+        return MSX_OK;
+    });
+}
+const void* msx_internal_staged_input(msx_plan* plan, const char* name) {
+    const HostInput* in = input_of(plan, name);
+    if (!in || plan->image < 0) return nullptr;
+    const std::vector<char>& displaced = plan->displaced[index_of(plan, *in)];
+    return displaced.empty() ? staged_value(plan, *in) : displaced.data();
+}
+int msx_internal_check_staged_input(msx_plan* plan, const char* name) {
+    return guarded(plan->device, [&]() -> int {
+        const HostInput* in = input_of(plan, name);
+        if (!in || plan->image < 0) return MSX_OK;
+        if (!plan->displaced[index_of(plan, *in)].empty()) {
+            const std::vector<char> back = std::move(plan->displaced[index_of(plan, *in)]);
+            stage_input(plan, *in, back.data(), true);
+        }
+        std::string why;
+        int rc = check_input(*in, staged_value(plan, *in), &why);
+        if (rc != MSX_OK) throw StatusError(rc, why);
+        return MSX_OK;
     });
 }
 
@@ -3205,13 +3311,13 @@ int msx_run(msx_plan* plan) {
         cuda_ok(cudaSetDevice(plan->device->ordinal), "cudaSetDevice");
         const int slot = static_cast<int>(plan->steps % kStagingSlots), at = static_cast<int>(plan->steps % kStepEvents);
         if (plan->steps >= kStagingSlots) {
-            int rc = wait_event(plan->step_done[(plan->steps - kStagingSlots) % kStepEvents], 600000u);
+            int rc = wait_step(plan, plan->steps - kStagingSlots, 600000u);
             if (rc != MSX_OK) throw StatusError(rc, "msx_run: a step submitted " + std::to_string(kStagingSlots) + " steps ago has not finished");
         }
         if (plan->clock_steps == 0) cuda_ok(cudaEventRecord(plan->clock_start, plan->stream), "cudaEventRecord");
         // A step submitted behind a running one begins where that one ends; only on an idle stream
         // does it need an event of its own (a recorded event costs the stream about 2 us).
-        plan->began_idle[at] = plan->steps == 0 || cudaEventQuery(plan->step_done[(plan->steps - 1) % kStepEvents]) == cudaSuccess;
+        plan->began_idle[at] = plan->steps == plan->finished || cudaEventQuery(plan->step_done[(plan->steps - 1) % kStepEvents]) == cudaSuccess;
         if (plan->began_idle[at]) {
             if (!plan->step_begin[at]) cuda_ok(cudaEventCreate(&plan->step_begin[at]), "cudaEventCreate");
             cuda_ok(cudaEventRecord(plan->step_begin[at], plan->stream), "cudaEventRecord");
@@ -3223,12 +3329,13 @@ int msx_run(msx_plan* plan) {
         ++plan->submits;
         plan->dispatches += plan->launches.size();
         plan->bytes_downloaded += (plan->loss_pos >= 0 ? 4 : 0) + 4;
-        const bool take_inputs = plan->input_bytes && plan->blob_dirty;
+        // (inputs that nothing has ever set are zeros)
+        const bool take_inputs = plan->input_bytes && (plan->image_open || plan->image < 0);
         if (take_inputs) {
-            make_input_slots(plan);
+            open_image(plan);
+            complete_image(plan);
             plan->bytes_uploaded += plan->input_bytes;
-            plan->blob_dirty = false;
-            std::memcpy(plan->pinned[slot], plan->blob.data(), plan->input_bytes);
+            plan->image_open = false;
             if (plan->d_staging) stage_inputs(plan, slot, plan->began_idle[at]);
         }
         if (plan->flags & MSX_PLAN_NO_GRAPH) {
@@ -3283,7 +3390,7 @@ int msx_loss_of(msx_plan* plan, uint64_t step_number, float* loss, uint32_t time
             throw StatusError(MSX_BAD_ARGUMENT, "msx_loss_of: only the last " + std::to_string(kStagingSlots) + " submitted steps keep their loss");
         if (plan->loss_pos < 0) throw StatusError(MSX_BAD_ARGUMENT, "msx_loss_of: the program has no rank-0 loss");
         int slot = static_cast<int>(step_number % kStagingSlots);
-        int rc = wait_event(plan->step_done[step_number % kStepEvents], timeout_ms == 0 ? 600000u : timeout_ms);
+        int rc = wait_step(plan, step_number, timeout_ms == 0 ? 600000u : timeout_ms);
         if (rc != MSX_OK) return rc;
         check_status(plan, slot);
         *loss = plan->pinned_loss[slot];
@@ -3313,9 +3420,9 @@ int msx_profile_step_repeated(msx_plan* plan, uint32_t repeats, float* launch_ms
         std::vector<cudaEvent_t> events(2 * count);
         for (cudaEvent_t& e : events) cuda_ok(cudaEventCreate(&e), "cudaEventCreate");
         if (plan->input_bytes) {
-            make_input_slots(plan);
-            std::memcpy(plan->pinned[0], plan->blob.data(), plan->input_bytes);
-            cuda_ok(cudaMemcpyAsync(plan->d_inputs, plan->pinned[0], plan->input_bytes, cudaMemcpyHostToDevice, plan->stream), "cudaMemcpyAsync");
+            open_image(plan);
+            complete_image(plan);
+            cuda_ok(cudaMemcpyAsync(plan->d_inputs, plan->pinned[plan->image], plan->input_bytes, cudaMemcpyHostToDevice, plan->stream), "cudaMemcpyAsync");
         }
         begin_side_work(plan);
         for (size_t l = 0; l < count; ++l) {

@@ -27,6 +27,10 @@
 
 // Defined beside msx_last_error: records a message on the device handle.
 extern "C" void msx_internal_set_error(msx_device* device, const char* message);
+// Defined beside msx_set_input: an input written into the slot its step reads, checked later.
+extern "C" int msx_internal_stage_input(msx_plan* plan, const char* name, const void* host, uint64_t bytes);
+extern "C" const void* msx_internal_staged_input(msx_plan* plan, const char* name);
+extern "C" int msx_internal_check_staged_input(msx_plan* plan, const char* name);
 
 struct msx_training {
     msx_device* device = nullptr;
@@ -59,7 +63,11 @@ struct msx_training {
     std::vector<std::string> packed_bound;  // the declared batch tensors, in source order
     uint32_t flags = 0;
     std::string error;
-    std::map<std::string, std::vector<char>> batch;  // declared inputs and targets, by name
+    // Declared inputs and targets, by name. Those of `staged` were written straight into the slot that the next
+    // step reads (once a step has run: a run that only infers needs no slots); `batch` holds their bytes once
+    // something else than the step reads them.
+    std::map<std::string, std::vector<char>> batch;
+    std::set<std::string> staged, uncopied;
     std::vector<std::string> sites;                  // dropout token inputs of the step
     std::set<std::string> step_inputs, forward_inputs;
     bool submitted = false;
@@ -102,6 +110,21 @@ const msx::DataDecl* declared(const msx_training* t, const std::string& name) {
     return nullptr;
 }
 
+// `batch` holds every input as it was last set.
+void copy_staged(msx_training* t) {
+    for (const std::string& name : t->uncopied) {
+        std::vector<char>& bytes = t->batch[name];
+        const char* from = static_cast<const char*>(msx_internal_staged_input(t->step, name.c_str()));
+        bytes.assign(from, from + bytes.size());
+    }
+    t->uncopied.clear();
+}
+// `batch` itself is written next, and staged from there.
+void unstage(msx_training* t) {
+    copy_staged(t);
+    t->staged.clear();
+}
+
 // The host side of the masked-row gather (crates/modelspec-runtime/src/train/masked.rs:88-128):
 // the rows of non-zero weight in ascending order with their labels and weights, then padding
 // rows of row 0, label 0 and weight +0.0; more selected rows than the capacity is refused.
@@ -112,6 +135,7 @@ void gather_masked(msx_training* t, uint64_t step, bool stage) {
     if (w == t->batch.end() || l == t->batch.end())
         throw Fail{MSX_BAD_INPUT, "E-DATA-012: the batch of step " + std::to_string(step) + " holds no `" +
                                       (w == t->batch.end() ? c.masked_weights : c.masked_labels) + "` to gather the masked rows from"};
+    if (t->uncopied.count(c.masked_weights) || t->uncopied.count(c.masked_labels)) copy_staged(t);
     const float* weights = reinterpret_cast<const float*>(w->second.data());
     const int32_t* labels = reinterpret_cast<const int32_t*>(l->second.data());
     size_t rows = w->second.size() / 4, capacity = c.masked_rows;
@@ -137,8 +161,12 @@ void gather_masked(msx_training* t, uint64_t step, bool stage) {
 }
 
 void stage_batch(msx_training* t, msx_plan* plan, const std::set<std::string>& reads) {
-    for (const auto& [name, bytes] : t->batch)
-        if (reads.count(name)) ok(t, msx_set_input(plan, name.c_str(), bytes.data(), bytes.size()));
+    if (plan != t->step) copy_staged(t);
+    for (const auto& [name, bytes] : t->batch) {
+        if (!reads.count(name)) continue;
+        if (plan == t->step && t->staged.count(name)) ok(t, msx_internal_check_staged_input(plan, name.c_str()));
+        else ok(t, msx_set_input(plan, name.c_str(), bytes.data(), bytes.size()));
+    }
 }
 
 }  // namespace
@@ -239,6 +267,14 @@ int msx_training_set_input(msx_training* t, const char* name, const void* host, 
         if (!d) throw Fail{MSX_BAD_ARGUMENT, std::string("the train block declares no `") + name + "`"};
         if (bytes != d->ty.count() * 4)
             throw Fail{MSX_BAD_ARGUMENT, std::string("`") + name + "` is " + d->ty.str() + ": " + std::to_string(d->ty.count() * 4) + " bytes"};
+        // (what the detour costs a small input is less than the names looked up for the direct way)
+        if (bytes >= 4096 && t->submitted && t->step_inputs.count(name)) {
+            ok(t, msx_internal_stage_input(t->step, name, host, bytes));
+            t->batch[name].resize(bytes);
+            t->staged.insert(name);
+            t->uncopied.insert(name);
+            return;
+        }
         const char* b = static_cast<const char*>(host);
         t->batch[name].assign(b, b + bytes);
     });
@@ -247,6 +283,7 @@ int msx_training_set_input(msx_training* t, const char* name, const void* host, 
 int msx_training_get_input(msx_training* t, const char* name, void* host, uint64_t bytes) {
     if (!t || !name || !host) return MSX_BAD_ARGUMENT;
     return guarded(t, [&] {
+        copy_staged(t);
         auto it = t->batch.find(name);
         if (it == t->batch.end() || it->second.size() != bytes) throw Fail{MSX_BAD_ARGUMENT, std::string("no batch input `") + name + "` of that size"};
         std::memcpy(host, it->second.data(), bytes);
@@ -256,6 +293,7 @@ int msx_training_get_input(msx_training* t, const char* name, void* host, uint64
 int msx_training_synthetic(msx_training* t) {
     if (!t) return MSX_BAD_ARGUMENT;
     return guarded(t, [&] {
+        unstage(t);
         const msx::Compiled& c = t->compiled;
         const msx::Program& fwd = c.forward;
         // Key masks: f32 inputs read only as the fourth operand of attention (data.rs:214-245).
@@ -356,6 +394,7 @@ int msx_training_step(msx_training* t, uint64_t step, uint64_t end) {
                 ok(t, msx_state_snapshot(t->step));
                 t->since_snapshot.clear();
             }
+            copy_staged(t);
             t->since_snapshot.push_back({step, end, t->batch});
         }
         submit_step(t, step, end);
@@ -384,6 +423,7 @@ int msx_training_rewind(msx_training* t, uint64_t step) {
         ok(t, msx_state_restore(t->step));
         t->since_snapshot.resize(last + 1);
         for (const msx_training::Replayed& r : t->since_snapshot) {
+            unstage(t);
             t->batch = r.batch;
             submit_step(t, r.step, r.end);
         }
@@ -691,6 +731,7 @@ int msx_training_feed_packed(msx_training* t, uint64_t step) {
         if (!t->packed) throw Fail{MSX_BAD_ARGUMENT, "no packed directory is bound"};
         std::vector<int32_t> labels;
         std::vector<float> weights;
+        unstage(t);
         draw_packed(t, MSX_SPLIT_TRAIN, step, &t->batch, &labels, &weights);
     });
 }
@@ -837,6 +878,7 @@ int msx_training_feed_dense(msx_training* t, uint64_t step) {
     return guarded(t, [&] {
         if (!t->dense) throw Fail{MSX_BAD_ARGUMENT, "no dense directory is bound"};
         const auto& decls = t->compiled.config.data;
+        unstage(t);
         for (uint32_t i = 0; i < decls.size(); ++i) {
             std::vector<char>& bytes = t->batch[decls[i].name];
             bytes.resize(msx_dense_batch_bytes(t->dense, i));
@@ -880,6 +922,7 @@ int msx_training_eval_dense(msx_training* t, const char* dir, double* loss, doub
             *at = best;
             return true;
         };
+        unstage(t);
         for (uint64_t b = 0; b < batches; ++b) {
             for (uint32_t i = 0; i < decls.size(); ++i) {
                 std::vector<char>& bytes = t->batch[decls[i].name];
@@ -1016,6 +1059,7 @@ int msx_training_infer_dense(msx_training* t, const char* dir, const char* out, 
                                           "\n  result: " + result.str() + "\n  batch: " + std::to_string(batch) + "\n  functions: " + listed_functions(c)};
         const uint64_t per_block = result.count(), count = samples / batch;
         std::vector<float> values(static_cast<size_t>(per_block * count));
+        unstage(t);
         for (uint64_t b = 0; b < count; ++b) {
             for (uint32_t i = 0; i < d.count(); ++i) {
                 std::vector<char>& bytes = t->batch[c.config.data[i].name];
