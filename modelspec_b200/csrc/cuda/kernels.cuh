@@ -435,6 +435,19 @@ void attention_bf16_backward(cudaStream_t s, const void* q, const void* k, const
                              void* dk, void* dv, void* p, void* ds, float* scores, AttentionShape shape, uint32_t* status,
                              bool p_ready = false);
 
+// The same ops with the scores on the chip (attention_f32.cu), for heads of up to 64 columns: the forward as one kernel
+// that leaves a row's maximum and sum in `stats` (attention_f32_stats_floats; or null) and, of up to 128 keys, the probabilities
+// in `p` (or null) for attention_tc_backward, the gradients as one kernel that reads those
+// and the forward's output; dq, dk and dv may each be null. `pays`: which shapes a kernel is the faster way for.
+bool attention_f32_fused_supported(AttentionShape shape);
+bool attention_f32_fused_forward_pays(AttentionShape shape);
+bool attention_f32_fused_backward_pays(AttentionShape shape);
+uint64_t attention_f32_stats_floats(AttentionShape shape);
+void attention_f32_forward(cudaStream_t s, const float* q, const float* k, const float* v, const float* mask, float* out, float* stats, float* p,
+                           AttentionShape shape, uint32_t* status);
+void attention_f32_backward(cudaStream_t s, const float* q, const float* k, const float* v, const float* mask, const float* g, const float* out,
+                            const float* stats, float* dq, float* dk, float* dv, AttentionShape shape, uint32_t* status);
+
 // Fused attention for mixed-precision plans (attention_fused.cu): the forward as one kernel that
 // never stores the scores (it writes O and, per (row, head), the softmax maximum and sum:
 // attention_fused_stats_floats(shape) floats), the three gradients as one kernel that reads those

@@ -315,7 +315,7 @@ void close_peer_reduce(msx_plan* P);
 // matmuls as jobs of one launch, 8 heavy launches with late readers on a side stream, 16
 // dropout_grad inside the layer-norm backward that makes or reads its operand and, in a
 // mixed-precision plan, gelu and gelu_grad inside the product that makes theirs, 32 the fused
-// attention kernels of a mixed-precision plan (off: batched products with row kernels between),
+// attention kernels (off: batched products with row kernels between),
 // 64 the keep decisions of a dropout site stored by the forward launch that draws them, one bit
 // per element, and read by the site's dropout_grad (off: every launch draws again).
 inline uint32_t fusion_mask() {
@@ -2177,20 +2177,44 @@ struct Scheduler {
             schedule_attention_bf16(at, shape, pair_flop);
             return;
         }
+        // The scores on the chip, when the shape fits: with its gradients where their kernel is the faster one too or
+        // where there are none; else with the probabilities of one key tile left for the products that form them.
+        const std::array<uint32_t, 5> key = {q, kk, v, mask, static_cast<uint32_t>(nd.heads)};
+        bool f32_fused = !simt && (fusion_mask() & 32u) && k::attention_f32_fused_supported(shape) && k::attention_f32_fused_forward_pays(shape);
+        bool leaves_probabilities = false;
+        if (f32_fused && !k::attention_f32_fused_backward_pays(shape))
+            for (uint32_t u : users[mask]) {
+                const Node& other = node(u);
+                if (other.op != Op::AttentionGradQ && other.op != Op::AttentionGradK && other.op != Op::AttentionGradV) continue;
+                if (other.heads != nd.heads || !std::equal(nd.operands.begin(), nd.operands.begin() + 4, other.operands.begin())) continue;
+                f32_fused = false;
+                leaves_probabilities = shape.k_len <= 128;
+            }
         if (nd.op == Op::Attention) {
             if (simt) {
                 Launch& l = emit("attention_forward", nd, {q, kk, v, mask}, {at}, [=](cudaStream_t s) {
                     k::attention_forward(s, plan->f(q), plan->f(kk), plan->f(v), plan->f(mask), plan->f(at), shape);
                 });
                 l.flop = 2 * pair_flop;
+            } else if (f32_fused) {
+                const uint32_t stats = scratch(k::attention_f32_stats_floats(shape) * 4);
+                fused_forward[key] = {stats, at};
+                Launch& l = emit("attention_forward", nd, {q, kk, v, mask}, {at, stats}, [=](cudaStream_t s) {
+                    k::attention_f32_forward(s, plan->f(q), plan->f(kk), plan->f(v), plan->f(mask), plan->f(at), plan->f(stats), nullptr, shape, plan->d_status);
+                });
+                l.flop = 2 * pair_flop;
             } else {
                 uint32_t probs = scratch(k::attention_tc_scratch_floats(shape) * 4);
                 // The backward of the same attention reads these probabilities instead of
                 // computing them again: the scratch then lives until that launch.
-                forward_probabilities[{q, kk, v, mask, static_cast<uint32_t>(nd.heads)}] = probs;
+                forward_probabilities[key] = probs;
                 Launch& l = emit("attention_forward", nd, {q, kk, v, mask}, {at, probs}, [=](cudaStream_t s) {
-                    k::attention_tc_forward(s, plan->f(q), plan->f(kk), plan->f(v), plan->f(mask), plan->f(at), plan->f(probs), shape,
-                                            plan->d_status);
+                    if (leaves_probabilities)
+                        k::attention_f32_forward(s, plan->f(q), plan->f(kk), plan->f(v), plan->f(mask), plan->f(at), nullptr, plan->f(probs), shape,
+                                                 plan->d_status);
+                    else
+                        k::attention_tc_forward(s, plan->f(q), plan->f(kk), plan->f(v), plan->f(mask), plan->f(at), plan->f(probs), shape,
+                                                plan->d_status);
                 });
                 l.flop = 2 * pair_flop;
             }
@@ -2215,8 +2239,24 @@ struct Scheduler {
                 make_arena(s, node(static_cast<uint32_t>(t)));
             }
         std::vector<uint32_t> reads = {q, kk, v, mask, g};
+        const auto forward = fused_forward.find(key);
+        if (f32_fused && forward != fused_forward.end()) {
+            const uint32_t stats = forward->second.first, o = forward->second.second;
+            reads.push_back(stats);
+            reads.push_back(o);
+            std::vector<uint32_t> writes;
+            for (int t : {dq, dk, dv})
+                if (t >= 0) writes.push_back(static_cast<uint32_t>(t));
+            auto or_null = [plan](int t) -> float* { return t >= 0 ? plan->f(static_cast<uint32_t>(t)) : nullptr; };
+            Launch& l = emit("attention_backward", nd, reads, writes, [=](cudaStream_t s) {
+                k::attention_f32_backward(s, plan->f(q), plan->f(kk), plan->f(v), plan->f(mask), plan->f(g), plan->f(o), plan->f(stats), or_null(dq),
+                                          or_null(dk), or_null(dv), shape, plan->d_status);
+            });
+            l.flop = pair_flop * (2u + (dv >= 0) + (dq >= 0) + (dk >= 0));
+            return;
+        }
         if (!simt) {
-            auto kept = forward_probabilities.find({q, kk, v, mask, static_cast<uint32_t>(nd.heads)});
+            auto kept = forward_probabilities.find(key);
             const bool p_ready = kept != forward_probabilities.end();
             uint32_t probs = p_ready ? kept->second : scratch(k::attention_tc_scratch_floats(shape) * 4);
             uint32_t dprobs = scratch(k::attention_tc_scratch_floats(shape) * 4);

@@ -1,0 +1,91 @@
+"""f32 attention with the scores on the chip, forward and gradients, element by element against float64 at the edges
+of its tiles: one query or key, 128 and one more of both, key tiles of 64 and 128 that end inside, heads that no 16-byte
+access fits, tiles whose keys are all masked."""
+import numpy as np
+import pytest
+
+import modelspec_b200 as M
+from helpers import ProgramText
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 1, 1, 1, 1), (2, 77, 77, 3, 33), (2, 128, 128, 2, 64), (1, 129, 130, 2, 40), (2, 16, 512, 1, 8), (1, 200, 65, 2, 64), (3, 64, 64, 2, 32),
+          (1, 300, 257, 1, 20), (1, 130, 512, 2, 61), (2, 33, 16, 5, 16), (1, 5, 385, 1, 64), (1, 256, 17, 1, 31),
+          # More blocks than the gradients' kernel is the faster way for: the forward leaves its probabilities, of rows on and
+          # off 16 bytes; and where neither kernel is.
+          (50, 100, 100, 4, 24), (60, 96, 99, 6, 7), (64, 20, 24, 12, 16)]
+
+
+def program(batch, q_len, k_len, heads, d, wanted):
+    h = heads * d
+    p = ProgramText()
+    q = p.input("q", "f32", [batch * q_len, h]); k = p.input("k", "f32", [batch * k_len, h])
+    v = p.input("v", "f32", [batch * k_len, h]); mask = p.input("mask", "f32", [batch, k_len])
+    g = p.input("g", "f32", [batch * q_len, h])
+    attr = "[heads = %d]" % heads
+    values = {"O": (p.op("Attention", [batch * q_len, h], [q, k, v, mask], attr=attr), q_len)}
+    for name in wanted:
+        rows = q_len if name == "Q" else k_len
+        values[name] = (p.op("AttentionGrad" + name, [batch * rows, h], [q, k, v, mask, g], attr=attr), rows)
+    for value, _ in values.values():
+        p.output(value)
+    return p.text(), values
+
+
+def float64(feed, batch, q_len, k_len, heads, d):
+    """The op and its gradients, and for each what the arithmetic of 11 + 11 bit operands and f32 sums can be off by."""
+    eps = 2.0 ** -20
+    split = lambda x, rows: x.astype(np.float64).reshape(batch, rows, heads, d).transpose(0, 2, 1, 3)
+    q, k, v, g = split(feed["q"], q_len), split(feed["k"], k_len), split(feed["v"], k_len), split(feed["g"], q_len)
+    kT, vT = k.transpose(0, 1, 3, 2), v.transpose(0, 1, 3, 2)
+    scale = 1.0 / np.sqrt(d)
+    s = q @ kT * scale
+    off_p = eps * (4 + (np.abs(q) @ np.abs(kT) * scale).max(axis=-1, keepdims=True))  # of itself
+    s = np.where(feed["mask"][:, None, None, :] != 0, s, -np.inf)
+    p = np.exp(s - s.max(axis=-1, keepdims=True))
+    p /= p.sum(axis=-1, keepdims=True)
+    out = p @ v
+    off_out = (2 * off_p + eps) * (p @ np.abs(v))
+    dP = g @ vT
+    dot = (out * g).sum(axis=-1, keepdims=True)
+    dS = p * (dP - dot) * scale
+    off_dP = eps * (np.abs(g) @ np.abs(vT)) + (off_out * np.abs(g)).sum(axis=-1, keepdims=True) + eps * (np.abs(out * g)).sum(axis=-1, keepdims=True)
+    off_dS = scale * p * (off_dP + 2 * off_p * (np.abs(dP) + np.abs(dot)))
+    T = lambda x: x.transpose(0, 1, 3, 2)
+    join = lambda x: x.transpose(0, 2, 1, 3).reshape(-1)
+    want = {"O": out, "Q": dS @ k, "K": T(dS) @ q, "V": T(p) @ g}
+    off = {"O": off_out, "Q": off_dS @ np.abs(k) + eps * (np.abs(dS) @ np.abs(k)), "K": T(off_dS) @ np.abs(q) + eps * (T(np.abs(dS)) @ np.abs(q)),
+           "V": T(2 * off_p * p) @ np.abs(g) + eps * (T(p) @ np.abs(g))}
+    return {n: (join(want[n]), join(off[n])) for n in want}
+
+
+@pytest.mark.parametrize("wanted", ["QKV", "V", "QK"])
+@pytest.mark.parametrize("batch,q_len,k_len,heads,d", SHAPES)
+def test_every_element_against_float64(device, batch, q_len, k_len, heads, d, wanted):
+    if wanted != "QKV" and (q_len, d) not in [(77, 33), (129, 40)]:
+        pytest.skip("some of the gradients: two shapes")
+    r = np.random.default_rng(q_len * 1000 + k_len + d)
+    draw = lambda rows: r.standard_normal((batch * rows, heads * d)).astype(np.float32)
+    feed = {"q": 2 * draw(q_len), "k": draw(k_len), "v": draw(k_len), "g": draw(q_len)}
+    mask = (r.random((batch, k_len)) < 0.8).astype(np.float32)
+    mask[0, : k_len - 1] = 0.0  # every tile but the last has no key of this sequence
+    mask[:, k_len - 1] = 1.0
+    feed["mask"] = mask
+    text, values = program(batch, q_len, k_len, heads, d, wanted)
+    plan = M.Plan(device, text, flags=M.PLAN_NO_GRAPH | M.PLAN_GUARD)
+    try:
+        for name, value in feed.items():
+            plan.set_input(name, value)
+        plan.run(); plan.sync(); plan.check_guards()
+        got = {name: plan.value(at, batch * rows * heads * d) for name, (at, rows) in values.items()}
+    finally:
+        plan.destroy()
+    want = float64(feed, batch, q_len, k_len, heads, d)
+    for name in got:
+        value, off = want[name]
+        bad = np.abs(got[name] - value) > off + 1e-30
+        assert not bad.any(), "%s: %d of %d outside; worst %g of its bound" % (
+            name, bad.sum(), bad.size, (np.abs(got[name] - value) / np.maximum(off, 1e-300)).max())
+    masked = np.repeat(mask.reshape(-1) == 0.0, heads * d)
+    for name in set("KV") & set(got):
+        assert not got[name][masked].any() and not np.signbit(got[name][masked]).any()
