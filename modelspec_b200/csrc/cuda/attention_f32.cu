@@ -690,25 +690,38 @@ bool on_16_bytes(std::initializer_list<const void*> pointers) {
 
 }  // namespace
 
-bool attention_f32_fused_supported(AttentionShape sh) {
+bool attention_f32_supported(AttentionShape sh) {
     return sh.head_dim >= 1 && sh.head_dim <= 64 && sh.k_len >= 1 && sh.k_len <= 512 && sh.q_len >= 1 &&
            static_cast<uint64_t>(sh.batch) * sh.heads * ((sh.q_len + QUERIES - 1) / QUERIES + 4) < (1ull << 31);
 }
 
-// The gradients' kernel takes 5 us and some 7 for every tile of 64 that one of its blocks walks, wave after wave of
-// blocks; the batched products grow with the work alone. Measured, us (this kernel, the products): one tile, 192 and 480
-// blocks 12.5, 24.7 and 28.8, 30.8, 1,024 blocks 65.7, 47.2; two tiles, 128 and 256 blocks 20.6, 28.7 and 34.9, 34.9, 512
-// blocks 45.7, 42.0; four tiles, 128 blocks 24.8 to 30.8, 34.0; eight 55.3, 47.2. Rows off 16 bytes keep the
-// products from their faster tiles: two tiles, 360 blocks 45.2, 62.6.
-bool attention_f32_fused_backward_pays(AttentionShape sh) {
-    const uint64_t tiles = (std::max(sh.q_len, sh.k_len) + BACKWARD_TILE - 1) / BACKWARD_TILE;
-    const uint64_t blocks = static_cast<uint64_t>(sh.batch) * sh.heads * ((sh.q_len + QUERIES - 1) / QUERIES + (sh.k_len + QUERIES - 1) / QUERIES);
-    return (blocks + SMS - 1) / SMS * tiles <= (sh.head_dim % 4 == 0 && sh.k_len % 4 == 0 ? 4u : 8u);
-}
-// The forward kernel is the faster way but for many heads of a few queries, whose blocks are mostly padding (768 heads
-// of 16 x 64: 37.0 us, the products 31.7; 192 heads 11.0, 16.9; 768 of 40 x 24 32.9, 35.8).
-bool attention_f32_fused_forward_pays(AttentionShape sh) {
-    return sh.q_len >= 32 || static_cast<uint64_t>(sh.batch) * sh.heads <= 4 * SMS;
+// Which way is the sooner one inside a step's graph, in us. The kernels here: their blocks in waves, each with a start
+// and, per tile, some 7 to 8 us for 64 columns (the most of it the tile's products), and 1.5 for code that is cold where
+// the products' is not. The batched products: three launches forward and four backward of a tile or two each, and
+// what the work adds, its tiles padded; more where rows off 16 bytes keep them from TMA. Measured (a launch alone less
+// the 2 us that it costs outside of a graph; these kernels, the products), forward: 64 heads of 128 x 64 10.7, 14.6; 16
+// heads 10.7, 11.1 (in a step 2 us slower than the products); 128 heads 12.3, 17.7; 96 of 40 x 24 6.4, 10.5; 768 of 16 x 64 35,
+// 26; 384 of 512 x 64 320, 390; off 16 bytes, 15 heads of 77 x 33 9.3, 11.6. Backward: 64 heads of 128 x 64 18.6, 20.7; 16 heads
+// 18.6, 17.7; 128 heads 32.9, 26.9; 96 of 40 x 24 10.4, 16.7; 240 of 64 x 32 26.8, 22.8; 8 of 256 x 64 31, 23; 15 of 77 x 33 17.7, 25.4.
+AttentionWay attention_f32_way(AttentionShape sh, bool gradients) {
+    if (!attention_f32_supported(sh)) return AttentionWay::Products;
+    auto up = [](uint64_t x, uint64_t to) { return (x + to - 1) / to; };
+    const uint64_t heads = static_cast<uint64_t>(sh.batch) * sh.heads, longest = std::max(sh.q_len, sh.k_len);
+    const bool aligned = sh.head_dim % 4 == 0 && sh.k_len % 4 == 0, narrow = sh.head_dim <= 32;
+    const uint64_t pad = longest <= 64 ? 64 : 128;
+    const double work = 1e-6 * static_cast<double>(heads * up(sh.q_len, pad) * up(sh.k_len, pad) * pad * pad * up(sh.head_dim, 32) * 32);
+    const double keys = static_cast<double>(up(sh.k_len, FORWARD_KEYS)) * std::min(1.0, up(sh.k_len, 16) * 16 / 128.0);
+    const double forward = 1.5 + static_cast<double>(up(heads * up(sh.q_len, QUERIES), SMS)) * (3.5 + keys * (narrow ? 4.0 : 7.5));
+    const double forward_products = aligned ? 10.5 + (longest <= 64 ? 0.10 : 0.06) * work : 13.0 + 0.09 * work;
+    if (!gradients) return forward < forward_products ? AttentionWay::Forward : AttentionWay::Products;
+    const double tile = 2.0 + (narrow ? 4.0 : 5.0) * std::min(1.0, up(longest, 16) * 16 / 64.0);
+    const double backward = 1.5 + static_cast<double>(up(heads * (up(sh.q_len, QUERIES) + up(sh.k_len, QUERIES)), SMS)) *
+                                      (3.5 + static_cast<double>(up(longest, BACKWARD_TILE)) * tile);
+    const double backward_products = aligned ? 17.0 + (longest <= 64 ? 0.17 : 0.07) * work : 23.0 + 0.16 * work;
+    // (the probabilities that the gradients' products read are left by the forward kernel where one tile holds a row)
+    const bool leaves = sh.k_len <= FORWARD_KEYS && forward < forward_products;
+    if (forward + backward < (leaves ? forward : forward_products) + backward_products) return AttentionWay::Both;
+    return leaves ? AttentionWay::Forward : AttentionWay::Products;
 }
 
 uint64_t attention_f32_stats_floats(AttentionShape sh) { return 2ull * sh.batch * sh.heads * sh.q_len; }

@@ -438,10 +438,12 @@ void attention_bf16_backward(cudaStream_t s, const void* q, const void* k, const
 // The same ops with the scores on the chip (attention_f32.cu), for heads of up to 64 columns: the forward as one kernel
 // that leaves a row's maximum and sum in `stats` (attention_f32_stats_floats; or null) and, of up to 128 keys, the probabilities
 // in `p` (or null) for attention_tc_backward, the gradients as one kernel that reads those
-// and the forward's output; dq, dk and dv may each be null. `pays`: which shapes a kernel is the faster way for.
-bool attention_f32_fused_supported(AttentionShape shape);
-bool attention_f32_fused_forward_pays(AttentionShape shape);
-bool attention_f32_fused_backward_pays(AttentionShape shape);
+// and the forward's output; dq, dk and dv may each be null. `attention_f32_way`
+// says which of the kernels a shape takes, of a program that has gradients of the op or none: neither, the forward (with the
+// probabilities left, where there are gradients), or both.
+bool attention_f32_supported(AttentionShape shape);
+enum class AttentionWay { Products, Forward, Both };
+AttentionWay attention_f32_way(AttentionShape shape, bool gradients);
 uint64_t attention_f32_stats_floats(AttentionShape shape);
 void attention_f32_forward(cudaStream_t s, const float* q, const float* k, const float* v, const float* mask, float* out, float* stats, float* p,
                            AttentionShape shape, uint32_t* status);

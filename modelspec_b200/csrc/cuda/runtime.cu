@@ -2180,16 +2180,18 @@ struct Scheduler {
         // The scores on the chip, when the shape fits: with its gradients where their kernel is the faster one too or
         // where there are none; else with the probabilities of one key tile left for the products that form them.
         const std::array<uint32_t, 5> key = {q, kk, v, mask, static_cast<uint32_t>(nd.heads)};
-        bool f32_fused = !simt && (fusion_mask() & 32u) && k::attention_f32_fused_supported(shape) && k::attention_f32_fused_forward_pays(shape);
-        bool leaves_probabilities = false;
-        if (f32_fused && !k::attention_f32_fused_backward_pays(shape))
+        k::AttentionWay way = k::AttentionWay::Products;
+        bool gradients = false;
+        if (!simt && (fusion_mask() & 32u)) {
             for (uint32_t u : users[mask]) {
                 const Node& other = node(u);
                 if (other.op != Op::AttentionGradQ && other.op != Op::AttentionGradK && other.op != Op::AttentionGradV) continue;
-                if (other.heads != nd.heads || !std::equal(nd.operands.begin(), nd.operands.begin() + 4, other.operands.begin())) continue;
-                f32_fused = false;
-                leaves_probabilities = shape.k_len <= 128;
+                gradients |= other.heads == nd.heads && std::equal(nd.operands.begin(), nd.operands.begin() + 4, other.operands.begin());
             }
+            way = k::attention_f32_way(shape, gradients);
+        }
+        const bool f32_fused = way == k::AttentionWay::Both || (way == k::AttentionWay::Forward && !gradients);
+        const bool leaves_probabilities = way == k::AttentionWay::Forward && gradients;
         if (nd.op == Op::Attention) {
             if (simt) {
                 Launch& l = emit("attention_forward", nd, {q, kk, v, mask}, {at}, [=](cudaStream_t s) {
@@ -3966,6 +3968,20 @@ int msx_op_matmul_bf16(const void* a, int a_transposed, const void* b, int b_tra
 
 uint64_t msx_op_matmul_bf16_workspace(uint64_t m, uint64_t n, uint64_t k) { return k::matmul_bf16_plan(m, n, k).workspace_floats; }
 
+int msx_op_attention_f32(const float* q, const float* k, const float* v, const float* mask, const float* g, float* out, float* dq, float* dk,
+                         float* dv, float* stats, float* p, uint32_t batch, uint32_t q_len, uint32_t k_len, uint32_t heads,
+                         uint32_t head_dim, uint32_t* status, void* stream) {
+    if (!q || !k || !v || !mask || !out || !status || (g && !stats)) return MSX_BAD_ARGUMENT;
+    return guarded(nullptr, [&]() -> int {
+        const k::AttentionShape shape = {batch, q_len, k_len, heads, head_dim};
+        if (!k::attention_f32_supported(shape) || (p && k_len > 128))
+            throw StatusError(MSX_UNSUPPORTED, "msx_op_attention_f32: heads of up to 64 columns, up to 512 keys (128 where the probabilities are wanted)");
+        cudaStream_t s = static_cast<cudaStream_t>(stream);
+        k::attention_f32_forward(s, q, k, v, mask, out, stats, p, shape, status);
+        if (g) k::attention_f32_backward(s, q, k, v, mask, g, out, stats, dq, dk, dv, shape, status);
+        return MSX_OK;
+    });
+}
 int msx_op_attention_bf16(const void* q, const void* k, const void* v, const float* mask, const void* g, void* out, void* dq, void* dk,
                           void* dv, float* stats, uint32_t batch, uint32_t q_len, uint32_t k_len, uint32_t heads, uint32_t head_dim,
                           uint32_t* status, void* stream) {

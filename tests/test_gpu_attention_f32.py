@@ -1,6 +1,8 @@
 """f32 attention with the scores on the chip, forward and gradients, element by element against float64 at the edges
 of its tiles: one query or key, 128 and one more of both, key tiles of 64 and 128 that end inside, heads that no 16-byte
 access fits, tiles whose keys are all masked."""
+import ctypes as C
+
 import numpy as np
 import pytest
 
@@ -10,10 +12,7 @@ from helpers import ProgramText
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 1, 1, 1, 1), (2, 77, 77, 3, 33), (2, 128, 128, 2, 64), (1, 129, 130, 2, 40), (2, 16, 512, 1, 8), (1, 200, 65, 2, 64), (3, 64, 64, 2, 32),
-          (1, 300, 257, 1, 20), (1, 130, 512, 2, 61), (2, 33, 16, 5, 16), (1, 5, 385, 1, 64), (1, 256, 17, 1, 31),
-          # More blocks than the gradients' kernel is the faster way for: the forward leaves its probabilities, of rows on and
-          # off 16 bytes; and where neither kernel is.
-          (50, 100, 100, 4, 24), (60, 96, 99, 6, 7), (64, 20, 24, 12, 16)]
+          (1, 300, 257, 1, 20), (1, 130, 512, 2, 61), (2, 33, 16, 5, 16), (1, 5, 385, 1, 64), (1, 256, 17, 1, 31)]
 
 
 def program(batch, q_len, k_len, heads, d, wanted):
@@ -59,11 +58,7 @@ def float64(feed, batch, q_len, k_len, heads, d):
     return {n: (join(want[n]), join(off[n])) for n in want}
 
 
-@pytest.mark.parametrize("wanted", ["QKV", "V", "QK"])
-@pytest.mark.parametrize("batch,q_len,k_len,heads,d", SHAPES)
-def test_every_element_against_float64(device, batch, q_len, k_len, heads, d, wanted):
-    if wanted != "QKV" and (q_len, d) not in [(77, 33), (129, 40)]:
-        pytest.skip("some of the gradients: two shapes")
+def feed_of(batch, q_len, k_len, heads, d):
     r = np.random.default_rng(q_len * 1000 + k_len + d)
     draw = lambda rows: r.standard_normal((batch * rows, heads * d)).astype(np.float32)
     feed = {"q": 2 * draw(q_len), "k": draw(k_len), "v": draw(k_len), "g": draw(q_len)}
@@ -71,21 +66,74 @@ def test_every_element_against_float64(device, batch, q_len, k_len, heads, d, wa
     mask[0, : k_len - 1] = 0.0  # every tile but the last has no key of this sequence
     mask[:, k_len - 1] = 1.0
     feed["mask"] = mask
-    text, values = program(batch, q_len, k_len, heads, d, wanted)
+    return feed
+
+
+def check(got, feed, shape):
+    want = float64(feed, *shape)
+    for name in got:
+        value, off = want[name]
+        bad = ~(np.abs(got[name] - value) <= off + 1e-30)
+        assert not bad.any(), "%s: %d of %d outside; worst %g of its bound" % (
+            name, bad.sum(), bad.size, (np.abs(got[name] - value) / np.maximum(off, 1e-300)).max())
+    masked = np.repeat(feed["mask"].reshape(-1) == 0.0, shape[3] * shape[4])
+    for name in set("KV") & set(got):
+        assert not got[name][masked].any() and not np.signbit(got[name][masked]).any()
+
+
+@pytest.mark.parametrize("shift", [0, 1])
+@pytest.mark.parametrize("wanted", ["QKV", "V", "QK"])
+@pytest.mark.parametrize("batch,q_len,k_len,heads,d", SHAPES)
+def test_every_element_of_the_kernels_against_float64(device, batch, q_len, k_len, heads, d, wanted, shift):
+    """`shift`: every operand a float behind a 16-byte boundary."""
+    if (wanted != "QKV" or shift) and (q_len, d) not in [(77, 33), (129, 40), (128, 64)]:
+        pytest.skip("some of the gradients, and unaligned operands: three shapes")
+    import torch
+    shape = (batch, q_len, k_len, heads, d)
+    feed = feed_of(*shape)
+    kept = []
+
+    def buffer(count, value=None):
+        t = torch.full((count + 8,), float("nan"), dtype=torch.float32, device="cuda")
+        if value is not None:
+            t[shift : shift + count] = torch.from_numpy(value.reshape(-1)).cuda()
+        kept.append(t)
+        return t[shift : shift + count]
+
+    ptr = lambda t: C.c_void_p(t.data_ptr()) if t is not None else None
+    operand = {n: buffer(v.size, v) for n, v in feed.items()}
+    rows = {"O": q_len, "Q": q_len, "K": k_len, "V": k_len}
+    out = {n: buffer(batch * rows[n] * heads * d) for n in "O" + wanted}
+    p = buffer(batch * heads * q_len * k_len) if k_len <= 128 else None
+    stats, status = torch.zeros(2 * batch * heads * q_len, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    if p is not None and k_len % 4 == 0 and shift:
+        p = None  # (a plan's scratch lies on 256 bytes)
+    rc = M.lib().msx_op_attention_f32(ptr(operand["q"]), ptr(operand["k"]), ptr(operand["v"]), ptr(operand["mask"]), ptr(operand["g"]), ptr(out["O"]),
+                                      ptr(out.get("Q")), ptr(out.get("K")), ptr(out.get("V")), ptr(stats), ptr(p), *shape, ptr(status), None)
+    assert rc == M.OK, M.lib().msx_last_error(None).decode()
+    torch.cuda.synchronize()
+    assert int(status.item()) == 0, "a bounded wait inside a kernel ran out"
+    check({n: t.cpu().numpy().astype(np.float64) for n, t in out.items()}, feed, shape)
+    for t in kept:  # nothing outside of an operand was written
+        assert torch.isnan(t[:shift]).all() and torch.isnan(t[-(8 - shift):]).all()
+    if p is not None:
+        sums = p.cpu().numpy().astype(np.float64).reshape(-1, k_len).sum(axis=1)
+        assert np.abs(sums - 1.0).max() <= 1e-5
+
+
+# One way each: both kernels, the forward with its probabilities left for the gradients' products (rows on and off 16 bytes),
+# neither.
+@pytest.mark.parametrize("batch,q_len,k_len,heads,d", [(32, 128, 128, 2, 64), (5, 77, 77, 3, 33), (32, 100, 100, 8, 32), (60, 96, 99, 6, 7), (2, 160, 256, 3, 16)])
+def test_a_plan_takes_each_way(device, batch, q_len, k_len, heads, d):
+    shape = (batch, q_len, k_len, heads, d)
+    feed = feed_of(*shape)
+    text, values = program(*shape, "QKV")
     plan = M.Plan(device, text, flags=M.PLAN_NO_GRAPH | M.PLAN_GUARD)
     try:
         for name, value in feed.items():
             plan.set_input(name, value)
         plan.run(); plan.sync(); plan.check_guards()
-        got = {name: plan.value(at, batch * rows * heads * d) for name, (at, rows) in values.items()}
+        check({name: plan.value(at, batch * rows * heads * d) for name, (at, rows) in values.items()}, feed, shape)
     finally:
         plan.destroy()
-    want = float64(feed, batch, q_len, k_len, heads, d)
-    for name in got:
-        value, off = want[name]
-        bad = np.abs(got[name] - value) > off + 1e-30
-        assert not bad.any(), "%s: %d of %d outside; worst %g of its bound" % (
-            name, bad.sum(), bad.size, (np.abs(got[name] - value) / np.maximum(off, 1e-300)).max())
-    masked = np.repeat(mask.reshape(-1) == 0.0, heads * d)
-    for name in set("KV") & set(got):
-        assert not got[name][masked].any() and not np.signbit(got[name][masked]).any()
