@@ -734,6 +734,29 @@ __device__ __forceinline__ void store_row(T* __restrict__ row, uint32_t lane, ui
     }
 }
 
+// The same as it was read, pairs of bf16 packed: rows that a kernel holds while others are on their way.
+template <int ITEMS, int V, class T> struct RawRow {
+    static constexpr bool HALF = sizeof(T) == 2;
+    static_assert(V == 1 || HALF);
+    uint32_t e[V == 2 ? ITEMS / 2 : ITEMS];
+    __device__ __forceinline__ void load(const T* __restrict__ row, uint32_t lane, uint32_t h) {
+        if constexpr (V == 2) {
+#pragma unroll
+            for (int j = 0; j < ITEMS / 2; ++j) e[j] = __ldg(reinterpret_cast<const uint32_t*>(row + min(j * 64 + lane * 2, h - 2)));
+        } else {
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) {
+                if constexpr (HALF) e[i] = __ldg(reinterpret_cast<const unsigned short*>(row) + min(i * 32 + lane, h - 1));
+                else e[i] = __ldg(reinterpret_cast<const uint32_t*>(row) + min(i * 32 + lane, h - 1));
+            }
+        }
+    }
+    __device__ __forceinline__ float operator[](int i) const {
+        if constexpr (V == 2) return i % 2 ? bf16_high(e[i / 2]) : bf16_low(e[i / 2]);
+        else return HALF ? bf16_low(e[i]) : __uint_as_float(e[i]);
+    }
+};
+
 // The keep decisions of one row as the warp holds it (bit i of `mask` = item i of this lane) to
 // and from their stored form: word w of the row holds columns 32 w .. 32 w + 31, bit = column
 // modulo 32. The row has a multiple of 32 columns, at most 1,024: one word per lane.
@@ -765,8 +788,7 @@ __device__ __forceinline__ void save_keep_bits(uint32_t* __restrict__ row_words,
     if (lane < h / 32) row_words[lane] = mine;
 }
 template <int ITEMS, int V>
-__device__ __forceinline__ uint32_t load_keep_bits(const uint32_t* __restrict__ row_words, uint32_t lane, uint32_t h) {
-    const uint32_t mine = lane < h / 32 ? __ldg(row_words + lane) : 0u;
+__device__ __forceinline__ uint32_t spread_keep_bits(uint32_t mine, uint32_t lane) {
     uint32_t mask = 0;
     if constexpr (V == 1) {
 #pragma unroll
@@ -780,12 +802,16 @@ __device__ __forceinline__ uint32_t load_keep_bits(const uint32_t* __restrict__ 
     }
     return mask;
 }
+// This lane's word of a row's stored decisions (0 where they are drawn).
+__device__ __forceinline__ uint32_t stored_keep_word(const DropoutDraw& draw, uint64_t row_at, uint32_t lane, uint32_t h) {
+    return draw.token != nullptr && draw.stored && draw.bits != nullptr && lane < h / 32 ? __ldg(draw.bits + row_at / 32 + lane) : 0u;
+}
 // The keep decisions of a row for one site: read when an earlier launch of the step stored them,
 // else drawn (element index_base + row h + column of Philox stream 4) and stored when asked.
 template <int ITEMS, int V>
-__device__ __forceinline__ uint32_t keep_mask(const DropoutDraw& draw, uint64_t row_at, uint32_t lane, uint32_t h) {
+__device__ __forceinline__ uint32_t keep_mask(const DropoutDraw& draw, uint64_t row_at, uint32_t lane, uint32_t h, uint32_t stored_word) {
     uint32_t* const row_words = draw.bits ? draw.bits + row_at / 32 : nullptr;
-    if (draw.stored && row_words != nullptr) return load_keep_bits<ITEMS, V>(row_words, lane, h);
+    if (draw.stored && row_words != nullptr) return spread_keep_bits<ITEMS, V>(stored_word, lane);
     const uint32_t id_lo = static_cast<uint32_t>(draw.token[0]), id_hi = static_cast<uint32_t>(draw.token[1]);
     uint32_t mask = 0;
 #pragma unroll
@@ -823,13 +849,22 @@ __global__ void __launch_bounds__(256, !EXACT ? 1 : ITEMS >= 32 ? 2 : ITEMS >= 2
     float v[ITEMS], xs[ITEMS];
     load_row<ITEMS, V>(x + base, lane, h, xs);
     if (residual != nullptr) load_row<ITEMS, V>(residual + base, lane, h, v);
+    const uint32_t x_word = stored_keep_word(x_draw, base, lane, h), out_word = stored_keep_word(out_draw, base, lane, h);
+    constexpr bool HELD_GAMMA = ITEMS <= 8;  // (wider rows have no registers left for it)
+    float gam[HELD_GAMMA ? ITEMS : 1], bet[HELD_GAMMA ? ITEMS : 1];
+    if constexpr (HELD_GAMMA) {
+        if (gamma != nullptr) {
+            load_row<ITEMS, V>(gamma, lane, h, gam);
+            load_row<ITEMS, V>(beta, lane, h, bet);
+        }
+    }
     // gelu(x) in the place of the sum (the head's transform: dense, gelu, layer norm).
     if (gelu_first) {
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) xs[i] = gelu_value_for<T>(xs[i]);
     }
     if (x_draw.token != nullptr) {
-        const uint32_t keep = keep_mask<ITEMS, V>(x_draw, base, lane, h);
+        const uint32_t keep = keep_mask<ITEMS, V>(x_draw, base, lane, h, x_word);
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i) xs[i] = (keep >> i) & 1u ? xs[i] * x_draw.scale : 0.0f;
     }
@@ -856,13 +891,13 @@ __global__ void __launch_bounds__(256, !EXACT ? 1 : ITEMS >= 32 ? 2 : ITEMS >= 2
             q = fmaf(d, d, q);
         }
     const float rstd = 1.0f / sqrtf(warp_sum(q) / width + kLayerNormEps);
-    const uint32_t keep_out = out_dropped != nullptr ? keep_mask<ITEMS, V>(out_draw, base, lane, h) : 0u;
+    const uint32_t keep_out = out_dropped != nullptr ? keep_mask<ITEMS, V>(out_draw, base, lane, h, out_word) : 0u;
     float dropped[ITEMS];
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const uint32_t c = column_of<V>(i, lane);
         const uint32_t cc = min(c, h - 1);
-        const float y = (v[i] - mean) * rstd * gamma[cc] + beta[cc];
+        const float y = HELD_GAMMA ? (v[i] - mean) * rstd * gam[HELD_GAMMA ? i : 0] + bet[HELD_GAMMA ? i : 0] : (v[i] - mean) * rstd * gamma[cc] + beta[cc];
         v[i] = y;
         dropped[i] = (out_dropped != nullptr && c < h && ((keep_out >> i) & 1u)) ? y * out_draw.scale : 0.0f;
     }
@@ -884,8 +919,10 @@ __global__ void __launch_bounds__(256, !EXACT ? 1 : ITEMS >= 32 ? 2 : ITEMS >= 2
 // EXACT: the row is ITEMS x 32 wide, so that no column has to be tested and the loads of gamma and the
 // updates of the column sums go out together (16,384 bf16 rows of 768 with an addend and a dropped
 // copy: 71 -> 44 us).
+// Blocks to an SM: four where 64 registers hold a row (4,096 bf16 rows of 128 in one wave: a BERT-tiny step 5 us less), else
+// two (as four, f32 rows of 128 spill: a BERT-tiny step 4 us more).
 template <int ITEMS, int V, bool EXACT, class T>
-__global__ void __launch_bounds__(256, ITEMS >= 16 ? 2 : 1) layer_norm_backward_kernel(
+__global__ void __launch_bounds__(256, ITEMS <= 2 || (ITEMS <= 4 && EXACT && sizeof(T) == 2) ? 4 : 2) layer_norm_backward_kernel(
     const T* __restrict__ x, const float* __restrict__ gamma, const T* __restrict__ g, const T* __restrict__ g1,
     const T* __restrict__ g2, const T* __restrict__ g3, T* __restrict__ dx,
     float* __restrict__ partial, uint32_t* __restrict__ counter, float* __restrict__ dgamma, float* __restrict__ dbeta,
@@ -923,13 +960,40 @@ __global__ void __launch_bounds__(256, ITEMS >= 16 ? 2 : 1) layer_norm_backward_
         }
     }
     for (uint32_t r = r0 + warp; r < r1; r += 8) {
-        // All loads of an array are issued before any is used: unconditional, from a clamped
-        // column (what a column past h reads is discarded below), one array after another. A load
-        // under a condition of its own would wait for the one before it.
+        // All loads of a row are issued before any is used: unconditional, from clamped columns (what a column
+        // past h reads is discarded below), the addends of the adjoint, the stored decisions and the
+        // pre-activations with the rest. A load behind a use of another one would wait for that
+        // (an addend or a pre-activation each a trip to the L2; inside a step 2,200 bf16 rows of 200 take 2.4 us less so,
+        // 4,096 f32 rows of 256 2.3). Wide f32 rows have registers for two arrays: their addends follow, out of the L2.
         const uint64_t row_at = static_cast<uint64_t>(r) * h;
+        constexpr int AHEAD = !WIDE ? 3 : sizeof(T) == 2 && V == 2 ? 1 : 0;  // addends held while x and g are on their way
+        const uint32_t adjoint_word = stored_keep_word(adjoint_draw, row_at, lane, h), dx_word = stored_keep_word(dx_draw, row_at, lane, h);
+        const T* const addends[3] = {g1, g2, g3};
         float xv[ITEMS], gv[ITEMS];
-        load_row<ITEMS, V>(x + row_at, lane, h, xv);
-        load_row<ITEMS, V>(g + row_at, lane, h, gv);
+        RawRow<!WIDE ? ITEMS : 2, V, T> pre_raw;
+        {
+            RawRow<ITEMS, V, T> x_raw, g_raw, more[AHEAD > 0 ? AHEAD : 1];
+            x_raw.load(x + row_at, lane, h);
+            g_raw.load(g + row_at, lane, h);
+#pragma unroll
+            for (int a = 0; a < AHEAD; ++a)
+                if (addends[a] != nullptr) more[a].load(addends[a] + row_at, lane, h);
+            if constexpr (!WIDE) {
+                if (pre_activation != nullptr) pre_raw.load(pre_activation + row_at, lane, h);
+            }
+#pragma unroll
+            for (int i = 0; i < ITEMS; ++i) {
+                xv[i] = x_raw[i];
+                gv[i] = g_raw[i];
+            }
+            // The adjoint as a sum the program spells as a chain of Adds: ((g + g1) + g2) + g3.
+#pragma unroll
+            for (int a = 0; a < AHEAD; ++a) {
+                if (addends[a] == nullptr) continue;
+#pragma unroll
+                for (int i = 0; i < ITEMS; ++i) gv[i] = gv[i] + more[a][i];
+            }
+        }
         if constexpr (WIDE) {
             // The warp's next row on its way into the L2, 128 bytes a lane.
             if (r + 8 < r1 && lane * 128u < h * sizeof(T)) {
@@ -938,18 +1002,18 @@ __global__ void __launch_bounds__(256, ITEMS >= 16 ? 2 : 1) layer_norm_backward_
                     if (from != nullptr) asm volatile("prefetch.global.L2 [%0];" ::"l"(reinterpret_cast<const char*>(from + next) + lane * 128u));
             }
         }
-        // The adjoint as a sum the program spells as a chain of Adds: ((g + g1) + g2) + g3.
-        for (const T* more : {g1, g2, g3}) {
-            if (more == nullptr) continue;
+#pragma unroll
+        for (int a = AHEAD; a < 3; ++a) {
+            if (addends[a] == nullptr) continue;
             float t[ITEMS];
-            load_row<ITEMS, V>(more + row_at, lane, h, t);
+            load_row<ITEMS, V>(addends[a] + row_at, lane, h, t);
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) gv[i] = gv[i] + t[i];
         }
         // An adjoint that the program passes through dropout_grad first: the draw of element
         // (r, c), on the sum.
         if (adjoint_draw.token != nullptr) {
-            const uint32_t keep = keep_mask<ITEMS, V>(adjoint_draw, row_at, lane, h);
+            const uint32_t keep = keep_mask<ITEMS, V>(adjoint_draw, row_at, lane, h, adjoint_word);
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) gv[i] = (keep >> i) & 1u ? gv[i] * adjoint_draw.scale : 0.0f;
         }
@@ -1008,9 +1072,16 @@ __global__ void __launch_bounds__(256, ITEMS >= 16 ? 2 : 1) layer_norm_backward_
             const float mean_gx = warp_sum(s1) / width, mean_gx_xhat = warp_sum(s2) / width;
             // The pre-activations of a gelu_grad on dx: loaded together, before the first is used.
             float pre[ITEMS];
-            if (pre_activation != nullptr) load_row<ITEMS, V>(pre_activation + row_at, lane, h, pre);
+            if (pre_activation != nullptr) {
+                if constexpr (!WIDE) {
+#pragma unroll
+                    for (int i = 0; i < ITEMS; ++i) pre[i] = pre_raw[i];
+                } else {
+                    load_row<ITEMS, V>(pre_activation + row_at, lane, h, pre);
+                }
+            }
             float second[ITEMS];
-            const uint32_t keep_dx = (pre_activation == nullptr && dx_dropped != nullptr) ? keep_mask<ITEMS, V>(dx_draw, row_at, lane, h) : 0u;
+            const uint32_t keep_dx = (pre_activation == nullptr && dx_dropped != nullptr) ? keep_mask<ITEMS, V>(dx_draw, row_at, lane, h, dx_word) : 0u;
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) {
                 const uint32_t c = column_of<V>(i, lane);
