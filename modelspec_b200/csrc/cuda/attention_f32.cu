@@ -37,6 +37,11 @@ namespace k {
 
 namespace {
 
+using tc::tmem_load;
+using tc::tmem_loaded;
+using tc::tmem_store;
+using tc::tmem_stored;
+
 constexpr int THREADS = 512;
 constexpr uint64_t SMS = 148;
 constexpr uint32_t QUERIES = 128, FORWARD_KEYS = 128, BACKWARD_TILE = 64;
@@ -61,37 +66,6 @@ __device__ __forceinline__ void mma_from_tmem(uint32_t d, uint32_t a, uint64_t d
                  ::"r"(d), "r"(a), "l"(desc_b), "r"(idesc), "r"(accumulate) : "memory");
 }
 
-// COUNT consecutive columns of this warp's 32 lanes.
-#define MSX_R4(a, i) "=r"(a[i]), "=r"(a[i + 1]), "=r"(a[i + 2]), "=r"(a[i + 3])
-#define MSX_S4(a, i) "r"(a[i]), "r"(a[i + 1]), "r"(a[i + 2]), "r"(a[i + 3])
-template <int COUNT> __device__ __forceinline__ void tmem_load(uint32_t at, uint32_t (&r)[COUNT]) {
-    static_assert(COUNT == 8 || COUNT == 16 || COUNT == 32);
-    if constexpr (COUNT == 8)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-                     : MSX_R4(r, 0), MSX_R4(r, 4) : "r"(at) : "memory");
-    else if constexpr (COUNT == 16)
-        asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                     : MSX_R4(r, 0), MSX_R4(r, 4), MSX_R4(r, 8), MSX_R4(r, 12) : "r"(at) : "memory");
-    else tc::tmem_load32(at, r);
-}
-template <int COUNT> __device__ __forceinline__ void tmem_store(uint32_t at, const uint32_t (&r)[COUNT]) {
-    static_assert(COUNT == 8 || COUNT == 16 || COUNT == 32);
-    if constexpr (COUNT == 8)
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%8], {%0, %1, %2, %3, %4, %5, %6, %7};"
-                     ::MSX_S4(r, 0), MSX_S4(r, 4), "r"(at) : "memory");
-    else if constexpr (COUNT == 16)
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%16], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15};"
-                     ::MSX_S4(r, 0), MSX_S4(r, 4), MSX_S4(r, 8), MSX_S4(r, 12), "r"(at) : "memory");
-    else
-        asm volatile("tcgen05.st.sync.aligned.32x32b.x32.b32 [%32], {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                     "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31};"
-                     ::MSX_S4(r, 0), MSX_S4(r, 4), MSX_S4(r, 8), MSX_S4(r, 12), MSX_S4(r, 16), MSX_S4(r, 20), MSX_S4(r, 24), MSX_S4(r, 28), "r"(at)
-                     : "memory");
-}
-#undef MSX_R4
-#undef MSX_S4
-__device__ __forceinline__ void tmem_loaded() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
-__device__ __forceinline__ void tmem_stored() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void before_sync() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ void after_sync() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 
