@@ -113,6 +113,7 @@ __device__ __forceinline__ void weighted_rows_phase(const float* __restrict__ sr
 __global__ void __launch_bounds__(THREADS) forward_kernel(const float* __restrict__ q, const float* __restrict__ k,
                                                            const float* __restrict__ v, const float* __restrict__ mask,
                                                            float* __restrict__ out, Dims dm) {
+    after_producers();
     extern __shared__ float smem[];
     const uint32_t ds = dm.d + 1, sstride = dm.s + 1;
     float* qs = smem;
@@ -139,6 +140,7 @@ __global__ void __launch_bounds__(THREADS) grad_q_kernel(const float* __restrict
                                                           const float* __restrict__ v, const float* __restrict__ mask,
                                                           const float* __restrict__ g, float* __restrict__ stats,
                                                           float* __restrict__ dq, Dims dm) {
+    after_producers();
     extern __shared__ float smem[];
     const uint32_t ds = dm.d + 1, sstride = dm.s + 1;
     float* qs = smem;
@@ -207,6 +209,7 @@ __global__ void __launch_bounds__(THREADS) grad_kv_kernel(const float* __restric
                                                            const float* __restrict__ v, const float* __restrict__ mask,
                                                            const float* __restrict__ g, const float* __restrict__ stats,
                                                            float* __restrict__ dk, float* __restrict__ dv, Dims dm) {
+    after_producers();
     extern __shared__ float smem[];
     const uint32_t ds = dm.d + 1;
     float* ks = smem;

@@ -177,6 +177,7 @@ __device__ __forceinline__ uint32_t begin(Control* c) {
     before_sync();
     __syncthreads();
     after_sync();
+    wait_for_producers();
     return c->tmem_slot;
 }
 __device__ __forceinline__ void finish(uint32_t tmem) {
@@ -267,10 +268,10 @@ __global__ void __launch_bounds__(THREADS, 1) attention_f32_forward_kernel(const
         vp.fetch(vb + static_cast<uint64_t>(j0) * sh.h, sh.h, rows, sh.d);
         mine = part * 32 + lane < rows ? __ldg(mb + j0 + part * 32 + lane) : 0.0f;
     };
+    const uint32_t tmem = begin(ctl), lanes = tmem + ((quarter * 32u) << 16);
     fetch(0);
     float x[OWN];
     fetch_row<DP, VEC>(q + q_at, sh.h, at.first + row, sh.l, part * OWN, sh.d, x);
-    const uint32_t tmem = begin(ctl), lanes = tmem + ((quarter * 32u) << 16);
     store_split(lanes + Q_HI + part * OWN, lanes + Q_LO + part * OWN, x);
     tmem_stored();
     before_sync();
@@ -373,6 +374,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_f32_forward_kernel(const
         j0 = next;
         if (!__syncthreads_and(alive && j0 < sh.s)) break;
     }
+    let_next_start();
     ctl->part2[part][row] = total;
     __syncthreads();
     total = (ctl->part2[0][row] + ctl->part2[1][row]) + (ctl->part2[2][row] + ctl->part2[3][row]);
@@ -438,12 +440,12 @@ template <int DP, bool VEC> __device__ __forceinline__ void backward_queries(cha
         vp.fetch(x.v + k_at + static_cast<uint64_t>(j0) * sh.h, sh.h, keys, sh.d);
         mine = lane < 16 && part * 16 + lane < keys ? __ldg(mb + j0 + part * 16 + lane) : 0.0f;
     };
+    const uint32_t tmem = begin(ctl), lanes = tmem + ((quarter * 32u) << 16);
     fetch(0);
     const float2 stat = at.first + row < sh.l ? __ldg(x.stats + (static_cast<uint64_t>(at.b) * sh.heads + at.a) * sh.l + at.first + row) : make_float2(0.f, 1.f);
     float own[OWN], other[OWN];
     fetch_row<DP, VEC>(x.q + q_at, sh.h, at.first + row, sh.l, part * OWN, sh.d, own);
     fetch_row<DP, VEC>(x.g + q_at, sh.h, at.first + row, sh.l, part * OWN, sh.d, other);
-    const uint32_t tmem = begin(ctl), lanes = tmem + ((quarter * 32u) << 16);
     store_split(lanes + ROWS_A_HI + part * OWN, lanes + ROWS_A_LO + part * OWN, own);
     store_split(lanes + ROWS_B_HI + part * OWN, lanes + ROWS_B_LO + part * OWN, other);
     tmem_stored();
@@ -511,6 +513,7 @@ template <int DP, bool VEC> __device__ __forceinline__ void backward_queries(cha
         j0 = next;
         if (!__syncthreads_and(alive && j0 < sh.s)) break;
     }
+    let_next_start();
     put_row<DP, VEC>(x.dq + q_at, sh.h, at.first + row, sh.l, part * OWN, sh.d, sum);
     finish(tmem);
 }
@@ -537,11 +540,11 @@ template <int DP, bool VEC> __device__ __forceinline__ void backward_keys(char* 
         op.fetch(x.out + from, sh.h, queries, sh.d);
         stat = tid < queries ? __ldg(stats + i0 + tid) : make_float2(0.f, 1.f);
     };
+    const uint32_t tmem = begin(ctl), lanes = tmem + ((quarter * 32u) << 16);
     fetch(0);
     const bool counted = at.first + row < sh.s && __ldg(x.mask + static_cast<uint64_t>(at.b) * sh.s + at.first + row) != 0.0f;
     float own[OWN];
     fetch_row<DP, VEC>(x.k + k_at, sh.h, at.first + row, sh.s, part * OWN, sh.d, own);
-    const uint32_t tmem = begin(ctl), lanes = tmem + ((quarter * 32u) << 16);
     store_split(lanes + ROWS_A_HI + part * OWN, lanes + ROWS_A_LO + part * OWN, own);
     fetch_row<DP, VEC>(x.v + k_at, sh.h, at.first + row, sh.s, part * OWN, sh.d, own);
     store_split(lanes + ROWS_B_HI + part * OWN, lanes + ROWS_B_LO + part * OWN, own);
@@ -633,6 +636,7 @@ template <int DP, bool VEC> __device__ __forceinline__ void backward_keys(char* 
         i0 = next;
         if (!__syncthreads_and(alive && i0 < sh.l)) break;
     }
+    let_next_start();
     if (x.dk) put_row<DP, VEC>(x.dk + k_at, sh.h, at.first + row, sh.s, part * OWN, sh.d, dk);
     if (x.dv) put_row<DP, VEC>(x.dv + k_at, sh.h, at.first + row, sh.s, part * OWN, sh.d, dv);
     finish(tmem);

@@ -146,6 +146,7 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_s = *tmem_slot, tmem_p = tmem_s + 128, tmem_pv = tmem_s + 192;
+    wait_for_producers();
 
     if (warp == FWD_ROW_WARPS) {
         if (lane == 0) {
@@ -166,6 +167,7 @@ attention_forward_kernel(const __grid_constant__ CUtensorMap map_q, const __grid
                 load_tile(smem_u32(v_tile(stage)), &map_v, bar(V_FULL0 + stage), args.order, j * TILE, head, seq);
                 ++issued_v;
             }
+            let_next_start();
             if (!alive || *abort_flag) {
                 // The copies already issued still write into this CTA's shared memory: wait (bounded).
                 for (uint32_t spin = 0; spin < WAIT_LIMIT && !mbar_try_wait(bar(Q_FULL), 0); ++spin) {}
@@ -392,6 +394,7 @@ __device__ __forceinline__ void backward_rows(const BackwardMaps& maps, const Fu
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem = *tmem_slot, tmem_s = tmem, tmem_dp = tmem + 64;
+    wait_for_producers();
     const uint32_t tmem_ds = KEYS ? tmem_dp : tmem + 128, tmem_dq = tmem + 160, tmem_dv = tmem + 128, tmem_dk = tmem + 192;
 
     if (warp == BWD_ROW_WARPS) {
@@ -409,6 +412,7 @@ __device__ __forceinline__ void backward_rows(const BackwardMaps& maps, const Fu
                 load_tile(smem_u32(a_tile(stage)), &maps.steps[KEYS ? MAP_Q : MAP_K], bar(FULL0 + stage), args.order, issued * BWD_STEP, head, seq);
                 load_tile(smem_u32(b_tile(stage)), &maps.steps[KEYS ? MAP_G : MAP_V], bar(FULL0 + stage), args.order, issued * BWD_STEP, head, seq);
             }
+            let_next_start();
             if (!alive || *abort_flag) {
                 // The copies already issued still write into this CTA's shared memory: wait (bounded).
                 for (uint32_t spin = 0; spin < WAIT_LIMIT && !mbar_try_wait(bar(XY_FULL), 0); ++spin) {}
@@ -666,6 +670,7 @@ attention_backward_whole_kernel(const __grid_constant__ CUtensorMap map_q, const
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
     const uint32_t tmem_sp = tmem_base, tmem_dv = tmem_base + 128, tmem_dk = tmem_base + 192, tmem_dq = tmem_base + 256;
+    wait_for_producers();
 
     if (warp == 0) {
         if (lane == 0) {
@@ -691,6 +696,7 @@ attention_backward_whole_kernel(const __grid_constant__ CUtensorMap map_q, const
                     armed_phase = (armed_phase & ~(2u << stage)) | ((use & 1u) << (1 + stage));
                 }
             }
+            let_next_start();
             if (!alive) {
                 if (armed & 1u) for (uint32_t spin = 0; spin < WAIT_LIMIT && !mbar_try_wait(bar(KV_FULL), armed_phase & 1u); ++spin) {}
                 for (uint32_t stage = 0; stage < 2; ++stage)

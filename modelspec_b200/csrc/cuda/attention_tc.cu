@@ -29,6 +29,7 @@ constexpr uint32_t ROW_BLOCK_WARPS = 8;
 template <int ITEMS, int V>
 __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(float* __restrict__ scores, const float* __restrict__ mask, uint32_t rows,
                                                                               uint32_t rows_per_sequence, uint32_t s, float scale) {
+    after_producers();
     const uint32_t row = blockIdx.x * ROW_BLOCK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
     float* p = scores + static_cast<uint64_t>(row) * s;
@@ -83,6 +84,7 @@ __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(fl
 template <int ITEMS>
 __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) score_grad_kernel(const float* __restrict__ p, float* __restrict__ dp, uint32_t rows, uint32_t s,
                                                                           float scale) {
+    after_producers();
     const uint32_t row = blockIdx.x * ROW_BLOCK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
     if (row >= rows) return;
     const float* pr = p + static_cast<uint64_t>(row) * s;
@@ -203,6 +205,7 @@ namespace {
 // One warp per score row: p = softmax over the unmasked keys of scores * scale, stored as bf16.
 __global__ void masked_softmax_half_kernel(const float* __restrict__ scores, const float* __restrict__ mask, bf16* __restrict__ p,
                                            uint32_t rows, uint32_t rows_per_sequence, uint32_t s, float scale) {
+    after_producers();
     uint32_t row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     int lane = threadIdx.x & 31;
@@ -222,6 +225,7 @@ __global__ void masked_softmax_half_kernel(const float* __restrict__ scores, con
 // dS = scale * P * (dP - sum_j P dP), stored as bf16.
 __global__ void score_grad_half_kernel(const bf16* __restrict__ p, const float* __restrict__ dp, bf16* __restrict__ ds, uint32_t rows,
                                        uint32_t s, float scale) {
+    after_producers();
     uint32_t row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     if (row >= rows) return;
     int lane = threadIdx.x & 31;

@@ -52,6 +52,23 @@ inline uint32_t device_sm_count() {
     return static_cast<uint32_t>(sms);
 }
 
+// ---- kernels that start while the one before them ends -------------------------------------------
+// In a step's graph a kernel may be launched as soon as every block of the kernel before it has come this far
+// (msx_run turns the edges between kernels into programmatic ones). Each waits here until that one is complete and
+// its writes are visible, and only then lets the next one start: whatever a kernel reads or writes in memory comes
+// after this call. Kernels whose blocks fill an SM wait first and let the next one start late, with their last loads
+// (blocks that stand there early keep the kernels of the side stream from the idle SMs, and gather on those: as early
+// as this, the f32 attention made a BERT-tiny step 21 us longer), and only with tensor memory of their own in hand: a block must not wait for tensor
+// memory that a block waiting for it has taken.
+// Between two kernels of a graph 0.85 us pass, 0.63 so, and a tensor-core kernel's barriers and tensor memory are set
+// up under the end of the kernel before.
+__device__ __forceinline__ void wait_for_producers() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+__device__ __forceinline__ void after_producers() {
+    wait_for_producers();
+    let_next_start();
+}
+
 // ---- elements of either storage type ------------------------------------------------------------
 // A mixed-precision plan stores activations as bf16; the kernels that touch them are templates on
 // the element type and compute in f32 whatever it is. One element, or four consecutive ones (16

@@ -24,6 +24,7 @@ template <class TI, class TO>
 __global__ void embedding_kernel(const TI* __restrict__ table, const int32_t* __restrict__ ids,
                                  TO* __restrict__ out, uint64_t n, uint32_t rows, uint32_t h,
                                  uint32_t* __restrict__ status) {
+    after_producers();
     // One warp per output row, 128-bit copies when the row length allows.
     uint64_t row = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
     int lane = threadIdx.x & 31;
@@ -51,6 +52,7 @@ constexpr int kOrderTile = 4096;
 __global__ void __launch_bounds__(256) order_kernel(const int32_t* __restrict__ ids, uint32_t n, uint32_t rows,
                                                     int32_t* __restrict__ sorted_id, int32_t* __restrict__ sorted_n,
                                                     uint32_t* __restrict__ status) {
+    after_producers();
     __shared__ int4 tile[kOrderTile / 4];
     const uint32_t i = blockIdx.x * 32 + threadIdx.x / 8, part = threadIdx.x & 7u;
     int32_t mine = i < n ? ids[i] : 0;
@@ -127,6 +129,7 @@ template <int VEC, class TG, class TO>
 __global__ void __launch_bounds__(256) scatter_kernel(const TG* __restrict__ g, const int32_t* __restrict__ sorted_id,
                                                       const int32_t* __restrict__ sorted_n, uint32_t n,
                                                       const float* base, TO* out, uint32_t rows, uint32_t h) {
+    after_producers();
     constexpr uint32_t span = VEC * 32;
     constexpr int LOADS = kHotChunk * span / VEC / 256;
     __shared__ float stage[kHotChunk][span];
@@ -291,6 +294,7 @@ template <int VEC, class TG, class TO>
 __global__ void __launch_bounds__(256) scatter_in_place_kernel(const TG* __restrict__ g, const int32_t* __restrict__ sorted_id,
                                                                const int32_t* __restrict__ sorted_n, uint32_t n, TO* out, uint32_t rows,
                                                                uint32_t h) {
+    after_producers();
     constexpr uint32_t span = VEC * 32;
     constexpr int LOADS = kHotChunk * span / VEC / 256;
     __shared__ float stage[kHotChunk][span];

@@ -183,6 +183,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) bf16_kernel(const __
     else __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    wait_for_producers();
 
     if (warp == 0) {
         // ---- the TMA warp: the k blocks of every unit of this CTA, in order -----------------------------
@@ -221,6 +222,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) bf16_kernel(const __
                 __syncwarp();
             }
         }
+        let_next_start();  // what is left of this kernel are its last products and their way out
         // A role gave up: the loads still in flight, of both CTAs, land (a bounded wait each on the first
         // one's barriers) before either CTA, and with it their shared-memory destination, goes away.
         if (*abort_flag && lane == 0 && rank == 0) {
@@ -437,6 +439,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) bf16_kernel(const __
 // The sum of the split-k partial tiles, ascending split order, into C (either type) with the bias.
 __global__ void splitk_reduce_bf16_kernel(const float* __restrict__ ws, void* __restrict__ c, uint32_t out_half, uint64_t m, uint32_t n,
                                           uint32_t ldc, uint32_t splits, const float* __restrict__ bias) {
+    after_producers();
     const uint64_t count = m * n, stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {
         float acc = ws[i];

@@ -67,6 +67,7 @@ __device__ __forceinline__ void cluster_barrier() {
 
 template <bool A_T, bool B_T, int COUNT>
 __global__ void __launch_bounds__(THREADS) matmul_small_kernel(const __grid_constant__ Problems<COUNT> problems) {
+    after_producers();
     extern __shared__ __align__(16) float shared[];
     uint32_t which = 0;
     while (which + 1 < problems.count && problems.p[which + 1].first_block <= blockIdx.x) ++which;

@@ -340,6 +340,7 @@ __global__ void __launch_bounds__(THREADS, Config<BM, BN>::CTAS_PER_SM) matmul_t
     // issued in the epilogue would be a round trip to memory with nothing to hide behind.
     const float* __restrict__ bias_row = (job_c || args.job_count) ? nullptr : args.bias[product];
     float bias_mine[4] = {0.f, 0.f, 0.f, 0.f};
+    wait_for_producers();
     if (warp < 8) {
         if (bias_row) {
             const uint32_t gn = n0 + (lane % (BN / 4)) * 4;
@@ -397,6 +398,7 @@ __global__ void __launch_bounds__(THREADS, Config<BM, BN>::CTAS_PER_SM) matmul_t
                 alive = deposit(kb, av[s], bv[s]);
             }
         }
+        let_next_start();
         // ---- epilogue: tensor memory -> shared memory -> global --------------------------------
         // Lanes 0-63 of tensor memory hold the A_hi rows, 64-127 the A_lo rows of the same 64 tile
         // rows; columns [0, BN) the products with B_hi, [BN, 2 BN) those with B_lo. A warp reads
@@ -521,6 +523,7 @@ __global__ void __launch_bounds__(THREADS, Config<BM, BN>::CTAS_PER_SM) matmul_t
 
 __global__ void splitk_reduce_kernel(const float* __restrict__ ws, float* __restrict__ c, uint64_t count, uint32_t splits,
                                      const float* __restrict__ bias, uint32_t n) {
+    after_producers();
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {
         float acc = ws[i];

@@ -201,6 +201,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
     else __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     const uint32_t tmem_base = *tmem_slot;
+    wait_for_producers();
 
     if (warp < T::LO_WARPS) {
         // ---- lo blocks: the word at an offset of the lo tile belongs to the word at the same offset of the
@@ -332,6 +333,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
                 __syncwarp();
             }
         }
+        let_next_start();  // what is left of this kernel are its last products and their way out
         // A role gave up: the loads still in flight land (a bounded wait each) before the CTA, and
         // with it their shared-memory destination, goes away.
         if (*abort_flag && lane == 0) {

@@ -83,6 +83,7 @@ __global__ void __launch_bounds__(THREADS) heldout_rows_kernel(const float* __re
                                                                 const int32_t* __restrict__ labels, const float* __restrict__ weights,
                                                                 uint32_t rows, uint32_t classes, double* __restrict__ terms,
                                                                 uint32_t* __restrict__ hits, HeldOutState* state) {
+    after_producers();
     __shared__ RowFacts warp_facts[THREADS / 32];
     __shared__ float warp_sums[THREADS / 32];
     __shared__ RowFacts row_facts;

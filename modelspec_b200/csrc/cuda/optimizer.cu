@@ -48,6 +48,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(const UpdateTensor* __restri
                                                      const uint32_t* __restrict__ chunk_start, uint32_t chunk, AdamWConstants c,
                                                      const float* __restrict__ lr_t, const float* __restrict__ c1,
                                                      const float* __restrict__ c2) {
+    after_producers();
     const float lr = lr_t[0], k1 = c1[0], k2 = c2[0];
     const Span s = span_of(tensors, chunk_tensor, chunk_start, chunk);
     const UpdateTensor& t = s.t;
@@ -105,6 +106,7 @@ __global__ void __launch_bounds__(256) adamw_kernel(const UpdateTensor* __restri
 
 // The bf16 working copy of a parameter from its f32 master (after an upload).
 __global__ void working_copy_kernel(const float* __restrict__ p, bf16* __restrict__ p16, uint64_t n) {
+    after_producers();
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) store1(p16 + i, p[i]);
 }
@@ -114,6 +116,7 @@ __global__ void __launch_bounds__(256) sgd_kernel(const UpdateTensor* __restrict
                                                    const uint32_t* __restrict__ chunk_tensor,
                                                    const uint32_t* __restrict__ chunk_start, uint32_t chunk,
                                                    const float* __restrict__ lr) {
+    after_producers();
     const float rate = lr[0];
     const Span s = span_of(tensors, chunk_tensor, chunk_start, chunk);
     const UpdateTensor& t = s.t;

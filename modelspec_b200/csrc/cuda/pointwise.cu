@@ -33,6 +33,7 @@ __device__ __forceinline__ float apply(Binary op, float a, float b) {
 template <bool A_SCALAR, bool B_SCALAR>
 __global__ void binary_kernel(Binary op, const float* __restrict__ a, const float* __restrict__ b,
                               float* __restrict__ out, uint64_t n) {
+    after_producers();
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     float sa = A_SCALAR ? a[0] : 0.0f, sb = B_SCALAR ? b[0] : 0.0f;
@@ -70,6 +71,7 @@ template <class T> __device__ __forceinline__ float apply_as(Unary op, float x) 
 
 template <class T>
 __global__ void unary_kernel(Unary op, const T* __restrict__ a, T* __restrict__ out, uint64_t n) {
+    after_producers();
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x;
     if constexpr (sizeof(T) == 2) {
@@ -102,6 +104,7 @@ __global__ void unary_kernel(Unary op, const T* __restrict__ a, T* __restrict__ 
 template <bool GELU, class T>
 __global__ void act_grad_kernel(const T* __restrict__ a, const T* __restrict__ g,
                                 T* __restrict__ out, uint64_t n) {
+    after_producers();
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     auto one = [](float x, float gg) { return GELU ? gelu_grad_value_for<T>(x, gg) : (x > 0.0f ? gg : 0.0f); };
     if constexpr (sizeof(T) == 2) {
@@ -140,6 +143,7 @@ __global__ void act_grad_kernel(const T* __restrict__ a, const T* __restrict__ g
 }
 
 __global__ void fill_kernel(const float* __restrict__ scalar, float* __restrict__ out, uint64_t n) {
+    after_producers();
     float v = scalar[0];
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t j = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += stride) out[j] = v;
@@ -147,6 +151,7 @@ __global__ void fill_kernel(const float* __restrict__ scalar, float* __restrict_
 
 __global__ void add_rows_kernel(const float* __restrict__ x, const float* __restrict__ b,
                                 float* __restrict__ out, uint64_t n, uint64_t h) {
+    after_producers();
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t j = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += stride)
         out[j] = x[j] + b[j % h];
@@ -155,6 +160,7 @@ __global__ void add_rows_kernel(const float* __restrict__ x, const float* __rest
 // 32 x 32 tiles through shared memory, padded against bank conflicts.
 __global__ void transpose_kernel(const float* __restrict__ a, float* __restrict__ out, uint32_t rows,
                                  uint32_t cols) {
+    after_producers();
     __shared__ float tile[32][33];
     uint32_t tiles_x = (cols + 31) / 32, tiles_y = (rows + 31) / 32;
     for (uint32_t t = blockIdx.x; t < tiles_x * tiles_y; t += gridDim.x) {
@@ -176,6 +182,7 @@ template <class T>
 __global__ void dropout_kernel(const T* __restrict__ x, const int32_t* __restrict__ token,
                                uint32_t seed_lo, uint32_t seed_hi, uint32_t threshold, float scale,
                                uint64_t index_base, T* __restrict__ out, uint64_t n) {
+    after_producers();
     uint32_t id_lo = static_cast<uint32_t>(token[0]), id_hi = static_cast<uint32_t>(token[1]);
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t j = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; j < n; j += stride) {

@@ -23,6 +23,7 @@ enum class Whole : int { Sum, SquaredDifference };
 template <Whole KIND>
 __global__ void whole_stage1(const float* __restrict__ a, const float* __restrict__ b, uint64_t n,
                              double* __restrict__ partial) {
+    after_producers();
     __shared__ double shared[33];
     double acc = 0.0;
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
@@ -40,6 +41,7 @@ __global__ void whole_stage1(const float* __restrict__ a, const float* __restric
 
 __global__ void whole_stage2(const double* __restrict__ partial, uint32_t blocks, double divisor,
                              float* __restrict__ out) {
+    after_producers();
     __shared__ double shared[33];
     double acc = 0.0;
     for (uint32_t j = threadIdx.x; j < blocks; j += blockDim.x) acc += partial[j];
@@ -60,6 +62,7 @@ uint32_t whole_blocks(uint64_t n) {
 template <class T>
 __global__ void sum_rows_stage1(const T* __restrict__ g, uint32_t rows, uint32_t h, uint32_t ld, uint32_t rows_per_chunk,
                                 float* __restrict__ partial, uint32_t* __restrict__ counters, float* __restrict__ out) {
+    after_producers();
     __shared__ float shared[8][32];
     __shared__ bool is_last;
     uint32_t c = blockIdx.x * 32 + threadIdx.x;
@@ -101,6 +104,7 @@ __global__ void sum_rows_stage1(const T* __restrict__ g, uint32_t rows, uint32_t
 template <class T>
 __global__ void sum_rows_stage1_wide(const T* __restrict__ g, uint32_t rows, uint32_t h, uint32_t ld, uint32_t rows_per_chunk,
                                      float* __restrict__ partial) {
+    after_producers();
     __shared__ float4 shared[8][32];
     const uint32_t c = (blockIdx.x * 32 + threadIdx.x) * 4;
     const uint32_t r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
@@ -153,6 +157,7 @@ __device__ __forceinline__ uint32_t job_of_block(const Job* __restrict__ jobs, u
 // The first stage of many column sums in one launch: block b works on the job whose block range
 // holds it, on one 32-column block and one chunk of rows, exactly as sum_rows_stage1 does.
 __global__ void sum_rows_batched_kernel(const RowSumJob* __restrict__ jobs, uint32_t count) {
+    after_producers();
     __shared__ float shared[8][32];
     __shared__ uint32_t which;
     const RowSumJob job = jobs[job_of_block(jobs, count, &which)];
@@ -188,6 +193,7 @@ __global__ void sum_rows_batched_kernel(const RowSumJob* __restrict__ jobs, uint
 
 __global__ void sum_rows_stage2(const float* __restrict__ partial, uint32_t chunks, uint32_t h,
                                 float* __restrict__ out) {
+    after_producers();
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= h) return;
     float total = partial[c];
@@ -196,6 +202,7 @@ __global__ void sum_rows_stage2(const float* __restrict__ partial, uint32_t chun
 }
 
 __global__ void finalize_sums_kernel(const SumJob* __restrict__ jobs, uint32_t count) {
+    after_producers();
     __shared__ float shared[8][32];
     __shared__ uint32_t which;
     const SumJob job = jobs[job_of_block(jobs, count, &which)];

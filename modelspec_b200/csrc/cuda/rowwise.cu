@@ -41,6 +41,7 @@ __device__ __forceinline__ void row_moments(const float* __restrict__ row, uint3
 __global__ void layer_norm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                   const float* __restrict__ beta, float* __restrict__ out, uint32_t rows,
                                   uint32_t h) {
+    after_producers();
     int lane = threadIdx.x & 31;
     uint32_t r = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (r >= rows) return;
@@ -54,6 +55,7 @@ __global__ void layer_norm_kernel(const float* __restrict__ x, const float* __re
 __global__ void layer_norm_grad_x_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
                                          const float* __restrict__ g, float* __restrict__ out, uint32_t rows,
                                          uint32_t h) {
+    after_producers();
     int lane = threadIdx.x & 31;
     uint32_t r = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (r >= rows) return;
@@ -80,6 +82,7 @@ __global__ void layer_norm_grad_x_kernel(const float* __restrict__ x, const floa
 
 __global__ void row_stats_kernel(const float* __restrict__ x, float* __restrict__ stats, uint32_t rows,
                                  uint32_t h) {
+    after_producers();
     int lane = threadIdx.x & 31;
     uint32_t r = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
     if (r >= rows) return;
@@ -97,6 +100,7 @@ __global__ void grad_gamma_stage1(const float* __restrict__ x, const float* __re
                                   const float* __restrict__ stats, uint32_t rows, uint32_t h,
                                   uint32_t rows_per_chunk, float* __restrict__ partial_gamma,
                                   float* __restrict__ partial_beta) {
+    after_producers();
     __shared__ float sg[8][32], sb[8][32];
     uint32_t c = blockIdx.x * 32 + threadIdx.x;
     uint32_t r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
@@ -126,6 +130,7 @@ __global__ void grad_gamma_stage1(const float* __restrict__ x, const float* __re
 __global__ void grad_gamma_stage2(const float* __restrict__ partial_gamma, const float* __restrict__ partial_beta,
                                   uint32_t chunks, uint32_t h, float* __restrict__ dgamma,
                                   float* __restrict__ dbeta) {
+    after_producers();
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= h) return;
     float tg = partial_gamma[c];
@@ -158,6 +163,7 @@ __device__ __forceinline__ void block_row_softmax(const T* __restrict__ row, uin
 }
 
 __global__ void softmax_kernel(const float* __restrict__ x, float* __restrict__ out, uint32_t k) {
+    after_producers();
     __shared__ float shared[33];
     const float* row = x + static_cast<uint64_t>(blockIdx.x) * k;
     float max, total;
@@ -168,6 +174,7 @@ __global__ void softmax_kernel(const float* __restrict__ x, float* __restrict__ 
 
 __global__ void softmax_grad_kernel(const float* __restrict__ y, const float* __restrict__ g,
                                     float* __restrict__ out, uint32_t k) {
+    after_producers();
     __shared__ float shared[33];
     const float* yr = y + static_cast<uint64_t>(blockIdx.x) * k;
     const float* gr = g + static_cast<uint64_t>(blockIdx.x) * k;
@@ -182,6 +189,7 @@ template <class T>
 __global__ void cross_entropy_rows_kernel(const T* __restrict__ logits, const int32_t* __restrict__ labels,
                                           const float* __restrict__ weights, float* __restrict__ row_loss,
                                           uint32_t v, uint32_t ld) {
+    after_producers();
     __shared__ float shared[33];
     uint32_t r = blockIdx.x;
     // A row of weight 0 adds w * l = 0 to the loss whatever its logits: skip its passes.
@@ -202,6 +210,7 @@ __global__ void cross_entropy_rows_kernel(const T* __restrict__ logits, const in
 // loss = sum_n w[n] l[n] / sum_n w[n], both sums in f64 (a tree over the block), one rounding.
 __global__ void cross_entropy_loss_kernel(const float* __restrict__ row_loss, const float* __restrict__ weights,
                                           uint32_t rows, const float* __restrict__ global_den, float* __restrict__ loss) {
+    after_producers();
     __shared__ double shared[33];
     double num = 0.0, den = 0.0;
     for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) {
@@ -217,6 +226,7 @@ __global__ void cross_entropy_loss_kernel(const float* __restrict__ row_loss, co
 }
 
 __global__ void weight_sum_kernel(const float* __restrict__ weights, uint32_t rows, float* __restrict__ out) {
+    after_producers();
     __shared__ double shared[33];
     double den = 0.0;
     for (uint32_t r = threadIdx.x; r < rows; r += blockDim.x) den += static_cast<double>(weights[r]);
@@ -228,6 +238,7 @@ __global__ void cross_entropy_grad_kernel(const float* __restrict__ logits, cons
                                           const float* __restrict__ weights, const float* __restrict__ g,
                                           const float* __restrict__ denominator, float* __restrict__ out,
                                           uint32_t v, uint32_t ld, uint32_t ld_out) {
+    after_producers();
     __shared__ float shared[33];
     uint32_t r = blockIdx.x;
     float* o = out + static_cast<uint64_t>(r) * ld_out;
@@ -255,6 +266,7 @@ __global__ void cross_entropy_fused_kernel(const T* __restrict__ logits, const i
                                            const float* __restrict__ weights, const float* __restrict__ g,
                                            const float* __restrict__ denominator, float* __restrict__ row_loss,
                                            T* __restrict__ out, uint32_t v, uint32_t ld, uint32_t ld_out) {
+    after_producers();
     __shared__ float shared[33];
     uint32_t r = blockIdx.x;
     T* o = out + static_cast<uint64_t>(r) * ld_out;
@@ -295,6 +307,7 @@ cross_entropy_fused_wide_kernel(const T* __restrict__ logits, const int32_t* __r
                                 const float* __restrict__ denominator, float* __restrict__ row_loss,
                                 T* __restrict__ out, uint32_t v, uint32_t ld, uint32_t ld_out,
                                 uint32_t* __restrict__ counter, float* __restrict__ loss) {
+    after_producers();
     // Element i of this thread is column column_of(i): consecutive threads take consecutive columns.
     auto column_of = [](int i, uint32_t tid) { return static_cast<uint32_t>(i) * kWideThreads + tid; };
     __shared__ float shared[33];
@@ -410,6 +423,7 @@ cross_entropy_row_kernel(const T* __restrict__ logits, const int32_t* __restrict
                          const float* __restrict__ g, const float* __restrict__ denominator, float* __restrict__ row_loss,
                          T* __restrict__ out, uint32_t rows, uint32_t v, uint32_t ld, uint32_t ld_out, uint32_t* __restrict__ counter,
                          float* __restrict__ loss) {
+    after_producers();
     static_assert(ROWS == 1 || THREADS == 32);
     constexpr bool HALF = sizeof(T) == 2;
     constexpr uint32_t E = 16 / sizeof(T), ALL = THREADS * ROWS, WARPS = ALL / 32;
@@ -573,6 +587,7 @@ cross_entropy_fused_split_kernel(const float* __restrict__ logits, const int32_t
                                  const float* __restrict__ denominator, float* __restrict__ row_loss,
                                  float* __restrict__ out, uint32_t v, uint32_t ld, uint32_t ld_out,
                                  uint32_t* __restrict__ counter, float* __restrict__ loss) {
+    after_producers();
     // Group k of this thread is the four columns from (k * threads + tid) * 4 on: groups 0..7 live in
     // registers, groups 8..15 in shared memory.
     extern __shared__ float4 parked[];  // [kSplitSharedItems / 4][kSplitThreads]
@@ -840,6 +855,7 @@ __global__ void __launch_bounds__(256, !EXACT ? 1 : ITEMS >= 32 ? 2 : ITEMS >= 2
     const T* __restrict__ x, const T* __restrict__ residual, DropoutDraw x_draw, const float* __restrict__ gamma,
     const float* __restrict__ beta, T* __restrict__ sum_out, T* __restrict__ out, DropoutDraw out_draw,
     T* __restrict__ out_dropped, uint32_t rows, uint32_t width_given, bool gelu_first) {
+    after_producers();
     const uint32_t h = EXACT ? 32u * ITEMS : width_given;
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t r = blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
@@ -928,6 +944,7 @@ __global__ void __launch_bounds__(256, ITEMS <= 2 || (ITEMS <= 4 && EXACT && siz
     float* __restrict__ partial, uint32_t* __restrict__ counter, float* __restrict__ dgamma, float* __restrict__ dbeta,
     uint32_t want, uint32_t rows, uint32_t width_given, uint32_t rows_per_chunk, DropoutDraw adjoint_draw, DropoutDraw dx_draw,
     T* __restrict__ dx_dropped, const T* __restrict__ pre_activation) {
+    after_producers();
     constexpr bool WIDE = ITEMS >= 16;
     const uint32_t h = EXACT ? 32u * ITEMS : width_given;
     extern __shared__ float backward_sums[];  // 8 * 32 * ITEMS floats, twice that for wide rows

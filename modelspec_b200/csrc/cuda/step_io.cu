@@ -20,6 +20,7 @@ constexpr int kTakeThreads = 256, kTakeChunks = 4;
 // reads of one host address are served one after the other, about a microsecond each.
 __global__ void __launch_bounds__(kTakeThreads) take_inputs_kernel(const __grid_constant__ InputSlots slots, uint64_t chunks, uint4* __restrict__ to,
                                                                     const uint32_t* __restrict__ turn) {
+    after_producers();
     const uint4* from = reinterpret_cast<const uint4*>(slots.at[*turn % slots.count]);
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kTakeThreads;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * kTakeThreads + threadIdx.x; i < chunks; i += kTakeChunks * stride) {
@@ -35,6 +36,7 @@ __global__ void __launch_bounds__(kTakeThreads) take_inputs_kernel(const __grid_
 
 __global__ void publish_step_kernel(const float* __restrict__ loss, const uint32_t* __restrict__ status, float* __restrict__ to_loss,
                                     uint32_t* __restrict__ to_status, uint32_t* __restrict__ turn, uint32_t slots) {
+    after_producers();
     const uint32_t slot = *turn;
     if (loss) to_loss[slot] = *loss;
     to_status[slot] = *status;

@@ -79,3 +79,22 @@ def test_a_bad_batch_is_refused_by_its_step_and_the_run_goes_on(device):
             assert good.loss_of(k) == bad.loss_of(k)
     finally:
         good.destroy(); bad.destroy()
+
+
+def test_kernels_that_start_early_give_the_same_bits(device):
+    """MSX_FUSE bit 128: kernels of a captured step launched while the one before them ends. The same kernels on the same
+    values: every loss, parameter and moment has the same bits with the bit on and off, in both precisions."""
+    import json
+    import os
+    import subprocess
+    import sys
+    here = os.path.dirname(os.path.abspath(__file__))
+    results = []
+    for mask in ("127", "255"):
+        env = dict(os.environ, MSX_FUSE=mask, PYTHONPATH=os.pathsep.join([os.path.dirname(here), here, os.environ.get("PYTHONPATH", "")]))
+        done = subprocess.run([sys.executable, os.path.join(here, "fuse_worker.py")], env=env, capture_output=True, text=True, timeout=600)
+        assert done.returncode == 0, done.stderr[-2000:]
+        results.append(json.loads(done.stdout.strip().splitlines()[-1]))
+    for precision in ("f32", "bf16"):
+        assert results[0][precision]["losses"] == results[1][precision]["losses"], precision
+        assert results[0][precision]["state"] == results[1][precision]["state"], precision
