@@ -198,6 +198,10 @@ template <class T> __device__ __forceinline__ float gelu_grad_value_for(float x,
     }
 }
 
+// relu and the two gradients' shared form, as the element kernels compute them.
+__device__ __forceinline__ float relu_value(float x) { return x > 0.0f ? x : 0.0f; }
+__device__ __forceinline__ float relu_grad_value(float x, float g) { return x > 0.0f ? g : 0.0f; }
+
 // ---- Philox4x32-10, word 0 of the block ------------------------------------------------------
 // Counter [c0, c1, c2, c3], key [k0, k1] (Salmon et al., SC 2011); the reference draws a dropout
 // decision from word 0 alone (crates/modelspec-runtime/src/train/init.rs:91-112, :160-165).

@@ -34,10 +34,12 @@ struct Problem {
     uint32_t splits;    // of k into partial results
     uint32_t first_block;
     uint32_t a_vec, b_vec;
+    float* beside;      // the epilogue's second matrix, of C's rows
 };
 template <int COUNT> struct Problems {
     uint32_t count;
     uint32_t cluster;  // CTAs that share one tile's k; splits are then 1
+    Epilogue epilogue;
     Problem p[COUNT];
 };
 
@@ -58,6 +60,7 @@ constexpr int THREADS = GROUP * G;
 constexpr int A_PITCH = BM + 4, B_PITCH = BN + 4;
 constexpr int SLAB = KS * (A_PITCH + B_PITCH);  // floats
 constexpr int SHARED_BYTES = G * 2 * SLAB * 4;
+static_assert(BM * BN / THREADS <= 2 && BM * BN % THREADS == 0, "a thread's elements");
 constexpr int A_FOURS = BM * KS / 4 / GROUP, B_FOURS = BN * KS / 4 / GROUP;
 static_assert(G * BM * BN <= G * 2 * SLAB, "the groups' sums take the slabs' place");
 
@@ -65,7 +68,8 @@ __device__ __forceinline__ void cluster_barrier() {
     asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
 
-template <bool A_T, bool B_T, int COUNT>
+// ACT: with an epilogue (an instantiation of its own: its code in every product cost a transformer block's step 2.7 %).
+template <bool A_T, bool B_T, int COUNT, bool ACT>
 __global__ void __launch_bounds__(THREADS) matmul_small_kernel(const __grid_constant__ Problems<COUNT> problems) {
     after_producers();
     extern __shared__ __align__(16) float shared[];
@@ -141,6 +145,22 @@ __global__ void __launch_bounds__(THREADS) matmul_small_kernel(const __grid_cons
     };
     auto group_barrier = [&] { asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(GROUP) : "memory"); };
 
+    // The arguments of the activations whose gradient this thread's elements take: fetched with the first slabs (behind
+    // the sums they would be a trip to memory of their own).
+    constexpr uint32_t OWN = BM * BN / THREADS;
+    const Epilogue epilogue = ACT ? problems.epilogue : Epilogue::None;
+    float argument[ACT ? OWN : 1];
+    if constexpr (ACT) {
+        if (epilogue == Epilogue::GeluGrad || epilogue == Epilogue::ReluGrad) {
+            const uint32_t share = BM * BN / cluster, end = (rank + 1) * share;
+#pragma unroll
+            for (uint32_t i = 0; i < OWN; ++i) {
+                const uint32_t e = rank * share + threadIdx.x + i * THREADS, row = m0 + e / BN, col = n0 + e % BN;
+                argument[i] = e < end && row < m && col < n ? __ldg(p.beside + static_cast<uint64_t>(row) * p.ldc + col) : 0.0f;
+            }
+        }
+    }
+
     const uint32_t tm = t / (BN / 4) * TM, tn = t % (BN / 4) * 4;
     float acc[TM][4];
 #pragma unroll
@@ -184,13 +204,23 @@ __global__ void __launch_bounds__(THREADS) matmul_small_kernel(const __grid_cons
         for (int g = 1; g < G; ++g) v += shared[g * BM * BN + e];
         return v;
     };
-    auto store = [&](uint32_t e, float v) {
+    // Element e of the tile, the thread's i-th.
+    auto store = [&](uint32_t e, uint32_t i, float v) {
         const uint32_t row = m0 + e / BN, col = n0 + e % BN;
-        if (row < m && col < n) out[static_cast<uint64_t>(row) * p.ldc + col] = bias ? v + __ldg(bias + col) : v;
+        if (row >= m || col >= n) return;
+        const uint64_t at = static_cast<uint64_t>(row) * p.ldc + col;
+        v = bias ? v + __ldg(bias + col) : v;
+        if constexpr (ACT) {
+            const float x = argument[OWN == 2 ? i & 1u : i];
+            if (epilogue == Epilogue::GeluGrad) v = gelu_grad_value(x, v);
+            else if (epilogue == Epilogue::ReluGrad) v = relu_grad_value(x, v);
+            else p.beside[at] = epilogue == Epilogue::Gelu ? gelu_value(v) : relu_value(v);
+        }
+        out[at] = v;
     };
     if (cluster == 1) {
 #pragma unroll
-        for (uint32_t e = threadIdx.x; e < BM * BN; e += THREADS) store(e, sum_of(e));
+        for (uint32_t i = 0; i < OWN; ++i) store(threadIdx.x + i * THREADS, i, sum_of(threadIdx.x + i * THREADS));
         return;
     }
     // Each CTA of the cluster adds its groups, then its share of the tile over the CTAs in ascending order.
@@ -202,7 +232,8 @@ __global__ void __launch_bounds__(THREADS) matmul_small_kernel(const __grid_cons
     for (int i = 0; i < BM * BN / THREADS; ++i) shared[threadIdx.x + i * THREADS] = total[i];
     cluster_barrier();
     const uint32_t share = BM * BN / cluster;
-    for (uint32_t e = rank * share + threadIdx.x; e < (rank + 1) * share; e += THREADS) {
+    uint32_t i = 0;
+    for (uint32_t e = rank * share + threadIdx.x; e < (rank + 1) * share; e += THREADS, ++i) {
         float v = 0.f;
         for (uint32_t r = 0; r < cluster; ++r) {
             float term;
@@ -210,13 +241,13 @@ __global__ void __launch_bounds__(THREADS) matmul_small_kernel(const __grid_cons
                          : "=f"(term) : "r"(static_cast<uint32_t>(__cvta_generic_to_shared(shared + e))), "r"(r) : "memory");
             v = r == 0 ? term : v + term;
         }
-        store(e, v);
+        store(e, i, v);
     }
     cluster_barrier();  // no CTA goes away while another reads its tile
 }
 
-template <bool A_T, bool B_T, int COUNT> void launch(cudaStream_t s, const Problems<COUNT>& problems, uint32_t blocks) {
-    auto kernel = matmul_small_kernel<A_T, B_T, COUNT>;
+template <bool A_T, bool B_T, bool ACT, int COUNT> void launch(cudaStream_t s, const Problems<COUNT>& problems, uint32_t blocks) {
+    auto kernel = matmul_small_kernel<A_T, B_T, COUNT, ACT>;
     static std::atomic<int> configured_device{-1};
     set_shared_memory(kernel, SHARED_BYTES, configured_device);
     cudaLaunchConfig_t config = {};
@@ -235,10 +266,19 @@ template <bool A_T, bool B_T, int COUNT> void launch(cudaStream_t s, const Probl
     check(cudaLaunchKernelEx(&config, kernel, problems), "matmul_small");
 }
 template <int COUNT> void launch_form(cudaStream_t s, bool a_t, bool b_t, const Problems<COUNT>& problems, uint32_t blocks) {
-    if (a_t && b_t) launch<true, true>(s, problems, blocks);
-    else if (a_t) launch<true, false>(s, problems, blocks);
-    else if (b_t) launch<false, true>(s, problems, blocks);
-    else launch<false, false>(s, problems, blocks);
+    if constexpr (COUNT == MAX_PRODUCTS) {
+        if (problems.epilogue != Epilogue::None) {
+            if (a_t && b_t) launch<true, true, true>(s, problems, blocks);
+            else if (a_t) launch<true, false, true>(s, problems, blocks);
+            else if (b_t) launch<false, true, true>(s, problems, blocks);
+            else launch<false, false, true>(s, problems, blocks);
+            return;
+        }
+    }
+    if (a_t && b_t) launch<true, true, false>(s, problems, blocks);
+    else if (a_t) launch<true, false, false>(s, problems, blocks);
+    else if (b_t) launch<false, true, false>(s, problems, blocks);
+    else launch<false, false, false>(s, problems, blocks);
 }
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
@@ -246,7 +286,7 @@ bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0;
 Problem problem_of(const float* a, const float* b, float* c, const float* bias, uint64_t m, uint64_t n, uint64_t k, uint64_t lda, uint64_t ldb, uint64_t ldc,
                    uint32_t splits, uint32_t first_block) {
     Problem p = {a, b, c, bias, static_cast<uint32_t>(m), static_cast<uint32_t>(n), static_cast<uint32_t>(k), static_cast<uint32_t>(lda),
-                 static_cast<uint32_t>(ldb), static_cast<uint32_t>(ldc), splits, first_block, 0, 0};
+                 static_cast<uint32_t>(ldb), static_cast<uint32_t>(ldc), splits, first_block, 0, 0, nullptr};
     p.a_vec = aligned16(a) && lda % 4 == 0;
     p.b_vec = aligned16(b) && ldb % 4 == 0;
     return p;
@@ -256,13 +296,15 @@ uint32_t blocks_of(uint64_t m, uint64_t n) { return static_cast<uint32_t>(((m + 
 }  // namespace
 
 void matmul_small(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* products, uint32_t count, bool a_t, bool b_t, uint64_t m, uint64_t n, uint64_t k,
-                  MatmulPitches pitches) {
+                  MatmulPitches pitches, Epilogue epilogue, float* beside) {
     Problems<MAX_PRODUCTS> problems = {};
     problems.cluster = p.cluster;
+    problems.epilogue = epilogue;
     uint32_t blocks = 0;
     for (uint32_t g = 0; g < count; ++g) {
         problems.p[problems.count++] = problem_of(products[g].a, products[g].b, products[g].c, products[g].bias, m, n, k, pitches.a ? pitches.a : (a_t ? m : k),
                                                   pitches.b ? pitches.b : (b_t ? k : n), pitches.c ? pitches.c : n, 1, blocks);
+        problems.p[g].beside = beside;
         blocks += blocks_of(m, n) * p.cluster;
     }
     launch_form(s, a_t, b_t, problems, blocks);

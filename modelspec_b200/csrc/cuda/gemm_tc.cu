@@ -75,6 +75,9 @@ struct TcArgs {
     uint32_t lda, ldb, ldc;        // row pitch, in elements, of each matrix as stored
     uint32_t a_vec, b_vec, c_vec;  // 16-byte accesses are aligned for this operand
     uint32_t c_padded;             // the columns of C between n and ldc are padding that may be overwritten
+    Epilogue epilogue;             // of one product
+    float* beside;
+    uint32_t beside_vec;
     // Batched products: grid.z = batch index z, split as (z / inner, z % inner); each matrix of
     // problem z starts at outer * stride_outer + inner * stride_inner elements. inner = 0: not batched.
     uint32_t batch_inner;
@@ -202,7 +205,8 @@ __device__ __forceinline__ void loaders_barrier(uint32_t threads) {
     asm volatile("bar.sync 1, %0;" ::"r"(threads) : "memory");
 }
 
-template <int BM, int BN, bool A_T, bool B_T>
+// ACT: with an epilogue.
+template <int BM, int BN, bool A_T, bool B_T, bool ACT>
 __global__ void __launch_bounds__(THREADS, Config<BM, BN>::CTAS_PER_SM) matmul_tc_kernel(TcArgs args) {
     using Cfg = Config<BM, BN>;
     constexpr int STAGES = Cfg::STAGES, SETS = Cfg::SETS;
@@ -459,6 +463,34 @@ __global__ void __launch_bounds__(THREADS, Config<BM, BN>::CTAS_PER_SM) matmul_t
 #pragma unroll
                 for (int q = 0; q < 4; ++q) v[q] = v[q] + bias_mine[q];
             }
+            if (ACT) {
+                // The second matrix has C's rows.
+                float* const at = args.beside + static_cast<uint64_t>(gm) * pldc + gn;
+                const bool whole = args.beside_vec && gn + 4 <= pn;
+                float other[4] = {0.f, 0.f, 0.f, 0.f};
+                if (args.epilogue == Epilogue::GeluGrad || args.epilogue == Epilogue::ReluGrad) {
+                    if (whole) {
+                        const float4 f = __ldg(reinterpret_cast<const float4*>(at));
+                        other[0] = f.x; other[1] = f.y; other[2] = f.z; other[3] = f.w;
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (gn + q < pn) other[q] = __ldg(at + q);
+                    }
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) v[q] = args.epilogue == Epilogue::GeluGrad ? gelu_grad_value(other[q], v[q]) : relu_grad_value(other[q], v[q]);
+                } else {
+#pragma unroll
+                    for (int q = 0; q < 4; ++q) other[q] = args.epilogue == Epilogue::Gelu ? gelu_value(v[q]) : relu_value(v[q]);
+                    if (whole) {
+                        *reinterpret_cast<float4*>(at) = make_float4(other[0], other[1], other[2], other[3]);
+                    } else {
+#pragma unroll
+                        for (int q = 0; q < 4; ++q)
+                            if (gn + q < pn) at[q] = other[q];
+                    }
+                }
+            }
             float* dst = out + static_cast<uint64_t>(gm) * pldc + gn;
             // Inside the pitch a whole float4 may be written: what lies past n is padding.
             if (args.c_vec && (gn + 4 <= pn || (args.c_padded && gn + 4 <= pldc))) {
@@ -532,25 +564,25 @@ __global__ void splitk_reduce_kernel(const float* __restrict__ ws, float* __rest
     }
 }
 
-template <int BM, int BN, bool A_T, bool B_T> void launch(cudaStream_t s, const TcArgs& args, dim3 grid) {
-    auto kernel = matmul_tc_kernel<BM, BN, A_T, B_T>;
+template <int BM, int BN, bool ACT, bool A_T, bool B_T> void launch(cudaStream_t s, const TcArgs& args, dim3 grid) {
+    auto kernel = matmul_tc_kernel<BM, BN, A_T, B_T, ACT>;
     static std::atomic<int> configured_device{-1};
     set_shared_memory(kernel, static_cast<int>(Config<BM, BN>::TOTAL), configured_device);
     kernel<<<grid, THREADS, Config<BM, BN>::TOTAL, s>>>(args);
     check_launch("matmul_tc");
 }
 
-template <int BM, int BN> void launch_forms(cudaStream_t s, const TcArgs& args, dim3 grid, bool a_t, bool b_t) {
-    if (a_t && b_t) launch<BM, BN, true, true>(s, args, grid);
-    else if (a_t) launch<BM, BN, true, false>(s, args, grid);
-    else if (b_t) launch<BM, BN, false, true>(s, args, grid);
-    else launch<BM, BN, false, false>(s, args, grid);
+template <int BM, int BN, bool ACT> void launch_forms(cudaStream_t s, const TcArgs& args, dim3 grid, bool a_t, bool b_t) {
+    if (a_t && b_t) launch<BM, BN, ACT, true, true>(s, args, grid);
+    else if (a_t) launch<BM, BN, ACT, true, false>(s, args, grid);
+    else if (b_t) launch<BM, BN, ACT, false, true>(s, args, grid);
+    else launch<BM, BN, ACT, false, false>(s, args, grid);
 }
 
-void launch_tile(cudaStream_t s, const TcArgs& args, dim3 grid, uint32_t bn, bool a_t, bool b_t) {
-    if (bn == 32) launch_forms<64, 32>(s, args, grid, a_t, b_t);
-    else if (bn == 64) launch_forms<64, 64>(s, args, grid, a_t, b_t);
-    else launch_forms<64, 128>(s, args, grid, a_t, b_t);
+template <bool ACT> void launch_tile(cudaStream_t s, const TcArgs& args, dim3 grid, uint32_t bn, bool a_t, bool b_t) {
+    if (bn == 32) launch_forms<64, 32, ACT>(s, args, grid, a_t, b_t);
+    else if (bn == 64) launch_forms<64, 64, ACT>(s, args, grid, a_t, b_t);
+    else launch_forms<64, 128, ACT>(s, args, grid, a_t, b_t);
 }
 
 bool aligned16(const void* p) { return reinterpret_cast<uintptr_t>(p) % 16 == 0; }
@@ -645,7 +677,7 @@ MatmulTcPlan matmul_tc_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t problem
 }
 
 void matmul_tc_group(cudaStream_t s, const MatmulOperands* products, uint32_t count, bool a_t, bool b_t, uint64_t m, uint64_t n,
-                     uint64_t k, uint32_t* status, bool leave_partials, MatmulPitches pitches) {
+                     uint64_t k, uint32_t* status, bool leave_partials, MatmulPitches pitches, Epilogue epilogue, float* beside) {
     if (m == 0 || n == 0 || count == 0) return;
     if (count > MAX_GROUP) throw std::invalid_argument("matmul_tc_group: more products than one launch carries");
     // The TMA-fed tiles want bases on 16 bytes and rows a multiple of 16 bytes apart.
@@ -653,8 +685,10 @@ void matmul_tc_group(cudaStream_t s, const MatmulOperands* products, uint32_t co
     for (uint32_t g = 0; g < count; ++g) tma_ok = tma_ok && aligned16(products[g].a) && aligned16(products[g].b);
     MatmulTcPlan p = matmul_tc_plan(m, n, k, 1, count, tma_ok);
     if (pitches.c && p.splits > 1) throw std::invalid_argument("matmul_tc_group: a pitched result with a split k");
+    if (epilogue != Epilogue::None && (count != 1 || pitches.c || !beside || !matmul_takes_epilogue(p)))
+        throw std::invalid_argument("matmul_tc_group: an epilogue for one dense product on the small tiles");
     if (p.fma) {
-        matmul_small(s, p, products, count, a_t, b_t, m, n, k, pitches);
+        matmul_small(s, p, products, count, a_t, b_t, m, n, k, pitches, epilogue, beside);
     } else if (p.bm >= 128) {
         matmul_tf32(s, p, products, count, a_t, b_t, m, n, k, 1, pitches, status);
     } else {
@@ -682,7 +716,12 @@ void matmul_tc_group(cudaStream_t s, const MatmulOperands* products, uint32_t co
             args.b_vec = args.b_vec && aligned16(products[g].b);
         }
         args.status = status;
-        launch_tile(s, args, dim3(static_cast<uint32_t>((n + p.bn - 1) / p.bn), static_cast<uint32_t>((m + p.bm - 1) / p.bm), p.splits * count), p.bn, a_t, b_t);
+        args.epilogue = epilogue;
+        args.beside = beside;
+        args.beside_vec = args.ldc % 4 == 0 && aligned16(beside);
+        const dim3 grid(static_cast<uint32_t>((n + p.bn - 1) / p.bn), static_cast<uint32_t>((m + p.bm - 1) / p.bm), p.splits * count);
+        if (epilogue != Epilogue::None) launch_tile<true>(s, args, grid, p.bn, a_t, b_t);
+        else launch_tile<false>(s, args, grid, p.bn, a_t, b_t);
     }
     if (p.splits > 1 && !leave_partials) {
         uint64_t total = m * n;
@@ -764,7 +803,7 @@ void matmul_tc_jobs(cudaStream_t s, const MatmulJob* jobs, uint32_t count, bool 
         args.b_vec = args.b_vec && aligned16(job.b) && to.ldb % 4 == 0;
         args.c_vec = args.c_vec && aligned16(to.c) && to.ldc % 4 == 0;
     }
-    launch_tile(s, args, dim3(blocks), 64, a_t, b_t);
+    launch_tile<false>(s, args, dim3(blocks), 64, a_t, b_t);
 }
 
 namespace {
@@ -795,7 +834,7 @@ void launch_batched(cudaStream_t s, const BatchedOperand& a, const BatchedOperan
     args.status = status;
     const MatmulTcPlan p = matmul_tc_plan(m, n, k, static_cast<uint64_t>(outer) * inner, 1, false, 1, true);
     dim3 grid(static_cast<uint32_t>((n + p.bn - 1) / p.bn), static_cast<uint32_t>((m + p.bm - 1) / p.bm), outer * inner);
-    launch_tile(s, args, grid, p.bn, a.transposed, b.transposed);
+    launch_tile<false>(s, args, grid, p.bn, a.transposed, b.transposed);
 }
 }  // namespace
 

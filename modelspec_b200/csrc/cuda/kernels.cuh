@@ -266,6 +266,9 @@ void matmul(cudaStream_t s, const float* a, bool a_t, const float* b, bool b_t, 
 // A wait that runs out inside the kernel raises bit 1 of *status instead of hanging. With
 // `leave_partials` a split k stops at the partial tiles, workspace[split][m][n], for
 // finalize_sums (no bias then).
+// What is applied to a result as it is stored: nothing; gelu or relu, stored in `beside` while C keeps their
+// argument; the gradient of either at the argument in `beside`, times the product, stored in C.
+enum class Epilogue : int { None, Gelu, GeluGrad, Relu, ReluGrad };
 struct MatmulTcPlan {
     uint32_t bm, bn, splits, kblocks_per_split;  // tile rows and width, k split
     bool fma;                                    // on the FMA units (gemm_small.cu),
@@ -297,8 +300,12 @@ struct MatmulOperands {
 struct MatmulPitches {
     uint32_t a = 0, b = 0, c = 0;
 };
+// An epilogue is for one product with a dense C that its plan gives to the FMA tiles or the 64-row tiles, k unsplit
+// (matmul_takes_epilogue); `beside` is dense as well.
 void matmul_tc_group(cudaStream_t s, const MatmulOperands* products, uint32_t count, bool a_t, bool b_t, uint64_t m, uint64_t n,
-                     uint64_t k, uint32_t* status, bool leave_partials = false, MatmulPitches pitches = {});
+                     uint64_t k, uint32_t* status, bool leave_partials = false, MatmulPitches pitches = {}, Epilogue epilogue = Epilogue::None,
+                     float* beside = nullptr);
+inline bool matmul_takes_epilogue(const MatmulTcPlan& p) { return p.splits == 1 && (p.fma || p.bm == 64); }
 
 // Products of different shapes, one storage form, in one launch (the weight gradients of a step,
 // which only the optimizer reads and which would each fill a fraction of the device for a few
@@ -317,7 +324,7 @@ void matmul_tf32(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* pr
                  uint32_t chain, MatmulPitches pitches, uint32_t* status);
 // Small products on the FMA units (gemm_small.cu).
 void matmul_small(cudaStream_t s, const MatmulTcPlan& p, const MatmulOperands* products, uint32_t count, bool a_t, bool b_t, uint64_t m, uint64_t n, uint64_t k,
-                  MatmulPitches pitches);
+                  MatmulPitches pitches, Epilogue epilogue = Epilogue::None, float* beside = nullptr);
 constexpr uint32_t kMatmulJobs = 24;  // jobs one launch carries
 MatmulTcPlan matmul_tc_job_plan(uint64_t m, uint64_t n, uint64_t k);
 // The jobs on the TMA-fed 128 x 128 tile, when TMA can address every operand and result; false when it
@@ -376,9 +383,6 @@ MatmulBf16Plan matmul_bf16_plan(uint64_t m, uint64_t n, uint64_t k, uint64_t pro
 // that runs out inside the kernel raises bit 1 of *status.
 void matmul_bf16(cudaStream_t s, const HalfMatrix& a, const HalfMatrix& b, const HalfResult& c, uint64_t m, uint64_t n, uint64_t k,
                  uint32_t outer, uint32_t inner, float* workspace, const float* bias, uint32_t* status, bool leave_partials = false);
-// What is applied to a bf16 result as it drains: nothing; gelu, stored in `beside` while C keeps its
-// argument; the gradient of gelu at the argument in `beside`, times the product, stored in C.
-enum class Epilogue { None, Gelu, GeluGrad };
 struct HalfProduct {
     HalfMatrix a, b;
     HalfResult c;

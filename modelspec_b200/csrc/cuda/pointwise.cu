@@ -62,7 +62,7 @@ __global__ void binary_kernel(Binary op, const float* __restrict__ a, const floa
 
 template <class T> __device__ __forceinline__ float apply_as(Unary op, float x) {
     switch (op) {
-        case Unary::Relu: return x > 0.0f ? x : 0.0f;
+        case Unary::Relu: return relu_value(x);
         case Unary::Sqrt: return sqrtf(x);
         case Unary::Gelu: return gelu_value_for<T>(x);
         default: return x;
@@ -106,7 +106,7 @@ __global__ void act_grad_kernel(const T* __restrict__ a, const T* __restrict__ g
                                 T* __restrict__ out, uint64_t n) {
     after_producers();
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    auto one = [](float x, float gg) { return GELU ? gelu_grad_value_for<T>(x, gg) : (x > 0.0f ? gg : 0.0f); };
+    auto one = [](float x, float gg) { return GELU ? gelu_grad_value_for<T>(x, gg) : relu_grad_value(x, gg); };
     if constexpr (sizeof(T) == 2) {
         // bf16: 16 bytes (eight elements) of each array per thread and turn.
         if ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(g)) % 16 == 0) {

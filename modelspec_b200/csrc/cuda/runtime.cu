@@ -1926,6 +1926,27 @@ struct Scheduler {
         k::MatmulPitches pitches;
         pitches.a = pitch_of(first.a);
         pitches.b = pitch_of(first.b);
+        // gelu, relu or the gradient of either behind a product of the small tiles, as it is stored (their own launch is 2 to 3 us
+        // of a step; on the TMA-fed tiles, whose drain sets their pace, they cost as much as it).
+        const int behind = count == 1 && k::matmul_takes_epilogue(tc) && !pitchable(first.result) ? activation_behind(first) : -1;
+        k::Epilogue epilogue = k::Epilogue::None;
+        uint32_t beside = 0, result_of_first = first.result;
+        if (behind >= 0) {
+            const uint32_t u = static_cast<uint32_t>(behind);
+            const Op op = node(u).op;
+            epilogue = op == Op::Gelu ? k::Epilogue::Gelu : op == Op::Relu ? k::Epilogue::Relu : op == Op::GeluGrad ? k::Epilogue::GeluGrad : k::Epilogue::ReluGrad;
+            handled[u] = 1;
+            make_arena(P->slots[u], node(u));
+            if (op == Op::Gelu || op == Op::Relu) {
+                beside = u;
+                writes.push_back(u);
+            } else {
+                beside = pos(node(u).operands[0]);
+                reads.push_back(beside);
+                P->slots[first.result].kind = Slot::Dead;
+                result_of_first = u;
+            }
+        }
         if (count == 1 && tc.splits == 1 && pitchable(first.result)) {
             set_pitch(first.result);
             pitches.c = P->slots[first.result].pitch;
@@ -1940,7 +1961,7 @@ struct Scheduler {
             }
             workspaces.push_back(ws);
             if (defer) deferred.push_back({static_cast<uint32_t>(ws), 0, tc.splits, m * n, p.result});
-            else writes.push_back(p.result);
+            else writes.push_back(behind >= 0 ? result_of_first : p.result);
         }
         Launch& l = emit("matmul", nd, reads, writes, [=](cudaStream_t s) {
             k::MatmulOperands operands[4];
@@ -1948,13 +1969,13 @@ struct Scheduler {
                 const Product& p = products[g];
                 operands[g].a = plan->f(p.a);
                 operands[g].b = plan->f(p.b);
-                operands[g].c = plan->f(p.result);
+                operands[g].c = plan->f(g == 0 ? result_of_first : p.result);
                 operands[g].bias = p.bias >= 0 ? plan->f(static_cast<uint32_t>(p.bias)) : nullptr;
                 operands[g].workspace = workspaces[g] >= 0 ? plan->f(static_cast<uint32_t>(workspaces[g])) : nullptr;
             }
             const bool a_t = plan->transposed(first.a) != a_t_flip, b_t = plan->transposed(first.b) != b_t_flip;
             if (chained && *chained) k::matmul_tf32(s, chain_plan, operands, count, a_t, b_t, m, n, kk, count, pitches, plan->d_status);
-            else k::matmul_tc_group(s, operands, count, a_t, b_t, m, n, kk, plan->d_status, defer, pitches);
+            else k::matmul_tc_group(s, operands, count, a_t, b_t, m, n, kk, plan->d_status, defer, pitches, epilogue, epilogue == k::Epilogue::None ? nullptr : plan->f(beside));
         });
         l.flop = 2 * m * n * kk * count;
     }
@@ -2077,6 +2098,27 @@ struct Scheduler {
             }
             if (un.op == Op::GeluGrad && users[p.result].size() == 1 && p.bias < 0 && pos(un.operands[1]) == p.result && pos(un.operands[0]) != p.result &&
                 pos(un.operands[0]) < p.node && arena_half(pos(un.operands[0])) && P->slots[pos(un.operands[0])].kind == Slot::Arena)
+                return static_cast<int>(u);
+        }
+        return -1;
+    }
+
+    // The same in an f32 plan, with relu and its gradient: the element kernels' own functions of the same values, so the same
+    // bits as a launch of their own gives.
+    int activation_behind(const Product& p) const {
+        if (!(fusion_mask() & 16u) || is_output_value(p.result)) return -1;
+        for (uint32_t u : users[p.result]) {
+            const Node& un = node(u);
+            if (handled[u] || is_output_value(u) || un.ty.rank() != 2) continue;
+            if (un.op == Op::Gelu || un.op == Op::Relu) {
+                for (uint32_t reader : users[u])
+                    if (un.op == Op::Gelu && node(reader).op == Op::LayerNorm) return -1;
+                return static_cast<int>(u);
+            }
+            if (un.op != Op::GeluGrad && un.op != Op::ReluGrad) continue;
+            const uint32_t argument = pos(un.operands[0]);
+            if (users[p.result].size() == 1 && p.bias < 0 && pos(un.operands[1]) == p.result && argument != p.result && argument < p.node &&
+                P->slots[argument].kind == Slot::Arena && P->slots[argument].pitch == 0)
                 return static_cast<int>(u);
         }
         return -1;
