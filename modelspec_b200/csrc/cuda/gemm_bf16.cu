@@ -177,6 +177,12 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) bf16_kernel(const __
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (warp == 0 && lane == 0 && first_unit < units) {
+        const uint32_t product = unit_of(args, first_unit).product;
+        prefetch_map(&maps.a[product]);
+        prefetch_map(&maps.b[product]);
+        prefetch_map(&maps.c[product]);
+    }
     if (warp == 1) tmem_alloc<CG>(smem_u32(tmem_slot), T::TMEM_COLUMNS);
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     if constexpr (CG == 2) cluster_barrier();  // the other CTA's barriers exist before anything arrives on them

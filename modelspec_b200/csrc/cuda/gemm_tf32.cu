@@ -193,6 +193,12 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
         *abort_flag = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
+    if (warp == T::TMA_WARP && lane == 0 && first_unit < units) {
+        const uint32_t product = unit_of(args, first_unit).product;
+        tc::prefetch_map(&maps.a[product]);
+        tc::prefetch_map(&maps.b[product]);
+        tc::prefetch_map(&maps.c[product]);
+    }
     if (warp == T::MMA_WARP) {
         tc::tmem_alloc<CG>(tc::smem_u32(tmem_slot), T::TMEM_COLUMNS);
     }

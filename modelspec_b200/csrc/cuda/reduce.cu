@@ -22,7 +22,7 @@ enum class Whole : int { Sum, SquaredDifference };
 
 template <Whole KIND>
 __global__ void whole_stage1(const float* __restrict__ a, const float* __restrict__ b, uint64_t n,
-                             double* __restrict__ partial) {
+                             double* __restrict__ partial, double divisor, float* __restrict__ out) {
     after_producers();
     __shared__ double shared[33];
     double acc = 0.0;
@@ -36,7 +36,9 @@ __global__ void whole_stage1(const float* __restrict__ a, const float* __restric
         }
     }
     double total = block_sum(acc, shared);
-    if (threadIdx.x == 0) partial[blockIdx.x] = total;
+    if (threadIdx.x != 0) return;
+    if (out != nullptr) out[0] = static_cast<float>(total / divisor);  // the only block: no second launch
+    else partial[blockIdx.x] = total;
 }
 
 __global__ void whole_stage2(const double* __restrict__ partial, uint32_t blocks, double divisor,
@@ -293,16 +295,19 @@ uint64_t reduce_scratch_doubles() { return kMaxBlocks; }
 
 void reduce_sum(cudaStream_t s, const float* a, uint64_t n, bool mean, double* scratch, float* out) {
     uint32_t blocks = whole_blocks(n);
-    whole_stage1<Whole::Sum><<<blocks, kThreads, 0, s>>>(a, nullptr, n, scratch);
+    const double divisor = mean ? static_cast<double>(n) : 1.0;
+    whole_stage1<Whole::Sum><<<blocks, kThreads, 0, s>>>(a, nullptr, n, scratch, divisor, blocks == 1 ? out : nullptr);
     check_launch("reduce_sum");
-    whole_stage2<<<1, kThreads, 0, s>>>(scratch, blocks, mean ? static_cast<double>(n) : 1.0, out);
+    if (blocks == 1) return;
+    whole_stage2<<<1, kThreads, 0, s>>>(scratch, blocks, divisor, out);
     check_launch("reduce_sum");
 }
 
 void mse(cudaStream_t s, const float* a, const float* b, uint64_t n, double* scratch, float* out) {
     uint32_t blocks = whole_blocks(n);
-    whole_stage1<Whole::SquaredDifference><<<blocks, kThreads, 0, s>>>(a, b, n, scratch);
+    whole_stage1<Whole::SquaredDifference><<<blocks, kThreads, 0, s>>>(a, b, n, scratch, static_cast<double>(n), blocks == 1 ? out : nullptr);
     check_launch("mse");
+    if (blocks == 1) return;
     whole_stage2<<<1, kThreads, 0, s>>>(scratch, blocks, static_cast<double>(n), out);
     check_launch("mse");
 }

@@ -220,6 +220,7 @@ struct msx_plan {
     // The captured step: [1] takes its inputs over first, [0] runs on what is staged already. Each is
     // made when a step of its kind first runs.
     cudaGraphExec_t graphs[2] = {};
+    std::set<cudaGraphNode_t> side_nodes;  // of the step being captured: its launches on the side stream
     cudaEvent_t clock_start = nullptr;  // before the first step since the last msx_elapsed_ms
     uint64_t clock_steps = 0;
 
@@ -2873,7 +2874,21 @@ void join_loss(msx_plan* P) {
 // A bucket closed this few launches before the optimizer has nothing left to hide behind.
 constexpr int kExposedLaunches = 6;
 
+// The nodes of the graph that `stream` is captured into; none where it is not.
+std::set<cudaGraphNode_t> captured_nodes(cudaStream_t stream) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    cudaGraph_t graph = nullptr;
+    cuda_ok(cudaStreamGetCaptureInfo_v2(stream, &status, nullptr, &graph, nullptr, nullptr), "cudaStreamGetCaptureInfo");
+    if (status != cudaStreamCaptureStatusActive || !graph) return {};
+    size_t count = 0;
+    cuda_ok(cudaGraphGetNodes(graph, nullptr, &count), "cudaGraphGetNodes");
+    std::vector<cudaGraphNode_t> nodes(count);
+    if (count) cuda_ok(cudaGraphGetNodes(graph, nodes.data(), &count), "cudaGraphGetNodes");
+    return {nodes.begin(), nodes.begin() + static_cast<std::ptrdiff_t>(count)};
+}
+
 void enqueue_all(msx_plan* P) {
+    P->side_nodes.clear();
     begin_side_work(P);
     std::vector<char> joined(P->launches.size(), 0);
     for (size_t l = 0; l < P->launches.size(); ++l) {
@@ -2892,7 +2907,10 @@ void enqueue_all(msx_plan* P) {
         if (P->launches[l].join_before >= 0 && P->side_stream && P->side_fork[l]) {
             cuda_ok(cudaEventRecord(P->side_fork[l], P->stream), "cudaEventRecord");
             cuda_ok(cudaStreamWaitEvent(P->side_stream, P->side_fork[l], 0), "cudaStreamWaitEvent");
+            const std::set<cudaGraphNode_t> before = captured_nodes(P->stream);
             P->launches[l].run(P->side_stream);
+            for (cudaGraphNode_t node : captured_nodes(P->stream))
+                if (!before.count(node)) P->side_nodes.insert(node);
             cuda_ok(cudaEventRecord(P->side_done[l], P->side_stream), "cudaEventRecord");
         } else {
             P->launches[l].run(P->stream);
@@ -3048,20 +3066,22 @@ void stage_input(msx_plan* P, const HostInput& in, const void* host, bool by_hos
 
 // The edges of a captured step between a kernel and the one kernel that follows it become programmatic: the
 // second may be launched once every block of the first has called after_producers (common.cuh), and waits there
-// itself until the first is complete. Left as they are: edges at a fork or a join (a kernel that starts early there would
-// take the place of the one beside it), kernels that are not the backend's or wait for other ranks, and edges to the FMA
+// itself until the first is complete. Left as they are: edges to and from the side stream's launches (`side`) and of a kernel
+// that one of those is forked from (the next kernel, standing there early, would take the idle SMs from it: a BERT-tiny step
+// 5 % longer), kernels that are not the backend's or wait for other ranks, and edges to the FMA
 // products, whose small blocks would gather on the few SMs that are idle early (a transformer block's step 267 us so, 261
 // without them starting early, 268 with none; the ragged f32 case 7,404, 7,270, 7,387 a pass).
 // Passes, without and with: MLP 1,310, 1,245; BERT-tiny f32 21,608, 21,128, mixed 15,080, 13,990; BERT-mini 30,228, 29,423.
-void chain_kernels(cudaGraph_t graph) {
+void chain_kernels(cudaGraph_t graph, const std::set<cudaGraphNode_t>& side) {
     size_t count = 0;
     cuda_ok(cudaGraphGetEdges_v2(graph, nullptr, nullptr, nullptr, &count), "cudaGraphGetEdges");
     std::vector<cudaGraphNode_t> from(count), to(count);
     std::vector<cudaGraphEdgeData> data(count);
     if (count) cuda_ok(cudaGraphGetEdges_v2(graph, from.data(), to.data(), data.data(), &count), "cudaGraphGetEdges");
-    std::map<cudaGraphNode_t, std::pair<int, int>> degrees;  // edges into and out of a node
+    std::map<cudaGraphNode_t, std::pair<int, int>> degrees;  // edges into and out of a node, on its own stream
+    auto crosses = [&](size_t e) { return side.count(from[e]) != side.count(to[e]); };
     for (size_t e = 0; e < count; ++e) {
-        ++degrees[to[e]].first;
+        if (!crosses(e)) ++degrees[to[e]].first;
         ++degrees[from[e]].second;
     }
     auto waits_for_producers = [](cudaGraphNode_t node, bool starts_early) {
@@ -3076,7 +3096,7 @@ void chain_kernels(cudaGraph_t graph) {
         return std::strstr(name, "msx") != nullptr && std::strstr(name, "peer_all_reduce") == nullptr;
     };
     for (size_t e = 0; e < count; ++e) {
-        if (data[e].type != cudaGraphDependencyTypeDefault || degrees[to[e]].first != 1 || degrees[from[e]].second != 1) continue;
+        if (crosses(e) || data[e].type != cudaGraphDependencyTypeDefault || degrees[to[e]].first != 1 || degrees[from[e]].second != 1) continue;
         if (!waits_for_producers(from[e], false) || !waits_for_producers(to[e], true)) continue;
         cudaGraphEdgeData early = {};
         early.from_port = cudaGraphKernelNodePortProgrammatic;
@@ -3480,7 +3500,7 @@ int msx_run(msx_plan* plan) {
                 cuda_ok(cudaStreamEndCapture(plan->stream, &graph), "cudaStreamEndCapture");
                 cudaError_t e = cudaSuccess;
                 try {
-                    if ((fusion_mask() & 128u) && !plan->comm) chain_kernels(graph);
+                    if ((fusion_mask() & 128u) && !plan->comm) chain_kernels(graph, plan->side_nodes);
                     e = cudaGraphInstantiate(&exec, graph, 0);
                 } catch (...) {
                     cudaGraphDestroy(graph);

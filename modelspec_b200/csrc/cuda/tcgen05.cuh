@@ -121,6 +121,9 @@ template <int COUNT> __device__ __forceinline__ void tmem_store(uint32_t at, con
 __device__ __forceinline__ void tmem_loaded() { asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory"); }
 __device__ __forceinline__ void tmem_stored() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
 
+// A tensor map (a kernel's parameter) on its way to where the copies read it.
+__device__ __forceinline__ void prefetch_map(const CUtensorMap* map) { asm volatile("prefetch.tensormap [%0];" ::"l"(map) : "memory"); }
+
 // One box of a 4-dimensional tensor map from shared memory to global memory (what lies outside the
 // tensor is not written), as a bulk group of the issuing thread.
 __device__ __forceinline__ void tma_store(const CUtensorMap* map, uint32_t src, uint32_t x, const uint32_t (&upper)[3]) {
