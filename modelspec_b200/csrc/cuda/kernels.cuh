@@ -84,9 +84,10 @@ struct RowSumJob {
     const void* g;
     float* partial;
     uint32_t rows, width, ld, rows_per_chunk, first_block, half;  // half: g holds bf16 elements
+    uint32_t columns;  // of a lane: 1 or 4
 };
 RowSumJob row_sum_job(In g, float* partial, uint64_t rows, uint64_t h, uint64_t ld, uint32_t first_block);
-uint32_t row_sum_job_blocks(uint64_t rows, uint64_t h);
+uint32_t row_sum_job_blocks(uint64_t rows, uint64_t h, uint64_t ld);
 void sum_rows_batched(cudaStream_t s, const RowSumJob* d_jobs, uint32_t jobs, uint32_t blocks);
 
 // Deferred second stages. A kernel that leaves `chunks` partial results of `width` floats each,

@@ -453,7 +453,7 @@ struct Scheduler {
                 const DeferredRows& d = deferred_rows[i];
                 reads.push_back(d.g);
                 writes.push_back(d.partial);
-                blocks += k::row_sum_job_blocks(d.rows, d.width);
+                blocks += k::row_sum_job_blocks(d.rows, d.width, d.ld);
             }
             Node pseudo;
             pseudo.id = node(deferred_rows[rows_finished].g).id;
@@ -2656,7 +2656,7 @@ void allocate(msx_plan* P, const Scheduler& sched) {
             if (std::find(sched.rows_cuts.begin(), sched.rows_cuts.end(), jobs.size()) != sched.rows_cuts.end()) first_block = 0;
             jobs.push_back(k::row_sum_job(P->in(d.g), static_cast<float*>(P->ptr(d.partial)), d.rows, d.width,
                                           d.ld, first_block));
-            first_block += k::row_sum_job_blocks(d.rows, d.width);
+            first_block += k::row_sum_job_blocks(d.rows, d.width, d.ld);
         }
         cuda_ok(cudaMemcpy(P->d_row_sum_jobs, jobs.data(), jobs.size() * sizeof(k::RowSumJob), cudaMemcpyHostToDevice), "cudaMemcpy(row sum jobs)");
     }
