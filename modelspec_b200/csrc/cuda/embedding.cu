@@ -124,9 +124,11 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const int32_t* __restrict__
 // order. A row nobody read gets `base` (or zero); when base is out itself, such a row is left
 // alone and only the rows some id names are read and written. VEC = 4 reads and writes 16 bytes
 // per lane and needs h % 4 == 0 and 16-byte aligned g, base and out.
+// Three blocks an SM: left alone the compiler takes 98 registers for the indices held ahead, which leaves room for
+// two (16,384 ids of 768 columns, three tables: bf16 168 -> 140 us, f32 171 -> 140).
 constexpr uint32_t kHotRow = 32, kHotChunk = 32, kTogether = 8, kCachedIds = 4096;
 template <int VEC, class TG, class TO>
-__global__ void __launch_bounds__(256) scatter_kernel(const TG* __restrict__ g, const int32_t* __restrict__ sorted_id,
+__global__ void __launch_bounds__(256, 3) scatter_kernel(const TG* __restrict__ g, const int32_t* __restrict__ sorted_id,
                                                       const int32_t* __restrict__ sorted_n, uint32_t n,
                                                       const float* base, TO* out, uint32_t rows, uint32_t h) {
     after_producers();
@@ -304,7 +306,7 @@ __global__ void __launch_bounds__(256) scatter_kernel(const TG* __restrict__ g, 
 // is what the launch waits for, so each group of columns has a block of its own (as a loop within the
 // block, 16,384 ids and 768 columns took 211 us; now 65).
 template <int VEC, class TG, class TO>
-__global__ void __launch_bounds__(256) scatter_in_place_kernel(const TG* __restrict__ g, const int32_t* __restrict__ sorted_id,
+__global__ void __launch_bounds__(256, 3) scatter_in_place_kernel(const TG* __restrict__ g, const int32_t* __restrict__ sorted_id,
                                                                const int32_t* __restrict__ sorted_n, uint32_t n, TO* out, uint32_t rows,
                                                                uint32_t h) {
     after_producers();
