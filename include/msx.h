@@ -298,7 +298,9 @@ int msx_training_comm_init(msx_training* training, int rank, int world, const vo
                            uint64_t rows_per_rank);
 
 /* Sets one declared `input` or `target` of the batch for the steps that follow (the dense feed
- * of train/data.rs:14-35; block k of a `--data` file is what the caller passes before step k). */
+ * of train/data.rs:14-35; block k of a `--data` file is what the caller passes before step k).
+ * Copied, without a wait for any step; checked by the msx_training_step that takes it, and not
+ * before that among the inputs of the step plan, which another caller may run. */
 int msx_training_set_input(msx_training* training, const char* name, const void* host, uint64_t bytes);
 
 /* The reference's synthetic batch (train/data.rs:189-212): the one f32 input standard normal,

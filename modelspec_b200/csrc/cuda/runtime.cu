@@ -12,6 +12,7 @@
 
 #include <algorithm>
 #include <array>
+#include <atomic>
 #include <chrono>
 #include <cstdio>
 #include <cstdlib>
@@ -28,6 +29,7 @@
 #include "kernels.cuh"
 #include "host_copy.hpp"
 #include "plan.hpp"
+#include "step_inputs.hpp"
 
 using msx::Launch;
 using msx::Node;
@@ -169,15 +171,7 @@ struct msx_plan {
     char* d_inputs = nullptr;
     char* d_shared_inputs = nullptr;  // those of a plan that shares its parameters, made with its slots
     uint64_t input_bytes = 0;
-    // The inputs as they were last set are the slot `image` (-1: none was made). While `image_open` it is the slot
-    // of the step that runs next: inputs of `image_set` have been written there, the others follow from
-    // `image_before` when the step is submitted.
-    int image = -1, image_before = -1;
-    bool image_open = false;
-    std::vector<char> image_set;
-    // Inputs that the host loop staged itself, and their bytes where msx_set_input has put others in their place.
-    std::vector<char> host_staged;
-    std::vector<std::vector<char>> displaced;
+    msx::StepInputs waiting;  // the inputs of the step that runs next, in the order of `inputs`
     msx::PinnedBlock pinned_together;
     char* pinned[kStagingSlots] = {};  // a slot of input_bytes each, pieces of pinned_together or requests of their own
     char* d_staging = nullptr;         // large inputs: kDeviceSlots slots on the device
@@ -214,7 +208,9 @@ struct msx_plan {
 
     int loss_pos = -1;
     uint64_t steps = 0;
-    uint64_t finished = 0;  // steps known to have run: the host has waited for the last of them
+    // Steps known to have run: the host has waited for the last of them, or asked. (Atomic: a thread may read losses while
+    // another sets inputs.)
+    std::atomic<uint64_t> finished{0};
     uint64_t shard_rows_before = 0;
 
     // The captured step: [1] takes its inputs over first, [0] runs on what is staged already. Each is
@@ -2508,7 +2504,7 @@ template <class T> cudaError_t plan_malloc(msx_plan* P, T** out, size_t bytes) {
 // never feed it. (An MLP of 200 KB a step: a run is made in 6.4 ms so, in 8.2 with the forward program's 200 KB on the
 // device beside the rest, which then takes one of the driver's 2 MB blocks more.)
 void make_input_slots(msx_plan* P, bool behind_its_own_steps = false) {
-    if (!P->image_set.empty()) return;
+    if (P->waiting.ready()) return;
     const uint64_t bytes = std::max<uint64_t>(P->input_bytes, kAlign);
     const uint64_t all = kStagingSlots * bytes;
     if (all <= kPinnedApart[0] || all > kPinnedApart[1]) {
@@ -2528,9 +2524,8 @@ void make_input_slots(msx_plan* P, bool behind_its_own_steps = false) {
         cuda_ok(cudaMemsetAsync(P->d_shared_inputs, 0, bytes, P->stream), "cudaMemset(inputs)");
         P->d_inputs = P->d_shared_inputs;
     }
-    P->host_staged.assign(P->inputs.size() + 1, 0);
-    P->displaced.resize(P->inputs.size() + 1);
-    P->image_set.assign(P->inputs.size() + 1, 0);
+    for (const HostInput& in : P->inputs) P->waiting.add(in.offset, in.bytes);
+    P->waiting.use_slots(P->pinned);
 }
 
 void allocate(msx_plan* P, const Scheduler& sched) {
@@ -2953,10 +2948,14 @@ int wait_event(cudaEvent_t event, uint32_t timeout_ms) {
 
 // Waits for step `step`. The driver is not asked about a step that is known to have run (a query costs the host
 // half a microsecond or more).
+void note_finished(msx_plan* P, uint64_t step) {
+    uint64_t known = P->finished;
+    while (known <= step && !P->finished.compare_exchange_weak(known, step + 1)) {}
+}
 int wait_step(msx_plan* P, uint64_t step, uint32_t timeout_ms) {
     if (step < P->finished) return MSX_OK;
     const int rc = wait_event(P->step_done[step % kStepEvents], timeout_ms);
-    if (rc == MSX_OK) P->finished = step + 1;
+    if (rc == MSX_OK) note_finished(P, step);
     return rc;
 }
 
@@ -3003,35 +3002,22 @@ void enqueue_step(msx_plan* P, bool take_inputs) {
                     P->d_turn, kStagingSlots);
 }
 
-// The slot of the step that runs next is open for its inputs: they are written where that step reads them, once
-// (through a host image of the plan's and from there into the slot a megabyte of inputs took 80 us more a step).
-// Waits until the step that last used the slot has run.
-void open_image(msx_plan* P) {
-    if (P->image_open) return;
-    if (P->image_set.empty()) {
+// The slot of the step that runs next is opened for its inputs when the step that used it last has run; this does not
+// wait for that.
+void open_inputs(msx_plan* P) {
+    if (P->waiting.open()) return;
+    if (!P->waiting.ready()) {
         cuda_ok(cudaSetDevice(P->device->ordinal), "cudaSetDevice");
         make_input_slots(P);
     }
     if (P->steps >= kStagingSlots) {
-        int rc = wait_step(P, P->steps - kStagingSlots, 600000u);
-        if (rc != MSX_OK) throw StatusError(rc, "a step submitted " + std::to_string(kStagingSlots) + " steps ago has not finished");
+        const uint64_t last = P->steps - kStagingSlots;
+        if (last >= P->finished) {
+            if (cudaEventQuery(P->step_done[last % kStepEvents]) != cudaSuccess) return;
+            note_finished(P, last);
+        }
     }
-    const int slot = static_cast<int>(P->steps % kStagingSlots);
-    std::fill(P->image_set.begin(), P->image_set.end(), static_cast<char>(slot == P->image));
-    P->image_before = P->image;
-    P->image = slot;
-    P->image_open = true;
-}
-
-// What was not set since the slot was opened comes from the slot before (zeros where there was none).
-void complete_image(msx_plan* P) {
-    for (size_t i = 0; i < P->inputs.size(); ++i) {
-        if (P->image_set[i]) continue;
-        char* const to = P->pinned[P->image] + P->inputs[i].offset;
-        if (P->image_before >= 0) std::memcpy(to, P->pinned[P->image_before] + P->inputs[i].offset, P->inputs[i].bytes);
-        else std::memset(to, 0, P->inputs[i].bytes);
-        P->image_set[i] = 1;
-    }
+    P->waiting.open(static_cast<int>(P->steps % kStagingSlots));
 }
 
 HostInput* input_of(msx_plan* P, const char* name) {
@@ -3041,28 +3027,6 @@ HostInput* input_of(msx_plan* P, const char* name) {
 }
 
 size_t index_of(const msx_plan* P, const HostInput& in) { return static_cast<size_t>(&in - P->inputs.data()); }
-
-// Where an input lies as it was last set (null: it never was).
-char* staged_value(msx_plan* P, const HostInput& in) {
-    if (P->image < 0) return nullptr;
-    const int slot = P->image_open && !P->image_set[index_of(P, in)] ? P->image_before : P->image;
-    return slot < 0 ? nullptr : P->pinned[slot] + in.offset;
-}
-
-// Input `in` of the step that runs next, unchecked.
-void stage_input(msx_plan* P, const HostInput& in, const void* host, bool by_host_loop) {
-    open_image(P);
-    const size_t i = index_of(P, in);
-    if (P->host_staged[i] && !by_host_loop) {
-        const char* now = staged_value(P, in);
-        P->displaced[i].assign(now, now + in.bytes);
-    } else if (by_host_loop) {
-        P->displaced[i].clear();
-    }
-    P->host_staged[i] = by_host_loop;
-    std::memcpy(P->pinned[P->image] + in.offset, host, in.bytes);
-    P->image_set[i] = 1;
-}
 
 // The edges of a captured step between a kernel and the one kernel that follows it become programmatic: the
 // second may be launched once every block of the first has called after_producers (common.cuh), and waits there
@@ -3395,41 +3359,40 @@ int msx_set_input(msx_plan* plan, const char* name, const void* host, uint64_t b
             std::string why;
             int rc = check_input(*in, host, &why);
             if (rc != MSX_OK) throw StatusError(rc, why);
-            stage_input(plan, *in, host, false);
+            open_inputs(plan);
+            plan->waiting.set(index_of(plan, *in), host);
             return MSX_OK;
         }
         throw StatusError(MSX_BAD_ARGUMENT, std::string("msx_set_input: the step reads no input `") + name + "`");
     });
 }
 
-// For the host loop above this file. An input written straight into the slot of the step that runs next; where
-// its value lies until the loop sets it again; its check before a step is submitted (on the value the loop set,
-// put back first where msx_set_input has displaced it).
+// For the host loop above this file (step_inputs.hpp). An input of the run's, unchecked, written straight into the slot
+// of the step that runs next: 1, or 0 where the run has to keep it itself. Where its value lies until the run sets it again. And its
+// check, with which it becomes the plan's.
 int msx_internal_stage_input(msx_plan* plan, const char* name, const void* host, uint64_t bytes) {
-    return guarded(plan->device, [&]() -> int {
+    try {
         const HostInput* in = input_of(plan, name);
-        if (!in || in->bytes != bytes) throw StatusError(MSX_BAD_ARGUMENT, std::string("no input `") + name + "` of that size");
-        stage_input(plan, *in, host, true);
-        return MSX_OK;
-    });
+        if (!in || in->bytes != bytes) return 0;
+        open_inputs(plan);
+        return plan->waiting.stage(index_of(plan, *in), host) ? 1 : 0;
+    } catch (const std::exception&) {
+        return 0;
+    }
 }
 const void* msx_internal_staged_input(msx_plan* plan, const char* name) {
     const HostInput* in = input_of(plan, name);
-    if (!in || plan->image < 0) return nullptr;
-    const std::vector<char>& displaced = plan->displaced[index_of(plan, *in)];
-    return displaced.empty() ? staged_value(plan, *in) : displaced.data();
+    return in ? plan->waiting.run_value(index_of(plan, *in)) : nullptr;
 }
-int msx_internal_check_staged_input(msx_plan* plan, const char* name) {
+int msx_internal_accept_input(msx_plan* plan, const char* name) {
     return guarded(plan->device, [&]() -> int {
         const HostInput* in = input_of(plan, name);
-        if (!in || plan->image < 0) return MSX_OK;
-        if (!plan->displaced[index_of(plan, *in)].empty()) {
-            const std::vector<char> back = std::move(plan->displaced[index_of(plan, *in)]);
-            stage_input(plan, *in, back.data(), true);
-        }
+        if (!in) throw StatusError(MSX_BAD_ARGUMENT, std::string("the step reads no input `") + name + "`");
         std::string why;
-        int rc = check_input(*in, staged_value(plan, *in), &why);
+        int rc = check_input(*in, plan->waiting.run_value(index_of(plan, *in)), &why);
         if (rc != MSX_OK) throw StatusError(rc, why);
+        open_inputs(plan);
+        plan->waiting.accept(index_of(plan, *in));
         return MSX_OK;
     });
 }
@@ -3475,14 +3438,14 @@ int msx_run(msx_plan* plan) {
         plan->dispatches += plan->launches.size();
         plan->bytes_downloaded += (plan->loss_pos >= 0 ? 4 : 0) + 4;
         // (inputs that nothing has ever set are zeros)
-        const bool take_inputs = plan->input_bytes && (plan->image_open || plan->image < 0);
+        const bool take_inputs = plan->input_bytes && plan->waiting.changed();
         if (take_inputs) {
-            open_image(plan);
-            complete_image(plan);
+            make_input_slots(plan);
+            plan->waiting.open(slot);
             plan->bytes_uploaded += plan->input_bytes;
-            plan->image_open = false;
-            if (plan->d_staging) stage_inputs(plan, slot, plan->began_idle[at]);
         }
+        plan->waiting.submitted();
+        if (take_inputs && plan->d_staging) stage_inputs(plan, slot, plan->began_idle[at]);
         if (plan->flags & MSX_PLAN_NO_GRAPH) {
             enqueue_step(plan, take_inputs);
         } else {
@@ -3572,9 +3535,9 @@ int msx_profile_step_repeated(msx_plan* plan, uint32_t repeats, float* launch_ms
         std::vector<cudaEvent_t> events(2 * count);
         for (cudaEvent_t& e : events) cuda_ok(cudaEventCreate(&e), "cudaEventCreate");
         if (plan->input_bytes) {
-            open_image(plan);
-            complete_image(plan);
-            cuda_ok(cudaMemcpyAsync(plan->d_inputs, plan->pinned[plan->image], plan->input_bytes, cudaMemcpyHostToDevice, plan->stream), "cudaMemcpyAsync");
+            open_inputs(plan);  // (every step has run)
+            const int from = plan->waiting.complete();
+            cuda_ok(cudaMemcpyAsync(plan->d_inputs, plan->pinned[from], plan->input_bytes, cudaMemcpyHostToDevice, plan->stream), "cudaMemcpyAsync");
         }
         begin_side_work(plan);
         for (size_t l = 0; l < count; ++l) {

@@ -27,10 +27,11 @@
 
 // Defined beside msx_last_error: records a message on the device handle.
 extern "C" void msx_internal_set_error(msx_device* device, const char* message);
-// Defined beside msx_set_input: an input written into the slot its step reads, checked later.
+// Defined beside msx_set_input: an input written into the slot its step reads (1; 0: not now), where it lies, and its check,
+// with which the step has it.
 extern "C" int msx_internal_stage_input(msx_plan* plan, const char* name, const void* host, uint64_t bytes);
 extern "C" const void* msx_internal_staged_input(msx_plan* plan, const char* name);
-extern "C" int msx_internal_check_staged_input(msx_plan* plan, const char* name);
+extern "C" int msx_internal_accept_input(msx_plan* plan, const char* name);
 
 struct msx_training {
     msx_device* device = nullptr;
@@ -64,8 +65,8 @@ struct msx_training {
     uint32_t flags = 0;
     std::string error;
     // Declared inputs and targets, by name. Those of `staged` were written straight into the slot that the next
-    // step reads (once a step has run: a run that only infers needs no slots); `batch` holds their bytes once
-    // something else than the step reads them.
+    // step reads (once a step has run: a run that only infers needs no slots), where they are this run's until its next step
+    // has checked them; `batch` holds the bytes of those of `uncopied` once something else than the step reads them.
     std::map<std::string, std::vector<char>> batch;
     std::set<std::string> staged, uncopied;
     std::vector<std::string> sites;                  // dropout token inputs of the step
@@ -164,7 +165,7 @@ void stage_batch(msx_training* t, msx_plan* plan, const std::set<std::string>& r
     if (plan != t->step) copy_staged(t);
     for (const auto& [name, bytes] : t->batch) {
         if (!reads.count(name)) continue;
-        if (plan == t->step && t->staged.count(name)) ok(t, msx_internal_check_staged_input(plan, name.c_str()));
+        if (plan == t->step && t->staged.count(name)) ok(t, msx_internal_accept_input(plan, name.c_str()));
         else ok(t, msx_set_input(plan, name.c_str(), bytes.data(), bytes.size()));
     }
 }
@@ -268,8 +269,7 @@ int msx_training_set_input(msx_training* t, const char* name, const void* host, 
         if (bytes != d->ty.count() * 4)
             throw Fail{MSX_BAD_ARGUMENT, std::string("`") + name + "` is " + d->ty.str() + ": " + std::to_string(d->ty.count() * 4) + " bytes"};
         // (what the detour costs a small input is less than the names looked up for the direct way)
-        if (bytes >= 4096 && t->submitted && t->step_inputs.count(name)) {
-            ok(t, msx_internal_stage_input(t->step, name, host, bytes));
+        if (bytes >= 4096 && t->submitted && t->step_inputs.count(name) && msx_internal_stage_input(t->step, name, host, bytes)) {
             t->batch[name].resize(bytes);
             t->staged.insert(name);
             t->uncopied.insert(name);
@@ -277,6 +277,8 @@ int msx_training_set_input(msx_training* t, const char* name, const void* host, 
         }
         const char* b = static_cast<const char*>(host);
         t->batch[name].assign(b, b + bytes);
+        t->staged.erase(name);
+        t->uncopied.erase(name);
     });
 }
 
