@@ -609,8 +609,9 @@ int msx_op_attention_bf16(const void* q, const void* k, const void* v, const flo
 
 /* The f32 attention kernels that keep the scores on the chip, on the caller's device buffers: as above with
  * q, k, v, g and the results f32, any strides a head width of up to 64 gives, up to 512 keys. Writes `out` and, where
- * not null, `stats` (needed with `g`) and, of up to 128 keys, the probabilities `p` [batch, heads, q_len, k_len]. A plan takes
- * these kernels where they are the faster way for its shape. */
+ * not null, `stats` (needed with `g`; on 8 bytes, else MSX_BAD_ARGUMENT) and, of up to 128 keys, the probabilities `p`
+ * [batch, heads, q_len, k_len]. Any other float pointer may lie on any float. A plan takes these kernels where they are the faster
+ * way for its shape. */
 int msx_op_attention_f32(const float* q, const float* k, const float* v, const float* mask, const float* g, float* out, float* dq, float* dk,
                          float* dv, float* stats, float* p, uint32_t batch, uint32_t q_len, uint32_t k_len, uint32_t heads,
                          uint32_t head_dim, uint32_t* status, void* stream);

@@ -150,6 +150,7 @@ struct Shape {
     uint32_t l, s, h, heads, d;              // queries, keys, row pitch, heads, head width
     uint32_t tiles, key_tiles, key_blocks;  // tiles of 128 queries and keys of a head; blocks of the backward that take keys
     float scale;
+    uint32_t p_vec;  // the probabilities' rows lie on 16 bytes
 };
 struct Place {
     uint32_t b, a, first;
@@ -352,7 +353,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_f32_forward_kernel(const
             for (int i = 0; i < 32; i += 4) {
                 const uint32_t c = part * 32 + i;
                 const float4 f = make_float4(p[i] * inverse, p[i + 1] * inverse, p[i + 2] * inverse, p[i + 3] * inverse);
-                if (sh.s % 4 == 0) {
+                if (sh.p_vec) {
                     if (c < sh.s) *reinterpret_cast<float4*>(to + i) = f;
                 } else {
                     if (c < sh.s) to[i] = f.x;
@@ -658,6 +659,7 @@ Shape shape_of(AttentionShape sh) {
     s.key_tiles = (sh.k_len + QUERIES - 1) / QUERIES;
     s.key_blocks = 0;
     s.scale = 1.0f / sqrtf(static_cast<float>(sh.head_dim));
+    s.p_vec = 0;
     return s;
 }
 bool on_16_bytes(std::initializer_list<const void*> pointers) {
@@ -707,7 +709,8 @@ uint64_t attention_f32_stats_floats(AttentionShape sh) { return 2ull * sh.batch 
 void attention_f32_forward(cudaStream_t s, const float* q, const float* k, const float* v, const float* mask, float* out, float* stats, float* p,
                            AttentionShape sh, uint32_t* status) {
     if (sh.batch == 0) return;
-    const Shape shape = shape_of(sh);
+    Shape shape = shape_of(sh);
+    shape.p_vec = sh.k_len % 4 == 0 && on_16_bytes({p});
     const bool vec = sh.head_dim % 4 == 0 && on_16_bytes({q, k, v, out});
     auto go = [&](auto kernel, int bytes, std::atomic<int>& configured_device) {
         set_shared_memory(kernel, bytes, configured_device);

@@ -4046,6 +4046,7 @@ int msx_op_attention_f32(const float* q, const float* k, const float* v, const f
                          uint32_t head_dim, uint32_t* status, void* stream) {
     if (!q || !k || !v || !mask || !out || !status || (g && !stats)) return MSX_BAD_ARGUMENT;
     return guarded(nullptr, [&]() -> int {
+        if (reinterpret_cast<uintptr_t>(stats) % 8 != 0) throw StatusError(MSX_BAD_ARGUMENT, "msx_op_attention_f32: `stats` on a boundary of 8 bytes");
         const k::AttentionShape shape = {batch, q_len, k_len, heads, head_dim};
         if (!k::attention_f32_supported(shape) || (p && k_len > 128))
             throw StatusError(MSX_UNSUPPORTED, "msx_op_attention_f32: heads of up to 64 columns, up to 512 keys (128 where the probabilities are wanted)");

@@ -107,8 +107,6 @@ def test_every_element_of_the_kernels_against_float64(device, batch, q_len, k_le
     p = buffer(batch * heads * q_len * k_len) if k_len <= 128 else None
     stats, status = torch.zeros(2 * batch * heads * q_len, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
     torch.cuda.synchronize()
-    if p is not None and k_len % 4 == 0 and shift:
-        p = None  # (a plan's scratch lies on 256 bytes)
     rc = M.lib().msx_op_attention_f32(ptr(operand["q"]), ptr(operand["k"]), ptr(operand["v"]), ptr(operand["mask"]), ptr(operand["g"]), ptr(out["O"]),
                                       ptr(out.get("Q")), ptr(out.get("K")), ptr(out.get("V")), ptr(stats), ptr(p), *shape, ptr(status), None)
     assert rc == M.OK, M.lib().msx_last_error(None).decode()
@@ -117,6 +115,10 @@ def test_every_element_of_the_kernels_against_float64(device, batch, q_len, k_le
     check({n: t.cpu().numpy().astype(np.float64) for n, t in out.items()}, feed, shape)
     for t in kept:  # nothing outside of an operand was written
         assert torch.isnan(t[:shift]).all() and torch.isnan(t[-(8 - shift):]).all()
+    # The statistics are pairs: refused where no pair can be stored.
+    assert M.lib().msx_op_attention_f32(ptr(operand["q"]), ptr(operand["k"]), ptr(operand["v"]), ptr(operand["mask"]), ptr(operand["g"]), ptr(out["O"]),
+                                        ptr(out.get("Q")), ptr(out.get("K")), ptr(out.get("V")), C.c_void_p(stats.data_ptr() + 4), ptr(p), *shape,
+                                        ptr(status), None) == M.BAD_ARGUMENT
     if p is not None:
         sums = p.cpu().numpy().astype(np.float64).reshape(-1, k_len).sum(axis=1)
         assert np.abs(sums - 1.0).max() <= 1e-5
