@@ -602,7 +602,8 @@ uint64_t msx_op_matmul_bf16_workspace(uint64_t m, uint64_t n, uint64_t k);
  * [batch, k_len] of 0 / 1. Writes `out` (bf16) and `stats` (2 floats per (row, head): the softmax
  * maximum and sum); with `g` not null also dq, dk, dv (bf16, each may be null). The op is the
  * reference's Attention / AttentionGradQ/K/V (cpu/interpreter.rs:1035-1119); the score matrix
- * stays on the SM. Heads of up to 64 columns (a multiple of 8), up to 512 keys and queries. */
+ * stays on the SM. Heads of up to 64 columns (a multiple of 8), up to 512 keys and queries. The bf16 matrices lie on
+ * 16 bytes, else MSX_BAD_ARGUMENT. */
 int msx_op_attention_bf16(const void* q, const void* k, const void* v, const float* mask, const void* g, void* out, void* dq, void* dk,
                           void* dv, float* stats, uint32_t batch, uint32_t q_len, uint32_t k_len, uint32_t heads, uint32_t head_dim,
                           uint32_t* status, void* stream);

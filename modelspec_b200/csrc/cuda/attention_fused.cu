@@ -488,8 +488,9 @@ __device__ __forceinline__ void backward_rows(const BackwardMaps& maps, const Fu
             *dot = 0.0f;
             if (query >= args.q_len) return;
             const uint64_t global_row = static_cast<uint64_t>(seq) * args.q_len + query;
-            const float2 st = __ldg(reinterpret_cast<const float2*>(args.stats + (global_row * args.heads + head) * 2));
-            if (st.y > 0.0f) *shift = fmaf(st.x, 1.4426950408889634f, log2f(st.y));
+            const float* const st = args.stats + (global_row * args.heads + head) * 2;
+            const float best = __ldg(st), total = __ldg(st + 1);
+            if (total > 0.0f) *shift = fmaf(best, 1.4426950408889634f, log2f(total));
             const bf16* o = static_cast<const bf16*>(args.o) + global_row * args.h + head * args.d;
             const bf16* g = static_cast<const bf16*>(args.g) + global_row * args.h + head * args.d;
             float sum = 0.0f;

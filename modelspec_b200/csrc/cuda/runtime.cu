@@ -4064,6 +4064,8 @@ int msx_op_attention_bf16(const void* q, const void* k, const void* v, const flo
         k::AttentionShape shape = {batch, q_len, k_len, heads, head_dim};
         if (!k::attention_fused_supported(shape))
             throw StatusError(MSX_UNSUPPORTED, "msx_op_attention_bf16: heads of up to 64 columns (a multiple of 8), up to 512 keys and queries");
+        for (const void* result : {static_cast<const void*>(out), static_cast<const void*>(dq), static_cast<const void*>(dk), static_cast<const void*>(dv)})
+            if (reinterpret_cast<uintptr_t>(result) % 16 != 0) throw StatusError(MSX_BAD_ARGUMENT, "msx_op_attention_bf16: a result off 16 bytes");
         try {
             cudaStream_t s = static_cast<cudaStream_t>(stream);
             k::attention_fused_forward(s, q, k, v, mask, out, stats, shape, status);

@@ -234,3 +234,32 @@ def test_every_element_of_the_fused_attention_against_float64(device, batch, seq
                                    ("dq", got_dq, ds @ k, off @ k.abs()), ("dk", got_dk, turn(ds) @ q, turn(off) @ q.abs())):
         ratio = float(((got - want).abs() / (r * moved + r * want.abs() + 1e-6)).max())
         assert ratio <= 1.0, (name, ratio)
+
+
+# Both kernels for the gradients (few heads, and many of one tile): statistics on any float give the same bits; the matrices that are
+# written or read 16 bytes at a time are refused elsewhere.
+@pytest.mark.parametrize("batch,seq,heads,d", [(1, 200, 2, 40), (40, 128, 12, 64)])
+def test_fused_attention_takes_statistics_on_any_float(device, batch, seq, heads, d):
+    import torch
+    gen = torch.Generator(device="cuda").manual_seed(seq)
+    h, rows = heads * d, batch * seq
+    t = {name: torch.randn((rows, h), device="cuda", generator=gen).to(torch.bfloat16) for name in "qkvg"}
+    mask = torch.ones((batch, seq), device="cuda")
+    status = torch.zeros(1, dtype=torch.int32, device="cuda")
+    at = lambda x, off=0: C.c_void_p(x.data_ptr() + off)
+    call = lambda out, offs, stats, shift: M.lib().msx_op_attention_bf16(
+        at(t["q"]), at(t["k"]), at(t["v"]), at(mask), at(t["g"]), *(at(o, off) for o, off in zip(out, offs)), at(stats, 4 * shift), batch, seq, seq, heads, d,
+        at(status), None)
+    results = []
+    for shift in (0, 1):
+        out = [torch.full((rows * h + 8,), float("nan"), dtype=torch.bfloat16, device="cuda") for _ in range(4)]
+        stats = torch.full((rows * heads * 2 + 2,), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        assert call(out, (0, 0, 0, 0), stats, shift) == M.OK, M.lib().msx_last_error(None).decode()
+        torch.cuda.synchronize()
+        assert int(status.item()) == 0
+        results.append([o[: rows * h].view(torch.int16).cpu() for o in out] + [stats[shift : shift + rows * heads * 2].cpu()])
+        for which in range(4):
+            assert call(out, [2 * (i == which) for i in range(4)], stats, 0) == M.BAD_ARGUMENT
+    for a, b in zip(*results):
+        assert torch.equal(a, b) and torch.isfinite(a.float()).all()
