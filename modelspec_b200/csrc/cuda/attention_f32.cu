@@ -50,9 +50,9 @@ constexpr uint32_t QUERIES = 128, FORWARD_KEYS = 128, BACKWARD_TILE = 64;
 // their sign, and with it the lo lo products that are left out: products come out low by some 2^-21 (8 to 10 10^-7 of
 // the norm of O). Both are therefore rounded: 0.7 2^-11 of a value added to it is between a third and two thirds of
 // its last kept bit (and, unlike an addition to the word, leaves a NaN one): 2 to 5 10^-7 of the norm of O and of the
-// gradients, as batched products 6 to 27 10^-7.
+// gradients, as batched products 6 to 27 10^-7. (The addition rounds towards zero: the largest finite values stay finite.)
 constexpr float kHalfBit = 0.7f / 2048.0f;
-__device__ __forceinline__ float high_of(float x) { return __uint_as_float(__float_as_uint(fmaf(x, kHalfBit, x)) & 0xffffe000u); }
+__device__ __forceinline__ float high_of(float x) { return __uint_as_float(__float_as_uint(__fmaf_rz(x, kHalfBit, x)) & 0xffffe000u); }
 __device__ __forceinline__ float low_of(float x, float h) {
     const float l = x - h;
     return fmaf(l, kHalfBit, l);

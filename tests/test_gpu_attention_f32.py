@@ -124,6 +124,31 @@ def test_every_element_of_the_kernels_against_float64(device, batch, q_len, k_le
         assert np.abs(sums - 1.0).max() <= 1e-5
 
 
+# The halves of an operand stay finite up to the largest float: rounding to the nearest would take what lies within 2^-11 of it to
+# infinity, and its remainder with it.
+@pytest.mark.parametrize("batch,q_len,k_len,heads,d", [(1, 33, 16, 2, 16), (1, 130, 300, 1, 64)])
+def test_values_next_to_the_largest_float(device, batch, q_len, k_len, heads, d):
+    import torch
+    shape = (batch, q_len, k_len, heads, d)
+    feed = feed_of(*shape)
+    feed["mask"][:] = 0.0
+    feed["mask"][:, 3] = 1.0  # one key: its probability is 1, and O the row of V itself
+    # A result is off by up to 2^-20 of itself (float64 above): as far below the largest float as that, it is finite.
+    largest = np.float32(3.4028235e38)
+    feed["v"][:] = np.where(np.random.default_rng(0).random(feed["v"].shape) < 0.5, -largest * np.float32(1 - 2.0 ** -13), largest * np.float32(1 - 2.0 ** -19))
+    operand = {n: torch.from_numpy(x.reshape(-1)).cuda() for n, x in feed.items()}
+    out, status = torch.zeros(batch * q_len * heads * d, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    rc = M.lib().msx_op_attention_f32(ptr(operand["q"]), ptr(operand["k"]), ptr(operand["v"]), ptr(operand["mask"]), None, ptr(out), None, None, None, None,
+                                      None, *shape, ptr(status), None)
+    assert rc == M.OK and int(status.item()) == 0
+    want = np.repeat(feed["v"].reshape(batch, 1, k_len, heads * d)[:, :, 3], q_len, axis=1).reshape(-1)
+    got = out.cpu().numpy()
+    assert np.isfinite(got).all()
+    assert np.abs(got.astype(np.float64) / want - 1.0).max() <= 2.0 ** -20
+
+
 # One way each: both kernels, the forward with its probabilities left for the gradients' products (rows on and off 16 bytes),
 # neither.
 @pytest.mark.parametrize("batch,q_len,k_len,heads,d", [(32, 128, 128, 2, 64), (5, 77, 77, 3, 33), (32, 100, 100, 8, 32), (60, 96, 99, 6, 7), (2, 160, 256, 3, 16)])
