@@ -110,9 +110,9 @@ __device__ __forceinline__ void weighted_rows_phase(const float* __restrict__ sr
 // Shared memory layout of the query-major kernels, in floats:
 //   qs[32][d + 1], gs[32][d + 1] (grad-q only), tile[64][d + 1], ss[32][s + 1],
 //   ds2[32][s + 1] (grad-q only), stat_max[32], stat_sum[32], stat_dot[32]
-__global__ void __launch_bounds__(THREADS) forward_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                                                           const float* __restrict__ v, const float* __restrict__ mask,
-                                                           float* __restrict__ out, Dims dm) {
+__global__ void __launch_bounds__(THREADS) forward_kernel(const float* q, const float* k,
+                                                           const float* v, const float* mask,
+                                                           float* out, Dims dm) {
     after_producers();
     extern __shared__ float smem[];
     const uint32_t ds = dm.d + 1, sstride = dm.s + 1;
@@ -136,10 +136,10 @@ __global__ void __launch_bounds__(THREADS) forward_kernel(const float* __restric
     }
 }
 
-__global__ void __launch_bounds__(THREADS) grad_q_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                                                          const float* __restrict__ v, const float* __restrict__ mask,
-                                                          const float* __restrict__ g, float* __restrict__ stats,
-                                                          float* __restrict__ dq, Dims dm) {
+__global__ void __launch_bounds__(THREADS) grad_q_kernel(const float* q, const float* k,
+                                                          const float* v, const float* mask,
+                                                          const float* g, float* stats,
+                                                          float* dq, Dims dm) {
     after_producers();
     extern __shared__ float smem[];
     const uint32_t ds = dm.d + 1, sstride = dm.s + 1;
@@ -205,10 +205,10 @@ __global__ void __launch_bounds__(THREADS) grad_q_kernel(const float* __restrict
 // Key-major: the CTA owns 32 keys and walks the queries of the sequence in ascending tiles.
 // Shared, in floats: ks[32][d+1], vs[32][d+1], qs[32][d+1], gs[32][d+1], ps[32][33], dss[32][33],
 // st[32][3].
-__global__ void __launch_bounds__(THREADS) grad_kv_kernel(const float* __restrict__ q, const float* __restrict__ k,
-                                                           const float* __restrict__ v, const float* __restrict__ mask,
-                                                           const float* __restrict__ g, const float* __restrict__ stats,
-                                                           float* __restrict__ dk, float* __restrict__ dv, Dims dm) {
+__global__ void __launch_bounds__(THREADS) grad_kv_kernel(const float* q, const float* k,
+                                                           const float* v, const float* mask,
+                                                           const float* g, const float* stats,
+                                                           float* dk, float* dv, Dims dm) {
     after_producers();
     extern __shared__ float smem[];
     const uint32_t ds = dm.d + 1;

@@ -102,9 +102,9 @@ __device__ __forceinline__ uint32_t instruction(uint32_t n, bool b_mn) {
 
 // Four elements from column c on of a row of d, zeros past its end.
 template <bool VEC> __device__ __forceinline__ float4 fetch4(const float* __restrict__ row, uint32_t c, uint32_t d) {
-    if constexpr (VEC) return c < d ? __ldg(reinterpret_cast<const float4*>(row + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
-    return make_float4(c < d ? __ldg(row + c) : 0.f, c + 1 < d ? __ldg(row + c + 1) : 0.f, c + 2 < d ? __ldg(row + c + 2) : 0.f,
-                       c + 3 < d ? __ldg(row + c + 3) : 0.f);
+    if constexpr (VEC) return c < d ? load_global(reinterpret_cast<const float4*>(row + c)) : make_float4(0.f, 0.f, 0.f, 0.f);
+    return make_float4(c < d ? load_global(row + c) : 0.f, c + 1 < d ? load_global(row + c + 1) : 0.f, c + 2 < d ? load_global(row + c + 2) : 0.f,
+                       c + 3 < d ? load_global(row + c + 3) : 0.f);
 }
 
 // `rows` rows of a head, as fetched by the block: piece i of a thread is row i 512/(DP/4) + tid / (DP/4), four
@@ -244,9 +244,9 @@ template <int DP, uint32_t STEPS> __device__ __forceinline__ void issue_product(
 template <int DP> constexpr int forward_bytes() { return 2 * (DP / 32) * 2 * FORWARD_KEYS * 128 + static_cast<int>(sizeof(Control)); }
 
 template <int DP, bool VEC>
-__global__ void __launch_bounds__(THREADS, 1) attention_f32_forward_kernel(const float* __restrict__ q, const float* __restrict__ k, const float* __restrict__ v,
-                                                                           const float* __restrict__ mask, float* __restrict__ out, float2* __restrict__ stats,
-                                                                           float* __restrict__ p_out, const Shape sh, uint32_t* __restrict__ status) {
+__global__ void __launch_bounds__(THREADS, 1) attention_f32_forward_kernel(const float* q, const float* k, const float* v,
+                                                                           const float* mask, float* out, float2* stats,
+                                                                           float* p_out, const Shape sh, uint32_t* status) {
     constexpr uint32_t PANELS = DP / 32, SCORES = 0, P_HI = 0, P_LO = 128, PV = 256, Q_HI = 384, Q_LO = 448, OWN = DP / 4;
     extern __shared__ __align__(1024) char smem[];
     char* const k_tile = smem;
@@ -267,7 +267,7 @@ __global__ void __launch_bounds__(THREADS, 1) attention_f32_forward_kernel(const
         const uint32_t rows = min(kt, sh.s - j0);
         kp.fetch(kb + static_cast<uint64_t>(j0) * sh.h, sh.h, rows, sh.d);
         vp.fetch(vb + static_cast<uint64_t>(j0) * sh.h, sh.h, rows, sh.d);
-        mine = part * 32 + lane < rows ? __ldg(mb + j0 + part * 32 + lane) : 0.0f;
+        mine = part * 32 + lane < rows ? load_global(mb + j0 + part * 32 + lane) : 0.0f;
     };
     const uint32_t tmem = begin(ctl), lanes = tmem + ((quarter * 32u) << 16);
     fetch(0);
@@ -439,11 +439,11 @@ template <int DP, bool VEC> __device__ __forceinline__ void backward_queries(cha
         const uint32_t keys = min(kt, sh.s - j0);
         kp.fetch(x.k + k_at + static_cast<uint64_t>(j0) * sh.h, sh.h, keys, sh.d);
         vp.fetch(x.v + k_at + static_cast<uint64_t>(j0) * sh.h, sh.h, keys, sh.d);
-        mine = lane < 16 && part * 16 + lane < keys ? __ldg(mb + j0 + part * 16 + lane) : 0.0f;
+        mine = lane < 16 && part * 16 + lane < keys ? load_global(mb + j0 + part * 16 + lane) : 0.0f;
     };
     const uint32_t tmem = begin(ctl), lanes = tmem + ((quarter * 32u) << 16);
     fetch(0);
-    const float2 stat = at.first + row < sh.l ? __ldg(x.stats + (static_cast<uint64_t>(at.b) * sh.heads + at.a) * sh.l + at.first + row) : make_float2(0.f, 1.f);
+    const float2 stat = at.first + row < sh.l ? load_global(x.stats + (static_cast<uint64_t>(at.b) * sh.heads + at.a) * sh.l + at.first + row) : make_float2(0.f, 1.f);
     float own[OWN], other[OWN];
     fetch_row<DP, VEC>(x.q + q_at, sh.h, at.first + row, sh.l, part * OWN, sh.d, own);
     fetch_row<DP, VEC>(x.g + q_at, sh.h, at.first + row, sh.l, part * OWN, sh.d, other);
@@ -539,11 +539,11 @@ template <int DP, bool VEC> __device__ __forceinline__ void backward_keys(char* 
         qp.fetch(x.q + from, sh.h, queries, sh.d);
         gp.fetch(x.g + from, sh.h, queries, sh.d);
         op.fetch(x.out + from, sh.h, queries, sh.d);
-        stat = tid < queries ? __ldg(stats + i0 + tid) : make_float2(0.f, 1.f);
+        stat = tid < queries ? load_global(stats + i0 + tid) : make_float2(0.f, 1.f);
     };
     const uint32_t tmem = begin(ctl), lanes = tmem + ((quarter * 32u) << 16);
     fetch(0);
-    const bool counted = at.first + row < sh.s && __ldg(x.mask + static_cast<uint64_t>(at.b) * sh.s + at.first + row) != 0.0f;
+    const bool counted = at.first + row < sh.s && load_global(x.mask + static_cast<uint64_t>(at.b) * sh.s + at.first + row) != 0.0f;
     float own[OWN];
     fetch_row<DP, VEC>(x.k + k_at, sh.h, at.first + row, sh.s, part * OWN, sh.d, own);
     store_split(lanes + ROWS_A_HI + part * OWN, lanes + ROWS_A_LO + part * OWN, own);

@@ -489,7 +489,7 @@ __device__ __forceinline__ void backward_rows(const BackwardMaps& maps, const Fu
             if (query >= args.q_len) return;
             const uint64_t global_row = static_cast<uint64_t>(seq) * args.q_len + query;
             const float* const st = args.stats + (global_row * args.heads + head) * 2;
-            const float best = __ldg(st), total = __ldg(st + 1);
+            const float best = load_global(st), total = load_global(st + 1);
             if (total > 0.0f) *shift = fmaf(best, 1.4426950408889634f, log2f(total));
             const bf16* o = static_cast<const bf16*>(args.o) + global_row * args.h + head * args.d;
             const bf16* g = static_cast<const bf16*>(args.g) + global_row * args.h + head * args.d;
@@ -504,7 +504,7 @@ __device__ __forceinline__ void backward_rows(const BackwardMaps& maps, const Fu
         bool counted = true;
         if (KEYS) {
             for (uint32_t query = tid; query < steps * BWD_STEP; query += 32 * BWD_ROW_WARPS) statistics(query, &row_shift[query], &row_dot[query]);
-            counted = row < args.k_len && __ldg(args.mask + static_cast<uint64_t>(seq) * args.k_len + row) != 0.0f;
+            counted = row < args.k_len && load_global(args.mask + static_cast<uint64_t>(seq) * args.k_len + row) != 0.0f;
             __syncwarp();
             if (lane == 0) mbar_arrive(bar(STATS_MET));
             alive = __all_sync(0xffffffffu, mbar_wait(bar(STATS_MET), 0, abort_flag, args.status));

@@ -27,7 +27,7 @@ constexpr uint32_t ROW_BLOCK_WARPS = 8;
 
 // p = softmax over the unmasked keys of acc * scale, in place.
 template <int ITEMS, int V>
-__global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(float* __restrict__ scores, const float* __restrict__ mask, uint32_t rows,
+__global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(float* scores, const float* mask, uint32_t rows,
                                                                               uint32_t rows_per_sequence, uint32_t s, float scale) {
     after_producers();
     const uint32_t row = blockIdx.x * ROW_BLOCK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -44,11 +44,11 @@ __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(fl
         if constexpr (V == 4) {
             const float4 x4 = *reinterpret_cast<const float4*>(p + j);
             x[i] = x4.x; x[i + 1] = x4.y; x[i + 2] = x4.z; x[i + 3] = x4.w;
-            mask4 = make_float4(__ldg(m + j), __ldg(m + j + 1), __ldg(m + j + 2), __ldg(m + j + 3));
+            mask4 = make_float4(load_global(m + j), load_global(m + j + 1), load_global(m + j + 2), load_global(m + j + 3));
             if (key_of(i) < s) counts |= ((mask4.x != 0.0f ? 1u : 0u) | (mask4.y != 0.0f ? 2u : 0u) | (mask4.z != 0.0f ? 4u : 0u) | (mask4.w != 0.0f ? 8u : 0u)) << i;
         } else {
             x[i] = p[j];
-            counts |= (key_of(i) < s && __ldg(m + j) != 0.0f ? 1u : 0u) << i;
+            counts |= (key_of(i) < s && load_global(m + j) != 0.0f ? 1u : 0u) << i;
         }
     }
     float best = -INFINITY;
@@ -82,7 +82,7 @@ __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) masked_softmax_kernel(fl
 
 // dS = scale * P * (dP - sum_j P dP), written over dP.
 template <int ITEMS>
-__global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) score_grad_kernel(const float* __restrict__ p, float* __restrict__ dp, uint32_t rows, uint32_t s,
+__global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) score_grad_kernel(const float* p, float* dp, uint32_t rows, uint32_t s,
                                                                           float scale) {
     after_producers();
     const uint32_t row = blockIdx.x * ROW_BLOCK_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
@@ -93,7 +93,7 @@ __global__ void __launch_bounds__(32 * ROW_BLOCK_WARPS) score_grad_kernel(const 
 #pragma unroll
     for (int i = 0; i < ITEMS; ++i) {
         const uint32_t j = min(lane + 32 * i, s - 1);
-        x[i] = __ldg(pr + j);
+        x[i] = load_global(pr + j);
         d[i] = dr[j];
     }
     float dot = 0.0f;
@@ -203,7 +203,7 @@ void attention_tc_backward(cudaStream_t s, const float* q, const float* k, const
 namespace {
 
 // One warp per score row: p = softmax over the unmasked keys of scores * scale, stored as bf16.
-__global__ void masked_softmax_half_kernel(const float* __restrict__ scores, const float* __restrict__ mask, bf16* __restrict__ p,
+__global__ void masked_softmax_half_kernel(const float* scores, const float* mask, bf16* p,
                                            uint32_t rows, uint32_t rows_per_sequence, uint32_t s, float scale) {
     after_producers();
     uint32_t row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
@@ -223,7 +223,7 @@ __global__ void masked_softmax_half_kernel(const float* __restrict__ scores, con
 }
 
 // dS = scale * P * (dP - sum_j P dP), stored as bf16.
-__global__ void score_grad_half_kernel(const bf16* __restrict__ p, const float* __restrict__ dp, bf16* __restrict__ ds, uint32_t rows,
+__global__ void score_grad_half_kernel(const bf16* p, const float* dp, bf16* ds, uint32_t rows,
                                        uint32_t s, float scale) {
     after_producers();
     uint32_t row = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);

@@ -69,19 +69,60 @@ __device__ __forceinline__ void after_producers() {
     let_next_start();
 }
 
+// A load of what another kernel of the step may have written. The read-only path (__ldg, ld.global.nc, a kernel's `const
+// __restrict__` parameter) is for memory that nobody writes while the kernel runs, which a kernel that starts early does not
+// know, and the compiler may move such a load in front of the wait above. So: ordinary loads, and no __restrict__ on
+// a kernel's parameters (on those of a function in its body it tells the accesses there apart, no more).
+template <class T> __device__ __forceinline__ T load_global(const T* p) { return *p; }
+
+// Where a kernel's stores keep the compiler from moving such loads together (they may be to the same memory, for all it
+// knows), and registers or unrolled loops ask for that: a pointer made here, behind the wait, and loads that the compiler may place
+// anywhere its value is known. For memory that the kernel itself does not write before it has read it.
+// (A BERT-tiny step in mixed precision 350 us, 355 with ordinary loads in the layer norms' gradients and the column sums.)
+template <class T> struct Settled {
+    const T* p;
+    __device__ __forceinline__ Settled operator+(uint64_t n) const { return {p + n}; }
+    __device__ __forceinline__ explicit operator bool() const { return p != nullptr; }
+};
+template <class T> __device__ __forceinline__ Settled<T> settled(const T* p) {
+    asm volatile("" : "+l"(p)::"memory");
+    return {p};
+}
+template <class V> __device__ __forceinline__ V load_settled(const void* p);
+template <> __device__ __forceinline__ uint16_t load_settled<uint16_t>(const void* p) {
+    uint16_t v;
+    asm("ld.global.u16 %0, [%1];" : "=h"(v) : "l"(p));
+    return v;
+}
+template <> __device__ __forceinline__ uint32_t load_settled<uint32_t>(const void* p) {
+    uint32_t v;
+    asm("ld.global.b32 %0, [%1];" : "=r"(v) : "l"(p));
+    return v;
+}
+template <> __device__ __forceinline__ uint2 load_settled<uint2>(const void* p) {
+    uint2 v;
+    asm("ld.global.v2.b32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+    return v;
+}
+template <> __device__ __forceinline__ uint4 load_settled<uint4>(const void* p) {
+    uint4 v;
+    asm("ld.global.v4.b32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+    return v;
+}
+
 // ---- elements of either storage type ------------------------------------------------------------
 // A mixed-precision plan stores activations as bf16; the kernels that touch them are templates on
 // the element type and compute in f32 whatever it is. One element, or four consecutive ones (16
 // bytes of f32, 8 bytes of bf16; the address a multiple of that).
 using bf16 = __nv_bfloat16;
-__device__ __forceinline__ float load1(const float* p) { return __ldg(p); }
+__device__ __forceinline__ float load1(const float* p) { return load_global(p); }
 __device__ __forceinline__ float load1(const bf16* p) { return __bfloat162float(*p); }
 __device__ __forceinline__ void store1(float* p, float v) { *p = v; }
 __device__ __forceinline__ void store1(bf16* p, float v) { *p = __float2bfloat16_rn(v); }
 // Two consecutive elements (the address a multiple of their size).
-__device__ __forceinline__ float2 load2(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
+__device__ __forceinline__ float2 load2(const float* p) { return load_global(reinterpret_cast<const float2*>(p)); }
 __device__ __forceinline__ float2 load2(const bf16* p) {
-    const uint32_t raw = __ldg(reinterpret_cast<const uint32_t*>(p));
+    const uint32_t raw = load_global(reinterpret_cast<const uint32_t*>(p));
     return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw));
 }
 __device__ __forceinline__ void store2(float* p, float2 v) { *reinterpret_cast<float2*>(p) = v; }
@@ -89,13 +130,20 @@ __device__ __forceinline__ void store2(bf16* p, float2 v) {
     const __nv_bfloat162 pair = __floats2bfloat162_rn(v.x, v.y);
     *reinterpret_cast<uint32_t*>(p) = *reinterpret_cast<const uint32_t*>(&pair);
 }
-__device__ __forceinline__ float4 load4(const float* p) { return __ldg(reinterpret_cast<const float4*>(p)); }
-__device__ __forceinline__ float4 load4(const bf16* p) {
-    const uint2 raw = __ldg(reinterpret_cast<const uint2*>(p));
+__device__ __forceinline__ float4 four_halves(const uint2& raw) {
     const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
     const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
     return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
+__device__ __forceinline__ float4 load4(const float* p) { return load_global(reinterpret_cast<const float4*>(p)); }
+__device__ __forceinline__ float4 load4(const bf16* p) { return four_halves(load_global(reinterpret_cast<const uint2*>(p))); }
+__device__ __forceinline__ float load1(Settled<float> s) { return __uint_as_float(load_settled<uint32_t>(s.p)); }
+__device__ __forceinline__ float load1(Settled<bf16> s) { return __uint_as_float(static_cast<uint32_t>(load_settled<uint16_t>(s.p)) << 16); }
+__device__ __forceinline__ float4 load4(Settled<float> s) {
+    const uint4 raw = load_settled<uint4>(s.p);
+    return make_float4(__uint_as_float(raw.x), __uint_as_float(raw.y), __uint_as_float(raw.z), __uint_as_float(raw.w));
+}
+__device__ __forceinline__ float4 load4(Settled<bf16> s) { return four_halves(load_settled<uint2>(s.p)); }
 __device__ __forceinline__ void store4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
 __device__ __forceinline__ void store4(bf16* p, float4 v) {
     const __nv_bfloat162 lo = __floats2bfloat162_rn(v.x, v.y), hi = __floats2bfloat162_rn(v.z, v.w);
@@ -108,14 +156,11 @@ __device__ __forceinline__ void store4(bf16* p, float4 v) {
 struct float8 {
     float4 lo, hi;
 };
-__device__ __forceinline__ float8 load8(const bf16* p) {
-    const uint4 raw = __ldg(reinterpret_cast<const uint4*>(p));
-    const float2 a = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
-    const float2 b = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
-    const float2 c = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.z));
-    const float2 d = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.w));
-    return {make_float4(a.x, a.y, b.x, b.y), make_float4(c.x, c.y, d.x, d.y)};
+__device__ __forceinline__ float8 eight_halves(const uint4& raw) {
+    return {four_halves(make_uint2(raw.x, raw.y)), four_halves(make_uint2(raw.z, raw.w))};
 }
+__device__ __forceinline__ float8 load8(const bf16* p) { return eight_halves(load_global(reinterpret_cast<const uint4*>(p))); }
+__device__ __forceinline__ float8 load8(Settled<bf16> s) { return eight_halves(load_settled<uint4>(s.p)); }
 __device__ __forceinline__ void store8(bf16* p, const float8& v) {
     const __nv_bfloat162 a = __floats2bfloat162_rn(v.lo.x, v.lo.y), b = __floats2bfloat162_rn(v.lo.z, v.lo.w);
     const __nv_bfloat162 c = __floats2bfloat162_rn(v.hi.x, v.hi.y), d = __floats2bfloat162_rn(v.hi.z, v.hi.w);

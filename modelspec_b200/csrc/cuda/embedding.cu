@@ -21,9 +21,9 @@ namespace k {
 namespace {
 
 template <class TI, class TO>
-__global__ void embedding_kernel(const TI* __restrict__ table, const int32_t* __restrict__ ids,
-                                 TO* __restrict__ out, uint64_t n, uint32_t rows, uint32_t h,
-                                 uint32_t* __restrict__ status) {
+__global__ void embedding_kernel(const TI* table, const int32_t* ids,
+                                 TO* out, uint64_t n, uint32_t rows, uint32_t h,
+                                 uint32_t* status) {
     after_producers();
     // One warp per output row, 128-bit copies when the row length allows.
     uint64_t row = (static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x) >> 5;
@@ -49,9 +49,9 @@ __global__ void embedding_kernel(const TI* __restrict__ table, const int32_t* __
 // 4096-id tile, read from shared memory as broadcast int4; an id outside the table sorts last and
 // is never matched by a row. n^2 / 8 comparisons per lane group: 2 M for n = 4096.
 constexpr int kOrderTile = 4096;
-__global__ void __launch_bounds__(256) order_kernel(const int32_t* __restrict__ ids, uint32_t n, uint32_t rows,
-                                                    int32_t* __restrict__ sorted_id, int32_t* __restrict__ sorted_n,
-                                                    uint32_t* __restrict__ status) {
+__global__ void __launch_bounds__(256) order_kernel(const int32_t* ids, uint32_t n, uint32_t rows,
+                                                    int32_t* sorted_id, int32_t* sorted_n,
+                                                    uint32_t* status) {
     after_producers();
     __shared__ int4 tile[kOrderTile / 4];
     const uint32_t i = blockIdx.x * 32 + threadIdx.x / 8, part = threadIdx.x & 7u;
@@ -128,8 +128,8 @@ __device__ __forceinline__ uint32_t warp_lower_bound(const int32_t* __restrict__
 // two (16,384 ids of 768 columns, three tables: bf16 168 -> 140 us, f32 171 -> 140).
 constexpr uint32_t kHotRow = 32, kHotChunk = 32, kTogether = 8, kCachedIds = 4096;
 template <int VEC, class TG, class TO>
-__global__ void __launch_bounds__(256, 3) scatter_kernel(const TG* __restrict__ g, const int32_t* __restrict__ sorted_id,
-                                                      const int32_t* __restrict__ sorted_n, uint32_t n,
+__global__ void __launch_bounds__(256, 3) scatter_kernel(const TG* g, const int32_t* sorted_id,
+                                                      const int32_t* sorted_n, uint32_t n,
                                                       const float* base, TO* out, uint32_t rows, uint32_t h) {
     after_producers();
     constexpr uint32_t span = VEC * 32;
@@ -172,7 +172,7 @@ __global__ void __launch_bounds__(256, 3) scatter_kernel(const TG* __restrict__ 
                 float acc[VEC];
 #pragma unroll
                 for (int q = 0; q < VEC; ++q) acc[q] = 0.0f;
-                const int32_t entry = lane < count ? __ldg(sorted_n + at + lane) : 0;
+                const int32_t entry = lane < count ? load_global(sorted_n + at + lane) : 0;
                 for (uint32_t done = 0; done < count; done += kTogether) {
                     const uint32_t here = min(kTogether, count - done);
                     float v[kTogether][VEC];
@@ -234,7 +234,7 @@ __global__ void __launch_bounds__(256, 3) scatter_kernel(const TG* __restrict__ 
 #pragma unroll
                 for (int j = 0; j < LOADS; ++j) {
                     const uint32_t r = (threadIdx.x + 256 * j) / (span / VEC);
-                    source[set][j] = chunk_start + r < count ? __ldg(sorted_n + at + chunk_start + r) : -1;
+                    source[set][j] = chunk_start + r < count ? load_global(sorted_n + at + chunk_start + r) : -1;
                 }
             };
             auto fetch = [&](int set) {
@@ -306,8 +306,8 @@ __global__ void __launch_bounds__(256, 3) scatter_kernel(const TG* __restrict__ 
 // is what the launch waits for, so each group of columns has a block of its own (as a loop within the
 // block, 16,384 ids and 768 columns took 211 us; now 65).
 template <int VEC, class TG, class TO>
-__global__ void __launch_bounds__(256, 3) scatter_in_place_kernel(const TG* __restrict__ g, const int32_t* __restrict__ sorted_id,
-                                                               const int32_t* __restrict__ sorted_n, uint32_t n, TO* out, uint32_t rows,
+__global__ void __launch_bounds__(256, 3) scatter_in_place_kernel(const TG* g, const int32_t* sorted_id,
+                                                               const int32_t* sorted_n, uint32_t n, TO* out, uint32_t rows,
                                                                uint32_t h) {
     after_producers();
     constexpr uint32_t span = VEC * 32;
@@ -341,7 +341,7 @@ __global__ void __launch_bounds__(256, 3) scatter_in_place_kernel(const TG* __re
                 float acc[VEC];
 #pragma unroll
                 for (int q = 0; q < VEC; ++q) acc[q] = 0.0f;
-                const int32_t entry = lane < count ? __ldg(sorted_n + p + lane) : 0;
+                const int32_t entry = lane < count ? load_global(sorted_n + p + lane) : 0;
                 for (uint32_t done = 0; done < count; done += kTogether) {
                     const uint32_t here = min(kTogether, count - done);
                     float v[kTogether][VEC];
@@ -392,7 +392,7 @@ __global__ void __launch_bounds__(256, 3) scatter_in_place_kernel(const TG* __re
 #pragma unroll
             for (int j = 0; j < LOADS; ++j) {
                 const uint32_t r = (threadIdx.x + 256 * j) / (span / VEC);
-                source[set][j] = chunk_start + r < count ? __ldg(sorted_n + at + chunk_start + r) : -1;
+                source[set][j] = chunk_start + r < count ? load_global(sorted_n + at + chunk_start + r) : -1;
             }
         };
         auto fetch = [&](int set) {

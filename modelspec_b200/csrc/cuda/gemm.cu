@@ -19,9 +19,9 @@ namespace {
 constexpr int BM = 64, BN = 64, BK = 16, TM = 4, TN = 4;
 
 template <bool A_T, bool B_T>
-__global__ void __launch_bounds__(256) matmul_kernel(const float* __restrict__ a, const float* __restrict__ b,
-                                                     float* __restrict__ c, uint32_t m, uint32_t n, uint32_t k,
-                                                     const float* __restrict__ bias) {
+__global__ void __launch_bounds__(256) matmul_kernel(const float* a, const float* b,
+                                                     float* c, uint32_t m, uint32_t n, uint32_t k,
+                                                     const float* bias) {
     after_producers();
     __shared__ float as[BK][BM + 4];
     __shared__ float bs[BK][BN + 4];

@@ -299,7 +299,7 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) bf16_kernel(const __
 #pragma unroll
             for (int i = 0; i < T::COLUMNS / 32; ++i) {
                 const uint32_t c = w.n0 + first_col + i * 32 + lane;
-                bias[i] = w.bias && c < w.n ? __ldg(w.bias + c) : 0.0f;
+                bias[i] = w.bias && c < w.n ? load_global(w.bias + c) : 0.0f;
             }
             alive = warp_wait<CG>(smem_u32(&acc_full[acc]), (turn >> 1) & 1u, abort_flag, args.status);
             if (!alive) break;
@@ -443,8 +443,8 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) bf16_kernel(const __
 }
 
 // The sum of the split-k partial tiles, ascending split order, into C (either type) with the bias.
-__global__ void splitk_reduce_bf16_kernel(const float* __restrict__ ws, void* __restrict__ c, uint32_t out_half, uint64_t m, uint32_t n,
-                                          uint32_t ldc, uint32_t splits, const float* __restrict__ bias) {
+__global__ void splitk_reduce_bf16_kernel(const float* ws, void* c, uint32_t out_half, uint64_t m, uint32_t n,
+                                          uint32_t ldc, uint32_t splits, const float* bias) {
     after_producers();
     const uint64_t count = m * n, stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {

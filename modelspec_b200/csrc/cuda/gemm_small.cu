@@ -45,12 +45,12 @@ template <int COUNT> struct Problems {
 
 // Four consecutive elements at p + index, `valid` of which exist.
 __device__ __forceinline__ float4 load_four(const float* __restrict__ p, uint64_t index, uint32_t valid, bool vec) {
-    if (valid == 4 && vec) return __ldg(reinterpret_cast<const float4*>(p + index));
+    if (valid == 4 && vec) return load_global(reinterpret_cast<const float4*>(p + index));
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (valid > 0) v.x = __ldg(p + index);
-    if (valid > 1) v.y = __ldg(p + index + 1);
-    if (valid > 2) v.z = __ldg(p + index + 2);
-    if (valid > 3) v.w = __ldg(p + index + 3);
+    if (valid > 0) v.x = load_global(p + index);
+    if (valid > 1) v.y = load_global(p + index + 1);
+    if (valid > 2) v.z = load_global(p + index + 2);
+    if (valid > 3) v.w = load_global(p + index + 3);
     return v;
 }
 __device__ __forceinline__ uint32_t inside(uint32_t start, uint32_t limit) { return start >= limit ? 0u : (limit - start >= 4u ? 4u : limit - start); }
@@ -156,7 +156,7 @@ __global__ void __launch_bounds__(THREADS) matmul_small_kernel(const __grid_cons
 #pragma unroll
             for (uint32_t i = 0; i < OWN; ++i) {
                 const uint32_t e = rank * share + threadIdx.x + i * THREADS, row = m0 + e / BN, col = n0 + e % BN;
-                argument[i] = e < end && row < m && col < n ? __ldg(p.beside + static_cast<uint64_t>(row) * p.ldc + col) : 0.0f;
+                argument[i] = e < end && row < m && col < n ? load_global(p.beside + static_cast<uint64_t>(row) * p.ldc + col) : 0.0f;
             }
         }
     }
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(THREADS) matmul_small_kernel(const __grid_cons
         const uint32_t row = m0 + e / BN, col = n0 + e % BN;
         if (row >= m || col >= n) return;
         const uint64_t at = static_cast<uint64_t>(row) * p.ldc + col;
-        v = bias ? v + __ldg(bias + col) : v;
+        v = bias ? v + load_global(bias + col) : v;
         if constexpr (ACT) {
             const float x = argument[OWN == 2 ? i & 1u : i];
             if (epilogue == Epilogue::GeluGrad) v = gelu_grad_value(x, v);

@@ -173,13 +173,13 @@ __device__ __forceinline__ float4 load4(const float* __restrict__ p, uint64_t in
     float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
     const float* at = p + index;
     if (valid == 4 && vec) {
-        asm volatile("ld.global.nc.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(at));
+        asm volatile("ld.global.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w) : "l"(at));
         return v;
     }
-    if (valid > 0) asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v.x) : "l"(at));
-    if (valid > 1) asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v.y) : "l"(at + 1));
-    if (valid > 2) asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v.z) : "l"(at + 2));
-    if (valid > 3) asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v.w) : "l"(at + 3));
+    if (valid > 0) asm volatile("ld.global.f32 %0, [%1];" : "=f"(v.x) : "l"(at));
+    if (valid > 1) asm volatile("ld.global.f32 %0, [%1];" : "=f"(v.y) : "l"(at + 1));
+    if (valid > 2) asm volatile("ld.global.f32 %0, [%1];" : "=f"(v.z) : "l"(at + 2));
+    if (valid > 3) asm volatile("ld.global.f32 %0, [%1];" : "=f"(v.w) : "l"(at + 3));
     return v;
 }
 
@@ -350,7 +350,7 @@ __global__ void __launch_bounds__(THREADS, Config<BM, BN>::CTAS_PER_SM) matmul_t
             const uint32_t gn = n0 + (lane % (BN / 4)) * 4;
 #pragma unroll
             for (int q = 0; q < 4; ++q)
-                if (gn + q < pn) bias_mine[q] = __ldg(bias_row + gn + q);
+                if (gn + q < pn) bias_mine[q] = load_global(bias_row + gn + q);
         }
 #pragma unroll
         for (int s = 0; s < SETS - 1; ++s)
@@ -470,12 +470,12 @@ __global__ void __launch_bounds__(THREADS, Config<BM, BN>::CTAS_PER_SM) matmul_t
                 float other[4] = {0.f, 0.f, 0.f, 0.f};
                 if (args.epilogue == Epilogue::GeluGrad || args.epilogue == Epilogue::ReluGrad) {
                     if (whole) {
-                        const float4 f = __ldg(reinterpret_cast<const float4*>(at));
+                        const float4 f = load_global(reinterpret_cast<const float4*>(at));
                         other[0] = f.x; other[1] = f.y; other[2] = f.z; other[3] = f.w;
                     } else {
 #pragma unroll
                         for (int q = 0; q < 4; ++q)
-                            if (gn + q < pn) other[q] = __ldg(at + q);
+                            if (gn + q < pn) other[q] = load_global(at + q);
                     }
 #pragma unroll
                     for (int q = 0; q < 4; ++q) v[q] = args.epilogue == Epilogue::GeluGrad ? gelu_grad_value(other[q], v[q]) : relu_grad_value(other[q], v[q]);
@@ -553,8 +553,8 @@ __global__ void __launch_bounds__(THREADS, Config<BM, BN>::CTAS_PER_SM) matmul_t
     }
 }
 
-__global__ void splitk_reduce_kernel(const float* __restrict__ ws, float* __restrict__ c, uint64_t count, uint32_t splits,
-                                     const float* __restrict__ bias, uint32_t n) {
+__global__ void splitk_reduce_kernel(const float* ws, float* c, uint64_t count, uint32_t splits,
+                                     const float* bias, uint32_t n) {
     after_producers();
     uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < count; i += stride) {

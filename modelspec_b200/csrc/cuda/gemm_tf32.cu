@@ -372,12 +372,12 @@ __global__ void __launch_bounds__(Tile<CG, BN>::THREADS, 1) tf32_kernel(const __
             const uint32_t bias_at = w.n0 + first_col + 4 * lane;
             if (w.bias && segment == 0 && lane < T::CHUNKS * 8u) {
                 if (bias_at + 4 <= w.n && reinterpret_cast<uintptr_t>(w.bias) % 16 == 0) {
-                    bias4 = __ldg(reinterpret_cast<const float4*>(w.bias + bias_at));
+                    bias4 = load_global(reinterpret_cast<const float4*>(w.bias + bias_at));
                 } else {
-                    if (bias_at < w.n) bias4.x = __ldg(w.bias + bias_at);
-                    if (bias_at + 1 < w.n) bias4.y = __ldg(w.bias + bias_at + 1);
-                    if (bias_at + 2 < w.n) bias4.z = __ldg(w.bias + bias_at + 2);
-                    if (bias_at + 3 < w.n) bias4.w = __ldg(w.bias + bias_at + 3);
+                    if (bias_at < w.n) bias4.x = load_global(w.bias + bias_at);
+                    if (bias_at + 1 < w.n) bias4.y = load_global(w.bias + bias_at + 1);
+                    if (bias_at + 2 < w.n) bias4.z = load_global(w.bias + bias_at + 2);
+                    if (bias_at + 3 < w.n) bias4.w = load_global(w.bias + bias_at + 3);
                 }
             }
             alive = tc::warp_wait<CG>(tc::smem_u32(&acc_full[acc]), (turn >> 1) & 1u, abort_flag, args.status);

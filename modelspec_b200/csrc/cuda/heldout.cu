@@ -57,7 +57,7 @@ __device__ __forceinline__ void see(RowFacts& f, float x, uint32_t i) {
 // 16 bytes at a time from the first 16-byte boundary of the row.
 template <class F> __device__ __forceinline__ void visit(const float* row, uint32_t classes, F f) {
     const uint32_t head = min(classes, static_cast<uint32_t>((16u - (reinterpret_cast<uintptr_t>(row) & 15u)) & 15u) / 4u);
-    if (threadIdx.x < head) f(__ldg(row + threadIdx.x), threadIdx.x);
+    if (threadIdx.x < head) f(load_global(row + threadIdx.x), threadIdx.x);
     const uint32_t body = (classes - head) / 4;
     const float4* wide = reinterpret_cast<const float4*>(row + head);
     auto four = [&](const float4& v, uint32_t i) {
@@ -68,21 +68,21 @@ template <class F> __device__ __forceinline__ void visit(const float* row, uint3
     };
     uint32_t j = threadIdx.x;
     for (; j + 3 * THREADS < body; j += 4 * THREADS) {  // four loads in flight per thread
-        const float4 a = __ldg(wide + j), b = __ldg(wide + j + THREADS), c = __ldg(wide + j + 2 * THREADS), d = __ldg(wide + j + 3 * THREADS);
+        const float4 a = load_global(wide + j), b = load_global(wide + j + THREADS), c = load_global(wide + j + 2 * THREADS), d = load_global(wide + j + 3 * THREADS);
         four(a, head + 4 * j);
         four(b, head + 4 * (j + THREADS));
         four(c, head + 4 * (j + 2 * THREADS));
         four(d, head + 4 * (j + 3 * THREADS));
     }
-    for (; j < body; j += THREADS) four(__ldg(wide + j), head + 4 * j);
+    for (; j < body; j += THREADS) four(load_global(wide + j), head + 4 * j);
     const uint32_t tail = head + 4 * body;
-    if (tail + threadIdx.x < classes) f(__ldg(row + tail + threadIdx.x), tail + threadIdx.x);
+    if (tail + threadIdx.x < classes) f(load_global(row + tail + threadIdx.x), tail + threadIdx.x);
 }
 
-__global__ void __launch_bounds__(THREADS) heldout_rows_kernel(const float* __restrict__ logits, uint64_t pitch,
-                                                                const int32_t* __restrict__ labels, const float* __restrict__ weights,
-                                                                uint32_t rows, uint32_t classes, double* __restrict__ terms,
-                                                                uint32_t* __restrict__ hits, HeldOutState* state) {
+__global__ void __launch_bounds__(THREADS) heldout_rows_kernel(const float* logits, uint64_t pitch,
+                                                                const int32_t* labels, const float* weights,
+                                                                uint32_t rows, uint32_t classes, double* terms,
+                                                                uint32_t* hits, HeldOutState* state) {
     after_producers();
     __shared__ RowFacts warp_facts[THREADS / 32];
     __shared__ float warp_sums[THREADS / 32];
@@ -138,7 +138,7 @@ __global__ void __launch_bounds__(THREADS) heldout_rows_kernel(const float* __re
                 row_total = total;
             }
             __syncthreads();
-            nll = m + logf(row_total) - __ldg(row + label);
+            nll = m + logf(row_total) - load_global(row + label);
         }
     }
     if (threadIdx.x == 0) {

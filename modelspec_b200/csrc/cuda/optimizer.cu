@@ -43,11 +43,11 @@ __device__ __forceinline__ Span span_of(const UpdateTensor* __restrict__ tensors
 }
 
 template <int VECTORS>
-__global__ void __launch_bounds__(256) adamw_kernel(const UpdateTensor* __restrict__ tensors,
-                                                     const uint32_t* __restrict__ chunk_tensor,
-                                                     const uint32_t* __restrict__ chunk_start, uint32_t chunk, AdamWConstants c,
-                                                     const float* __restrict__ lr_t, const float* __restrict__ c1,
-                                                     const float* __restrict__ c2) {
+__global__ void __launch_bounds__(256) adamw_kernel(const UpdateTensor* tensors,
+                                                     const uint32_t* chunk_tensor,
+                                                     const uint32_t* chunk_start, uint32_t chunk, AdamWConstants c,
+                                                     const float* lr_t, const float* c1,
+                                                     const float* c2) {
     after_producers();
     const float lr = lr_t[0], k1 = c1[0], k2 = c2[0];
     const Span s = span_of(tensors, chunk_tensor, chunk_start, chunk);
@@ -105,17 +105,17 @@ __global__ void __launch_bounds__(256) adamw_kernel(const UpdateTensor* __restri
 }
 
 // The bf16 working copy of a parameter from its f32 master (after an upload).
-__global__ void working_copy_kernel(const float* __restrict__ p, bf16* __restrict__ p16, uint64_t n) {
+__global__ void working_copy_kernel(const float* p, bf16* p16, uint64_t n) {
     after_producers();
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t i = static_cast<uint64_t>(blockIdx.x) * blockDim.x + threadIdx.x; i < n; i += stride) store1(p16 + i, p[i]);
 }
 
 template <int VECTORS>
-__global__ void __launch_bounds__(256) sgd_kernel(const UpdateTensor* __restrict__ tensors,
-                                                   const uint32_t* __restrict__ chunk_tensor,
-                                                   const uint32_t* __restrict__ chunk_start, uint32_t chunk,
-                                                   const float* __restrict__ lr) {
+__global__ void __launch_bounds__(256) sgd_kernel(const UpdateTensor* tensors,
+                                                   const uint32_t* chunk_tensor,
+                                                   const uint32_t* chunk_start, uint32_t chunk,
+                                                   const float* lr) {
     after_producers();
     const float rate = lr[0];
     const Span s = span_of(tensors, chunk_tensor, chunk_start, chunk);

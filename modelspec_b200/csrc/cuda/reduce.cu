@@ -21,8 +21,8 @@ constexpr uint32_t kMaxBlocks = 592;  // 4 per SM
 enum class Whole : int { Sum, SquaredDifference };
 
 template <Whole KIND>
-__global__ void whole_stage1(const float* __restrict__ a, const float* __restrict__ b, uint64_t n,
-                             double* __restrict__ partial, double divisor, float* __restrict__ out) {
+__global__ void whole_stage1(const float* a, const float* b, uint64_t n,
+                             double* partial, double divisor, float* out) {
     after_producers();
     __shared__ double shared[33];
     double acc = 0.0;
@@ -41,8 +41,8 @@ __global__ void whole_stage1(const float* __restrict__ a, const float* __restric
     else partial[blockIdx.x] = total;
 }
 
-__global__ void whole_stage2(const double* __restrict__ partial, uint32_t blocks, double divisor,
-                             float* __restrict__ out) {
+__global__ void whole_stage2(const double* partial, uint32_t blocks, double divisor,
+                             float* out) {
     after_producers();
     __shared__ double shared[33];
     double acc = 0.0;
@@ -62,8 +62,8 @@ uint32_t whole_blocks(uint64_t n) {
 // column block to finish adds the chunk sums in ascending chunk order (what sum_rows_stage2 does
 // as a second launch) and writes `out`.
 template <class T>
-__global__ void sum_rows_stage1(const T* __restrict__ g, uint32_t rows, uint32_t h, uint32_t ld, uint32_t rows_per_chunk,
-                                float* __restrict__ partial, uint32_t* __restrict__ counters, float* __restrict__ out) {
+__global__ void sum_rows_stage1(const T* g, uint32_t rows, uint32_t h, uint32_t ld, uint32_t rows_per_chunk,
+                                float* partial, uint32_t* counters, float* out) {
     after_producers();
     __shared__ float shared[8][32];
     __shared__ bool is_last;
@@ -104,7 +104,7 @@ __global__ void sum_rows_stage1(const T* __restrict__ g, uint32_t rows, uint32_t
 // 128 columns, and a column's sum takes its terms in the order of the one-column form. Only the chunk sum is written
 // (the second stage is the step's finalize launch or sum_rows_stage2).
 template <class T>
-__device__ __forceinline__ void chunk_sum_of_four(const T* __restrict__ g, uint32_t c, uint32_t r0, uint32_t r1, uint32_t h, uint32_t ld,
+__device__ __forceinline__ void chunk_sum_of_four(Settled<T> g, uint32_t c, uint32_t r0, uint32_t r1, uint32_t h, uint32_t ld,
                                                   float4 (*shared)[32], float* __restrict__ to) {
     float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
     if (c < h) {  // the pitch covers the whole float4; columns past h hold padding and are not written below
@@ -138,12 +138,12 @@ __device__ __forceinline__ void chunk_sum_of_four(const T* __restrict__ g, uint3
 }
 
 template <class T>
-__global__ void sum_rows_stage1_wide(const T* __restrict__ g, uint32_t rows, uint32_t h, uint32_t ld, uint32_t rows_per_chunk,
-                                     float* __restrict__ partial) {
+__global__ void sum_rows_stage1_wide(const T* g, uint32_t rows, uint32_t h, uint32_t ld, uint32_t rows_per_chunk,
+                                     float* partial) {
     after_producers();
     __shared__ float4 shared[8][32];
     const uint32_t r0 = blockIdx.y * rows_per_chunk, r1 = min(rows, r0 + rows_per_chunk);
-    chunk_sum_of_four(g, (blockIdx.x * 32 + threadIdx.x) * 4, r0, r1, h, ld, shared, partial + static_cast<uint64_t>(blockIdx.y) * h);
+    chunk_sum_of_four(settled(g), (blockIdx.x * 32 + threadIdx.x) * 4, r0, r1, h, ld, shared, partial + static_cast<uint64_t>(blockIdx.y) * h);
 }
 
 // The job whose block range holds this block: the last one whose first block is not past it. Thread
@@ -162,7 +162,7 @@ __device__ __forceinline__ uint32_t job_of_block(const Job* __restrict__ jobs, u
 
 // The first stage of many column sums in one launch: block b works on the job whose block range
 // holds it, on one block of columns and one chunk of rows, as sum_rows_stage1 and sum_rows_stage1_wide do.
-__global__ void sum_rows_batched_kernel(const RowSumJob* __restrict__ jobs, uint32_t count) {
+__global__ void sum_rows_batched_kernel(const RowSumJob* jobs, uint32_t count) {
     after_producers();
     __shared__ float4 shared4[8][32];
     __shared__ uint32_t which;
@@ -172,8 +172,8 @@ __global__ void sum_rows_batched_kernel(const RowSumJob* __restrict__ jobs, uint
     const uint32_t r0 = chunk * job.rows_per_chunk, r1 = min(job.rows, r0 + job.rows_per_chunk);
     if (job.columns == 4) {  // one form per block
         float* to = job.partial + static_cast<uint64_t>(chunk) * job.width;
-        if (job.half) chunk_sum_of_four(static_cast<const bf16*>(job.g), c, r0, r1, job.width, job.ld, shared4, to);
-        else chunk_sum_of_four(static_cast<const float*>(job.g), c, r0, r1, job.width, job.ld, shared4, to);
+        if (job.half) chunk_sum_of_four(settled(static_cast<const bf16*>(job.g)), c, r0, r1, job.width, job.ld, shared4, to);
+        else chunk_sum_of_four(settled(static_cast<const float*>(job.g)), c, r0, r1, job.width, job.ld, shared4, to);
         return;
     }
     float (*shared)[32] = reinterpret_cast<float (*)[32]>(shared4);
@@ -204,8 +204,8 @@ __global__ void sum_rows_batched_kernel(const RowSumJob* __restrict__ jobs, uint
     }
 }
 
-__global__ void sum_rows_stage2(const float* __restrict__ partial, uint32_t chunks, uint32_t h,
-                                float* __restrict__ out) {
+__global__ void sum_rows_stage2(const float* partial, uint32_t chunks, uint32_t h,
+                                float* out) {
     after_producers();
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= h) return;
@@ -214,7 +214,7 @@ __global__ void sum_rows_stage2(const float* __restrict__ partial, uint32_t chun
     out[c] = total;
 }
 
-__global__ void finalize_sums_kernel(const SumJob* __restrict__ jobs, uint32_t count) {
+__global__ void finalize_sums_kernel(const SumJob* jobs, uint32_t count) {
     after_producers();
     __shared__ float shared[8][32];
     __shared__ uint32_t which;

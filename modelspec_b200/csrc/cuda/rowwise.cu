@@ -38,8 +38,8 @@ __device__ __forceinline__ void row_moments(const float* __restrict__ row, uint3
     *rstd = 1.0f / sqrtf(variance + kLayerNormEps);
 }
 
-__global__ void layer_norm_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
-                                  const float* __restrict__ beta, float* __restrict__ out, uint32_t rows,
+__global__ void layer_norm_kernel(const float* x, const float* gamma,
+                                  const float* beta, float* out, uint32_t rows,
                                   uint32_t h) {
     after_producers();
     int lane = threadIdx.x & 31;
@@ -49,11 +49,13 @@ __global__ void layer_norm_kernel(const float* __restrict__ x, const float* __re
     float mean, rstd;
     row_moments(row, h, lane, &mean, &rstd);
     float* o = out + static_cast<uint64_t>(r) * h;
-    for (uint32_t j = lane; j < h; j += 32) o[j] = (row[j] - mean) * rstd * gamma[j] + beta[j];
+    const Settled<float> values = settled(row), by = settled(gamma), plus = settled(beta);
+#pragma unroll 4
+    for (uint32_t j = lane; j < h; j += 32) o[j] = (load1(values + j) - mean) * rstd * load1(by + j) + load1(plus + j);
 }
 
-__global__ void layer_norm_grad_x_kernel(const float* __restrict__ x, const float* __restrict__ gamma,
-                                         const float* __restrict__ g, float* __restrict__ out, uint32_t rows,
+__global__ void layer_norm_grad_x_kernel(const float* x, const float* gamma,
+                                         const float* g, float* out, uint32_t rows,
                                          uint32_t h) {
     after_producers();
     int lane = threadIdx.x & 31;
@@ -80,7 +82,7 @@ __global__ void layer_norm_grad_x_kernel(const float* __restrict__ x, const floa
     }
 }
 
-__global__ void row_stats_kernel(const float* __restrict__ x, float* __restrict__ stats, uint32_t rows,
+__global__ void row_stats_kernel(const float* x, float* stats, uint32_t rows,
                                  uint32_t h) {
     after_producers();
     int lane = threadIdx.x & 31;
@@ -96,10 +98,10 @@ __global__ void row_stats_kernel(const float* __restrict__ x, float* __restrict_
 
 // Block (32, 8) over a 32-column tile and a chunk of rows: partial column sums of g * xhat and,
 // when wanted, of g.
-__global__ void grad_gamma_stage1(const float* __restrict__ x, const float* __restrict__ g,
-                                  const float* __restrict__ stats, uint32_t rows, uint32_t h,
-                                  uint32_t rows_per_chunk, float* __restrict__ partial_gamma,
-                                  float* __restrict__ partial_beta) {
+__global__ void grad_gamma_stage1(const float* x, const float* g,
+                                  const float* stats, uint32_t rows, uint32_t h,
+                                  uint32_t rows_per_chunk, float* partial_gamma,
+                                  float* partial_beta) {
     after_producers();
     __shared__ float sg[8][32], sb[8][32];
     uint32_t c = blockIdx.x * 32 + threadIdx.x;
@@ -127,9 +129,9 @@ __global__ void grad_gamma_stage1(const float* __restrict__ x, const float* __re
     }
 }
 
-__global__ void grad_gamma_stage2(const float* __restrict__ partial_gamma, const float* __restrict__ partial_beta,
-                                  uint32_t chunks, uint32_t h, float* __restrict__ dgamma,
-                                  float* __restrict__ dbeta) {
+__global__ void grad_gamma_stage2(const float* partial_gamma, const float* partial_beta,
+                                  uint32_t chunks, uint32_t h, float* dgamma,
+                                  float* dbeta) {
     after_producers();
     uint32_t c = blockIdx.x * blockDim.x + threadIdx.x;
     if (c >= h) return;
@@ -162,7 +164,7 @@ __device__ __forceinline__ void block_row_softmax(const T* __restrict__ row, uin
     *total = block_sum(s, shared);
 }
 
-__global__ void softmax_kernel(const float* __restrict__ x, float* __restrict__ out, uint32_t k) {
+__global__ void softmax_kernel(const float* x, float* out, uint32_t k) {
     after_producers();
     __shared__ float shared[33];
     const float* row = x + static_cast<uint64_t>(blockIdx.x) * k;
@@ -172,8 +174,8 @@ __global__ void softmax_kernel(const float* __restrict__ x, float* __restrict__ 
     for (uint32_t c = threadIdx.x; c < k; c += blockDim.x) o[c] = expf(row[c] - max) / total;
 }
 
-__global__ void softmax_grad_kernel(const float* __restrict__ y, const float* __restrict__ g,
-                                    float* __restrict__ out, uint32_t k) {
+__global__ void softmax_grad_kernel(const float* y, const float* g,
+                                    float* out, uint32_t k) {
     after_producers();
     __shared__ float shared[33];
     const float* yr = y + static_cast<uint64_t>(blockIdx.x) * k;
@@ -186,8 +188,8 @@ __global__ void softmax_grad_kernel(const float* __restrict__ y, const float* __
 }
 
 template <class T>
-__global__ void cross_entropy_rows_kernel(const T* __restrict__ logits, const int32_t* __restrict__ labels,
-                                          const float* __restrict__ weights, float* __restrict__ row_loss,
+__global__ void cross_entropy_rows_kernel(const T* logits, const int32_t* labels,
+                                          const float* weights, float* row_loss,
                                           uint32_t v, uint32_t ld) {
     after_producers();
     __shared__ float shared[33];
@@ -208,8 +210,8 @@ __global__ void cross_entropy_rows_kernel(const T* __restrict__ logits, const in
 }
 
 // loss = sum_n w[n] l[n] / sum_n w[n], both sums in f64 (a tree over the block), one rounding.
-__global__ void cross_entropy_loss_kernel(const float* __restrict__ row_loss, const float* __restrict__ weights,
-                                          uint32_t rows, const float* __restrict__ global_den, float* __restrict__ loss) {
+__global__ void cross_entropy_loss_kernel(const float* row_loss, const float* weights,
+                                          uint32_t rows, const float* global_den, float* loss) {
     after_producers();
     __shared__ double shared[33];
     double num = 0.0, den = 0.0;
@@ -225,7 +227,7 @@ __global__ void cross_entropy_loss_kernel(const float* __restrict__ row_loss, co
     if (threadIdx.x == 0) loss[0] = den == 0.0 ? 0.0f : static_cast<float>(num / den);
 }
 
-__global__ void weight_sum_kernel(const float* __restrict__ weights, uint32_t rows, float* __restrict__ out) {
+__global__ void weight_sum_kernel(const float* weights, uint32_t rows, float* out) {
     after_producers();
     __shared__ double shared[33];
     double den = 0.0;
@@ -234,9 +236,9 @@ __global__ void weight_sum_kernel(const float* __restrict__ weights, uint32_t ro
     if (threadIdx.x == 0) out[0] = static_cast<float>(den);
 }
 
-__global__ void cross_entropy_grad_kernel(const float* __restrict__ logits, const int32_t* __restrict__ labels,
-                                          const float* __restrict__ weights, const float* __restrict__ g,
-                                          const float* __restrict__ denominator, float* __restrict__ out,
+__global__ void cross_entropy_grad_kernel(const float* logits, const int32_t* labels,
+                                          const float* weights, const float* g,
+                                          const float* denominator, float* out,
                                           uint32_t v, uint32_t ld, uint32_t ld_out) {
     after_producers();
     __shared__ float shared[33];
@@ -262,10 +264,10 @@ __global__ void cross_entropy_grad_kernel(const float* __restrict__ logits, cons
 // scale * (p - onehot) while the row is still in cache. The same formulas, in the same order, as
 // the two separate kernels.
 template <class T>
-__global__ void cross_entropy_fused_kernel(const T* __restrict__ logits, const int32_t* __restrict__ labels,
-                                           const float* __restrict__ weights, const float* __restrict__ g,
-                                           const float* __restrict__ denominator, float* __restrict__ row_loss,
-                                           T* __restrict__ out, uint32_t v, uint32_t ld, uint32_t ld_out) {
+__global__ void cross_entropy_fused_kernel(const T* logits, const int32_t* labels,
+                                           const float* weights, const float* g,
+                                           const float* denominator, float* row_loss,
+                                           T* out, uint32_t v, uint32_t ld, uint32_t ld_out) {
     after_producers();
     __shared__ float shared[33];
     uint32_t r = blockIdx.x;
@@ -302,11 +304,11 @@ __global__ void cross_entropy_fused_kernel(const T* __restrict__ logits, const i
 constexpr int kWideThreads = 1024, kWideItems = 32;
 template <class T>
 __global__ void __launch_bounds__(kWideThreads, 1)
-cross_entropy_fused_wide_kernel(const T* __restrict__ logits, const int32_t* __restrict__ labels,
-                                const float* __restrict__ weights, const float* __restrict__ g,
-                                const float* __restrict__ denominator, float* __restrict__ row_loss,
-                                T* __restrict__ out, uint32_t v, uint32_t ld, uint32_t ld_out,
-                                uint32_t* __restrict__ counter, float* __restrict__ loss) {
+cross_entropy_fused_wide_kernel(const T* logits, const int32_t* labels,
+                                const float* weights, const float* g,
+                                const float* denominator, float* row_loss,
+                                T* out, uint32_t v, uint32_t ld, uint32_t ld_out,
+                                uint32_t* counter, float* loss) {
     after_producers();
     // Element i of this thread is column column_of(i): consecutive threads take consecutive columns.
     auto column_of = [](int i, uint32_t tid) { return static_cast<uint32_t>(i) * kWideThreads + tid; };
@@ -419,10 +421,10 @@ __device__ __forceinline__ float bf16_high(uint32_t pair) { return __uint_as_flo
 // 24.9 -> 10.6, 832 x 30,522 bf16 47.6 -> 32.4, 2,880 x 30,522 bf16 177 -> 107 (a 1,024-thread block a row before).
 template <int THREADS, int ROWS, int GROUPS, int BLOCKS, class T>
 __global__ void __launch_bounds__(THREADS * ROWS, BLOCKS)
-cross_entropy_row_kernel(const T* __restrict__ logits, const int32_t* __restrict__ labels, const float* __restrict__ weights,
-                         const float* __restrict__ g, const float* __restrict__ denominator, float* __restrict__ row_loss,
-                         T* __restrict__ out, uint32_t rows, uint32_t v, uint32_t ld, uint32_t ld_out, uint32_t* __restrict__ counter,
-                         float* __restrict__ loss) {
+cross_entropy_row_kernel(const T* logits, const int32_t* labels, const float* weights,
+                         const float* g, const float* denominator, float* row_loss,
+                         T* out, uint32_t rows, uint32_t v, uint32_t ld, uint32_t ld_out, uint32_t* counter,
+                         float* loss) {
     after_producers();
     static_assert(ROWS == 1 || THREADS == 32);
     constexpr bool HALF = sizeof(T) == 2;
@@ -444,7 +446,7 @@ cross_entropy_row_kernel(const T* __restrict__ logits, const int32_t* __restrict
     if (w != 0.0f) {
         const uint32_t last = (v - 1) / E * E;
 #pragma unroll
-        for (int k = 0; k < GROUPS; ++k) x[k] = __ldg(reinterpret_cast<const uint4*>(row + min(column_of(k), last)));
+        for (int k = 0; k < GROUPS; ++k) x[k] = load_global(reinterpret_cast<const uint4*>(row + min(column_of(k), last)));
         if (t == 0 && label < v) picked = load1(row + label);
     }
     // The weight sum: given (the whole batch's, data parallel), or summed here by every block in the same
@@ -582,11 +584,11 @@ cross_entropy_row_kernel(const T* __restrict__ logits, const int32_t* __restrict
 constexpr int kSplitRegisterItems = 32, kSplitSharedItems = 32;
 template <int kSplitThreads>
 __global__ void __launch_bounds__(kSplitThreads, 1024 / kSplitThreads)
-cross_entropy_fused_split_kernel(const float* __restrict__ logits, const int32_t* __restrict__ labels,
-                                 const float* __restrict__ weights, const float* __restrict__ g,
-                                 const float* __restrict__ denominator, float* __restrict__ row_loss,
-                                 float* __restrict__ out, uint32_t v, uint32_t ld, uint32_t ld_out,
-                                 uint32_t* __restrict__ counter, float* __restrict__ loss) {
+cross_entropy_fused_split_kernel(const float* logits, const int32_t* labels,
+                                 const float* weights, const float* g,
+                                 const float* denominator, float* row_loss,
+                                 float* out, uint32_t v, uint32_t ld, uint32_t ld_out,
+                                 uint32_t* counter, float* loss) {
     after_producers();
     // Group k of this thread is the four columns from (k * threads + tid) * 4 on: groups 0..7 live in
     // registers, groups 8..15 in shared memory.
@@ -629,7 +631,7 @@ cross_entropy_fused_split_kernel(const float* __restrict__ logits, const int32_t
             }
         asm volatile("cp.async.commit_group;" ::: "memory");
 #pragma unroll
-        for (int k = 0; k < kRegisterGroups; ++k) x[k] = __ldg(reinterpret_cast<const float4*>(row + min(column_of(k), last)));
+        for (int k = 0; k < kRegisterGroups; ++k) x[k] = load_global(reinterpret_cast<const float4*>(row + min(column_of(k), last)));
         auto mask = [v](float4 f, uint32_t c) {
             if (c >= v) f.x = -INFINITY;
             if (c + 1 >= v) f.y = -INFINITY;
@@ -754,15 +756,15 @@ template <int ITEMS, int V, class T> struct RawRow {
     static constexpr bool HALF = sizeof(T) == 2;
     static_assert(V == 1 || HALF);
     uint32_t e[V == 2 ? ITEMS / 2 : ITEMS];
-    __device__ __forceinline__ void load(const T* __restrict__ row, uint32_t lane, uint32_t h) {
+    __device__ __forceinline__ void load(Settled<T> row, uint32_t lane, uint32_t h) {
         if constexpr (V == 2) {
 #pragma unroll
-            for (int j = 0; j < ITEMS / 2; ++j) e[j] = __ldg(reinterpret_cast<const uint32_t*>(row + min(j * 64 + lane * 2, h - 2)));
+            for (int j = 0; j < ITEMS / 2; ++j) e[j] = load_settled<uint32_t>((row + min(j * 64 + lane * 2, h - 2)).p);
         } else {
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) {
-                if constexpr (HALF) e[i] = __ldg(reinterpret_cast<const unsigned short*>(row) + min(i * 32 + lane, h - 1));
-                else e[i] = __ldg(reinterpret_cast<const uint32_t*>(row) + min(i * 32 + lane, h - 1));
+                if constexpr (HALF) e[i] = load_settled<uint16_t>((row + min(i * 32 + lane, h - 1)).p);
+                else e[i] = load_settled<uint32_t>((row + min(i * 32 + lane, h - 1)).p);
             }
         }
     }
@@ -819,7 +821,7 @@ __device__ __forceinline__ uint32_t spread_keep_bits(uint32_t mine, uint32_t lan
 }
 // This lane's word of a row's stored decisions (0 where they are drawn).
 __device__ __forceinline__ uint32_t stored_keep_word(const DropoutDraw& draw, uint64_t row_at, uint32_t lane, uint32_t h) {
-    return draw.token != nullptr && draw.stored && draw.bits != nullptr && lane < h / 32 ? __ldg(draw.bits + row_at / 32 + lane) : 0u;
+    return draw.token != nullptr && draw.stored && draw.bits != nullptr && lane < h / 32 ? load_global(draw.bits + row_at / 32 + lane) : 0u;
 }
 // The keep decisions of a row for one site: read when an earlier launch of the step stored them,
 // else drawn (element index_base + row h + column of Philox stream 4) and stored when asked.
@@ -852,9 +854,9 @@ __device__ __forceinline__ uint32_t keep_mask(const DropoutDraw& draw, uint64_t 
 // integer units busier than the two of 92 (68 -> 59 us).
 template <int ITEMS, int V, bool EXACT, class T>
 __global__ void __launch_bounds__(256, !EXACT ? 1 : ITEMS >= 32 ? 2 : ITEMS >= 24 ? 3 : 4) dropout_add_layer_norm_kernel(
-    const T* __restrict__ x, const T* __restrict__ residual, DropoutDraw x_draw, const float* __restrict__ gamma,
-    const float* __restrict__ beta, T* __restrict__ sum_out, T* __restrict__ out, DropoutDraw out_draw,
-    T* __restrict__ out_dropped, uint32_t rows, uint32_t width_given, bool gelu_first) {
+    const T* x, const T* residual, DropoutDraw x_draw, const float* gamma,
+    const float* beta, T* sum_out, T* out, DropoutDraw out_draw,
+    T* out_dropped, uint32_t rows, uint32_t width_given, bool gelu_first) {
     after_producers();
     const uint32_t h = EXACT ? 32u * ITEMS : width_given;
     const uint32_t lane = threadIdx.x & 31;
@@ -939,12 +941,13 @@ __global__ void __launch_bounds__(256, !EXACT ? 1 : ITEMS >= 32 ? 2 : ITEMS >= 2
 // two (as four, f32 rows of 128 spill: a BERT-tiny step 4 us more).
 template <int ITEMS, int V, bool EXACT, class T>
 __global__ void __launch_bounds__(256, ITEMS <= 2 || (ITEMS <= 4 && EXACT && sizeof(T) == 2) ? 4 : 2) layer_norm_backward_kernel(
-    const T* __restrict__ x, const float* __restrict__ gamma, const T* __restrict__ g, const T* __restrict__ g1,
-    const T* __restrict__ g2, const T* __restrict__ g3, T* __restrict__ dx,
-    float* __restrict__ partial, uint32_t* __restrict__ counter, float* __restrict__ dgamma, float* __restrict__ dbeta,
+    const T* x, const float* gamma, const T* g, const T* g1,
+    const T* g2, const T* g3, T* dx,
+    float* partial, uint32_t* counter, float* dgamma, float* dbeta,
     uint32_t want, uint32_t rows, uint32_t width_given, uint32_t rows_per_chunk, DropoutDraw adjoint_draw, DropoutDraw dx_draw,
-    T* __restrict__ dx_dropped, const T* __restrict__ pre_activation) {
+    T* dx_dropped, const T* pre_activation) {
     after_producers();
+    const Settled<T> x_rows = settled(x), g_rows = settled(g), pre_rows = settled(pre_activation), added_rows[3] = {settled(g1), settled(g2), settled(g3)};
     constexpr bool WIDE = ITEMS >= 16;
     const uint32_t h = EXACT ? 32u * ITEMS : width_given;
     extern __shared__ float backward_sums[];  // 8 * 32 * ITEMS floats, twice that for wide rows
@@ -990,13 +993,13 @@ __global__ void __launch_bounds__(256, ITEMS <= 2 || (ITEMS <= 4 && EXACT && siz
         RawRow<!WIDE ? ITEMS : 2, V, T> pre_raw;
         {
             RawRow<ITEMS, V, T> x_raw, g_raw, more[AHEAD > 0 ? AHEAD : 1];
-            x_raw.load(x + row_at, lane, h);
-            g_raw.load(g + row_at, lane, h);
+            x_raw.load(x_rows + row_at, lane, h);
+            g_raw.load(g_rows + row_at, lane, h);
 #pragma unroll
             for (int a = 0; a < AHEAD; ++a)
-                if (addends[a] != nullptr) more[a].load(addends[a] + row_at, lane, h);
+                if (added_rows[a]) more[a].load(added_rows[a] + row_at, lane, h);
             if constexpr (!WIDE) {
-                if (pre_activation != nullptr) pre_raw.load(pre_activation + row_at, lane, h);
+                if (pre_rows) pre_raw.load(pre_rows + row_at, lane, h);
             }
 #pragma unroll
             for (int i = 0; i < ITEMS; ++i) {
@@ -1065,7 +1068,7 @@ __global__ void __launch_bounds__(256, ITEMS <= 2 || (ITEMS <= 4 && EXACT && siz
         auto gamma_of = [&](int i) -> float {
             if constexpr (!WIDE) return gam[i];
             else if constexpr (ROW_GAMMA) return row_gamma[i];
-            else return want_dx ? __ldg(gamma + column_of<V>(i, lane)) : 0.0f;
+            else return want_dx ? load_global(gamma + column_of<V>(i, lane)) : 0.0f;
         };
 #pragma unroll
         for (int i = 0; i < ITEMS; ++i)

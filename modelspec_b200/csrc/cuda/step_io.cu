@@ -18,8 +18,8 @@ constexpr int kTakeThreads = 256, kTakeChunks = 4;
 
 // 16-byte chunks, four in flight per thread. No word in pinned memory is read by more than one warp:
 // reads of one host address are served one after the other, about a microsecond each.
-__global__ void __launch_bounds__(kTakeThreads) take_inputs_kernel(const __grid_constant__ InputSlots slots, uint64_t chunks, uint4* __restrict__ to,
-                                                                    const uint32_t* __restrict__ turn) {
+__global__ void __launch_bounds__(kTakeThreads) take_inputs_kernel(const __grid_constant__ InputSlots slots, uint64_t chunks, uint4* to,
+                                                                    const uint32_t* turn) {
     after_producers();
     const uint4* from = reinterpret_cast<const uint4*>(slots.at[*turn % slots.count]);
     const uint64_t stride = static_cast<uint64_t>(gridDim.x) * kTakeThreads;
@@ -34,8 +34,8 @@ __global__ void __launch_bounds__(kTakeThreads) take_inputs_kernel(const __grid_
     }
 }
 
-__global__ void publish_step_kernel(const float* __restrict__ loss, const uint32_t* __restrict__ status, float* __restrict__ to_loss,
-                                    uint32_t* __restrict__ to_status, uint32_t* __restrict__ turn, uint32_t slots) {
+__global__ void publish_step_kernel(const float* loss, const uint32_t* status, float* to_loss,
+                                    uint32_t* to_status, uint32_t* turn, uint32_t slots) {
     after_producers();
     const uint32_t slot = *turn;
     if (loss) to_loss[slot] = *loss;
