@@ -7,8 +7,10 @@
 #include <atomic>
 #include <cstdint>
 #include <initializer_list>
+#include <set>
 #include <stdexcept>
 #include <string>
+#include <vector>
 
 namespace msx {
 namespace k {
@@ -67,6 +69,33 @@ __device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.
 __device__ __forceinline__ void after_producers() {
     wait_for_producers();
     let_next_start();
+}
+
+// What the launches of a step being captured on this thread say of their kernels, while the runtime asks.
+struct CaptureNotes {
+    std::set<cudaGraphNode_t> side;      // on the side stream
+    std::set<cudaGraphNode_t> in_order;  // better started when the kernel before has ended
+};
+inline thread_local CaptureNotes* capture_notes = nullptr;
+struct NoteCapture {
+    explicit NoteCapture(CaptureNotes* notes) { capture_notes = notes; }
+    ~NoteCapture() { capture_notes = nullptr; }
+    NoteCapture(const NoteCapture&) = delete;
+    NoteCapture& operator=(const NoteCapture&) = delete;
+};
+// The nodes that the next one captured on `s` will follow: after a launch, its kernel.
+inline std::vector<cudaGraphNode_t> captured_last(cudaStream_t s) {
+    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
+    const cudaGraphNode_t* last = nullptr;
+    size_t count = 0;
+    check(cudaStreamGetCaptureInfo_v2(s, &status, nullptr, nullptr, &last, &count), "cudaStreamGetCaptureInfo");
+    if (status != cudaStreamCaptureStatusActive) return {};
+    return {last, last + count};
+}
+// The kernel just launched on `s` is one of those.
+inline void starts_in_order(cudaStream_t s) {
+    if (!capture_notes) return;
+    for (cudaGraphNode_t node : captured_last(s)) capture_notes->in_order.insert(node);
 }
 
 // A load of what another kernel of the step may have written. The read-only path (__ldg, ld.global.nc, a kernel's `const

@@ -264,6 +264,7 @@ template <bool A_T, bool B_T, bool ACT, int COUNT> void launch(cudaStream_t s, c
         config.numAttrs = 1;
     }
     check(cudaLaunchKernelEx(&config, kernel, problems), "matmul_small");
+    starts_in_order(s);  // (its small blocks would gather on the few SMs that are idle early)
 }
 template <int COUNT> void launch_form(cudaStream_t s, bool a_t, bool b_t, const Problems<COUNT>& problems, uint32_t blocks) {
     if constexpr (COUNT == MAX_PRODUCTS) {

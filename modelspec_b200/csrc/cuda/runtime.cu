@@ -21,6 +21,7 @@
 #include <memory>
 #include <set>
 #include <thread>
+#include <unordered_map>
 
 #include "../../../include/msx.h"
 #include "../core/frontend.hpp"
@@ -216,7 +217,6 @@ struct msx_plan {
     // The captured step: [1] takes its inputs over first, [0] runs on what is staged already. Each is
     // made when a step of its kind first runs.
     cudaGraphExec_t graphs[2] = {};
-    std::set<cudaGraphNode_t> side_nodes;  // of the step being captured: its launches on the side stream
     cudaEvent_t clock_start = nullptr;  // before the first step since the last msx_elapsed_ms
     uint64_t clock_steps = 0;
 
@@ -2869,21 +2869,24 @@ void join_loss(msx_plan* P) {
 // A bucket closed this few launches before the optimizer has nothing left to hide behind.
 constexpr int kExposedLaunches = 6;
 
-// The nodes of the graph that `stream` is captured into; none where it is not.
-std::set<cudaGraphNode_t> captured_nodes(cudaStream_t stream) {
-    cudaStreamCaptureStatus status = cudaStreamCaptureStatusNone;
-    cudaGraph_t graph = nullptr;
-    cuda_ok(cudaStreamGetCaptureInfo_v2(stream, &status, nullptr, &graph, nullptr, nullptr), "cudaStreamGetCaptureInfo");
-    if (status != cudaStreamCaptureStatusActive || !graph) return {};
-    size_t count = 0;
-    cuda_ok(cudaGraphGetNodes(graph, nullptr, &count), "cudaGraphGetNodes");
-    std::vector<cudaGraphNode_t> nodes(count);
-    if (count) cuda_ok(cudaGraphGetNodes(graph, nodes.data(), &count), "cudaGraphGetNodes");
-    return {nodes.begin(), nodes.begin() + static_cast<std::ptrdiff_t>(count)};
+// What a launch has put on the side stream of a step being captured: its kernels, from the last one back to what
+// `before` held, the main stream's last nodes as it was forked.
+void note_side_launch(k::CaptureNotes* notes, cudaStream_t side, const std::vector<cudaGraphNode_t>& before) {
+    std::vector<cudaGraphNode_t> open = k::captured_last(side);
+    while (!open.empty()) {
+        const cudaGraphNode_t node = open.back();
+        open.pop_back();
+        if (std::find(before.begin(), before.end(), node) != before.end() || !notes->side.insert(node).second) continue;
+        size_t count = 0;
+        cuda_ok(cudaGraphNodeGetDependencies_v2(node, nullptr, nullptr, &count), "cudaGraphNodeGetDependencies");
+        std::vector<cudaGraphNode_t> from(count);
+        std::vector<cudaGraphEdgeData> data(count);
+        if (count) cuda_ok(cudaGraphNodeGetDependencies_v2(node, from.data(), data.data(), &count), "cudaGraphNodeGetDependencies");
+        open.insert(open.end(), from.begin(), from.end());
+    }
 }
 
 void enqueue_all(msx_plan* P) {
-    P->side_nodes.clear();
     begin_side_work(P);
     std::vector<char> joined(P->launches.size(), 0);
     for (size_t l = 0; l < P->launches.size(); ++l) {
@@ -2902,10 +2905,10 @@ void enqueue_all(msx_plan* P) {
         if (P->launches[l].join_before >= 0 && P->side_stream && P->side_fork[l]) {
             cuda_ok(cudaEventRecord(P->side_fork[l], P->stream), "cudaEventRecord");
             cuda_ok(cudaStreamWaitEvent(P->side_stream, P->side_fork[l], 0), "cudaStreamWaitEvent");
-            const std::set<cudaGraphNode_t> before = captured_nodes(P->stream);
+            k::CaptureNotes* const notes = k::capture_notes;
+            const std::vector<cudaGraphNode_t> before = notes ? k::captured_last(P->stream) : std::vector<cudaGraphNode_t>();
             P->launches[l].run(P->side_stream);
-            for (cudaGraphNode_t node : captured_nodes(P->stream))
-                if (!before.count(node)) P->side_nodes.insert(node);
+            if (notes) note_side_launch(notes, P->side_stream, before);
             cuda_ok(cudaEventRecord(P->side_done[l], P->side_stream), "cudaEventRecord");
         } else {
             P->launches[l].run(P->stream);
@@ -3030,44 +3033,50 @@ size_t index_of(const msx_plan* P, const HostInput& in) { return static_cast<siz
 
 // The edges of a captured step between a kernel and the one kernel that follows it become programmatic: the
 // second may be launched once every block of the first has called after_producers (common.cuh), and waits there
-// itself until the first is complete. Left as they are: edges to and from the side stream's launches (`side`) and of a kernel
+// itself until the first is complete. Left as they are: edges to and from the side stream's launches and of a kernel
 // that one of those is forked from (the next kernel, standing there early, would take the idle SMs from it: a BERT-tiny step
-// 5 % longer), kernels that are not the backend's or wait for other ranks, and edges to the FMA
-// products, whose small blocks would gather on the few SMs that are idle early (a transformer block's step 267 us so, 261
-// without them starting early, 268 with none; the ragged f32 case 7,404, 7,270, 7,387 a pass).
+// 5 % longer), nodes that are no kernels, and edges to kernels that say so (starts_in_order: a transformer block's step 267 us
+// where the FMA products start early, 261 where the others alone do, 268 with none; the ragged f32 case 7,404, 7,270, 7,387 a pass).
+// The plan has no communicator: every kernel of the graph is the backend's, and none waits for another rank.
 // Passes, without and with: MLP 1,310, 1,245; BERT-tiny f32 21,608, 21,128, mixed 15,080, 13,990; BERT-mini 30,228, 29,423.
-void chain_kernels(cudaGraph_t graph, const std::set<cudaGraphNode_t>& side) {
+void chain_kernels(cudaGraph_t graph, const k::CaptureNotes& notes) {
     size_t count = 0;
     cuda_ok(cudaGraphGetEdges_v2(graph, nullptr, nullptr, nullptr, &count), "cudaGraphGetEdges");
     std::vector<cudaGraphNode_t> from(count), to(count);
     std::vector<cudaGraphEdgeData> data(count);
     if (count) cuda_ok(cudaGraphGetEdges_v2(graph, from.data(), to.data(), data.data(), &count), "cudaGraphGetEdges");
-    std::map<cudaGraphNode_t, std::pair<int, int>> degrees;  // edges into and out of a node, on its own stream
-    auto crosses = [&](size_t e) { return side.count(from[e]) != side.count(to[e]); };
+    struct Facts {
+        int in = 0, out = 0;  // edges into it on its own stream, and out of it
+        bool kernel = false;
+    };
+    std::unordered_map<cudaGraphNode_t, Facts> nodes;
+    auto crosses = [&](size_t e) { return notes.side.count(from[e]) != notes.side.count(to[e]); };
     for (size_t e = 0; e < count; ++e) {
-        if (!crosses(e)) ++degrees[to[e]].first;
-        ++degrees[from[e]].second;
+        if (!crosses(e)) ++nodes[to[e]].in;
+        ++nodes[from[e]].out;
+        nodes[to[e]];
     }
-    auto waits_for_producers = [](cudaGraphNode_t node, bool starts_early) {
+    for (auto& [node, facts] : nodes) {
         cudaGraphNodeType type;
         cuda_ok(cudaGraphNodeGetType(node, &type), "cudaGraphNodeGetType");
-        if (type != cudaGraphNodeTypeKernel) return false;
-        cudaKernelNodeParams params = {};
-        cuda_ok(cudaGraphKernelNodeGetParams(node, &params), "cudaGraphKernelNodeGetParams");
-        const char* name = nullptr;
-        cuda_ok(cudaFuncGetName(&name, params.func), "cudaFuncGetName");
-        if (starts_early && std::strstr(name, "matmul_small")) return false;
-        return std::strstr(name, "msx") != nullptr && std::strstr(name, "peer_all_reduce") == nullptr;
-    };
-    for (size_t e = 0; e < count; ++e) {
-        if (crosses(e) || data[e].type != cudaGraphDependencyTypeDefault || degrees[to[e]].first != 1 || degrees[from[e]].second != 1) continue;
-        if (!waits_for_producers(from[e], false) || !waits_for_producers(to[e], true)) continue;
-        cudaGraphEdgeData early = {};
-        early.from_port = cudaGraphKernelNodePortProgrammatic;
-        early.type = cudaGraphDependencyTypeProgrammatic;
-        cuda_ok(cudaGraphRemoveDependencies_v2(graph, &from[e], &to[e], &data[e], 1), "cudaGraphRemoveDependencies");
-        cuda_ok(cudaGraphAddDependencies_v2(graph, &from[e], &to[e], &early, 1), "cudaGraphAddDependencies");
+        facts.kernel = type == cudaGraphNodeTypeKernel;
     }
+    size_t early = 0;  // the edges to change, moved to the front
+    for (size_t e = 0; e < count; ++e) {
+        const Facts &a = nodes[from[e]], &b = nodes[to[e]];
+        if (crosses(e) || data[e].type != cudaGraphDependencyTypeDefault || !a.kernel || !b.kernel || b.in != 1 || a.out != 1 || notes.in_order.count(to[e])) continue;
+        std::swap(from[early], from[e]);
+        std::swap(to[early], to[e]);
+        std::swap(data[early], data[e]);
+        ++early;
+    }
+    if (early == 0) return;
+    cudaGraphEdgeData programmatic = {};
+    programmatic.from_port = cudaGraphKernelNodePortProgrammatic;
+    programmatic.type = cudaGraphDependencyTypeProgrammatic;
+    const std::vector<cudaGraphEdgeData> changed(early, programmatic);
+    cuda_ok(cudaGraphRemoveDependencies_v2(graph, from.data(), to.data(), data.data(), early), "cudaGraphRemoveDependencies");
+    cuda_ok(cudaGraphAddDependencies_v2(graph, from.data(), to.data(), changed.data(), early), "cudaGraphAddDependencies");
 }
 
 // A large step's inputs from its pinned slot to its slot on the device: on the plan's stream when that is
@@ -3452,6 +3461,9 @@ int msx_run(msx_plan* plan) {
             cudaGraphExec_t& exec = plan->graphs[take_inputs ? 1 : 0];
             if (!exec) {
                 cudaGraph_t graph = nullptr;
+                const bool chained = (fusion_mask() & 128u) && !plan->comm;
+                k::CaptureNotes notes;
+                k::NoteCapture noting(chained ? &notes : nullptr);
                 cuda_ok(cudaStreamBeginCapture(plan->stream, cudaStreamCaptureModeThreadLocal), "cudaStreamBeginCapture");
                 try {
                     enqueue_step(plan, take_inputs);
@@ -3463,7 +3475,7 @@ int msx_run(msx_plan* plan) {
                 cuda_ok(cudaStreamEndCapture(plan->stream, &graph), "cudaStreamEndCapture");
                 cudaError_t e = cudaSuccess;
                 try {
-                    if ((fusion_mask() & 128u) && !plan->comm) chain_kernels(graph, plan->side_nodes);
+                    if (chained) chain_kernels(graph, notes);
                     e = cudaGraphInstantiate(&exec, graph, 0);
                 } catch (...) {
                     cudaGraphDestroy(graph);
