@@ -150,17 +150,30 @@ def test_values_next_to_the_largest_float(device, batch, q_len, k_len, heads, d)
 
 
 # One way each: both kernels, the forward with its probabilities left for the gradients' products (rows on and off 16 bytes),
-# neither.
-@pytest.mark.parametrize("batch,q_len,k_len,heads,d", [(32, 128, 128, 2, 64), (5, 77, 77, 3, 33), (32, 100, 100, 8, 32), (60, 96, 99, 6, 7), (2, 160, 256, 3, 16)])
-def test_a_plan_takes_each_way(device, batch, q_len, k_len, heads, d):
+# neither. Which way a plan takes shows in what its gradients read (the statistics and O, or probabilities), and in the bits of O.
+@pytest.mark.parametrize("batch,q_len,k_len,heads,d,way", [(32, 128, 128, 2, 64, "both"), (5, 77, 77, 3, 33, "both"), (32, 100, 100, 8, 32, "forward"),
+                                                          (60, 96, 99, 6, 7, "forward"), (2, 160, 256, 3, 16, "products")])
+def test_a_plan_takes_each_way(device, batch, q_len, k_len, heads, d, way):
+    import torch
     shape = (batch, q_len, k_len, heads, d)
     feed = feed_of(*shape)
     text, values = program(*shape, "QKV")
+    backward = next(line for line in M.schedule_describe(text).splitlines() if " attention_backward " in line)
+    assert (" %%%d " % values["O"][0] in backward.split("writes")[0]) == (way == "both"), backward
     plan = M.Plan(device, text, flags=M.PLAN_NO_GRAPH | M.PLAN_GUARD)
     try:
         for name, value in feed.items():
             plan.set_input(name, value)
         plan.run(); plan.sync(); plan.check_guards()
-        check({name: plan.value(at, batch * rows * heads * d) for name, (at, rows) in values.items()}, feed, shape)
+        got = {name: plan.value(at, batch * rows * heads * d) for name, (at, rows) in values.items()}
+        check(got, feed, shape)
     finally:
         plan.destroy()
+    operand = {n: torch.from_numpy(x.reshape(-1)).cuda() for n, x in feed.items()}
+    out, status = torch.zeros(batch * q_len * heads * d, device="cuda"), torch.zeros(1, dtype=torch.int32, device="cuda")
+    torch.cuda.synchronize()
+    ptr = lambda t: C.c_void_p(t.data_ptr())
+    rc = M.lib().msx_op_attention_f32(ptr(operand["q"]), ptr(operand["k"]), ptr(operand["v"]), ptr(operand["mask"]), None, ptr(out), None, None, None, None,
+                                      None, *shape, ptr(status), None)
+    assert rc == M.OK and int(status.item()) == 0
+    assert (out.cpu().numpy().tobytes() == np.ascontiguousarray(got["O"]).tobytes()) == (way != "products")

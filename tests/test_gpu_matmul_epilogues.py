@@ -1,5 +1,6 @@
 """relu, gelu and their gradients inside the f32 product whose result they take (the FMA tiles, with and without a cluster, and
-the 64-row tiles, aligned and not): the bits of the launches of their own, which a program gets whose product is an output."""
+the 64-row tiles 32, 64 and 128 wide, with rows on and off 16 bytes): the bits of the launches of their own, which a program gets
+whose product is an output."""
 import numpy as np
 import pytest
 
@@ -25,7 +26,8 @@ def program(m, n, k, act, bias, apart):
 
 @pytest.mark.parametrize("act", ["Relu", "Gelu"])
 @pytest.mark.parametrize("m,n,k,bias", [(1, 1, 1, True), (33, 31, 17, False), (64, 128, 784, True), (5, 7, 300, True), (385, 250, 99, True), (700, 250, 99, False),
-                                        (1500, 130, 250, True), (64, 66, 2000, True), (900, 33, 130, False)])
+                                        (1500, 130, 250, True), (64, 66, 2000, True), (900, 33, 130, False), (1500, 128, 249, True), (1500, 512, 249, False),
+                                        (1500, 2048, 249, True)])
 def test_an_activation_inside_a_product_has_the_bits_of_its_own_launch(device, m, n, k, bias, act):
     r = np.random.default_rng(m * 1000 + n)
     x, g = (r.standard_normal((m, depth)).astype(np.float32) for depth in (k, k + 4))  # (of one shape they would share a launch)
@@ -34,7 +36,8 @@ def test_an_activation_inside_a_product_has_the_bits_of_its_own_launch(device, m
     results, launches = [], []
     for apart in (False, True):
         text, ends = program(m, n, k, act, bias, apart)
-        launches.append(M.schedule_describe(text).count(": matmul "))
+        listed = [line.split(": ")[1].split()[0] for line in M.schedule_describe(text).splitlines() if ": " in line]
+        launches.append((listed.count("matmul"), sum(kernel.startswith((act.lower(), "unary")) for kernel in listed)))
         plan = M.Plan(device, text, flags=M.PLAN_NO_GRAPH | M.PLAN_GUARD)
         try:
             plan.set_input("x", x); plan.set_input("g", g)
@@ -44,7 +47,7 @@ def test_an_activation_inside_a_product_has_the_bits_of_its_own_launch(device, m
             results.append([plan.value(e, m * n) for e in ends])
         finally:
             plan.destroy()
-    assert launches == [2, 2]
+    assert launches == [(2, 0), (2, 2)], "the activation and its gradient: inside the products, and apart"
     for name, inside, own in zip((act, act + "Grad"), *results):
         assert_bits_equal(inside, own, name)
     z = x.astype(np.float64) @ w.astype(np.float64) + (b if bias else 0.0)
