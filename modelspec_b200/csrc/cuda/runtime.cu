@@ -310,9 +310,9 @@ void close_peer_reduce(msx_plan* P);
 // Tuning switch: MSX_FUSE is a bit mask of optional fusions (default: all). 1 sublayer tails
 // (dropout + residual + layer norm), 2 adjoint sums inside layer-norm backward, 4 weight-gradient
 // matmuls as jobs of one launch, 8 heavy launches with late readers on a side stream, 16
-// dropout_grad inside the layer-norm backward that makes or reads its operand and, in a
-// mixed-precision plan, gelu and gelu_grad inside the product that makes theirs, 32 the fused
-// attention kernels (off: batched products with row kernels between),
+// dropout_grad inside the layer-norm backward that makes or reads its operand, gelu and gelu_grad inside
+// the product that makes theirs (mixed precision), relu, gelu and their gradients inside small f32 products,
+// 32 the fused attention kernels (off: batched products with row kernels between),
 // 64 the keep decisions of a dropout site stored by the forward launch that draws them, one bit
 // per element, and read by the site's dropout_grad (off: every launch draws again), 128 kernels of a
 // captured step that start while the one before them ends.
